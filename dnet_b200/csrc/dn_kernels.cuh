@@ -394,6 +394,8 @@ typedef OpOProj OpDown;  // identical dataflow: a=[T][ffn], w=[H][ffn], resid=h,
 //   OpGateUpMoe   act_j = SwiGLU of expert sel[j]           (j = 0..k-1; same epilogue as the dense OpGateUp)
 //   OpDownMoe     y_j = T(act_j Wd[sel[j]]^T); term_j = T(y_j * score_j); acc = T(acc + term_j) in selection order;
 //                 the last j writes out = T(h + acc)
+// A prompt's tokens (16 and more) take k_moe_route and the grouped GEMM instead: every expert's matrices are read once for all the
+// tokens that chose it (moe_ffn_tc in dn_api.cu), with the same rounding points; k_moe_join adds a token's pairs.
 // ---------------------------------------------------------------------------------
 struct OpRouter {
   static constexpr int ALIGN = 1;
@@ -415,9 +417,8 @@ struct OpRouter {
 };
 
 constexpr int MOE_MAX_E = 64, MOE_MAX_K = 8;
-__global__ void __launch_bounds__(32) k_moe_select(const float* __restrict__ logits, int E, int k, int32_t* __restrict__ sel,
-                                                   float* __restrict__ score) {
-  if (threadIdx.x != 0) return;
+// one token's choice (a single thread)
+__device__ __forceinline__ void moe_select(const float* logits, int E, int k, int32_t* sel, float* score) {
   float v[MOE_MAX_K];
   int id[MOE_MAX_K];
   unsigned long long taken = 0ull;
@@ -431,6 +432,54 @@ __global__ void __launch_bounds__(32) k_moe_select(const float* __restrict__ log
   float sum = 0.f, ex[MOE_MAX_K];
   for (int j = 0; j < k; ++j) { ex[j] = expf(v[j] - v[0]); sum += ex[j]; }
   for (int j = 0; j < k; ++j) { sel[j] = id[j]; score[j] = bf16r(ex[j] / sum); }
+}
+__global__ void __launch_bounds__(32) k_moe_select(const float* __restrict__ logits, int E, int k, int32_t* __restrict__ sel,
+                                                   float* __restrict__ score) {
+  if (threadIdx.x == 0) moe_select(logits, E, k, sel, score);
+}
+
+// a prompt's tokens, one block each: router logits of the normed row, then the choice of k_moe_select
+__global__ void __launch_bounds__(256) k_moe_route(const bf16* __restrict__ xn, const bf16* __restrict__ w, int K, int E, int k,
+                                                   int32_t* __restrict__ sel, float* __restrict__ score) {
+  __shared__ float lg[MOE_MAX_E];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bf16* x = xn + (size_t)t * K;
+  for (int e = warp; e < E; e += 8) {
+    float a = 0.f;
+    for (int i = lane * 8; i < K; i += 256) {
+      const uint4 v = *reinterpret_cast<const uint4*>(x + i);
+      const float xf[8] = {bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y), bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w)};
+      a = dot8(*reinterpret_cast<const uint4*>(w + (size_t)e * K + i), xf, a);
+    }
+    a = warp_sum(a);
+    if (lane == 0) lg[e] = bf16r(a);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) moe_select(lg, E, k, sel + (size_t)t * k, score + (size_t)t * k);
+}
+// a prompt's tokens: out = T(h + acc), acc = T(acc + T(y_j score_j)) over the token's pairs in selection order (OpDownMoe's rounding)
+__global__ void __launch_bounds__(256) k_moe_join(const bf16* __restrict__ y, const int32_t* __restrict__ pos, const float* __restrict__ score,
+                                                  int k, int H, const bf16* __restrict__ h, bf16* __restrict__ out) {
+  const int t = blockIdx.x;
+  for (int i = threadIdx.x * 8; i < H; i += 256 * 8) {
+    float acc[8];
+    for (int j = 0; j < k; ++j) {
+      const uint4 v = *reinterpret_cast<const uint4*>(y + (size_t)pos[t * k + j] * H + i);
+      const float f[8] = {bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y), bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w)};
+      const float sc = score[t * k + j];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float term = bf16r(__fmul_rn(f[q], sc));
+        acc[q] = j == 0 ? term : bf16r(__fadd_rn(acc[q], term));
+      }
+    }
+    const uint4 v = *reinterpret_cast<const uint4*>(h + (size_t)t * H + i);
+    const float f[8] = {bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y), bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w)};
+    __align__(16) bf16 o[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) o[q] = __float2bfloat16_rn(__fadd_rn(f[q], acc[q]));
+    *reinterpret_cast<uint4*>(out + (size_t)t * H + i) = *reinterpret_cast<const uint4*>(o);
+  }
 }
 
 struct OpGateUpMoe {

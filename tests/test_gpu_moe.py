@@ -101,3 +101,33 @@ def test_step_kernel_refuses_moe(moe, cuda_lib):
         assert rc < 0 and "MoE" in _cabi.last_error()
     finally:
         rt.unload_model_core()
+
+
+@pytest.mark.parametrize("T", [16, 63, 65, 200, 512])
+def test_prompt_experts_in_one_grouped_launch(moe, T):
+    """Prompt chunks of 16 tokens and more sort their (token, choice) pairs by expert and run all experts in one grouped launch
+    (moe_ffn_tc): experts with no rows, one row, whole tiles and remainders.  Against the oracle's token-by-token loop on the same
+    inputs; a result may differ where the last bf16 rounding does (as above)."""
+    from oracle.llama_oracle import LlamaOracle, OracleConfig, OracleKV
+
+    g, w = moe
+    cfgd = g["config"]
+    rt = make_runtime(cfgd, w, range(1), cuda_graphs=False, megakernel=False, max_tokens=1024)
+    try:
+        msg = token_message(rt, "probe", g["prompt"].tolist())
+        to_bind = rt.policy._bind_layer_weights([0], msg)
+        torch.cuda.synchronize()
+        rt.model.load_weights(list(to_bind.items()))
+        gen = torch.Generator().manual_seed(T)
+        x = torch.randn(T, cfgd["hidden_size"], generator=gen).to(torch.bfloat16)
+        oracle = LlamaOracle(OracleConfig.from_dict(cfgd), w, exact_linear=True)
+        ref = oracle.apply_single_layer(0, x, OracleKV())
+        ns = rt.get_or_make_kv("grouped")
+        got = rt.model.apply_single_layer(0, x.cuda().unsqueeze(0), ns.kv)[0]
+        torch.cuda.synchronize()
+        got = got.cpu()
+        frac = float((ulp_diff(got, ref) > 0).float().mean())
+        worst = float((got.float() - ref.float()).abs().max() / ref.float().abs().max())
+        assert frac < 0.03 and worst <= 2 * 2.0 ** -8, f"T {T}: {frac:.4f} mismatching, worst {worst:.2e}"
+    finally:
+        rt.unload_model_core()
