@@ -6,6 +6,7 @@
 #include "dn_kvquant.cuh"
 #include "dn_megakernel.cuh"
 #include "dn_gemm_tc.cuh"
+#include "dn_attn_tc.cuh"
 #include "dn_moe.cuh"
 #include "../../include/dnet_b200.h"
 
@@ -116,7 +117,7 @@ struct LayerW {
 constexpr int TPF_MAX = 512;   // tokens per tensor-core prefill chunk (weights are streamed once per chunk)
 static int g_tc_prefill = 1;
 static int g_gemm_bn256 = 0;   // prefill GEMMs: 256-token tiles (one accumulator set for SwiGLU); measured slower than 128-token tiles with two sets (30.7K vs 32.6K tok/s at 2048 tokens)
-static int g_tc_attn = 1;      // prefill attention on tcgen05 (GQA groups dividing 128), else the CUDA-core kernel
+static int g_tc_attn = 1;      // prefill attention on tcgen05, else the CUDA-core kernel
 
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -274,7 +275,7 @@ static cudaError_t init_kernel_attrs() {
 #undef PRS
 #undef PRE
 #define ATA(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
-  ATA(1) ATA(2) ATA(4) ATA(8)
+  ATA(1) ATA(2) ATA(4) ATA(5) ATA(7) ATA(8)
 #undef ATA
   return cudaSuccess;
 }
@@ -855,6 +856,25 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   return DN_OK;
 }
 
+// clusters span the grid's z
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, const Args&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = grid.z;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (g_capturing) g_capture_launches++; else g_launches++;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
   auto it = m->abs2local.find(abs_layer);
   if (it == m->abs2local.end()) return fail(DN_ENOENT, "Layer %d not hosted on this model instance", abs_layer);
@@ -890,16 +910,16 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   if (kvq) {
     const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, s);
     if (rc) return rc;
-  } else if (g_tc_attn && m->tm_kv_ok && (m->G == 1 || m->G == 2 || m->G == 4 || m->G == 8)) {
+  } else if (g_tc_attn && m->tm_kv_ok) {
     AtParams a;
     a.q = m->pf_q; a.out = m->pf_attn; a.block_table = kv->block_table; a.st = kv->st;
     a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.T = T; a.err = err;
-    const int tb = 128 / m->G;
-    dim3 grid(c.n_kv_heads, (T + tb - 1) / tb);
-#define PFT(Gv) case Gv: k_attn_prefill_tc<Gv><<<grid, 256, AT_SMEM, s>>>(m->tm_kv[li], a); break;
-    switch (m->G) { PFT(1) PFT(2) PFT(4) PFT(8) default: break; }
+    const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
+    // (how the keys are shared out only decides the order of the sums; the kernel reads the position from the step state)
+    const int Z = attn_prefill_split(c.n_kv_heads * blocks, kv->host_pos + T, g_sms);
+#define PFT(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_tc<Gv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, m->tm_kv[li], a)); break;
+    switch (m->G) { PFT(1) PFT(2) PFT(4) PFT(5) PFT(7) PFT(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT
-    g_launches++;
   } else {
     dim3 grid(c.n_kv_heads, (T + 3) / 4);
 #define PFA(Gv) case Gv: k_attn_prefill<Gv, 4><<<grid, Gv * 32, 0, s>>>(m->pf_q, pool, kv->block_table, kv->st, m->pf_attn, c.n_heads, c.n_kv_heads, T); break;

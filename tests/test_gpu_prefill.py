@@ -1,0 +1,77 @@
+"""-m gpu: the kernels of a prompt chunk's layer alone, at the sizes where they can go wrong: one decoder layer of a small model through
+``apply_single_layer``, against another path of the library that forms the same sums in another order.
+
+Bound: both paths store bf16 between a layer's operations and differ in the order of fp32 sums, so a stored value may differ by its last
+rounding (2^-8 relative).  A flipped rounding of one operand of the following products moves their results by far less than their own
+rounding, so results agree to a few last roundings of the largest value.  How many differ at all: the attention's sums differ by some
+2^-16 of their terms, which flips about p = 1 in 100 of its roundings; a product of such rows is then off by sqrt(p) 2^-9 of its size,
+a tenth of the distance of two roundings, which flips one result in ten, and the feed-forward does the same once more: below a quarter
+(a wrong key, row or head changes all of them)."""
+import pytest
+import torch
+
+from tests.helpers import rel_inf
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(kv_heads, group, seed=0, pages=48, kv_bits=0, hidden=512, ffn=512):
+    from dnet_b200.core.models.llama import LlamaRingModel
+
+    cfg = dict(hidden_size=hidden, num_attention_heads=kv_heads * group, num_key_value_heads=kv_heads, head_dim=128, intermediate_size=ffn,
+               vocab_size=256, num_hidden_layers=1, rms_norm_eps=1e-5, rope_theta=10000.0, model_type="llama", torch_dtype="bfloat16")
+    g = torch.Generator().manual_seed(seed)
+    p = "model.layers.0."
+    rows = {"q": kv_heads * group * 128, "k": kv_heads * 128, "v": kv_heads * 128}
+
+    def t(*shape, std):
+        return (torch.randn(*shape, generator=g) * std).to(torch.bfloat16).cuda()
+
+    w = {f"{p}self_attn.{c}_proj.weight": t(n, hidden, std=(2.0 if c in "qk" else 1.0) * hidden ** -0.5) for c, n in rows.items()}
+    w.update({f"{p}self_attn.{c}_proj.bias": t(n, std=0.5) for c, n in rows.items()})
+    w[p + "self_attn.o_proj.weight"] = t(hidden, rows["q"], std=rows["q"] ** -0.5)
+    w[p + "mlp.gate_proj.weight"], w[p + "mlp.up_proj.weight"] = t(ffn, hidden, std=hidden ** -0.5), t(ffn, hidden, std=hidden ** -0.5)
+    w[p + "mlp.down_proj.weight"] = t(hidden, ffn, std=ffn ** -0.5)
+    for n in ("input_layernorm", "post_attention_layernorm"):
+        w[f"{p}{n}.weight"] = torch.ones(hidden, dtype=torch.bfloat16).cuda()
+    m = LlamaRingModel(cfg, [0], kv_pool_pages=pages, kv_bits=kv_bits)
+    m.load_weights(w)
+    return m
+
+
+def _call(m, kv, x, context):
+    """the layer's outputs of the tokens behind `context`"""
+    kv.seek(0)
+    if context:
+        m.apply_single_layer(0, x[:context].clone(), kv)
+        kv.seek(context)
+    y = m.apply_single_layer(0, x[context:].clone(), kv)
+    torch.cuda.synchronize()
+    return y.float().cpu()
+
+
+def _agree(a, b):
+    assert torch.isfinite(a).all()
+    assert rel_inf(a, b) <= 3 * 2.0 ** -8, rel_inf(a, b)
+    assert float((a != b).float().mean()) < 0.25
+
+
+@pytest.mark.parametrize("group", [1, 2, 4, 5, 7, 8])
+@pytest.mark.parametrize("context,T", [(0, 16), (0, 127), (129, 26), (1000, 300), (2490, 16)])
+def test_prefill_attention_groups_and_key_shares(cuda_lib, group, context, T):
+    """k_attn_prefill_tc against the CUDA-core kernel: groups that leave MMA rows empty (5, 7), row blocks with a remainder, one key tile
+    (the second side has none), tiles cut by the causal edge, and contexts whose keys the CTAs of a cluster share (few tokens far back)."""
+    m = _model(2, group, seed=group)
+    kv = m.make_cache(max_tokens=2560)
+    x = torch.randn(context + T, 512, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    out = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_attn", tc)
+            out[tc] = _call(m, kv, x, context)
+        assert cuda_lib.dn_step_error(m._h, 0) == 0
+    finally:
+        cuda_lib.dn_set_option(b"tc_attn", 1)
+        kv.free()
+        m.destroy()
+    _agree(out[1], out[0])
