@@ -104,7 +104,7 @@ static cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
 struct LayerW {
   const bf16* w[DN_W_COUNT];
   bool bound = false;
-  CUtensorMap tm[7];          // TMA descriptors of q,k,v,o,gate,up,down ([rows, K] bf16, box 128 x 64, SWIZZLE_128B)
+  CUtensorMap tm[7];          // TMA descriptors of q,k,v,o,gate,up,down ([rows, K] bf16, box 64 x 64, SWIZZLE_128B)
   bool tm_ok = false;
   // sparse MoE layers (cfg.n_experts > 0): router [E][H] and a device table [3][E] of expert pointers (gate, up, down)
   const bf16* router = nullptr;
@@ -116,7 +116,6 @@ struct LayerW {
 
 constexpr int TPF_MAX = 512;   // tokens per tensor-core prefill chunk (weights are streamed once per chunk)
 static int g_tc_prefill = 1;
-static int g_gemm_bn256 = 0;   // prefill GEMMs: 256-token tiles (one accumulator set for SwiGLU); measured slower than 128-token tiles with two sets (30.7K vs 32.6K tok/s at 2048 tokens)
 static int g_tc_attn = 1;      // prefill attention on tcgen05, else the CUDA-core kernel
 
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -164,7 +163,7 @@ struct dn_model {
   int32_t *moe_psel = nullptr, *moe_plan = nullptr;      // choices [P]; rows of pairs [P], tokens of rows [P], tile table [3][max tiles] + 1
   float* moe_pscore = nullptr;
   CUtensorMap* moe_maps = nullptr;                       // [local layers][3][E]
-  CUtensorMap tm_moe_xg[2], tm_moe_act[2];               // row boxes of 64 / 128
+  CUtensorMap tm_moe_xg, tm_moe_act;
   int moe_max_tiles = 0;
   bool moe_tc_ok = false;
   StepState* null_state = nullptr;      // zeroed step state + block table for launches without a nonce (head-part only)
@@ -180,7 +179,7 @@ struct dn_model {
   bf16 *xa = nullptr, *xb = nullptr;
   // tensor-core prefill scratch ([TPF_MAX][...]) and the TMA descriptors of the activation buffers
   bf16 *pf_xn = nullptr, *pf_qkv = nullptr, *pf_q = nullptr, *pf_attn = nullptr, *pf_h = nullptr, *pf_act = nullptr;
-  CUtensorMap tm_xn[4], tm_attn[4], tm_act[4];   // token-tile boxes of 32 / 64 / 128 / 256 rows
+  CUtensorMap tm_xn, tm_attn, tm_act;
   std::vector<CUtensorMap> tm_kv;                // per local layer: KV pool as [pages*2*n_kv*64 rows][128] bf16, box 64 x 64
   bool tm_kv_ok = false;
   bool pf_ok = false;
@@ -307,7 +306,7 @@ extern "C" int dn_set_option(const char* key, int64_t value) {
   if (!strcmp(key, "pdl")) { g_pdl = value ? 1 : 0; return DN_OK; }
   if (!strcmp(key, "l2_prefetch_kb")) { g_l2_prefetch_kb = (int)value; return DN_OK; }
   if (!strcmp(key, "tc_prefill")) { g_tc_prefill = value ? 1 : 0; return DN_OK; }
-  if (!strcmp(key, "gemm_bn256")) { g_gemm_bn256 = value ? 1 : 0; return DN_OK; }
+  if (!strcmp(key, "gemm_bn256")) return DN_OK;      // (the width of a tile is planned for every launch)
   if (!strcmp(key, "tc_attn")) { g_tc_attn = value ? 1 : 0; return DN_OK; }
   if (!strcmp(key, "attn_single")) { g_attn_single = (int)value; return DN_OK; }
   if (!strcmp(key, "attn_last")) { g_attn_last = value ? 1 : 0; return DN_OK; }
@@ -443,12 +442,8 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
     CK(util_fill0(m->pf_act, (size_t)TPF_MAX * cfg->ffn * 2));
     m->pf_ok = (H % 128 == 0) && (qd % 128 == 0) && (cfg->ffn % 128 == 0) && ((cfg->n_kv_heads * HD) % 128 == 0) &&
                true;
-    for (int b = 0; b < 4 && m->pf_ok; ++b) {
-      const int box = 32 << b;
-      m->pf_ok = make_tmap(&m->tm_xn[b], m->pf_xn, TPF_MAX, H, box) == DN_OK &&
-                 make_tmap(&m->tm_attn[b], m->pf_attn, TPF_MAX, qd, box) == DN_OK &&
-                 make_tmap(&m->tm_act[b], m->pf_act, TPF_MAX, cfg->ffn, box) == DN_OK;
-    }
+    m->pf_ok = m->pf_ok && make_tmap(&m->tm_xn, m->pf_xn, TPF_MAX, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_attn, m->pf_attn, TPF_MAX, qd, TC_XBOX) == DN_OK &&
+               make_tmap(&m->tm_act, m->pf_act, TPF_MAX, cfg->ffn, TC_XBOX) == DN_OK;
     if (cfg->n_experts > 0 && m->pf_ok) {
       const int P = TPF_MAX * cfg->top_k, E = cfg->n_experts;
       m->moe_max_tiles = P / 64 + E;
@@ -463,10 +458,7 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
       CK(util_fill0(m->moe_xg, (size_t)P * H * 2));
       CK(util_fill0(m->moe_act, (size_t)P * cfg->ffn * 2));
       for (int i = 0; i < n_layers; ++i) m->layers[i].emaps = m->moe_maps + (size_t)i * 3 * E;
-      m->moe_tc_ok = true;
-      for (int b = 0; b < 2; ++b)
-        m->moe_tc_ok = m->moe_tc_ok && make_tmap(&m->tm_moe_xg[b], m->moe_xg, P, H, 64 << b) == DN_OK &&
-                       make_tmap(&m->tm_moe_act[b], m->moe_act, P, cfg->ffn, 64 << b) == DN_OK;
+      m->moe_tc_ok = make_tmap(&m->tm_moe_xg, m->moe_xg, P, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_moe_act, m->moe_act, P, cfg->ffn, TC_XBOX) == DN_OK;
     }
   }
   *out = m;
@@ -510,7 +502,7 @@ extern "C" int dn_bind_layer(dn_model* m, int abs_layer, const void* const* dev_
     const int cols[7] = {H, H, H, qd, H, H, c.ffn};
     L.tm_ok = m->pf_ok;
     const int n_tm = m->cfg.n_experts > 0 ? 4 : 7;       // MoE layers: the expert FFN runs token by token, no GEMM descriptors
-    for (int i = 0; i < n_tm && L.tm_ok; ++i) L.tm_ok = make_tmap(&L.tm[i], L.w[i], rows[i], cols[i], TC_BM) == DN_OK;
+    for (int i = 0; i < n_tm && L.tm_ok; ++i) L.tm_ok = make_tmap(&L.tm[i], L.w[i], rows[i], cols[i], TC_WBOX) == DN_OK;
   }
   MkLayer& ML = m->mk_host[it->second];
   for (int i = 0; i < DN_W_COUNT; ++i) ML.w[i] = L.w[i];
@@ -541,7 +533,7 @@ extern "C" int dn_bind_layer_experts(dn_model* m, int abs_layer, const void* rou
     bool ok = true;
     for (int i = 0; i < 3 * n_experts && ok; ++i) {
       const bool is_down = i >= 2 * n_experts;
-      ok = make_tmap(&maps[i], tab[i], is_down ? m->cfg.hidden : m->cfg.ffn, is_down ? m->cfg.ffn : m->cfg.hidden, TC_BM) == DN_OK;
+      ok = make_tmap(&maps[i], tab[i], is_down ? m->cfg.hidden : m->cfg.ffn, is_down ? m->cfg.ffn : m->cfg.hidden, TC_WBOX) == DN_OK;
     }
     if (ok) CK(util_h2d(L.emaps, maps.data(), maps.size() * sizeof(CUtensorMap)));
     L.emaps_ok = ok;
@@ -782,51 +774,22 @@ static int head_common(dn_model* m, const void* x, int T, dn_kv* kv, int32_t* to
                        float* logits_f32, cudaStream_t s);
 
 // ---- tensor-core prefill path (16 <= T <= TPF_MAX): tcgen05 GEMMs fed by TMA (dn_gemm_tc.cuh)
-template <int BN, int EPI, int STAGES>
-static cudaError_t launch_tc(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, const TcParams& p, cudaStream_t s) {
-  constexpr int NA = epi_two_weights(EPI) ? 2 : 1;
-  constexpr size_t smem = (size_t)STAGES * (NA * TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024 + 256;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, EPI, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  const int tiles = ((p.N + TC_BM - 1) / TC_BM) * ((p.T + BN - 1) / BN);
-  int grid = tiles < g_sms ? tiles : g_sms;
-  if (g_capturing) g_capture_launches++; else g_launches++;
-  k_gemm_tc<BN, EPI, STAGES><<<grid, TC_THREADS, smem, s>>>(w, w2, x, p);
-  return cudaGetLastError();
-}
-// token-tile width: the widest tile that still yields >= ~100 CTAs (a 4096-row matrix has only 32
-// row tiles; narrower token tiles re-read W from L2, not from HBM -- concurrent CTAs share the tile)
+// one launch: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
-static cudaError_t gemm_tc(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap* x /*[4]: 32,64,128,256*/,
-                           const TcParams& p, cudaStream_t s) {
-  const int n_tiles = (p.N + TC_BM - 1) / TC_BM;
-  auto tiles = [&](int bn) { return n_tiles * ((p.T + bn - 1) / bn); };
-  // 256-token tiles halve the L2 -> shared-memory re-reads of W at 512-token chunks (the GEMMs are L2-bound there)
-  if (g_gemm_bn256 && p.T > 128 && tiles(256) >= 100) return launch_tc<256, EPI, (EPI == EPI_SWIGLU ? 3 : 4)>(w, w2, x[3], p, s);
-  if (p.T > 64 && tiles(128) >= 100) return launch_tc<128, EPI, (EPI == EPI_SWIGLU ? 4 : 6)>(w, w2, x[2], p, s);
-  if (p.T > 32 && tiles(64) >= 100) return launch_tc<64, EPI, (EPI == EPI_SWIGLU ? 5 : 8)>(w, w2, x[1], p, s);
-  if (p.T > 32 && tiles(32) < 100 && tiles(64) * 2 > tiles(32)) return launch_tc<64, EPI, (EPI == EPI_SWIGLU ? 5 : 8)>(w, w2, x[1], p, s);
-  return launch_tc<32, EPI, (EPI == EPI_SWIGLU ? 5 : 8)>(w, w2, x[0], p, s);
+static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, cudaStream_t s) {
+  int n_tiles = 0;
+  for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + tc_tile_rows<EPI>() - 1) / tc_tile_rows<EPI>();
+  if (g_capturing) g_capture_launches++; else g_launches++;
+  return tc_launch<EPI, false>(maps, p, tc_plan(n_tiles, p.T, p.K, g_sms), s);
 }
 
-template <int EPI, int BN>
-static cudaError_t gemm_tc_grouped(const CUtensorMap& x, const TcParams& p, cudaStream_t s) {
-  constexpr int NA = epi_two_weights(EPI) ? 2 : 1;
-  constexpr int STAGES = BN == 128 ? (NA == 2 ? 4 : 6) : (NA == 2 ? 5 : 8);
-  constexpr size_t smem = (size_t)STAGES * (NA * TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024 + 256;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, EPI, STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+template <int EPI>
+static cudaError_t gemm_tc_grouped(const CUtensorMap& x, TcParams& p, int width, cudaStream_t s) {
+  TcMaps maps;
+  for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = x;      // (the weights' descriptors lie in global memory)
+  maps.x = x;
   if (g_capturing) g_capture_launches++; else g_launches++;
-  k_gemm_tc<BN, EPI, STAGES, true><<<g_sms, TC_THREADS, smem, s>>>(x, x, x, p);
-  return cudaGetLastError();
+  return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s);
 }
 
 // sparse MoE FFN of a prompt chunk's layer (16 .. TPF_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up
@@ -836,22 +799,19 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   const dn_model_cfg& c = m->cfg;
   const int H = c.hidden, E = c.n_experts, k = c.top_k, P = T * k, mt = m->moe_max_tiles, Pmax = TPF_MAX * k;
   MoePlan pl{m->moe_plan, m->moe_plan + Pmax, m->moe_plan + 2 * Pmax, m->moe_plan + 2 * Pmax + mt, m->moe_plan + 2 * Pmax + 2 * mt, m->moe_plan + 2 * Pmax + 3 * mt};
-  // rows of a token tile: 128 once the experts' average share needs more than one of 64 (the tensor cores then read a weight tile once)
-  const bool wide = P / E > 64;
+  const int width = tc_grouped_width((c.ffn + 127) / 128, E, P, g_sms);
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, false, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   CK(launch(k_moe_route, dim3(T), dim3(256), 0, s, false, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
-  CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, false, (const int32_t*)m->moe_psel, P, k, E, wide ? 128 : 64, pl, E));
+  CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, false, (const int32_t*)m->moe_psel, P, k, E, width, pl, E));
   CK(launch(k_moe_gather<bf16>, dim3(P), dim3(128), 0, s, false, (const bf16*)m->pf_xn, (const int32_t*)pl.row_tok, H, m->moe_xg));
   TcParams p;
   memset(&p, 0, sizeof(p));
   p.err = m->mk_sync + 2;
   p.g_tile_e = pl.tile_e; p.g_tile_r0 = pl.tile_r0; p.g_tile_rows = pl.tile_rows; p.g_ntiles = pl.n_tiles;
-  p.T = P; p.N = c.ffn; p.K = H; p.ldy = c.ffn; p.Y = m->moe_act; p.g_mapW = L.emaps; p.g_mapW2 = L.emaps + E;
-  if (wide) CK((gemm_tc_grouped<EPI_SWIGLU, 128>(m->tm_moe_xg[1], p, s)));
-  else CK((gemm_tc_grouped<EPI_SWIGLU, 64>(m->tm_moe_xg[0], p, s)));
-  p.N = H; p.K = c.ffn; p.ldy = H; p.Y = m->moe_out; p.g_mapW = p.g_mapW2 = L.emaps + 2 * E;
-  if (wide) CK((gemm_tc_grouped<EPI_STORE, 128>(m->tm_moe_act[1], p, s)));
-  else CK((gemm_tc_grouped<EPI_STORE, 64>(m->tm_moe_act[0], p, s)));
+  p.T = P; p.K = H; p.nseg = 1; p.seg[0] = TcSeg{c.ffn, c.ffn, m->moe_act, nullptr, 0}; p.g_mapW = L.emaps; p.g_mapW2 = L.emaps + E;
+  CK(gemm_tc_grouped<EPI_SWIGLU>(m->tm_moe_xg, p, width, s));
+  p.K = c.ffn; p.seg[0] = TcSeg{H, H, m->moe_out, nullptr, 0}; p.g_mapW = p.g_mapW2 = L.emaps + 2 * E;
+  CK(gemm_tc_grouped<EPI_STORE>(m->tm_moe_act, p, width, s));
   CK(launch(k_moe_join, dim3(T), dim3(256), 0, s, false, (const bf16*)m->moe_out, (const int32_t*)pl.pos, (const float*)m->moe_pscore, k, H, h, out));
   return DN_OK;
 }
@@ -893,14 +853,14 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   EV(0);
   k_rmsnorm_rows<<<T, 256, 0, s>>>(x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps);
   g_launches++;
-  p.K = H; p.Y = m->pf_qkv; p.ldy = qkvd;
-  p.N = qd; p.col0 = 0; p.bias = L.w[DN_W_QB];
-  CK(gemm_tc<EPI_STORE>(L.tm[0], L.tm[0], m->tm_xn, p, s));
-  p.N = kd; p.col0 = qd; p.bias = L.w[DN_W_KB];
-  CK(gemm_tc<EPI_STORE>(L.tm[1], L.tm[1], m->tm_xn, p, s));
-  p.col0 = qd + kd; p.bias = L.w[DN_W_VB];
-  CK(gemm_tc<EPI_STORE>(L.tm[2], L.tm[2], m->tm_xn, p, s));
-  p.bias = nullptr;
+  TcMaps maps;
+  for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = L.tm[i < 3 ? i : 0];
+  maps.x = m->tm_xn;
+  p.K = H; p.nseg = 3;      // q, k and v in one launch
+  p.seg[0] = TcSeg{qd, qkvd, m->pf_qkv, L.w[DN_W_QB], 0};
+  p.seg[1] = TcSeg{kd, qkvd, m->pf_qkv + qd, L.w[DN_W_KB], 0};
+  p.seg[2] = TcSeg{kd, qkvd, m->pf_qkv + qd + kd, L.w[DN_W_VB], 0};
+  CK(gemm_tc<EPI_STORE>(maps, p, s));
   const bool kvq = c.kv_bits != 0;
   k_rope_append<<<dim3(c.n_heads + 2 * c.n_kv_heads, T), 128, 0, s>>>(m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
                                                                         kvq ? m->kvq_stage_bt : kv->block_table, kv->st, m->inv_freq,
@@ -928,8 +888,9 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     g_launches++;
   }
   EV(2);
-  p.K = qd; p.N = H; p.Y = m->pf_h; p.ldy = H; p.col0 = 0; p.resid = x; p.ldr = H;
-  CK(gemm_tc<EPI_RESID>(L.tm[3], L.tm[3], m->tm_attn, p, s));
+  p.K = qd; p.nseg = 1; p.seg[0] = TcSeg{H, H, m->pf_h, nullptr, 0}; p.resid = x; p.ldr = H;
+  maps.w[0] = L.tm[3]; maps.x = m->tm_attn;
+  CK(gemm_tc<EPI_RESID>(maps, p, s));
   EV(3);
   if (c.n_experts > 0) {
     if (!L.experts_bound) return fail(DN_ENOENT, "MoE layer has no experts bound (dn_bind_layer_experts)");
@@ -939,11 +900,13 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   }
   k_rmsnorm_rows<<<T, 256, 0, s>>>(m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps);
   g_launches++;
-  p.K = H; p.N = c.ffn; p.Y = m->pf_act; p.ldy = c.ffn; p.resid = nullptr;
-  CK(gemm_tc<EPI_SWIGLU>(L.tm[4], L.tm[5], m->tm_xn, p, s));
+  p.K = H; p.seg[0] = TcSeg{c.ffn, c.ffn, m->pf_act, nullptr, 0};
+  maps.w[0] = L.tm[4]; maps.w[1] = L.tm[5]; maps.x = m->tm_xn;
+  CK(gemm_tc<EPI_SWIGLU>(maps, p, s));
   EV(4);
-  p.K = c.ffn; p.N = H; p.Y = x; p.ldy = H; p.resid = m->pf_h; p.ldr = H;
-  CK(gemm_tc<EPI_RESID>(L.tm[6], L.tm[6], m->tm_act, p, s));
+  p.K = c.ffn; p.seg[0] = TcSeg{H, H, x, nullptr, 0}; p.resid = m->pf_h; p.ldr = H;
+  maps.w[0] = L.tm[6]; maps.x = m->tm_act;
+  CK(gemm_tc<EPI_RESID>(maps, p, s));
   EV(5);
 #undef EV
   CK(cudaGetLastError());

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
 // CTAs that share a row block's keys: what makes (waves of CTAs) x (key tiles of a CTA + 4 for its start, joining and end) smallest.
 // The grid alone (heads x row blocks) leaves most SMs idle when a chunk is short, and a last wave nearly empty when it is long:
 // 40 heads in groups of 5, 512 tokens give 168 CTAs for 148 SMs.
-inline int attn_prefill_split(int ctas, int kv_len, int sms) {
+static inline int attn_prefill_split(int ctas, int kv_len, int sms) {
   const int tiles = (kv_len + 127) / 128;
   int best = 1;
   long long cost = 0;

@@ -1,39 +1,45 @@
-// dn_gemm_tc.cuh -- prefill GEMMs on the 5th-gen tensor cores (tcgen05 + TMEM), operands staged
-// by TMA (cp.async.bulk.tensor.2d, SWIZZLE_128B), warp-specialised: warp 0 = TMA producer, warp 1 =
-// single-thread tcgen05.mma issuer, warp 2 = TMEM allocator, warps 4-7 = epilogue (tcgen05.ld).
+// dn_gemm_tc.cuh -- GEMMs of prompt portions on the 5th-gen tensor cores (tcgen05 + TMEM), operands staged by TMA
+// (cp.async.bulk.tensor.2d, SWIZZLE_128B), two CTAs on one tile (cta_group::2), warp-specialised: warp 0 = TMA producer,
+// warp 1 = MMA issuer (one thread of the leading CTA), warp 2 = TMEM allocator, warps 4-11 = epilogue (tcgen05.ld).
 //
 //   Y[T, N] = X[T, K] . W[N, K]^T        bf16 operands, fp32 accumulate in TMEM
 //
-// "swap-AB" orientation: the WEIGHT tile is the MMA's A operand (M = 128 output features per CTA
-// tile, one TMEM lane each) and the TOKEN tile is B (N = BN tokens = TMEM columns), because prefill
-// chunks have few tokens and many output features; both operands are K-major in shared memory,
-// exactly what TMA produces from the row-major [rows, K] tensors.  Each CTA walks n-tiles
-// persistently; per k-step (64 columns = one 128-byte swizzle span) four UMMA_K=16 instructions.
+// "swap-AB" orientation: the WEIGHT tile is the MMA's A operand (M = 256 rows per pair of CTAs, 128 each, one TMEM lane a row) and
+// the TOKEN tile is B (up to 256 tokens = TMEM columns, half of them staged by each CTA), because prefill chunks have few tokens
+// and many output features; both operands are K-major in shared memory, exactly what TMA produces from row-major [rows, K] tensors.
+// An SM takes about 64 bytes a cycle from L2: a 128 x 128 tile of one CTA needs 128 for full tensor rate, 128 x 256 of a pair's
+// half 64.  A tile is therefore as wide in tokens as the chunk allows (TcPlan), and where that leaves too few tiles for the SMs
+// the reduction is split over the S pairs of a cluster, which add their accumulators through distributed shared memory in a fixed
+// order.  Whole rounds of tiles are walked persistently with two accumulator sets in TMEM; the tiles of a last, mostly empty round
+// are cut into narrower pieces.
+//
+// Up to TC_SEGS products that read the same X run in one launch (q, k, v): tiles of all of them fill the SMs together.
 //
 // Epilogues (fused, same rounding points as the decode kernels / oracle):
-//   EPI_STORE  : y = T(acc + bias)                        -> Y[t][col0 + n]
+//   EPI_STORE  : y = T(acc + bias)                        -> Y[t][n]
 //   EPI_RESID  : y = T(resid[t][n] + T(acc))              -> Y[t][n]
-//   EPI_SWIGLU : two weight tiles (gate, up) share the token tile; g = T(acc_g), u = T(acc_u),
+//   EPI_SWIGLU : gate and up rows share the token tile; g = T(acc_g), u = T(acc_u),
 //                s = T(sigmoid g), a = T(g s), m = T(a u)  -> Y[t][n]
-//   EPI_STORE_F32 : the fp32 accumulator itself               -> ((float*)Y)[t][col0 + n]   (outputs that join an fp32
+//   EPI_STORE_F32 : the fp32 accumulator itself (+ bias)      -> ((float*)Y)[t][n]   (outputs that join an fp32
 //                residual or feed fp32 gates)
-//   EPI_GEGLU  : two weight tiles like EPI_SWIGLU; y = T(gelu_tanh(acc_g) * acc_u), the activation and the product
+//   EPI_GEGLU  : two weights like EPI_SWIGLU; y = T(gelu_tanh(acc_g) * acc_u), the activation and the product
 //                in fp32 with one rounding                     -> Y[t][n]
 //   EPI_TANH   : y = T(tanh(acc))                              -> Y[t][n]
-//   EPI_CGLU   : two weight tiles; g = min(acc_g, limit), u = clamp(acc_u, -limit, limit), y = T(g sigmoid(1.702 g) (u + 1))
-//   EPI_SGLU   : two weight tiles; y = T(silu(acc_g) * acc_u), in fp32 with one rounding
+//   EPI_CGLU   : two weights; g = min(acc_g, limit), u = clamp(acc_u, -limit, limit), y = T(g sigmoid(1.702 g) (u + 1))
+//   EPI_SGLU   : two weights; y = T(silu(acc_g) * acc_u), in fp32 with one rounding
 //   EPI_RELU2  : y = T(relu(acc + bias)^2)
-//   (EPI_STORE_F32 adds the bias too when there is one)
 //   EPI_GELU_TAB : y = T(gelu_tanh(acc) * tab[row[t] tab_ld + n]), in fp32 with one rounding
 //   EPI_JOIN   : an fp32 residual takes the product in, x[t][n] += acc mul ls[n], and the norm that follows is elementwise:
 //                nh[t][n] = T(tanh(alpha x) w + b), or T(x) without an alpha (ls, nh optional; no Y)
+// Two-weight forms stage 64 gate and 64 up rows a CTA.
 //
 // GROUPED: one launch over many weight matrices of one shape (routed experts).  The token rows are sorted by matrix
-// into tiles of BN rows that never span two matrices; a device table gives every token tile its matrix, first row
+// into tiles that never span two matrices; a device table gives every token tile its matrix, first row
 // and row count, and the weights' TMA descriptors lie in an array in global memory (written by the host before the
 // launch).  The number of token tiles is read from device memory, so the host never learns the routing.
 #pragma once
 #include <cuda.h>
+#include <string.h>
 #include "dn_megakernel.cuh"
 
 namespace dn {
@@ -41,26 +47,48 @@ namespace dn {
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_STORE_F32 = 3, EPI_GEGLU = 4, EPI_CGLU = 5, EPI_TANH = 6, EPI_SGLU = 7, EPI_RELU2 = 8, EPI_GELU_TAB = 9, EPI_JOIN = 10 };
 __host__ __device__ constexpr bool epi_two_weights(int epi) { return epi == EPI_SWIGLU || epi == EPI_GEGLU || epi == EPI_CGLU || epi == EPI_SGLU; }
 
-constexpr int TC_BM = 128;        // weight rows per tile (MMA M)
 constexpr int TC_BK = 64;         // k-step: 64 bf16 = 128 bytes = one swizzle span
-constexpr int TC_THREADS = 256;
+constexpr int TC_WBOX = 64;       // rows of a weight descriptor's box
+constexpr int TC_XBOX = 32;       // rows of an activation descriptor's box
+constexpr int TC_WMAX = 256;      // tokens of a tile at most
+constexpr int TC_THREADS = 384;
+constexpr int TC_EWARPS = 8;
+constexpr int TC_SEGS = 4;
+constexpr int TC_A_BYTES = 128 * TC_BK * 2;                       // a CTA's weight rows of a stage
+constexpr int TC_RING = 6 * (TC_A_BYTES + 128 * TC_BK * 2);       // bytes of all stages; also holds a split tile's partial sums
+constexpr int TC_MAX_STAGES = 10;
+constexpr int TC_PITCH = 36, TC_BOX = 16 * TC_PITCH;              // an epilogue warp's [16 tokens][32 features] in floats (16-byte rows, no bank conflicts)
+constexpr int TC_XCH = TC_EWARPS * TC_BOX * 4;
+constexpr int TC_SMEM = TC_RING + TC_XCH + 1024 + 512;
 
-struct TcParams {
-  int T, N, K;                    // tokens, output features, reduction
-  int ldy, col0;                  // output leading dimension (elements) and column offset
+struct TcSeg {                    // one product of a launch
+  int N, ldy;                     // output features, leading dimension of Y (elements)
   bf16* Y;
+  const bf16* bias;               // [N] or null
+  int vec;                        // rows of Y (and of what the epilogue reads) start on 16-byte boundaries (set by tc_launch)
+};
+struct TcMaps {
+  CUtensorMap w[TC_SEGS];         // two-weight forms: [0] gate, [1] up
+  CUtensorMap x;
+};
+struct TcParams {
+  int T, K;                       // tokens, reduction
+  int nseg;
+  TcSeg seg[TC_SEGS];
   const bf16* resid;              // [T][ldr]
   int ldr;
-  const bf16* bias;               // [N] or null
   unsigned int* err;
   float limit;                    // EPI_CGLU
   const bf16* tab; const int32_t* row; int tab_ld;       // EPI_GELU_TAB
-  float* x; const bf16* ls; float mul; const bf16 *nw, *nb, *nalpha; bf16* nh;      // EPI_JOIN, leading dimension ldy
+  float* x; const bf16* ls; float mul; const bf16 *nw, *nb, *nalpha; bf16* nh;      // EPI_JOIN, leading dimension seg[0].ldy
   // GROUPED: token tile tt uses the matrix g_tile_e[tt] on the rows [g_tile_r0[tt], + g_tile_rows[tt]) of X and Y
   const int32_t *g_tile_e, *g_tile_r0, *g_tile_rows, *g_ntiles;
   const CUtensorMap *g_mapW, *g_mapW2;      // [matrices], 64-byte aligned, in global memory
+  // the plan (tc_plan)
+  int width, split, stages;       // tokens of a tile, pairs that share a tile's reduction, stages of the ring
 };
 
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 // address of this CTA's shared object in the cluster's CTA `rank`
 __device__ __forceinline__ uint32_t dsmem_addr(const void* p, uint32_t rank) {
   uint32_t a;
@@ -73,10 +101,30 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
+// bounded wait as mbar_wait, for a barrier that threads of other CTAs arrive on
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned int* err) {
+  if (mbar_try_wait_cluster(bar, parity)) return;
+  const unsigned long long t0 = gtimer();
+  for (unsigned it = 1; !mbar_try_wait_cluster(bar, parity); ++it)
+    if ((it & 1023u) == 0 && gtimer() - t0 > MK_TIMEOUT_NS) { atomicExch(err, 2u); return; }
+}
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+               : "memory");
+}
+// into this CTA's shared memory, counted on a barrier of the pair's leading CTA (`bar`: its cluster address)
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1)
                : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -84,12 +132,25 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// arrives on the barrier at this offset in every CTA of `mask` once the pair's MMAs so far have retired
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t mask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask) : "memory");
+}
 // D[tmem] (+)= A[smem] . B[smem]^T   (kind::f16: bf16 x bf16 -> fp32)
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// the same on both CTAs of a pair: A rows 0-127 (128-255) and the first (second) half of B's rows from the leading (other) CTA
+__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
@@ -121,19 +182,6 @@ __device__ __forceinline__ uint64_t tc_smem_desc(const void* smem_ptr) {
 __device__ __forceinline__ uint32_t tc_instr_desc(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-// 32 lanes x 16 consecutive fp32 columns of this warp's TMEM quarter
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // MN-major, SWIZZLE_128B operand: 64 contiguous elements along N per 128-byte row, 8 k-rows per
 // 1024-byte atom; LBO = bytes between N atoms (dims 0-63 -> 64-127), SBO = bytes between k groups
 __device__ __forceinline__ uint64_t tc_smem_desc_mn(const void* smem_ptr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -151,6 +199,18 @@ __device__ __forceinline__ uint32_t at_swz(int r, int c) {
   return (uint32_t)((c >> 3) * 16384 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
 }
 
+// 32 lanes x 16 consecutive fp32 columns of this warp's TMEM quarter
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
 // 32 consecutive 32-bit columns of this warp's TMEM quarter; the registers are valid after tm_wait_ld and tm_pin
 __device__ __forceinline__ void tm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -171,212 +231,479 @@ __device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sy
 // exponential of the special-function unit (a few units in the last place of fp32, far inside what the bf16 operands carry)
 __device__ __forceinline__ float tc_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
-template <int BN, int EPI, int STAGES, bool GROUPED = false>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-k_gemm_tc(const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapW2,
-          const __grid_constant__ CUtensorMap mapX, const TcParams p) {
-  constexpr int NA = epi_two_weights(EPI) ? 2 : 1;
-  constexpr int A_BYTES = TC_BM * TC_BK * 2;      // 16 KB
-  constexpr int B_BYTES = BN * TC_BK * 2;
-  constexpr int STAGE_BYTES = NA * A_BYTES + B_BYTES;
-  // two accumulator sets when they fit the 512 TMEM columns: the epilogue of tile i drains one while
-  // the MMAs of tile i+1 fill the other
-  constexpr int NACC = (2 * NA * BN <= 512) ? 2 : 1;
-  constexpr int ACC_COLS = NA * BN;
-  constexpr uint32_t TMEM_COLS = (NACC * ACC_COLS <= 32) ? 32 : (NACC * ACC_COLS <= 64) ? 64 : (NACC * ACC_COLS <= 128) ? 128 : (NACC * ACC_COLS <= 256) ? 256 : 512;
+// a launch's tiles.  Rounds of whole tiles, then the last tiles cut `cut` times along the tokens, so that their round is shorter
+struct TcTiles {
+  int t_tiles, whole, cut, units;
+};
+__host__ __device__ __forceinline__ TcTiles tc_tiles(int n_tiles, int t_tiles, int width, int split, int pairs) {
+  TcTiles r;
+  r.t_tiles = t_tiles;
+  const int total = n_tiles * t_tiles, rest = total % pairs;
+  r.cut = split > 1 || rest == 0 ? 1 : rest * 4 <= pairs && width % 128 == 0 ? 4 : rest * 2 <= pairs && width % 64 == 0 ? 2 : 1;
+  r.whole = r.cut > 1 ? total - rest : total;
+  r.units = r.whole + (total - r.whole) * r.cut;
+  return r;
+}
+template <int EPI>
+__host__ __device__ constexpr int tc_tile_rows() { return epi_two_weights(EPI) ? 128 : 256; }      // output features of a pair's tile
+
+template <int EPI, bool GROUPED = false>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant__ TcMaps maps, const __grid_constant__ TcParams p) {
+  constexpr bool GLU = epi_two_weights(EPI);
+  constexpr int ROWS = tc_tile_rows<EPI>();
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)STAGES * STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tmem_full = empty + STAGES;          // [2]
-  uint64_t* tmem_empty = tmem_full + 2;          // [2]
+  float* xch = reinterpret_cast<float*>(smem + TC_RING);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + TC_RING + TC_XCH);      // counted in the leading CTA
+  uint64_t* empty = full + TC_MAX_STAGES;
+  uint64_t* tmem_full = empty + TC_MAX_STAGES;   // [2]
+  uint64_t* tmem_empty = tmem_full + 2;          // [2], counted in the leading CTA
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = (p.N + TC_BM - 1) / TC_BM;
-  const int t_tiles = GROUPED ? *p.g_ntiles : (p.T + BN - 1) / BN;
-  const int total_tiles = n_tiles * t_tiles;
-  const int k_steps = p.K / TC_BK;
+  const uint32_t crank = cluster_rank(), lead = crank & ~1u;
+  const int rank = (int)(crank & 1u), part = (int)(crank >> 1);      // place in the pair; which share of a split reduction
+  const int S = p.split, W = p.width, stages = p.stages;
+  int n_tiles = 0;
+  for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + ROWS - 1) / ROWS;
+  const int pairs = (int)gridDim.x / (2 * S), pair = (int)blockIdx.x / (2 * S);      // (a cluster counts once)
+  const TcTiles tl = tc_tiles(n_tiles, GROUPED ? *p.g_ntiles : (p.T + W - 1) / W, W, S, pairs);
+  const int k_all = p.K / TC_BK, k0 = (int)((long long)k_all * part / S), k1 = (int)((long long)k_all * (part + 1) / S);
+  const int stage_bytes = TC_A_BYTES + (W / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], 4); }   // 4: one arrival per epilogue warp
+    for (int i = 0; i < stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], 2 * TC_EWARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 2) {                // TMEM allocation (whole warp), address lands in shared memory
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)), "n"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (warp == 2) {                // TMEM allocation (a warp of each CTA of the pair), address lands in shared memory
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_base_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
+  // a unit's tile: segment and first row of the weights, first token and how many
+  struct Tile { int seg, n0, e, t0, t_end, cols; };
+  auto tile_of = [&](int u) {
+    Tile r;
+    int tile = u, sub = 0;
+    if (u >= tl.whole) { tile = tl.whole + (u - tl.whole) / tl.cut; sub = (u - tl.whole) % tl.cut; }
+    const int w = u >= tl.whole ? W / tl.cut : W;
+    const int tt = tile % tl.t_tiles;             // token tiles of one weight tile run back to back (weights hit L2)
+    int nt = tile / tl.t_tiles;
+    r.seg = 0;
+    while (r.seg + 1 < p.nseg && nt >= (p.seg[r.seg].N + ROWS - 1) / ROWS) { nt -= (p.seg[r.seg].N + ROWS - 1) / ROWS; ++r.seg; }
+    r.n0 = nt * ROWS;
+    r.e = 0;
+    if (GROUPED) {
+      r.e = p.g_tile_e[tt];
+      r.t0 = p.g_tile_r0[tt] + sub * w;
+      r.t_end = min(r.t0 + w, p.g_tile_r0[tt] + p.g_tile_rows[tt]);
+    } else {
+      r.t0 = tt * W + sub * w;
+      r.t_end = min(r.t0 + w, p.T);
+    }
+    r.cols = S > 1 ? W : min(w, (max(r.t_end - r.t0, 1) + 15) & ~15);      // a pair computes whole sixteens of tokens
+    return r;
+  };
+
   if (warp == 0) {
-    // ===================== TMA producer =====================
+    // ===================== TMA producer (each CTA its own rows; bytes counted by the leading CTA) =====================
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-        const int tt = tile % t_tiles, nt = tile / t_tiles;     // token tiles of one weight tile run back to back (weights hit L2)
+      for (int u = pair; u < tl.units; u += pairs) {
+        const Tile tl_ = tile_of(u);
+        const CUtensorMap *mw = &maps.w[tl_.seg], *mw2 = &maps.w[GLU ? 1 : tl_.seg];
         if (GROUPED) {      // descriptors read from global memory: make the host's writes visible to the TMA unit
-          asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(p.g_mapW + p.g_tile_e[tt]) : "memory");
-          if (NA == 2) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(p.g_mapW2 + p.g_tile_e[tt]) : "memory");
+          mw = p.g_mapW + tl_.e;
+          mw2 = GLU ? p.g_mapW2 + tl_.e : mw;
+          asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(mw) : "memory");
+          if (GLU) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(mw2) : "memory");
         }
-        for (int ks = 0; ks < k_steps; ++ks) {
+        const int r0 = GLU ? tl_.n0 + rank * 64 : tl_.n0 + rank * 128, r1 = GLU ? r0 : r0 + 64;
+        const int x0 = tl_.t0 + rank * (tl_.cols / 2), boxes = (tl_.cols / 2 + TC_XBOX - 1) / TC_XBOX;
+        const uint32_t bytes = 2u * (TC_A_BYTES + boxes * (TC_XBOX * TC_BK * 2));
+        for (int ks = k0; ks < k1; ++ks) {
           mbar_wait(&empty[stage], phase ^ 1u, p.err);
-          mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
-          unsigned char* sa = smem + (size_t)stage * STAGE_BYTES;
-          tma_load_2d(sa, GROUPED ? p.g_mapW + p.g_tile_e[tt] : &mapW, ks * TC_BK, nt * TC_BM, &full[stage]);
-          if (NA == 2) tma_load_2d(sa + A_BYTES, GROUPED ? p.g_mapW2 + p.g_tile_e[tt] : &mapW2, ks * TC_BK, nt * TC_BM, &full[stage]);
-          tma_load_2d(sa + NA * A_BYTES, &mapX, ks * TC_BK, GROUPED ? p.g_tile_r0[tt] : tt * BN, &full[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          const uint32_t bar = dsmem_addr(&full[stage], lead);
+          if (rank == 0) mbar_arrive_expect_tx(&full[stage], bytes);
+          unsigned char* sa = smem + (size_t)stage * stage_bytes;
+          tma_load_2d_pair(sa, mw, ks * TC_BK, r0, bar);
+          tma_load_2d_pair(sa + TC_A_BYTES / 2, mw2, ks * TC_BK, r1, bar);
+          for (int i = 0; i < boxes; ++i)
+            tma_load_2d_pair(sa + TC_A_BYTES + i * (TC_XBOX * TC_BK * 2), &maps.x, ks * TC_BK, x0 + i * TC_XBOX, bar);
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
-    // ===================== MMA issuer (one thread) =====================
-    if (lane == 0) {
-      const uint32_t idesc = tc_instr_desc(TC_BM, BN);
+    // ===================== MMA issuer (one thread of the leading CTA) =====================
+    if (lane == 0 && rank == 0) {
+      const uint16_t both = (uint16_t)(3u << lead);
       int stage = 0; uint32_t phase = 0;
       uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-        const uint32_t ab = (NACC == 2) ? (it & 1u) : 0u;              // accumulator set of this tile
-        const uint32_t acc_phase = ((NACC == 2) ? (it >> 1) : it) & 1u;
-        const uint32_t tacc = tmem_base + ab * ACC_COLS;
-        mbar_wait(&tmem_empty[ab], acc_phase ^ 1u, p.err); // epilogue drained this accumulator set
+      for (int u = pair; u < tl.units; u += pairs, ++it) {
+        const uint32_t idesc = tc_instr_desc(256, tile_of(u).cols);
+        const uint32_t ab = it & 1u, acc_phase = (it >> 1) & 1u, tacc = tmem_base + ab * TC_WMAX;
+        mbar_wait_cluster(&tmem_empty[ab], acc_phase ^ 1u, p.err);    // both CTAs' epilogues drained this accumulator set
         tc_fence_after();
-        for (int ks = 0; ks < k_steps; ++ks) {
-          mbar_wait(&full[stage], phase, p.err);
+        for (int ks = k0; ks < k1; ++ks) {
+          mbar_wait(&full[stage], phase, p.err);      // (bytes of both CTAs' copies; arrived on by this CTA alone)
           tc_fence_after();
-          unsigned char* sa = smem + (size_t)stage * STAGE_BYTES;
-          const uint64_t bdesc = tc_smem_desc(sa + NA * A_BYTES);
+          unsigned char* sa = smem + (size_t)stage * stage_bytes;
+          const uint64_t adesc = tc_smem_desc(sa), bdesc = tc_smem_desc(sa + TC_A_BYTES);
 #pragma unroll
-          for (int a = 0; a < NA; ++a) {
-            const uint64_t adesc = tc_smem_desc(sa + a * A_BYTES);
-#pragma unroll
-            for (int k = 0; k < TC_BK / 16; ++k)      // +32 bytes (>>4 = 2) per UMMA_K inside the swizzle span
-              tc_mma(tacc + a * BN, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (ks | k) ? 1u : 0u);
-          }
-          tc_commit(&empty[stage]);                   // smem stage reusable once these MMAs retire
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          for (int k = 0; k < TC_BK / 16; ++k)      // +32 bytes (>>4 = 2) per UMMA_K inside the swizzle span
+            tc_mma_pair(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (ks > k0 || k) ? 1u : 0u);
+          tc_commit_pair(&empty[stage], both);        // both CTAs' stages are reusable once these MMAs retire
+          if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
-        tc_commit(&tmem_full[ab]);                    // accumulator complete -> epilogue
+        tc_commit_pair(&tmem_full[ab], both);         // accumulator complete -> both epilogues
       }
     }
-  } else if (warp >= 4) {
-    // ===================== epilogue: TMEM -> registers -> global =====================
-    const int ew = warp - 4;                          // TMEM lanes [32 ew, 32 ew + 32)
-    uint32_t it = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-      const int tt = tile % t_tiles, nt = tile / t_tiles;     // token tiles of one weight tile run back to back (weights hit L2)
-      const int n = nt * TC_BM + ew * 32 + lane;      // output feature owned by this thread
-      const uint32_t ab = (NACC == 2) ? (it & 1u) : 0u;
-      const uint32_t acc_phase = ((NACC == 2) ? (it >> 1) : it) & 1u;
-      // what a joining epilogue reads is asked for 32 tokens ahead, the first of them before the products are done
-      constexpr bool OPS = EPI == EPI_JOIN || EPI == EPI_GELU_TAB;
-      float jls = 0.f, jw = 0.f, jb = 0.f, ja = 0.f, jx[OPS ? 32 : 1];
-      auto ahead = [&](int c) {
+  }
+
+  // ===================== epilogue: TMEM -> registers -> shared memory -> global =====================
+  const int qd = warp & 3, half = (warp - 4) >> 2;    // TMEM lanes [32 qd, 32 qd + 32); half of the columns
+  const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+  // Columns [c_lo, c_hi) of the accumulator at tacc, sixteen at a time.  A TMEM lane is a feature and a column a token; global memory wants the
+  // features of a token side by side, so every chunk turns in shared memory (`box`, [16 tokens][32 features] a warp) and a thread finishes
+  // eight features of a token: 16-byte loads and stores, 64 bytes a token and warp.  (Straight from the lanes every store is 2 bytes a thread:
+  // the epilogue of a 256 x 256 tile then took longer than its 64 k-steps.)
+  // With parts: `got` holds the other parts' sums [S][per][128], added in the order of the parts, whichever of them adds.
+  float* box = xch + (warp - 4) * TC_BOX;
+  const int tq = lane >> 2, fq = (lane & 3) * 8, up = qd >> 1;
+  constexpr int PASSES = GLU ? 1 : 2;       // of eight tokens
+  auto emit = [&](const Tile& tl_, uint32_t tacc, int c_lo, int c_hi, const float* got, int per) {
+    const TcSeg& sg = p.seg[tl_.seg];
+    const int n = GLU ? tl_.n0 + rank * 64 + (qd & 1) * 32 + fq : tl_.n0 + rank * 128 + qd * 32 + fq;      // first of the thread's eight features
+    const int n_have = min(8, sg.N - n);
+    const bool vec = n_have == 8 && sg.vec;
+    float bias[8], jls[8], jw[8], jb[8], ja = 0.f;
+    if (EPI == EPI_STORE || EPI == EPI_STORE_F32 || EPI == EPI_RELU2)
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int t = tt * BN + c + j;
-          if (t < p.T) jx[OPS ? j : 0] = EPI == EPI_JOIN ? p.x[(size_t)t * p.ldy + n] : __bfloat162float(p.tab[(size_t)p.row[t] * p.tab_ld + n]);
-        }
-      };
-      if (OPS && n < p.N) {
-        ahead(0);
+      for (int i = 0; i < 8; ++i) bias[i] = sg.bias != nullptr && i < n_have ? __bfloat162float(sg.bias[n + i]) : 0.f;
+    if (EPI == EPI_JOIN) {
+      if (p.nalpha) ja = 2.885390081777927f * __bfloat162float(*p.nalpha);      // 2 log2(e) alpha
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        jls[i] = p.ls && i < n_have ? p.mul * __bfloat162float(p.ls[n + i]) : p.mul;
+        jw[i] = p.nalpha && i < n_have ? __bfloat162float(p.nw[n + i]) : 0.f;
+        jb[i] = p.nalpha && i < n_have ? __bfloat162float(p.nb[n + i]) : 0.f;
+      }
+    }
+    // what a joining epilogue reads is asked for a chunk ahead
+    constexpr bool OPS = EPI == EPI_JOIN || EPI == EPI_GELU_TAB || EPI == EPI_RESID;
+    float nxt[OPS ? 2 : 1][8], op[OPS ? 2 : 1][8];
+    auto ahead = [&](int c) {
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        const int cc = c + z * 8 + tq, t = tl_.t0 + cc;
+        if (t >= tl_.t_end || cc >= c_hi || n_have <= 0) continue;
+        float* d = nxt[OPS ? z : 0];
         if (EPI == EPI_JOIN) {
-          jls = p.ls ? p.mul * __bfloat162float(p.ls[n]) : p.mul;
-          if (p.nalpha) { ja = 2.885390081777927f * __bfloat162float(*p.nalpha); jw = __bfloat162float(p.nw[n]); jb = __bfloat162float(p.nb[n]); }      // 2 log2(e) alpha
-        }
-      }
-      mbar_wait(&tmem_full[ab], acc_phase, p.err);
-      tc_fence_after();
-      const uint32_t trow = tmem_base + ab * ACC_COLS + ((uint32_t)(ew * 32) << 16);
-      float bias = 0.f;
-      if ((EPI == EPI_STORE || EPI == EPI_STORE_F32 || EPI == EPI_RELU2) && p.bias != nullptr && n < p.N) bias = __bfloat162float(p.bias[n]);
-      const int t_base = GROUPED ? p.g_tile_r0[tt] : tt * BN;
-      const int t_end = GROUPED ? t_base + p.g_tile_rows[tt] : p.T;
-      if constexpr (OPS) {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          float v[32];
-          tc_ld16(trow + c, *reinterpret_cast<float(*)[16]>(v));
-          tc_ld16(trow + c + 16, *reinterpret_cast<float(*)[16]>(v + 16));
-          if (n >= p.N) continue;
-          float op[32];
+          const float* src = p.x + (size_t)t * sg.ldy + n;
+          if (vec) {
+            *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(src);
+            *reinterpret_cast<float4*>(d + 4) = *reinterpret_cast<const float4*>(src + 4);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) op[j] = jx[j];
-          if (c + 32 < BN) ahead(c + 32);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int t = tt * BN + c + j;
-            if (t >= p.T) continue;
-            if (EPI == EPI_JOIN) {
-              const float xn = op[j] + v[j] * jls;
-              p.x[(size_t)t * p.ldy + n] = xn;
-              // tanh(z) = 1 - 2 / (1 + e^2z): an absolute error of a few 1e-7, far below the rounding of the result
-              if (p.nh) p.nh[(size_t)t * p.ldy + n] = __float2bfloat16_rn(p.nalpha ? fmaf(1.f - __fdividef(2.f, 1.f + exp2f(fminf(ja * xn, 80.f))), jw, jb) : xn);
-            } else {
-              const float g = v[j];
-              p.Y[(size_t)t * p.ldy + p.col0 + n] = __float2bfloat16_rn(0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * op[j]);
-            }
+            for (int i = 0; i < 8; ++i) if (i < n_have) d[i] = src[i];
           }
-        }
-      } else {
-#pragma unroll 1
-      for (int c = 0; c < BN; c += 16) {
-        float v[16], v2[16];
-        tc_ld16(trow + c, v);
-        if (NA == 2) tc_ld16(trow + BN + c, v2);
-        if (n < p.N) {
+        } else {
+          const bf16* src = EPI == EPI_RESID ? p.resid + (size_t)t * p.ldr + n : p.tab + (size_t)p.row[t] * p.tab_ld + n;
+          if (vec) {
+            const uint4 v = *reinterpret_cast<const uint4*>(src);
+            d[0] = bf_lo(v.x); d[1] = bf_hi(v.x); d[2] = bf_lo(v.y); d[3] = bf_hi(v.y); d[4] = bf_lo(v.z); d[5] = bf_hi(v.z); d[6] = bf_lo(v.w); d[7] = bf_hi(v.w);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int t = t_base + c + j;
-            if (t < t_end) {
-              if (EPI == EPI_STORE_F32) {
-                reinterpret_cast<float*>(p.Y)[(size_t)t * p.ldy + p.col0 + n] = v[j] + bias;
-                continue;
-              }
-              float y;
-              if (EPI == EPI_GEGLU) {
-                const float g = v[j];
-                y = 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * v2[j];
-              } else if (EPI == EPI_TANH) {
-                y = tanhf(v[j]);
-              } else if (EPI == EPI_SGLU) {
-                y = v[j] / (1.0f + expf(-v[j])) * v2[j];
-              } else if (EPI == EPI_RELU2) {
-                const float r = fmaxf(v[j] + bias, 0.f);
-                y = r * r;
-              } else if (EPI == EPI_CGLU) {
-                const float g = fminf(v[j], p.limit), u = fminf(fmaxf(v2[j], -p.limit), p.limit);
-                y = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-              } else if (EPI == EPI_STORE) {
-                y = v[j] + bias;
-              } else if (EPI == EPI_RESID) {
-                y = __fadd_rn(__bfloat162float(p.resid[(size_t)t * p.ldr + n]), bf16r(v[j]));
-              } else {
-                const float g = bf16r(v[j]), u = bf16r(v2[j]);
-                const float s = bf16r(1.0f / (1.0f + expf(-g)));
-                y = __fmul_rn(bf16r(__fmul_rn(g, s)), u);
-              }
-              p.Y[(size_t)t * p.ldy + p.col0 + n] = __float2bfloat16_rn(y);
-            }
+            for (int i = 0; i < 8; ++i) if (i < n_have) d[i] = __bfloat162float(src[i]);
           }
         }
       }
+    };
+    if (OPS) ahead(c_lo);
+#pragma unroll 1
+    for (int c = c_lo; c < c_hi; c += 16) {
+      float v[16];
+      tc_ld16(tacc + lane_off + c, v);
+      if (S > 1) {
+        float s[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s[j] = 0.f;
+        for (int q = 0; q < S; ++q)
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < c_hi) s[j] += q == part ? v[j] : got[((size_t)q * per + (c + j - part * per)) * 128 + qd * 32 + lane];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = s[j];
       }
-      tc_fence_before();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) box[j * TC_PITCH + lane] = v[j];
+      if (OPS) {
+#pragma unroll
+        for (int z = 0; z < 2; ++z)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) op[OPS ? z : 0][i] = nxt[OPS ? z : 0][i];
+        if (c + 16 < c_hi) ahead(c + 16);
+      }
+      // (two weights: lanes 0-63 hold the gate products and 64-127 the up products of the same features; each of the two warps finishes
+      // eight of the sixteen tokens)
+      if (GLU) asm volatile("bar.sync %0, 64;" ::"r"(2 + half * 2 + (qd & 1)) : "memory");
+      else __syncwarp();
+      const float* box_g = GLU ? xch + (warp - 4 - 2 * up) * TC_BOX : box;
+      const float* box_u = GLU ? box_g + 2 * TC_BOX : box;
+#pragma unroll
+      for (int z = 0; z < PASSES; ++z) {
+        const int j = (GLU ? up : z) * 8 + tq, t = tl_.t0 + c + j;
+        if (t >= tl_.t_end || c + j >= c_hi || n_have <= 0) continue;
+        float a[8], b[8], y[8];
+        *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(box_g + j * TC_PITCH + fq);
+        *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(box_g + j * TC_PITCH + fq + 4);
+        if (GLU) {
+          *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(box_u + j * TC_PITCH + fq);
+          *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(box_u + j * TC_PITCH + fq + 4);
+        }
+        const float* o = op[OPS ? z : 0];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (EPI == EPI_STORE || EPI == EPI_STORE_F32) {
+            y[i] = a[i] + bias[i];
+          } else if (EPI == EPI_JOIN) {
+            y[i] = o[i] + a[i] * jls[i];
+          } else if (EPI == EPI_GELU_TAB) {
+            y[i] = 0.5f * a[i] * (1.0f + tanhf(0.7978845608028654f * (a[i] + 0.044715f * a[i] * a[i] * a[i]))) * o[i];
+          } else if (EPI == EPI_GEGLU) {
+            y[i] = 0.5f * a[i] * (1.0f + tanhf(0.7978845608028654f * (a[i] + 0.044715f * a[i] * a[i] * a[i]))) * b[i];
+          } else if (EPI == EPI_TANH) {
+            y[i] = tanhf(a[i]);
+          } else if (EPI == EPI_SGLU) {
+            y[i] = a[i] / (1.0f + expf(-a[i])) * b[i];
+          } else if (EPI == EPI_RELU2) {
+            const float r = fmaxf(a[i] + bias[i], 0.f);
+            y[i] = r * r;
+          } else if (EPI == EPI_CGLU) {
+            const float g = fminf(a[i], p.limit), u = fminf(fmaxf(b[i], -p.limit), p.limit);
+            y[i] = g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
+          } else if (EPI == EPI_RESID) {
+            y[i] = __fadd_rn(o[i], bf16r(a[i]));
+          } else {
+            const float g = bf16r(a[i]), u = bf16r(b[i]);
+            const float s = bf16r(1.0f / (1.0f + expf(-g)));
+            y[i] = __fmul_rn(bf16r(__fmul_rn(g, s)), u);
+          }
+        }
+        if (EPI == EPI_STORE_F32 || EPI == EPI_JOIN) {
+          float* dst = (EPI == EPI_JOIN ? p.x : reinterpret_cast<float*>(sg.Y)) + (size_t)t * sg.ldy + n;
+          if (vec) {
+            *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(y);
+            *reinterpret_cast<float4*>(dst + 4) = *reinterpret_cast<const float4*>(y + 4);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) if (i < n_have) dst[i] = y[i];
+          }
+          if (EPI == EPI_STORE_F32 || !p.nh) continue;
+        }
+        if (EPI == EPI_JOIN) {      // the norm that follows.  tanh(z) = 1 - 2 / (1 + e^2z): an absolute error of a few 1e-7, far below the rounding of the result
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (p.nalpha) y[i] = fmaf(1.f - __fdividef(2.f, 1.f + exp2f(fminf(ja * y[i], 80.f))), jw[i], jb[i]);
+        }
+        bf16* dst = (EPI == EPI_JOIN ? p.nh : sg.Y) + (size_t)t * sg.ldy + n;
+        if (vec) {
+          __align__(16) bf16 w[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) w[i] = __float2bfloat16_rn(y[i]);
+          *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(w);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) if (i < n_have) dst[i] = __float2bfloat16_rn(y[i]);
+        }
+      }
+      // the box may be written again
+      if (GLU) asm volatile("bar.sync %0, 64;" ::"r"(2 + half * 2 + (qd & 1)) : "memory");
+      else __syncwarp();
+    }
+  };
+
+  if (S == 1) {
+    if (warp >= 4) {
+      uint32_t it = 0;
+      for (int u = pair; u < tl.units; u += pairs, ++it) {
+        const Tile tl_ = tile_of(u);
+        const uint32_t ab = it & 1u, acc_phase = (it >> 1) & 1u;
+        const int hw = tl_.cols / 2;
+        mbar_wait(&tmem_full[ab], acc_phase, p.err);
+        __syncwarp();
+        tc_fence_after();
+        emit(tl_, tmem_base + ab * TC_WMAX, half * hw, half * hw + hw, nullptr, 0);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(dsmem_addr(&tmem_empty[ab], lead));
+      }
+    }
+  } else {
+    // one tile a cluster: the S pairs' accumulators meet, every pair finishes 1 / S of the columns
+    float* got = reinterpret_cast<float*>(smem);      // [S][per][128], over the ring: no stage is in use any more
+    const int per = W / S;
+    const Tile tl_ = tile_of(pair);
+    if (warp >= 4) {
+      mbar_wait(&tmem_full[0], 0u, p.err);
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[ab]);
+      tc_fence_after();
+    }
+    __syncwarp();
+    cluster_sync();                   // every pair's MMAs have read their stages
+    if (warp >= 4) {
+      const int row = qd * 32 + lane;
+      for (int q = 0; q < S; ++q) {
+        if (q == part) continue;
+        const uint32_t dst = dsmem_addr(got + (size_t)part * per * 128 + row, (uint32_t)(2 * q + rank));
+        for (int c = half * (per / 2); c < (half + 1) * (per / 2); c += 8) {
+          uint32_t r[8];
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                       : "r"(tmem_base + lane_off + q * per + c));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j) dsmem_st(dst + (uint32_t)((c + j) * 512), __uint_as_float(r[j]));
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync();                   // the other pairs' sums are here
+    if (warp >= 4) {
+      const int lo = part * per + half * (per / 2);
+      emit(tl_, tmem_base, lo, lo + per / 2, got, per);
     }
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();                     // nobody leaves while the pair's other CTA may still read its memory or count on its barriers
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
+}
+
+// ---------------------------------------------------------------------------------
+// the plan of a launch (host).  Internal linkage: a process may load both libraries, and the statics of shared inline functions would be one object
+// ---------------------------------------------------------------------------------
+struct TcPlan { int width, split, stages, grid; };
+static inline int tc_stages(int width) {
+  const int s = TC_RING / (TC_A_BYTES + (width / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2));
+  return s < TC_MAX_STAGES ? s : TC_MAX_STAGES;
+}
+static inline void tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int grid, int cluster, cudaStream_t s) {
+  memset(cfg, 0, sizeof(*cfg));
+  cfg->gridDim = dim3(grid);
+  cfg->blockDim = dim3(TC_THREADS);
+  cfg->dynamicSmemBytes = TC_SMEM;
+  cfg->stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = cluster;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+}
+// clusters of 2 S CTAs that run at once (asked of the device once; the SMs of a processing cluster hold whole ones: 33 of 4, 15 of 8)
+static inline int tc_clusters(int S, int sms) {
+  static int n[5] = {0, 0, 0, 0, 0};
+  if (n[S] == 0) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    int c = 0;
+    tc_config(&cfg, at, 2 * S * sms, 2 * S, 0);
+    if (cudaFuncSetAttribute(k_gemm_tc<EPI_STORE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&c, k_gemm_tc<EPI_STORE, false>, &cfg) != cudaSuccess || c < 1) {
+      cudaGetLastError();
+      c = sms / (2 * S) * 3 / 4;
+    }
+    n[S] = c > 0 ? c : 1;
+  }
+  return n[S];
+}
+// What a plan is expected to take, in microseconds.  A k-step takes at least 0.28 (the way of a stage through the ring) and otherwise as long
+// as its bytes from L2, of which all SMs together get 10.8 TB/s (a 256-token tile's MMAs take as long as its bytes); a launch that fills
+// more than half of the SMs with pairs does no better than 120 of them would.  The weights come out of DRAM at 5.6 TB/s at best.  Start and
+// end of a launch cost 6, 10.5 where partial sums meet, and the epilogue of the last tile, which nothing hides, grows with its tokens.
+// Against all widths and splits at 47 shapes (2,048 .. 27,648 features, reductions of 2,048 .. 27,648, 16 .. 2,048 tokens) the plan so
+// chosen was the fastest or within a tenth of it at 45.
+static inline double tc_step(int active, int w) {
+  const int bytes = TC_A_BYTES + (w / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
+  if (active > 72 && active < 120) active = 120;
+  const double t = active * (double)bytes / 10.8e6;
+  return t > 0.28 ? t : 0.28;
+}
+static inline double tc_cost(int n_tiles, int T, int K, int w, int S, int sms) {
+  const int pairs = sms / 2, t_tiles = (T + w - 1) / w, ks = K / TC_BK;
+  const double dram = n_tiles * 256.0 * K * 2.0 / 5.6e6 + 7.0;
+  double c;
+  if (S > 1) {
+    const int at_once = tc_clusters(S, sms), total = n_tiles * t_tiles, rounds = (total + at_once - 1) / at_once;
+    c = rounds * ((ks + S - 1) / S * tc_step((total < at_once ? total : at_once) * 2 * S, w) + 10.5 + 0.035 * w);
+  } else {
+    const TcTiles tl = tc_tiles(n_tiles, t_tiles, w, 1, pairs);
+    c = tl.whole / pairs * (ks * tc_step(sms, w)) + 6.0 + 0.024 * w;
+    if (tl.whole % pairs) c += ks * tc_step(2 * (tl.whole % pairs), w);
+    if (tl.cut > 1) c += ks * tc_step(2 * (tl.units - tl.whole), w / tl.cut);
+  }
+  return c > dram ? c : dram;
+}
+static inline TcPlan tc_plan(int n_tiles, int T, int K, int sms) {
+  TcPlan best{0, 1, 0, 0};
+  double cost = 0;
+  const int ks = K / TC_BK;
+  for (int S = 1; S <= 4; ++S) {
+    if (S > 1 && ks < 8 * S) break;
+    for (int w = 64; w <= TC_WMAX; w += 32) {
+      if (w % (16 * S) || (w > 96 && w >= T + 32)) continue;
+      const double c = tc_cost(n_tiles, T, K, w, S, sms);
+      if (!best.width || c < cost * 0.999) { cost = c; best.width = w; best.split = S; }
+    }
+  }
+  best.stages = tc_stages(best.width);
+  const TcTiles tl = tc_tiles(n_tiles, (T + best.width - 1) / best.width, best.width, best.split, sms / 2);
+  best.grid = best.split > 1 ? 2 * best.split * tl.units : 2 * (tl.units < sms / 2 ? tl.units : sms / 2);
+  return best;
+}
+// rows of a grouped launch's tiles: P rows over E matrices, taken as equal shares (a tile computes no more rows than it has)
+static inline int tc_grouped_width(int n_tiles, int E, int P, int sms) {
+  const int avg = (P + E - 1) / E, pairs = sms / 2;
+  int best = 64;
+  long long cost = 0;
+  for (int w = 64; w <= TC_WMAX; w *= 2) {
+    const int cols = avg < w ? (avg + 15) & ~15 : w;
+    const long long c = (long long)(n_tiles * E * ((avg + w - 1) / w) + pairs - 1) / pairs * (256 + cols);
+    if (w == 64 || c < cost) { cost = c; best = w; }
+  }
+  return best;
+}
+template <int EPI, bool GROUPED>
+static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPlan& pl, cudaStream_t s) {
+  p.width = pl.width; p.split = pl.split; p.stages = pl.stages;
+  for (int i = 0; i < p.nseg; ++i) {
+    TcSeg& sg = p.seg[i];
+    bool v = sg.ldy % 8 == 0 && ((uintptr_t)sg.Y & 15) == 0;
+    if (EPI == EPI_RESID) v = v && p.ldr % 8 == 0 && ((uintptr_t)p.resid & 15) == 0;
+    if (EPI == EPI_GELU_TAB) v = v && p.tab_ld % 8 == 0 && ((uintptr_t)p.tab & 15) == 0;
+    if (EPI == EPI_JOIN) v = v && (((uintptr_t)p.x | (uintptr_t)p.nh) & 15) == 0;
+    sg.vec = v;
+  }
+  static bool attr = false;
+  if (!attr) {
+    const cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<EPI, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  tc_config(&cfg, at, pl.grid, 2 * pl.split, s);
+  return cudaLaunchKernelEx(&cfg, k_gemm_tc<EPI, GROUPED>, maps, p);
 }
 
 // ---------------------------------------------------------------------------------

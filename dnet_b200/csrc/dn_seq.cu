@@ -22,6 +22,7 @@
 #include <new>
 #include <type_traits>
 #include <vector>
+#include <initializer_list>
 
 using namespace dnseq;
 
@@ -54,7 +55,7 @@ static size_t g_max_smem = 0;
 
 // weight matrices and the activation buffers they multiply get TMA descriptors in bf16 mode
 struct XMaps {
-  CUtensorMap m[3];     // token tiles of 32 / 64 / 128 rows
+  CUtensorMap m;
   bool ok = false;
 };
 struct SeqLayer {
@@ -73,7 +74,7 @@ struct SeqLayer {
   const void** etab_d;
   CUtensorMap* emaps_d;              // [3][E] TMA descriptors of the experts' matrices, in device memory (bf16 mode)
   std::vector<char> emap_ok;
-  CUtensorMap x_eact[2];             // the experts' activations [pairs, ff], 64- and 128-row boxes
+  CUtensorMap x_eact;                // the experts' activations [pairs, ff]
   bool x_eact_ok;
 };
 // One run of a layer.  A layer inside the loop runs loop_times times on the same weights; every run has its own
@@ -92,7 +93,7 @@ struct dn_seq_model {
   std::vector<Run> runs;
   const void *embed = nullptr, *final_norm = nullptr, *head = nullptr;
   const void* mw[16] = {nullptr};     // the other model tensors, by (which - DN_SQ_EMBED)
-  CUtensorMap tm_loop_in, x_xg[2];    // x_xg: the tokens' rows sorted by expert [pairs, W], 64- and 128-row boxes
+  CUtensorMap tm_loop_in, x_xg;       // x_xg: the tokens' rows sorted by expert [pairs, W]
   bool tm_loop_ok = false, x_xg_ok = false;
   void* xg = nullptr;
   float* attn_part = nullptr;         // partials of split attention rows [AT_SPLIT_ROWS][heads][AT_MAX_SPLITS][2 + vdim padded]
@@ -208,9 +209,7 @@ static bool sig_tc_sizes(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {
          (c.dim == 64 || c.dim == 128) && (c.vdim == 64 || c.vdim == 128) && (size_t)c.heads * dist_span(cfg, c) <= DIST_TAB_MAX;
 }
 static void make_xmaps(XMaps* x, const void* base, int rows, int cols) {
-  x->ok = true;
-  const int br[3] = {32, 64, 128};
-  for (int i = 0; i < 3; i++) x->ok = x->ok && make_tmap(&x->m[i], base, rows, cols, br[i]);
+  x->ok = make_tmap(&x->m, base, rows, cols, dn::TC_XBOX);
 }
 
 static int n_maps(const dn_seq_layer_cfg& c) { return c.maps == 2 ? 2 : 1; }
@@ -597,10 +596,10 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
       if (fa > 0) make_xmaps(&l.x_act, m->act, m->MB, fa);
     }
     if (m->xg) {
-      m->x_xg_ok = make_tmap(&m->x_xg[0], m->xg, m->MB * mpairs, cfg->width, 64) && make_tmap(&m->x_xg[1], m->xg, m->MB * mpairs, cfg->width, 128);
+      m->x_xg_ok = make_tmap(&m->x_xg, m->xg, m->MB * mpairs, cfg->width, dn::TC_XBOX);
       for (auto& l : m->L)
         if (l.c.mlp_kind == DN_MLP_MOE && l.c.ff > 0)
-          l.x_eact_ok = make_tmap(&l.x_eact[0], m->eact, m->MB * l.c.top, l.c.ff, 64) && make_tmap(&l.x_eact[1], m->eact, m->MB * l.c.top, l.c.ff, 128);
+          l.x_eact_ok = make_tmap(&l.x_eact, m->eact, m->MB * l.c.top, l.c.ff, dn::TC_XBOX);
     }
     if (cfg->side_dim > 0) make_xmaps(&m->x_side, m->act, m->MB, cfg->side_dim);
     if (m->cat) make_xmaps(&m->x_cat, m->cat, m->MB, 2 * cfg->width);
@@ -629,10 +628,10 @@ extern "C" int dn_seq_bind(dn_seq_model* m, int layer, int which, const void* p)
     else if (which == DN_SQ_FINAL_NORM) m->final_norm = p;
     else if (which == DN_SQ_HEAD) {
       m->head = p;
-      m->tm_head_ok = b16 && make_tmap(&m->tm_head, p, m->cfg.vocab, m->cfg.width, dn::TC_BM);
+      m->tm_head_ok = b16 && make_tmap(&m->tm_head, p, m->cfg.vocab, m->cfg.width, dn::TC_WBOX);
     } else if (which > DN_SQ_HEAD && which <= DN_SQ_SIDE_EMBED) {
       m->mw[which - DN_SQ_EMBED] = p;
-      if (which == DN_SQ_LOOP_IN) m->tm_loop_ok = b16 && make_tmap(&m->tm_loop_in, p, m->cfg.width, 2 * m->cfg.width, dn::TC_BM);
+      if (which == DN_SQ_LOOP_IN) m->tm_loop_ok = b16 && make_tmap(&m->tm_loop_in, p, m->cfg.width, 2 * m->cfg.width, dn::TC_WBOX);
     } else return fail(DN_EINVAL, "tensor %d is not a model tensor", which);
     return DN_OK;
   }
@@ -666,7 +665,7 @@ extern "C" int dn_seq_bind(dn_seq_model* m, int layer, int which, const void* p)
   }
   if (l.c.mlp_kind == DN_MLP_MOE && (which == DN_SQ_GATE || which == DN_SQ_UP || which == DN_SQ_DOWN))
     return fail(DN_EINVAL, "layer %d: the matrices of routed experts are bound with dn_seq_bind_expert", layer);
-  l.tm_ok[which] = b16 && rows > 0 && make_tmap(&l.tm[which], p, rows, cols, dn::TC_BM);
+  l.tm_ok[which] = b16 && rows > 0 && make_tmap(&l.tm[which], p, rows, cols, dn::TC_WBOX);
   return DN_OK;
 }
 
@@ -684,7 +683,7 @@ extern "C" int dn_seq_bind_expert(dn_seq_model* m, int layer, int expert, int wh
   if (l.emaps_d) {
     CUtensorMap tm;
     const bool down = which == DN_SQ_E_DOWN;
-    l.emap_ok[at] = make_tmap(&tm, p, down ? m->cfg.width : l.c.ff, down ? l.c.ff : m->cfg.width, dn::TC_BM) ? 1 : 0;
+    l.emap_ok[at] = make_tmap(&tm, p, down ? m->cfg.width : l.c.ff, down ? l.c.ff : m->cfg.width, dn::TC_WBOX) ? 1 : 0;
     if (l.emap_ok[at]) CK(cudaMemcpy(l.emaps_d + at, &tm, sizeof(tm), cudaMemcpyHostToDevice));
   }
   return DN_OK;
@@ -753,30 +752,21 @@ extern "C" int dn_seq_free_pages(dn_seq_model* m) { return m ? (int)m->free_page
 extern "C" int dn_seq_free_slots(dn_seq_model* m) { return m ? (int)m->free_slots.size() : DN_EINVAL; }
 
 // ---------------------------------------------------------------------------------------------------------------
-template <int BN, int EPI, int STAGES>
-static cudaError_t launch_tc(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, const dn::TcParams& p, cudaStream_t s) {
-  constexpr int NA = dn::epi_two_weights(EPI) ? 2 : 1;
-  constexpr size_t smem = (size_t)STAGES * (NA * dn::TC_BM * dn::TC_BK * 2 + BN * dn::TC_BK * 2) + 1024 + 256;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(dn::k_gemm_tc<BN, EPI, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  const int tiles = ((p.N + dn::TC_BM - 1) / dn::TC_BM) * ((p.T + BN - 1) / BN);
-  g_launches++;
-  dn::k_gemm_tc<BN, EPI, STAGES><<<tiles < g_sms ? tiles : g_sms, dn::TC_THREADS, smem, s>>>(w, w2, x, p);
-  return cudaGetLastError();
-}
-// token-tile width: the widest that still gives about one CTA per SM
+// one launch of the tcgen05 GEMM: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
-static cudaError_t gemm_tc(const CUtensorMap& w, const CUtensorMap& w2, const XMaps& x, const dn::TcParams& p, cudaStream_t s) {
-  constexpr bool two = dn::epi_two_weights(EPI);
-  const int n_tiles = (p.N + dn::TC_BM - 1) / dn::TC_BM;
-  auto tiles = [&](int bn) { return n_tiles * ((p.T + bn - 1) / bn); };
-  if (p.T > 64 && tiles(128) >= 100) return launch_tc<128, EPI, (two ? 4 : 6)>(w, w2, x.m[2], p, s);
-  if (p.T > 32 && (tiles(64) >= 100 || tiles(64) * 2 > tiles(32))) return launch_tc<64, EPI, (two ? 5 : 8)>(w, w2, x.m[1], p, s);
-  return launch_tc<32, EPI, (two ? 5 : 8)>(w, w2, x.m[0], p, s);
+static cudaError_t gemm_tc(const dn::TcMaps& maps, dn::TcParams& p, cudaStream_t s) {
+  int n_tiles = 0;
+  for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + dn::tc_tile_rows<EPI>() - 1) / dn::tc_tile_rows<EPI>();
+  g_launches++;
+  return dn::tc_launch<EPI, false>(maps, p, dn::tc_plan(n_tiles, p.T, p.K, g_sms), s);
+}
+template <int EPI>
+static cudaError_t gemm_tc(const CUtensorMap& w, const CUtensorMap& w2, const XMaps& x, dn::TcParams& p, cudaStream_t s) {
+  dn::TcMaps maps;
+  maps.w[0] = maps.w[2] = maps.w[3] = w;
+  maps.w[1] = w2;
+  maps.x = x.m;
+  return gemm_tc<EPI>(maps, p, s);
 }
 
 // One product Y[N, O] = X[N, K] W[O, K]^T (act: an ACT_* epilogue, the two-operand ones on X W^T and X W2^T).  bf16 batches of 16 tokens and more run on
@@ -794,7 +784,7 @@ static cudaError_t linear(dn_seq_model* m, cudaStream_t s, const T* X, const voi
       (act == ACT_NONE || act == ACT_TANH || act == ACT_RELU2 || act == ACT_GELU_TAB || act == ACT_JOIN || (act_two(act) && tm.w2))) {
     dn::TcParams p;
     memset(&p, 0, sizeof(p));
-    p.T = N; p.N = O; p.K = K; p.ldy = O; p.Y = (dn::bf16*)Y; p.err = m->tc_err; p.limit = alim; p.bias = (const dn::bf16*)bias;
+    p.T = N; p.K = K; p.nseg = 1; p.seg[0] = dn::TcSeg{O, O, (dn::bf16*)Y, (const dn::bf16*)bias, 0}; p.err = m->tc_err; p.limit = alim;
     if (act == ACT_CGLU) return gemm_tc<dn::EPI_CGLU>(*tm.w, *tm.w2, *tm.x, p, s);
     if (act == ACT_SWIGLU) return gemm_tc<dn::EPI_SGLU>(*tm.w, *tm.w2, *tm.x, p, s);
     if (act == ACT_RELU2) return gemm_tc<dn::EPI_RELU2>(*tm.w, *tm.w, *tm.x, p, s);
@@ -1008,20 +998,13 @@ static cudaError_t mark(dn_seq_model* m, int phase, cudaStream_t s) {
 }
 
 // one launch of the tcgen05 GEMM over all experts of a layer (token tiles of MOE_ROWS rows from the plan)
-template <int EPI, int BN>
-static cudaError_t gemm_tc_grouped(const CUtensorMap& x, const dn::TcParams& p, cudaStream_t s) {
-  constexpr int NA = dn::epi_two_weights(EPI) ? 2 : 1;
-  constexpr int STAGES = BN == 128 ? (NA == 2 ? 4 : 6) : (NA == 2 ? 5 : 8);
-  constexpr size_t smem = (size_t)STAGES * (NA * dn::TC_BM * dn::TC_BK * 2 + BN * dn::TC_BK * 2) + 1024 + 256;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(dn::k_gemm_tc<BN, EPI, STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+template <int EPI>
+static cudaError_t gemm_tc_grouped(const CUtensorMap& x, dn::TcParams& p, int width, cudaStream_t s) {
+  dn::TcMaps maps;
+  for (int i = 0; i < dn::TC_SEGS; ++i) maps.w[i] = x;      // (the weights' descriptors lie in global memory)
+  maps.x = x;
   g_launches++;
-  dn::k_gemm_tc<BN, EPI, STAGES, true><<<g_sms, dn::TC_THREADS, smem, s>>>(x, x, x, p);
-  return cudaGetLastError();
+  return dn::tc_launch<EPI, true>(maps, p, dn::TcPlan{width, 1, dn::tc_stages(width), g_sms / 2 * 2}, s);
 }
 
 // the expert products of a routed feed-forward: h [N, W] -> m->y [N, W] (routed sum), m->y2 (shared expert, if any);
@@ -1057,9 +1040,8 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
     const int mt = std::min(m->max_tiles, P / MOE_ROWS + E + 1);
     bool tc = std::is_same<T, bf16>::value && m->x_xg_ok && l.x_eact_ok && l.emaps_d && lc.ff >= 32 && W >= 32;
     for (size_t i = gated ? 0 : E; i < l.emap_ok.size(); i++) tc = tc && l.emap_ok[i];
-    // rows of a token tile: 128 (the tensor cores read the weight tile once for twice the tokens) when an expert gets
-    // two such tiles on average, else 64 (less padding); the CUDA-core tiles are 64 rows
-    const int tile_rows = tc && P / E >= 256 ? 128 : MOE_ROWS;
+    // rows of a token tile: by the plan of the tcgen05 GEMM; the CUDA-core tiles are 64 rows
+    const int feat = gated ? 128 : 256, tile_rows = tc ? dn::tc_grouped_width((lc.ff + feat - 1) / feat, E, P, g_sms) : MOE_ROWS;
     CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * Et + 1) * 4, s, (const int32_t*)m->ridx, P, top, Et, tile_rows, pl, E));
     if (tc) {     // bf16 with TMA-able shapes: every expert's tiles in one launch of the tcgen05 GEMM
       CK(launch(k_moe_gather<T>, dim3(P), dim3(128), 0, s, (const T*)m->h, (const int32_t*)m->rtok, W, (T*)m->xg));
@@ -1068,20 +1050,15 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
       p.err = m->tc_err; p.limit = lc.limit;
       p.g_tile_e = pl.tile_e; p.g_tile_r0 = pl.tile_r0; p.g_tile_rows = pl.tile_rows; p.g_ntiles = pl.n_tiles;
       CK(mark(m, DN_SEQ_PH_MOE_UP, s));
-      p.T = P; p.N = lc.ff; p.K = W; p.ldy = lc.ff; p.Y = (dn::bf16*)m->eact; p.g_mapW = l.emaps_d; p.g_mapW2 = l.emaps_d + E;
+      p.T = P; p.K = W; p.nseg = 1; p.seg[0] = dn::TcSeg{lc.ff, lc.ff, (dn::bf16*)m->eact, nullptr, 0}; p.g_mapW = l.emaps_d; p.g_mapW2 = l.emaps_d + E;
       if (eact == ACT_RELU2) {
         p.g_mapW = p.g_mapW2;      // the up matrices
-        if (tile_rows == 128) CK(gemm_tc_grouped<dn::EPI_RELU2, 128>(m->x_xg[1], p, s));
-        else CK(gemm_tc_grouped<dn::EPI_RELU2, 64>(m->x_xg[0], p, s));
-      } else if (eact == ACT_SWIGLU) {
-        if (tile_rows == 128) CK(gemm_tc_grouped<dn::EPI_SGLU, 128>(m->x_xg[1], p, s));
-        else CK(gemm_tc_grouped<dn::EPI_SGLU, 64>(m->x_xg[0], p, s));
-      } else if (tile_rows == 128) CK(gemm_tc_grouped<dn::EPI_CGLU, 128>(m->x_xg[1], p, s));
-      else CK(gemm_tc_grouped<dn::EPI_CGLU, 64>(m->x_xg[0], p, s));
+        CK(gemm_tc_grouped<dn::EPI_RELU2>(m->x_xg, p, tile_rows, s));
+      } else if (eact == ACT_SWIGLU) CK(gemm_tc_grouped<dn::EPI_SGLU>(m->x_xg, p, tile_rows, s));
+      else CK(gemm_tc_grouped<dn::EPI_CGLU>(m->x_xg, p, tile_rows, s));
       CK(mark(m, DN_SEQ_PH_MOE_DOWN, s));
-      p.N = W; p.K = lc.ff; p.ldy = W; p.Y = (dn::bf16*)m->eo; p.g_mapW = l.emaps_d + 2 * E; p.g_mapW2 = l.emaps_d + 2 * E;
-      if (tile_rows == 128) CK(gemm_tc_grouped<dn::EPI_STORE_F32, 128>(l.x_eact[1], p, s));
-      else CK(gemm_tc_grouped<dn::EPI_STORE_F32, 64>(l.x_eact[0], p, s));
+      p.K = lc.ff; p.seg[0] = dn::TcSeg{W, W, (dn::bf16*)m->eo, nullptr, 0}; p.g_mapW = p.g_mapW2 = l.emaps_d + 2 * E;
+      CK(gemm_tc_grouped<dn::EPI_STORE_F32>(l.x_eact, p, tile_rows, s));
     } else {
       CK(mark(m, DN_SEQ_PH_MOE_UP, s));
       CK(launch(k_moe_tiles<T, true>, dim3((lc.ff + 63) / 64, mt), dim3(256), 0, s, (const T*)m->h, (const void* const*)l.etab_d, E, pl, m->eact, lc.ff, W, lc.limit, eact));
@@ -1219,6 +1196,33 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
                  lc.ff_act == DN_FF_RELU2 ? l.w[DN_SQ_DOWN_B] : nullptr, ep));
     return DN_OK;
   };
+  // products that read the same rows X [N, K]: one launch of the tcgen05 GEMM where all of them can take it.  o32: fp32 results
+  struct Lin { int which; void* y; int rows; };
+  auto lins = [&](SeqLayer& l, const T* X, const XMaps& xm, int K, bool o32, std::initializer_list<Lin> ls) -> cudaError_t {
+    dn::TcMaps maps;
+    dn::TcParams p;
+    memset(&p, 0, sizeof(p));
+    bool ok = std::is_same<T, bf16>::value && N >= 16 && xm.ok;
+    for (const Lin& q : ls)
+      if (q.rows > 0 && ok) {
+        ok = l.tm_ok[q.which] && p.nseg < dn::TC_SEGS;
+        if (!ok) break;
+        maps.w[p.nseg] = l.tm[q.which];
+        p.seg[p.nseg++] = dn::TcSeg{q.rows, q.rows, (dn::bf16*)q.y, nullptr, 0};
+      }
+    if (ok && p.nseg > 1) {
+      for (int i = p.nseg; i < dn::TC_SEGS; ++i) maps.w[i] = maps.w[0];
+      maps.x = xm.m;
+      p.T = N; p.K = K; p.err = m->tc_err;
+      return o32 ? gemm_tc<dn::EPI_STORE_F32>(maps, p, s) : gemm_tc<dn::EPI_STORE>(maps, p, s);
+    }
+    for (const Lin& q : ls)
+      if (q.rows > 0) {
+        const cudaError_t e = linear<T>(m, s, X, l.w[q.which], nullptr, q.y, N, q.rows, K, o32, 0, LinMaps{l.tm_ok[q.which] ? &l.tm[q.which] : nullptr, nullptr, &xm});
+        if (e != cudaSuccess) return e;
+      }
+    return cudaSuccess;
+  };
   bool h_ready = !pre;
   for (int ri = 0; ri < (int)m->runs.size(); ri++) {
     const Run& run = m->runs[ri];
@@ -1283,9 +1287,9 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         if (ride) add(nullptr, DN_SQ_UP, m->act, lc.ff, 0, ACT_RELU2);
         CK(run_segs());
       } else {
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_Q], nullptr, m->uq, N, l.Cq, W, false, 0, LinMaps{wm(DN_SQ_Q), nullptr, &m->x_h}));
-        if (l.Ck) CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_K], nullptr, m->uk, N, l.Ck, W, false, 0, LinMaps{wm(DN_SQ_K), nullptr, &m->x_h}));
-        if (l.Cv) CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_V], nullptr, m->uv, N, l.Cv, W, false, 0, LinMaps{wm(DN_SQ_V), nullptr, &m->x_h}));
+        const bool delta = lc.mixer == DN_MIX_DELTA;
+        CK(lins(l, (const T*)m->h, m->x_h, W, false, {{DN_SQ_Q, m->uq, l.Cq}, {DN_SQ_K, m->uk, l.Ck}, {DN_SQ_V, m->uv, l.Cv}, {DN_SQ_G, m->gt, delta ? l.Co : 0}}));
+        if (delta) CK(lins(l, (const T*)m->h, m->x_h, W, true, {{DN_SQ_A, m->pa, lc.heads}, {DN_SQ_B, m->pb, lc.heads}}));
         if (lc.mixer != DN_MIX_DELTA && lc.out_gate)
           CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_HEAD_GATE], nullptr, m->pa, N, lc.heads, W, true, 0, LinMaps{wm(DN_SQ_HEAD_GATE), nullptr, &m->x_h}));
       }
@@ -1363,8 +1367,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         if (lc.out_gate) add(nullptr, DN_SQ_HEAD_GATE, m->pa, lc.heads, 1);
         CK(run_segs());
       } else {
-        CK(linear<T>(m, s, (const T*)m->h, l.w[q1t], nullptr, q1, N, q1w, W, false, 0, LinMaps{wm(q1t), nullptr, &m->x_h}));
-        if (lc.kv_from < 0) CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_DKV], nullptr, m->uk, N, l.Ck, W, false, 0, LinMaps{wm(DN_SQ_DKV), nullptr, &m->x_h}));
+        CK(lins(l, (const T*)m->h, m->x_h, W, false, {{q1t, q1, q1w}, {DN_SQ_DKV, m->uk, lc.kv_from < 0 ? l.Ck : 0}}));
         if (lc.out_gate)
           CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_HEAD_GATE], nullptr, m->pa, N, lc.heads, W, true, 0, LinMaps{wm(DN_SQ_HEAD_GATE), nullptr, &m->x_h}));
       }
@@ -1415,11 +1418,6 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(launch(k_linear_heads<T>, dim3((lc.vdim + 63) / 64, (N + 63) / 64, lc.heads), dim3(256), 0, s, (const T*)m->gt, w(DN_SQ_UV), (T*)m->mo, N, lc.vdim, R,
                   HeadsGeom{l.Col, R, l.Co, lc.vdim, (size_t)lc.vdim * R, R, 1}));
     } else if (lc.mixer == DN_MIX_DELTA) {
-      if (!few) {
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_A], nullptr, m->pa, N, lc.heads, W, true, 0, LinMaps{wm(DN_SQ_A), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_B], nullptr, m->pb, N, lc.heads, W, true, 0, LinMaps{wm(DN_SQ_B), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_G], nullptr, m->gt, N, l.Co, W, false, 0, LinMaps{wm(DN_SQ_G), nullptr, &m->x_h}));
-      }
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
       CK(launch(k_delta_prep<T>, dim3(N), dim3(256), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
@@ -1520,10 +1518,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         sg.act[sg.n - 1] = ACT_TANH;
         CK(run_segs());
       } else {
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_Q], nullptr, m->uq, N, l.Rc, W, false, 0, LinMaps{wm(DN_SQ_R_Q), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_K], nullptr, m->uk, N, l.Rc, W, false, 0, LinMaps{wm(DN_SQ_R_K), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_V], nullptr, m->uv, N, l.Rv, W, false, 0, LinMaps{wm(DN_SQ_R_V), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_G], nullptr, m->gt, N, l.Rv, W, false, 0, LinMaps{wm(DN_SQ_R_G), nullptr, &m->x_h}));
+        CK(lins(l, (const T*)m->h, m->x_h, W, false, {{DN_SQ_R_Q, m->uq, l.Rc}, {DN_SQ_R_K, m->uk, l.Rc}, {DN_SQ_R_V, m->uv, l.Rv}, {DN_SQ_R_G, m->gt, l.Rv}}));
         CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_A], nullptr, m->aun, N, l.Rc, W, true, 0, LinMaps{wm(DN_SQ_R_A), nullptr, &m->x_h}));
         CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_DECAY1], nullptr, m->lr, N, lc.rank, W, false, ACT_TANH, LinMaps{wm(DN_SQ_DECAY1), nullptr, &m->x_h}));
       }
@@ -1576,10 +1571,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         add(nullptr, DN_SQ_R_G, m->gt, l.Rv, 0); add(nullptr, DN_SQ_DECAY1, m->lr, lc.rank, 0);
         CK(run_segs());
       } else {
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_Q], nullptr, m->uq, N, l.Rc, W, false, 0, LinMaps{wm(DN_SQ_R_Q), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_K], nullptr, m->uk, N, l.Rc, W, false, 0, LinMaps{wm(DN_SQ_R_K), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_V], nullptr, m->uv, N, l.Rv, W, false, 0, LinMaps{wm(DN_SQ_R_V), nullptr, &m->x_h}));
-        CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_R_G], nullptr, m->gt, N, l.Rv, W, false, 0, LinMaps{wm(DN_SQ_R_G), nullptr, &m->x_h}));
+        CK(lins(l, (const T*)m->h, m->x_h, W, false, {{DN_SQ_R_Q, m->uq, l.Rc}, {DN_SQ_R_K, m->uk, l.Rc}, {DN_SQ_R_V, m->uv, l.Rv}, {DN_SQ_R_G, m->gt, l.Rv}}));
         CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_DECAY1], nullptr, m->lr, N, lc.rank, W, false, 0, LinMaps{wm(DN_SQ_DECAY1), nullptr, &m->x_h}));
       }
       CK(linear<T>(m, s, (const T*)m->lr, l.w[DN_SQ_DECAY2], nullptr, m->dz, N, l.Rc, lc.rank, true, 0, LinMaps{wm(DN_SQ_DECAY2), nullptr, &l.x_lr}));

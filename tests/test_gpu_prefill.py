@@ -75,3 +75,25 @@ def test_prefill_attention_groups_and_key_shares(cuda_lib, group, context, T):
         kv.free()
         m.destroy()
     _agree(out[1], out[0])
+
+
+@pytest.mark.parametrize("hidden,ffn,kv_heads,group,T", [(256, 8192, 2, 1, 16), (256, 8192, 2, 1, 45), (768, 1280, 1, 2, 65), (1024, 14336, 2, 4, 129),
+                                                         (512, 2048, 2, 2, 300), (768, 27648, 1, 4, 512)])
+def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_heads, group, T):
+    """k_gemm_tc (tiles of a CTA pair) against the row kernels: features and tokens that leave part of a tile empty, q, k and v in one launch
+    with fewer rows than a tile, reductions shared by the pairs of a cluster, widths of 64 to 256 tokens, last tiles cut narrower."""
+    x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    out = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_prefill", tc)
+            m = _model(kv_heads, group, seed=T, hidden=hidden, ffn=ffn)
+            assert m.max_prefill_chunk == (512 if tc else 0)
+            kv = m.make_cache(max_tokens=576)
+            out[tc] = _call(m, kv, x, 0)
+            assert cuda_lib.dn_step_error(m._h, 0) == 0
+            kv.free()
+            m.destroy()
+    finally:
+        cuda_lib.dn_set_option(b"tc_prefill", 1)
+    _agree(out[1], out[0])
