@@ -7,6 +7,7 @@
 #include "dn_megakernel.cuh"
 #include "dn_gemm_tc.cuh"
 #include "dn_attn_tc.cuh"
+#include "dn_attn_q.cuh"
 #include "dn_moe.cuh"
 #include "../../include/dnet_b200.h"
 
@@ -276,6 +277,10 @@ static cudaError_t init_kernel_attrs() {
 #define ATA(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
   ATA(1) ATA(2) ATA(4) ATA(5) ATA(7) ATA(8)
 #undef ATA
+#define ATQ(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess || \
+                    (e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess) return e;
+  ATQ(1) ATQ(2) ATQ(4) ATQ(5) ATQ(7) ATQ(8)
+#undef ATQ
   return cudaSuccess;
 }
 
@@ -664,8 +669,43 @@ extern "C" int dn_embed(dn_model* m, const int32_t* ids_dev, int T, void* x_out,
   return DN_OK;
 }
 
+// clusters span the grid's z
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, const Args&... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = grid.z;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (g_capturing) g_capture_launches++; else g_launches++;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// a prompt chunk's attention over the quantised pages (T >= 16)
+template <int BITS>
+static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf16* out, int T, dn_kv* kv, cudaStream_t s) {
+  const dn_model_cfg& c = m->cfg;
+  AqParams a;
+  a.a.q = q; a.a.out = out; a.a.block_table = kv->block_table; a.a.st = kv->st;
+  a.a.n_heads = c.n_heads; a.a.n_kv = c.n_kv_heads; a.a.T = T; a.a.err = m->mk_sync + 2;
+  a.pool = pool;
+  const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
+  const dim3 grid(c.n_kv_heads, blocks, attn_prefill_split(c.n_kv_heads * blocks, kv->host_pos + T, g_sms));
+#define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, a)); break;
+  switch (m->G) { PFQ(1) PFQ(2) PFQ(4) PFQ(5) PFQ(7) PFQ(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
+#undef PFQ
+  return DN_OK;
+}
+
 // quantised KV: after the (unchanged) append kernels wrote the T new K/V rows as bf16 into the staging pool, quantise
-// them into the packed pool and run the two-pass quantised attention (dn_kvquant.cuh)
+// them into the packed pool and run the two-pass quantised attention (dn_kvquant.cuh; prompt chunks: dn_attn_q.cuh)
 static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   unsigned char* pool = reinterpret_cast<unsigned char*>(m->kv_pool) + (size_t)li * m->kv_layer_bytes;
@@ -673,6 +713,13 @@ static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_
   const int kv_len_max = g_capturing ? kv->max_tokens : kv->host_pos + T;
   const size_t smem = ((size_t)((kv_len_max + 31) / 32 * 32) + AQ_WARPS * 132) * sizeof(float);
   if (smem > 200 * 1024) return fail(DN_EINVAL, "quantised-KV attention outside the step kernel supports contexts up to ~50K tokens (got %d)", kv_len_max);
+  const dim3 ga(T, 2 * c.n_kv_heads), gq(c.n_heads, T);
+  if (c.kv_bits == 8) {
+    CK(launch(k_kv_quant_append<8>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
+  } else {
+    CK(launch(k_kv_quant_append<4>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
+  }
+  if (T >= 16 && g_tc_attn) return c.kv_bits == 8 ? attend_q_tc<8>(m, pool, q, attn_out, T, kv, s) : attend_q_tc<4>(m, pool, q, attn_out, T, kv, s);
   static size_t smem_set[2] = {0, 0};
   const int bi = c.kv_bits == 8 ? 1 : 0;
   if (smem > smem_set[bi]) {
@@ -682,12 +729,9 @@ static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_
     if (e != cudaSuccess) return fail(DN_ECUDA, "k_attn_q smem attribute: %s", cudaGetErrorString(e));
     smem_set[bi] = want;
   }
-  const dim3 ga(T, 2 * c.n_kv_heads), gq(c.n_heads, T);
   if (c.kv_bits == 8) {
-    CK(launch(k_kv_quant_append<8>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
     CK(launch(k_attn_q<8>, gq, dim3(AQ_WARPS * 32), smem, s, false, q, (const unsigned char*)pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, attn_out, c.n_heads, c.n_kv_heads));
   } else {
-    CK(launch(k_kv_quant_append<4>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
     CK(launch(k_attn_q<4>, gq, dim3(AQ_WARPS * 32), smem, s, false, q, (const unsigned char*)pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, attn_out, c.n_heads, c.n_kv_heads));
   }
   return DN_OK;
@@ -814,25 +858,6 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   CK(gemm_tc_grouped<EPI_STORE>(m->tm_moe_act, p, width, s));
   CK(launch(k_moe_join, dim3(T), dim3(256), 0, s, false, (const bf16*)m->moe_out, (const int32_t*)pl.pos, (const float*)m->moe_pscore, k, H, h, out));
   return DN_OK;
-}
-
-// clusters span the grid's z
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, const Args&... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = grid.z;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  if (g_capturing) g_capture_launches++; else g_launches++;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
 static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {

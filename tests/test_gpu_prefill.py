@@ -97,3 +97,25 @@ def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_h
     finally:
         cuda_lib.dn_set_option(b"tc_prefill", 1)
     _agree(out[1], out[0])
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("group,context,T", [(4, 0, 16), (1, 0, 130), (2, 100, 29), (5, 129, 64), (7, 1000, 40), (8, 2490, 16), (4, 1500, 512)])
+def test_prefill_attention_over_quantised_pages(cuda_lib, bits, group, context, T):
+    """k_attn_prefill_q against the CUDA-core kernel on the same pages: both widths of code, groups with empty rows, tiles cut by the causal
+    edge, shares of a cluster.  Scores and probabilities are rounded to bf16 in both, so a score whose sum lies near an edge may flip: a
+    weight is then off by 2^-8 of itself, less than what the stored outputs may be."""
+    m = _model(2, group, seed=group + bits, kv_bits=bits)
+    kv = m.make_cache(max_tokens=2560)
+    x = torch.randn(context + T, 512, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    out = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_attn", tc)
+            out[tc] = _call(m, kv, x, context)
+        assert cuda_lib.dn_step_error(m._h, 0) == 0
+    finally:
+        cuda_lib.dn_set_option(b"tc_attn", 1)
+        kv.free()
+        m.destroy()
+    _agree(out[1], out[0])
