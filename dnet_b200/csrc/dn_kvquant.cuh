@@ -55,6 +55,36 @@ __device__ __forceinline__ void kvq_load_sb(const unsigned char* unit, int tok, 
   bi = __uint_as_float((uint32_t)__ldcg(s + PAGE * 2 + tok * 2 + g) << 16);
 }
 
+// A tile of up to 32 rows for a whole warp with every load in flight at once: cw[j] = this lane's 4 codes of row row0 + j, and of row
+// row0 + lane the scales and biases of both groups (two bf16 a word); rows from nt on are zero.  (Row by row each load waited for the
+// one before: behind 8,192 tokens a step of two layers and the head took 824 us with the pages not in L2, 546 with; now 417 without.)
+template <int BITS>
+__device__ __forceinline__ void kvq_load_tile(const unsigned char* unit, int row0, int nt, int lane, uint32_t (&cw)[32], uint32_t& sp, uint32_t& bp) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if (BITS == 8) cw[j] = j < nt ? __ldcg(reinterpret_cast<const uint32_t*>(unit + (size_t)(row0 + j) * 128) + lane) : 0u;
+    else cw[j] = j < nt ? (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(unit + (size_t)(row0 + j) * 64) + lane) : 0u;
+  }
+  const uint32_t* sb = reinterpret_cast<const uint32_t*>(unit + KvQ<BITS>::CODES_BYTES);
+  sp = lane < nt ? __ldcg(sb + row0 + lane) : 0u;
+  bp = lane < nt ? __ldcg(sb + PAGE + row0 + lane) : 0u;
+}
+template <int BITS>
+__device__ __forceinline__ void kvq_unpack(uint32_t w, float (&c)[4]) {
+  if (BITS == 8) { c[0] = (float)(w & 0xffu); c[1] = (float)((w >> 8) & 0xffu); c[2] = (float)((w >> 16) & 0xffu); c[3] = (float)(w >> 24); }
+  else { c[0] = (float)(w & 0xfu); c[1] = (float)((w >> 4) & 0xfu); c[2] = (float)((w >> 8) & 0xfu); c[3] = (float)((w >> 12) & 0xfu); }
+}
+template <int BITS>
+__device__ __forceinline__ uint32_t kvq_pack(const float (&c)[4]) {
+  if (BITS == 8) return (uint32_t)c[0] | ((uint32_t)c[1] << 8) | ((uint32_t)c[2] << 16) | ((uint32_t)c[3] << 24);
+  return (uint32_t)c[0] | ((uint32_t)c[1] << 4) | ((uint32_t)c[2] << 8) | ((uint32_t)c[3] << 12);
+}
+// of row j of the tile: the scale (or bias) of this lane's group, out of the lane that holds the row's pair.  pick: kvq_pick(lane)
+__device__ __forceinline__ uint32_t kvq_pick(int lane) { return (lane >> 4) ? 0x3244u : 0x1044u; }
+__device__ __forceinline__ float kvq_of_row(uint32_t pair, int j, uint32_t pick) {
+  return __uint_as_float(__byte_perm(__shfl_sync(0xffffffffu, pair, j), 0u, pick));
+}
+
 // Quantise one 128-dim row held as 4 values per lane (warp-collective).  Returns this lane's 4 codes and the
 // bf16-rounded (scale, bias) of its group -- the values dequantisation uses.
 template <int BITS>

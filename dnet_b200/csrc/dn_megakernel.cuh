@@ -1106,30 +1106,49 @@ __device__ __forceinline__ void mk_attention_q(const MkParams& p, const MkLayer&
       kvq_store_row<BITS>(const_cast<unsigned char*>(kvq_unit<BITS>(pool, pg, 1, kvh, p.n_kv)), pos % PAGE, lane, vc, vsc, vbi);
     }
   }
+  // a tile's codes, scales and biases are asked for a tile ahead; the new token's row, which the pool may not hold yet, takes its place in them
+  const uint32_t pick = kvq_pick(lane);
+  uint32_t cw_a[32], sp_a = 0u, bp_a = 0u;
+  auto fetch = [&](int tile, int kv) {
+    const int t0 = tile << 5;
+    kvq_load_tile<BITS>(kvq_unit<BITS>(pool, p.block_table[t0 / PAGE], kv, kvh, p.n_kv), t0 % PAGE, min(32, kv_len - t0), lane, cw_a, sp_a, bp_a);
+  };
+  auto take = [&](int tile, const float (&nc)[4], float nsc, float nbi, uint32_t (&cwv)[32], uint32_t& sp, uint32_t& bp) {
+    const bool has_new = tile == last_tile;
+    const uint32_t w = kvq_pack<BITS>(nc);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) cwv[j] = has_new && j == jnew ? w : cw_a[j];
+    sp = sp_a; bp = bp_a;
+    if (has_new) {      // (warp-uniform)
+      const uint32_t s2 = (__float_as_uint(__shfl_sync(0xffffffffu, nsc, 0)) >> 16) | (__float_as_uint(__shfl_sync(0xffffffffu, nsc, 16)) & 0xffff0000u);
+      const uint32_t b2 = (__float_as_uint(__shfl_sync(0xffffffffu, nbi, 0)) >> 16) | (__float_as_uint(__shfl_sync(0xffffffffu, nbi, 16)) & 0xffff0000u);
+      if (lane == jnew) { sp = s2; bp = b2; }
+    }
+  };
   // ---- pass A
   float m = -INFINITY;
+  if (tile0 + cw < tile1) fetch(tile0 + cw, 0);
 #pragma unroll 1
   for (int tile = tile0 + cw; tile < tile1; tile += MK_CW) {
     const int t0 = tile << 5, nt = min(32, kv_len - t0);
-    const unsigned char* ku = kvq_unit<BITS>(pool, p.block_table[t0 / PAGE], 0, kvh, p.n_kv);
-    const bool has_new = tile == last_tile;
+    uint32_t cwv[32], sp, bp;
+    take(tile, kc, ksc, kbi, cwv, sp, bp);
+    if (tile + MK_CW < tile1) fetch(tile + MK_CW, 0);
     float sc[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-      sc[j] = 0.f;
-      if (j < nt) {
-        float c[4], s1, b1;
-        if (has_new && j == jnew) { c[0] = kc[0]; c[1] = kc[1]; c[2] = kc[2]; c[3] = kc[3]; s1 = ksc; b1 = kbi; }
-        else { kvq_load_codes<BITS>(ku, (t0 % PAGE) + j, lane, c); kvq_load_sb<BITS>(ku, (t0 % PAGE) + j, lane, s1, b1); }
-        const float dot = fmaf(qv[0], c[0], fmaf(qv[1], c[1], fmaf(qv[2], c[2], qv[3] * c[3])));
-        sc[j] = fmaf(s1, dot, b1 * qsum);
-      }
+      float c[4];
+      kvq_unpack<BITS>(cwv[j], c);
+      const float s1 = kvq_of_row(sp, j, pick), b1 = kvq_of_row(bp, j, pick);
+      const float dot = fmaf(qv[0], c[0], fmaf(qv[1], c[1], fmaf(qv[2], c[2], qv[3] * c[3])));
+      sc[j] = fmaf(s1, dot, b1 * qsum);
     }
     transpose_reduce32(sc, lane);
     const float s = (lane < nt) ? bf16r(sc[0]) : -INFINITY;
     scb[t0 + lane] = s;
     m = fmaxf(m, warp_max(s));
   }
+  if (tile0 + cw < tile1) fetch(tile0 + cw, 1);      // the first value tile is on its way while the sums meet
   if (lane == 0) wpart[cw * 132 + 128] = m;
   cbar_sync();
   float M = -INFINITY;
@@ -1176,15 +1195,17 @@ __device__ __forceinline__ void mk_attention_q(const MkParams& p, const MkLayer&
 #pragma unroll 1
   for (int tile = tile0 + cw; tile < tile1; tile += MK_CW) {
     const int t0 = tile << 5, nt = min(32, kv_len - t0);
-    const unsigned char* vu = kvq_unit<BITS>(pool, p.block_table[t0 / PAGE], 1, kvh, p.n_kv);
-    const bool has_new = tile == last_tile;
+    uint32_t cwv[32], sp, bp;
+    take(tile, vc, vsc, vbi, cwv, sp, bp);
+    if (tile + MK_CW < tile1) fetch(tile + MK_CW, 1);
     const float sl = scb[t0 + lane];
-    const float pl = (lane < nt) ? bf16r(exp2f((sl - M) * LOG2E) * invL) : 0.f;
-    for (int j = 0; j < nt; ++j) {
+    const float pl = (lane < nt) ? bf16r(exp2f((sl - M) * LOG2E) * invL) : 0.f;      // (rows from nt on add zeros)
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
       const float pj = __shfl_sync(0xffffffffu, pl, j);
-      float c[4], s1, b1;
-      if (has_new && j == jnew) { c[0] = vc[0]; c[1] = vc[1]; c[2] = vc[2]; c[3] = vc[3]; s1 = vsc; b1 = vbi; }
-      else { kvq_load_codes<BITS>(vu, (t0 % PAGE) + j, lane, c); kvq_load_sb<BITS>(vu, (t0 % PAGE) + j, lane, s1, b1); }
+      float c[4];
+      kvq_unpack<BITS>(cwv[j], c);
+      const float s1 = kvq_of_row(sp, j, pick), b1 = kvq_of_row(bp, j, pick);
       const float ws = pj * s1;
       o[0] = fmaf(ws, c[0], o[0]); o[1] = fmaf(ws, c[1], o[1]); o[2] = fmaf(ws, c[2], o[2]); o[3] = fmaf(ws, c[3], o[3]);
       ob = fmaf(pj, b1, ob);

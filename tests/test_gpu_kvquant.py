@@ -117,3 +117,32 @@ def test_quantised_kv_pool_is_smaller(cuda_lib):
     assert C.sizeof(_cabi.ModelCfg) == 17 * 4
     unit = {8: 64 * 128 + 64 * 8, 4: 64 * 64 + 64 * 8}
     assert unit[8] * 2 * 8 / 64 == 2176 and unit[4] * 2 * 8 / 64 == 1152
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("n", [30, 62, 126, 255])
+def test_quantised_kv_step_kernel_around_tiles_of_32_rows(cuda_lib, bits, n):
+    """The step kernel asks for a tile of 32 cached rows at a time: contexts that end just before, on and just behind a tile and a page,
+    the new row (not in the pool yet) in a tile of its own and at a tile's end, against the oracle within its order sensitivity."""
+    g = load_golden("tiny_llama")
+    cfgd = g["config"]
+    w = oracle_weights(cfgd, g["wseed"])
+    prompt = np.random.Generator(np.random.PCG64(n)).integers(0, cfgd["vocab_size"], size=n).tolist()
+    steps = 5
+    toks, ref, gaps = _oracle_run(cfgd, w, prompt, steps, bits)
+    alt = _teacher_forced_logits(cfgd, w, prompt, toks, f64=True, kv_bits=bits)
+    tol = max(2e-3, 4.0 * max(rel_inf(ref[i], alt[i]) for i in range(steps)))
+    rt = make_runtime(cfgd, w, range(cfgd["num_hidden_layers"]), megakernel=True, cuda_graphs=False, kv_bits=f"{bits}bit", max_tokens=512)
+    try:
+        ids = prompt
+        for step in range(steps):
+            rt.policy.process(token_message(rt, "edge", ids))
+            res = rt.activation_send_queue.get_nowait()
+            f32, _ = rt.model.head_logits(rt._kv_by_nonce["edge"].x_view(len(ids)))
+            torch.cuda.synchronize()
+            assert rel_inf(f32.cpu(), ref[step]) <= tol, step
+            assert res.token_id == toks[step] or gaps[step] < 3.0
+            ids = [toks[step]]
+        assert cuda_lib.dn_step_error(rt.model._h, rt.compute_stream_ptr) == 0
+    finally:
+        rt.unload_model_core()
