@@ -802,6 +802,16 @@ static cudaError_t linear(dn_seq_model* m, cudaStream_t s, const T* X, const voi
     if (out32) return gemm_tc<dn::EPI_STORE_F32>(*tm.w, *tm.w, *tm.x, p, s);
     return gemm_tc<dn::EPI_STORE>(*tm.w, *tm.w, *tm.x, p, s);
   }
+  if constexpr (std::is_same<T, bf16>::value)
+    if (N <= 8 && (O >= ROWS_SPLIT || act_two(act)) && dn::rows_mma_ok(K, X, W, act_two(act) ? W2 : nullptr)) {
+      const bool own = act == ACT_JOIN || act == ACT_GELU_TAB;      // an epilogue with operands of its own
+#define LM(MODE, EPv) launch(k_linear_mma<MODE, EPv>, dim3((O + (MODE == 1 ? 31 : 15)) / (MODE == 1 ? 32 : 16)), dim3(dn::RM_THREADS), 0, s, (const bf16*)X, (const bf16*)W, \
+                             (const bf16*)W2, Y, out32 ? 1 : 0, N, O, K, act, alim, (const bf16*)bias, epi)
+      if (act_two(act)) return LM(2, false);
+      if (O >= LM_WIDE) return own ? LM(1, true) : LM(1, false);
+      return own ? LM(0, true) : LM(0, false);
+#undef LM
+    }
   if (N <= 8 && O < ROWS_SPLIT && !act_two(act)) {      // few features: the warps of a block split the reduction
 #define LS(NT) launch(k_linear_rows_split<T, NT>, dim3((O + 1) / 2), dim3(256), 0, s, X, (const T*)W, Y, out32 ? 1 : 0, N, O, K, act, alim, (const T*)bias, epi)
     return N == 1 ? LS(1) : N == 2 ? LS(2) : N <= 4 ? LS(4) : LS(8);
@@ -1271,6 +1281,16 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     auto run_segs = [&]() {
       int blocks = 0, rows = 0;
       for (int i = 0; i < sg.n; i++) rows += sg.O[i];
+      if constexpr (std::is_same<T, bf16>::value) {
+        bool mma = true;
+        for (int i = 0; i < sg.n; i++) mma = mma && dn::rows_mma_ok(sg.K[i] > 0 ? sg.K[i] : W, sg.X[i] ? sg.X[i] : m->h, sg.W[i], nullptr);
+        if (mma) {
+          const int per = rows >= LM_WIDE ? 32 : 16;
+          for (int i = 0; i < sg.n; i++) blocks += (sg.O[i] + per - 1) / per;
+          return per == 32 ? launch(k_linear_mma_multi<1>, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W)
+                           : launch(k_linear_mma_multi<0>, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W);
+        }
+      }
       const bool pair = rows >= ROWS_PAIR;
       for (int i = 0; i < sg.n; i++) blocks += pair ? (sg.O[i] + 15) / 16 : (sg.O[i] + 7) / 8;
 #define LR(NT) (pair ? launch(k_linear_rows_multi<T, NT, true>, dim3(blocks), dim3(256), 0, s, (const T*)m->h, sg, N, W) \

@@ -4,7 +4,8 @@
 // a prompt or a single decoded token).  Entry e owns the rows [ent_start[e], ent_start[e+1]) of every [N, *]
 // buffer; its tokens sit at positions ent_pos0[e].. of the sequence in state slot ent_slot[e].  Everything a token
 // computes depends only on its own row, its sequence's cache pages and its slot's recurrent state, and every
-// reduction runs in an order that does not depend on N, E or the page / slot numbers.
+// reduction runs in an order that does not depend on N, E or the page / slot numbers (the matrix products in one that
+// depends on the kernel which N selects: up to 8 rows, up to 15, and from 16 on the plan of the tcgen05 GEMM).
 //
 // Mechanisms (each with its constants as arguments, none tied to one model family):
 //   * residual streams ("hyper-connections"): S fp32 copies of the residual, a learned read-out before a sublayer
@@ -37,6 +38,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "dn_rows_mma.cuh"
 
 namespace dnseq {
 
@@ -915,6 +917,53 @@ __global__ void __launch_bounds__(256) k_linear_rows_multi(const T* __restrict__
   if (o >= sg.O[i]) return;
   linear_rows_at<T, NT, TWO, false>(sg.X[i] ? (const T*)sg.X[i] : X, (const T*)sg.W[i], (const T*)nullptr, sg.Y[i], sg.out32[i] != 0, N, sg.O[i],
                              sg.K[i] > 0 ? sg.K[i] : K, sg.act[i], o, 0.f, (const T*)nullptr, LinEpi<T>{});
+}
+
+// The same products on the tensor cores (bf16, K a multiple of 32, 16-byte rows; dn_rows_mma.cuh).  MODE 0: a block takes 16 features;
+// 1: 32 (each token row is read for twice the weights; from LM_WIDE features on, which fill three blocks an SM either way); 2: 16 of two matrices.
+// The order of a feature's sums is the same in all of them.
+constexpr int LM_WIDE = 7104;
+template <int MODE, bool EP>
+__device__ __forceinline__ void linear_mma_block(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt, const __nv_bfloat16* __restrict__ W2, void* __restrict__ Y,
+                                                 bool out32, int N, int O, int K, int act, int o0, float alim, const __nv_bfloat16* __restrict__ bias,
+                                                 const LinEpi<__nv_bfloat16>& ep) {
+  constexpr int TILES = MODE == 0 ? 1 : 2;
+  __shared__ float red[dn::RM_WARPS * TILES * 128];
+  const int tile = threadIdx.x >> 7, at = threadIdx.x & 127, n = at & 7, o = o0 + (MODE == 1 ? 16 * tile : 0) + (at >> 3);
+  const bool live = n < N && o < O && (MODE == 1 || tile == 0);
+  EpiArgs<__nv_bfloat16> ea;
+  if (EP && live) ea.load(ep, act, n, o, O);      // what the epilogue reads is asked for before the product
+  const __nv_bfloat16* w[TILES];
+  int r0[TILES];
+#pragma unroll
+  for (int i = 0; i < TILES; i++) { w[i] = MODE == 2 && i == 1 ? W2 : Wt; r0[i] = o0 + (MODE == 1 ? 16 * i : 0); }
+  dn::rows_mma_block<TILES>(w, r0, O, X, N, K, red);
+  if (!live) return;
+  const float v = dn::rows_mma_sum<TILES>(red, MODE == 1 ? tile : 0, at) + (bias ? ldf(bias + o) : 0.f);
+  if (EP) { ea.finish(ep, act, v, n, o, O, Y, out32, alim); return; }
+  const float y = act_apply(act, v, MODE == 2 ? dn::rows_mma_sum<TILES>(red, 1, at) : 0.f, alim);
+  if (out32) ((float*)Y)[(size_t)n * O + o] = y;
+  else stf((__nv_bfloat16*)Y + (size_t)n * O + o, y);
+}
+template <int MODE, bool EP>
+__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 ? 3 : 2) k_linear_mma(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt,
+                                                                                const __nv_bfloat16* __restrict__ W2, void* __restrict__ Y, int out32, int N, int O, int K,
+                                                                                int act, float alim, const __nv_bfloat16* __restrict__ bias,
+                                                                                const __grid_constant__ LinEpi<__nv_bfloat16> ep) {
+  linear_mma_block<MODE, EP>(X, Wt, W2, Y, out32 != 0, N, O, K, act, blockIdx.x * (MODE == 1 ? 32 : 16), alim, bias, ep);
+}
+template <int MODE>
+__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 ? 3 : 2) k_linear_mma_multi(const __nv_bfloat16* __restrict__ X, LinSegs sg, int N, int K) {
+  constexpr int PER = MODE == 1 ? 32 : 16;
+  int blk = blockIdx.x, i = 0;
+  for (; i < sg.n; i++) {
+    const int nb = (sg.O[i] + PER - 1) / PER;
+    if (blk < nb) break;
+    blk -= nb;
+  }
+  if (i >= sg.n) return;
+  linear_mma_block<MODE, false>(sg.X[i] ? (const __nv_bfloat16*)sg.X[i] : X, (const __nv_bfloat16*)sg.W[i], nullptr, sg.Y[i], sg.out32[i] != 0, N, sg.O[i],
+                                sg.K[i] > 0 ? sg.K[i] : K, sg.act[i], blk * PER, 0.f, nullptr, LinEpi<__nv_bfloat16>{});
 }
 
 // ---------------------------------------------------------------------------------------------------------------
