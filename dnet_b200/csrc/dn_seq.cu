@@ -1132,6 +1132,8 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
   const float rmul = c.residual_mult != 0.f ? c.residual_mult : 1.f;
   const bool pre = !c.no_pre_norm;      // false: the sublayers read the residual itself, h = T(x)
   auto mwp = [&](int which) { return (const T*)m->mw[which - DN_SQ_EMBED]; };
+  // threads of a mixer's preparation: 16 bytes of channels each, 512 at most (a function of the model only)
+  auto prep_threads = [&](int channels) { return dim3((unsigned)std::min(512, std::max(128, (channels * (int)sizeof(T) / 16 + 31) / 32 * 32))); };
   auto write_back = [&](const T* mix, const T* out) {
     if (W % 4 == 0) return launch(k_write_back<T, 4>, dim3(ew4), dim3(256), 0, s, m->xs, N, W, S, mix, out, (const float*)m->y);
     return launch(k_write_back<T, 1>, dim3(ew), dim3(256), 0, s, m->xs, N, W, S, mix, out, (const float*)m->y);
@@ -1145,6 +1147,24 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
   auto next_norm = [&](const SeqLayer& nl, int which) {
     return NextNorm<T>{(const T*)nl.w[which], (const T*)nl.w[which == DN_SQ_NORM1 ? DN_SQ_NORM1_B : DN_SQ_NORM2_B],
                        (const T*)nl.w[which == DN_SQ_NORM1 ? DN_SQ_NORM1_ALPHA : DN_SQ_NORM2_ALPHA], (T*)m->h};
+  };
+  // A write-back waits for the norm that follows it, which then takes both in one pass (k_turn), or for the next reader of the streams.
+  // (Rows wider than TURN_MAX, more than TURN_STREAMS streams and norms of another kind than RMS keep the kernels apart.)
+  constexpr int TURN_STREAMS = 4;
+  const bool turn = pre && !dyt && lnorm == 0 && W % 4 == 0 && W <= TURN_MAX && S <= TURN_STREAMS;
+  struct { bool due; const T *mix, *out; } owed{false, nullptr, nullptr};
+  auto settle = [&]() -> cudaError_t {
+    if (!owed.due) return cudaSuccess;
+    owed.due = false;
+    return write_back(owed.mix, owed.out);
+  };
+  // rows: the gathered rows of the last norm
+  auto turn_norm = [&](const T* hc_in, const T* nw, int sum_all, int n_rows, const int32_t* rows, T* dst) -> cudaError_t {
+    const bool due = owed.due;
+    owed.due = false;
+    const dim3 thr((unsigned)std::max(32, (W / 4 + 63) / 64 * 32));
+    return launch(S <= 1 ? k_turn<T, 1> : k_turn<T, TURN_STREAMS>, dim3(n_rows), thr, 0, s, m->xs, N, W, S, due ? owed.mix : (const T*)nullptr, due ? owed.out : (const T*)nullptr,
+                  due ? (const float*)m->y : (const float*)nullptr, hc_in, nw, wmode, sum_all, c.eps, rows, dst);
   };
   const MoeSrc<T> no_moe{nullptr, nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, nullptr};
   auto join = [&](SeqLayer& l, int post, int hc_mix, int hc_out, float a, const float* y2, float bb, NextNorm<T> nx, const MoeSrc<T>* ms = nullptr) -> cudaError_t {
@@ -1163,11 +1183,15 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       cudaError_t e = launch(k_axpby, dim3(ew), dim3(256), 0, s, m->y, NW, a, y2 ? y2 : (const float*)m->y, y2 ? bb : 0.f);
       if (e != cudaSuccess) return e;
     }
+    if (turn) {
+      owed = {true, w(hc_mix), w(hc_out)};
+      return cudaSuccess;
+    }
     return write_back(w(hc_mix), w(hc_out));
   };
 #define PH(id) CK(mark(m, id, s))
   PH(DN_SEQ_PH_EMBED);
-  CK(launch(k_embed<T>, dim3(N), dim3(128), 0, s, (const T*)m->embed, b, c.embed_scale, W, S1, m->xs, mwp(DN_SQ_EMBED_NORM), mwp(DN_SQ_EMBED_NORM_B),
+  CK(launch(W % 4 == 0 ? k_embed<T, 4> : k_embed<T, 1>, dim3(N, (W + (W % 4 == 0 ? 511 : 127)) / (W % 4 == 0 ? 512 : 128)), dim3(128), 0, s, (const T*)m->embed, b, c.embed_scale, W, S1, m->xs, mwp(DN_SQ_EMBED_NORM), mwp(DN_SQ_EMBED_NORM_B),
             c.embed_norm ? mwp(DN_SQ_EMBED_NORM_ALPHA) : (const T*)nullptr, m->x0, pre ? (T*)nullptr : (T*)m->h,
             c.bigram_buckets > 0 ? mwp(DN_SQ_BIGRAM) : (const T*)nullptr, c.max_positions > 0 ? mwp(DN_SQ_POS) : (const T*)nullptr));
   // the norm before a sublayer and, where the model has them, the sublayer's input convolution with its carried rows
@@ -1178,8 +1202,13 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     T* dst = taps > 0 && !fused ? (T*)m->hn : (T*)m->h;
     T* cst = taps > 0 ? (T*)m->conv_state + run.canon_off[q] : (T*)nullptr;
     const T* cwq = taps > 0 ? w(q == 0 ? DN_SQ_CANON1 : DN_SQ_CANON2) : (const T*)nullptr;
+    if (turn && !fused && ((uintptr_t)w(nrm) & (4 * sizeof(T) - 1)) == 0)
+      CK(turn_norm(w(q == 0 ? DN_SQ_HC1_IN : DN_SQ_HC2_IN), w(nrm), 0, N, nullptr, dst));
+    else {
+    CK(settle());
     CK(launch(k_read_norm<T>, dim3(N), nthr, nsm, s, m->xs, N, W, S, w(q == 0 ? DN_SQ_HC1_IN : DN_SQ_HC2_IN), w(nrm), wmode, 0, c.eps, (const int32_t*)nullptr, dst,
               w(nb), dyt ? w(na) : (const T*)nullptr, lnorm, fused ? cwq : (const T*)nullptr, taps, b.slot, cst, m->conv_stride));
+    }
     if (taps > 0 && !fused) {
       CK(mark(m, DN_SEQ_PH_CANON, s));
       const int thr = 128, per = thr * (16 / (int)sizeof(T));
@@ -1242,6 +1271,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     auto wm = [&](int i) { return l.tm_ok[i] ? &l.tm[i] : (const CUtensorMap*)nullptr; };
     if (run.inject) {       // a pass of the loop starts: x <- W_in [x; x0]
       PH(DN_SEQ_PH_OTHER);
+      CK(settle());
       CK(launch(k_loop_cat<T>, dim3((unsigned)((2 * NW + 255) / 256)), dim3(256), 0, s, (const float*)m->xs, (const float*)m->x0, N, W, (T*)m->cat));
       CK(linear<T>(m, s, (const T*)m->cat, m->mw[DN_SQ_LOOP_IN - DN_SQ_EMBED], nullptr, m->xs, N, W, 2 * W, true, 0,
                    LinMaps{m->tm_loop_ok ? &m->tm_loop_in : nullptr, nullptr, &m->x_cat}));
@@ -1347,7 +1377,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(launch(k_attn_prep_rot<T>, dim3(N, (units + per * PREP_WARPS - 1) / (per * PREP_WARPS)), dim3(32 * PREP_WARPS), 0, s, a, b, per, (const T*)m->uq, (const T*)m->uk,
                   (const T*)m->uv, w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), (T*)m->qb, (T*)m->kpool[run.kv_index], (T*)m->vpool[run.kv_index]));
       } else
-        CK(launch(k_attn_prep<T>, dim3(N), dim3(256), sm, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv, w(DN_SQ_Q_CONV),
+        CK(launch(k_attn_prep<T>, dim3(N), prep_threads(l.Cq + l.Ck + l.Cv), sm, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv, w(DN_SQ_Q_CONV),
                   w(DN_SQ_K_CONV), w(DN_SQ_V_CONV), w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), cst, m->conv_stride, (T*)m->qb,
                   (T*)m->kpool[run.kv_index], (T*)m->vpool[run.kv_index]));
       if (lc.pool > 0)      // blocks that this step's tokens complete get their mean key and value
@@ -1440,7 +1470,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     } else if (lc.mixer == DN_MIX_DELTA) {
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
-      CK(launch(k_delta_prep<T>, dim3(N), dim3(256), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
+      CK(launch(k_delta_prep<T>, dim3(N), prep_threads(2 * l.Cq + l.Cv), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
                 w(DN_SQ_Q_CONV), w(DN_SQ_K_CONV), w(DN_SQ_V_CONV), (const float*)m->pa, (const float*)m->pb, w(DN_SQ_A_LOG),
                 w(DN_SQ_DT_BIAS), (const T*)cst, m->conv_stride, m->qn, m->kn, m->vv, m->beta, m->decay));
       int R, P;
@@ -1645,6 +1675,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     // ---- token input: x <- x + rms(W_p (gelu(W_g x) * e)) w, and the next run's norm
     if (c.side_dim > 0) {
       PH(DN_SEQ_PH_SIDE);
+      CK(settle());
       const LinEpi<T> ep{mwp(DN_SQ_SIDE_EMBED) + (size_t)run.layer * c.side_dim, b.tok, c.n_layers * c.side_dim, nullptr, nullptr, 1.f, no_next};
       CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_SIDE_GATE], nullptr, m->act, N, c.side_dim, W, false, ACT_GELU_TAB, LinMaps{wm(DN_SQ_SIDE_GATE), nullptr, &m->x_h}, 0.f,
                    nullptr, &ep));
@@ -1653,13 +1684,22 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       h_ready = nx_run.alpha != nullptr;
     }
     PH(DN_SEQ_PH_OTHER);
-    if (trace) CK(launch(k_stream_sum, dim3(ew), dim3(256), 0, s, (const float*)m->xs, N, W, S1, trace + (size_t)ri * N * W));
+    if (trace) {
+      CK(settle());
+      CK(launch(k_stream_sum, dim3(ew), dim3(256), 0, s, (const float*)m->xs, N, W, S1, trace + (size_t)ri * N * W));
+    }
   }
+  // (the streams end here: nothing reads them after the step, and rows that are not wanted are left where they are)
   if (n_want > 0) {
     PH(DN_SEQ_PH_NORM);
+    if (turn && (((uintptr_t)m->final_norm) & (4 * sizeof(T) - 1)) == 0)
+      CK(turn_norm((const T*)nullptr, (const T*)m->final_norm, 1, n_want, want_dev, (T*)m->h));
+    else {
+    CK(settle());
     CK(launch(k_read_norm<T>, dim3(n_want), nthr, nsm, s, m->xs, N, W, S, (const T*)nullptr, (const T*)m->final_norm, wmode, 1, c.eps, want_dev, (T*)m->h,
               mwp(DN_SQ_FINAL_NORM_B), dyt ? mwp(DN_SQ_FINAL_NORM_ALPHA) : (const T*)nullptr, lnorm, (const T*)nullptr, 0, (const int32_t*)nullptr, (T*)nullptr,
               (size_t)0));
+    }
     PH(DN_SEQ_PH_HEAD);
     CK(linear<T>(m, s, (const T*)m->h, m->head, nullptr, logits, n_want, c.vocab, W, true, 0, LinMaps{m->tm_head_ok ? &m->tm_head : nullptr, nullptr, &m->x_h}));
     if (c.logit_softcap > 0.f)

@@ -38,6 +38,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include "dn_rows_mma.cuh"
 
 namespace dnseq {
@@ -75,6 +76,20 @@ __device__ __forceinline__ void stv(bf16* p, const float* o) {
 #pragma unroll
   for (int i = 0; i < 4; i++) h[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
   *reinterpret_cast<uint4*>(p) = v;
+}
+// the same for four numbers
+__device__ __forceinline__ void ld4(const float* p, float (&o)[4]) { *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void ld4(const bf16* p, float (&o)[4]) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+}
+__device__ __forceinline__ void st4(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
+__device__ __forceinline__ void st4(bf16* p, const float (&o)[4]) {
+  uint2 v;
+  *reinterpret_cast<__nv_bfloat162*>(&v.x) = __floats2bfloat162_rn(o[0], o[1]);
+  *reinterpret_cast<__nv_bfloat162*>(&v.y) = __floats2bfloat162_rn(o[2], o[3]);
+  *reinterpret_cast<uint2*>(p) = v;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -165,24 +180,44 @@ struct Batch {
 // embedding -> residual streams
 // nalpha != null: the embedding is dynamic-tanh normed; x0 != null: it is also kept aside (the loop's injection reads it);
 // hout != null: also in the products' number format (models whose sublayers read the residual without a norm)
-template <class T>
+// A thread takes four columns (VEC 4: W a multiple of 4) and gridDim.y blocks share a row: every load of a row is in flight at once.
+// (One block of 128 threads a row, a number at a time: 21 us for four rows of 4,096 into four streams; now 2.5.)
+template <class T, int VEC>
 __global__ void k_embed(const T* __restrict__ embed, Batch b, float scale, int W, int S1, float* __restrict__ xs, const T* __restrict__ nw,
                         const T* __restrict__ nb, const T* __restrict__ nalpha, float* __restrict__ x0, T* __restrict__ hout,
                         const T* __restrict__ bigram, const T* __restrict__ ptab) {
-  const int n = blockIdx.x;
-  const size_t row = (size_t)b.tok[n] * W;
-  const float alpha = nalpha ? ldf(nalpha) : 0.f;
-  const T* brow = bigram ? bigram + (size_t)b.brow[n] * W : nullptr;
-  const T* prow = ptab ? ptab + (size_t)b.pos[n] * W : nullptr;      // learned position row
-  for (int c = threadIdx.x; c < W; c += blockDim.x) {
-    float v = ldf(embed + row + c) * scale;
-    if (brow) v += ldf(brow + c);      // the hashed (previous token, token) row, summed in fp32
-    if (prow) v += ldf(prow + c);
-    if (nalpha) v = dyt_f(v, alpha, nw, nb, c);
-    for (int s = 0; s < S1; s++) xs[((size_t)s * b.N + n) * W + c] = v;
-    if (x0) x0[(size_t)n * W + c] = v;
-    if (hout) stf(hout + (size_t)n * W + c, v);      // the first sublayer reads the residual itself
+  const int n = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+  if (c >= W) return;
+  auto ld = [](const T* p, float (&o)[VEC]) {
+    if constexpr (VEC == 4) ld4(p, o);
+    else o[0] = ldf(p);
+  };
+  auto st = [](auto* p, const float (&o)[VEC]) {
+    if constexpr (VEC == 4) st4(p, o);
+    else stf(p, o[0]);
+  };
+  float v[VEC], t[VEC];
+  ld(embed + (size_t)b.tok[n] * W + c, v);
+#pragma unroll
+  for (int i = 0; i < VEC; i++) v[i] *= scale;
+  if (bigram) {      // the hashed (previous token, token) row, summed in fp32
+    ld(bigram + (size_t)b.brow[n] * W + c, t);
+#pragma unroll
+    for (int i = 0; i < VEC; i++) v[i] += t[i];
   }
+  if (ptab) {      // learned position row
+    ld(ptab + (size_t)b.pos[n] * W + c, t);
+#pragma unroll
+    for (int i = 0; i < VEC; i++) v[i] += t[i];
+  }
+  if (nalpha) {
+    const float alpha = ldf(nalpha);
+#pragma unroll
+    for (int i = 0; i < VEC; i++) v[i] = dyt_f(v[i], alpha, nw, nb, c + i);
+  }
+  for (int s = 0; s < S1; s++) st(xs + ((size_t)s * b.N + n) * W + c, v);
+  if (x0) st(x0 + (size_t)n * W + c, v);
+  if (hout) st(hout + (size_t)n * W + c, v);      // the first sublayer reads the residual itself
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -357,6 +392,93 @@ __global__ void k_write_back(float* __restrict__ xs, int N, int W, int S, const 
     for (int v = 0; v < VEC; v++) a[v] += ot * yy[v];
     if (VEC == 4) *reinterpret_cast<float4*>(xs + (size_t)t * NW + i) = *reinterpret_cast<float4*>(a);
     else xs[(size_t)t * NW + i] = a[0];
+  }
+}
+
+// Between two sublayers: the write-back of one (y null: there is none; S = 0: x <- x + y) and the read-out and RMS norm of the next, a row
+// in registers from its streams to the product's input.
+// Bound by the streams' bytes in prompts and by the chain of loads in steps of a few tokens.  Apart, the norm read the streams a second
+// time: 2,048 tokens, 4 streams of 4,096: 48 + 54 us, together 41 (6.9 TB/s); 4 tokens: 2.6 + 5.1 us, together 4.4.
+// A thread owns two runs of four columns (rows up to TURN_MAX wide), and the norm's weights are asked for before the row's sum is known.
+// Sums and products in the order of k_write_back and k_read_norm.  rows != null: only these are needed, and the streams end here (nothing
+// is written back).
+constexpr int TURN_MAX = 4096;
+template <class T, int SMAX>
+__global__ void __launch_bounds__(512, 2) k_turn(float* __restrict__ xs, int N, int W, int S, const T* __restrict__ mix, const T* __restrict__ out,
+                                                 const float* __restrict__ y, const T* __restrict__ hc_in, const T* __restrict__ nw, int wmode, int sum_all, float eps,
+                                                 const int32_t* __restrict__ rows, T* __restrict__ h) {
+  __shared__ float cm[SMAX * SMAX + 2 * SMAX], red[33];
+  const int r = blockIdx.x, n = rows ? rows[r] : r, S1 = S > 0 ? S : 1;
+  for (int i = threadIdx.x; i < S1 * S1 + 2 * S1; i += blockDim.x) {      // mix [S][S], out [S], in [S]
+    float v = 1.f;
+    if (i >= S1 * S1 + S1) { if (S > 0 && !sum_all) v = ldf(hc_in + (i - S1 * S1 - S1)); }
+    else if (S > 0 && y) v = i < S1 * S1 ? ldf(mix + i) : ldf(out + (i - S1 * S1));
+    cm[i] = v;
+  }
+  __syncthreads();
+  const size_t NW = (size_t)N * W;
+  float u[2][4], ss = 0.f;
+#pragma unroll
+  for (int it = 0; it < 2; it++) {
+    const int c = (it * blockDim.x + threadIdx.x) * 4;
+    u[it][0] = u[it][1] = u[it][2] = u[it][3] = 0.f;
+    if (c >= W) continue;
+    float* xp = xs + (size_t)n * W + c;
+    float x[SMAX][4], yy[4];
+#pragma unroll
+    for (int s = 0; s < SMAX; s++)
+      if (s < S1) ld4(xp + (size_t)s * NW, x[s]);
+    if (y) ld4(y + (size_t)n * W + c, yy);
+#pragma unroll
+    for (int t = 0; t < SMAX; t++) {
+      if (t >= S1) continue;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      if (y) {
+#pragma unroll
+        for (int s = 0; s < SMAX; s++)
+          if (s < S1) {
+            const float m = cm[s * S1 + t];
+#pragma unroll
+            for (int v = 0; v < 4; v++) a[v] += m * x[s][v];
+          }
+        const float ot = cm[S1 * S1 + t];
+#pragma unroll
+        for (int v = 0; v < 4; v++) a[v] += ot * yy[v];
+        if (!rows) st4(xp + (size_t)t * NW, a);
+      } else {
+#pragma unroll
+        for (int v = 0; v < 4; v++) a[v] = x[t][v];
+      }
+      const float ci = cm[S1 * S1 + S1 + t];
+#pragma unroll
+      for (int v = 0; v < 4; v++) u[it][v] += ci * a[v];
+    }
+#pragma unroll
+    for (int v = 0; v < 4; v++) ss += u[it][v] * u[it][v];
+  }
+  float g[2][4];
+#pragma unroll
+  for (int it = 0; it < 2; it++) {
+    const int c = (it * blockDim.x + threadIdx.x) * 4;
+    if (c >= W) continue;
+    if (wmode == NW_SCALAR) g[it][0] = g[it][1] = g[it][2] = g[it][3] = norm_weight(nw, c, wmode);
+    else {
+      ld4(nw + c, g[it]);
+      if (wmode == NW_ONE_PLUS)
+#pragma unroll
+        for (int v = 0; v < 4; v++) g[it][v] = 1.f + g[it][v];
+    }
+  }
+  ss = block_sum(ss, red);
+  const float rinv = 1.f / sqrtf(ss / (float)W + eps);
+#pragma unroll
+  for (int it = 0; it < 2; it++) {
+    const int c = (it * blockDim.x + threadIdx.x) * 4;
+    if (c >= W) continue;
+    float o[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) o[v] = u[it][v] * rinv * g[it][v];
+    st4(h + (size_t)r * W + c, o);
   }
 }
 
@@ -997,6 +1119,42 @@ __device__ __forceinline__ float conv_carry_at(const T* __restrict__ U, int ldu,
   return a + ldf(cw + (size_t)c * taps + taps - 1) * x;
 }
 
+// The same for V = 16 bytes of adjacent channels, every load in flight at once.  carry: the token is the only one of its entry, and its
+// input takes its place among the carried ones.  (A number at a time each channel's loads waited for one another: 4 tokens of 4,096 + 2 x 1,024
+// channels took k_attn_prep 27 us, now 6.9; k_delta_prep 20, now 7.5.)
+constexpr int CONV_MAX_TAPS = 4;
+template <class T, int TAPS>
+__device__ __forceinline__ void conv_vec(const T* __restrict__ U, int ldu, const T* __restrict__ cw, int c, int n, int local, T* st, int ldst, bool carry,
+                                         float (&v)[Vec16<T>::n]) {
+  constexpr int V = Vec16<T>::n;
+  if constexpr (TAPS == 0) ldv(U + (size_t)n * ldu + c, v);
+  else {
+    float wl[V * TAPS], x[TAPS][V];
+    canon_weights<T, TAPS>(cw, c, wl);
+#pragma unroll
+    for (int j = 0; j < TAPS; j++) {
+      const int back = TAPS - 1 - j;
+      ldv(back <= local ? U + (size_t)(n - back) * ldu + c : st + (size_t)(TAPS - 1 - (back - local)) * ldst + c, x[j]);
+    }
+#pragma unroll
+    for (int i = 0; i < V; i++) v[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < TAPS; j++)
+#pragma unroll
+      for (int i = 0; i < V; i++) v[i] += wl[i * TAPS + j] * x[j][i];
+    if (carry)
+#pragma unroll
+      for (int j = 1; j < TAPS; j++) stv(st + (size_t)(j - 1) * ldst + c, x[j]);
+  }
+}
+// whether the three inputs of a layer can be read so
+template <class T>
+__device__ __forceinline__ bool conv_vec_ok(int Cq, int Ck, int Cv, size_t slot_stride, const void* cwq, const void* cwk, const void* cwv, const void* st, int taps) {
+  constexpr int V = Vec16<T>::n;
+  return taps <= CONV_MAX_TAPS && (Cq % V | Ck % V | Cv % V) == 0 && slot_stride % V == 0 &&
+         (((uintptr_t)cwq | (uintptr_t)(Ck ? cwk : cwq) | (uintptr_t)(Cv ? cwv : cwq) | (uintptr_t)st) & 15) == 0;
+}
+
 // after a step: the last taps-1 inputs of every entry become its slot's carried inputs; blockIdx.z picks the
 // projection (q, k, v; a width of 0 means the layer has none of its own)
 template <class T>
@@ -1091,11 +1249,11 @@ struct AttnPrep {
 // head) -> rotary (angles, cos and sin fp32, one table a token) -> query scale -> q to scratch, k / v into the
 // sequence's pages.  One block per token.  Shared memory: Cq + Ck + 34 + H + G + rot floats.
 template <class T>
-__global__ void k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const T* __restrict__ Uk, const T* __restrict__ Uv,
+__global__ void __launch_bounds__(512) k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const T* __restrict__ Uk, const T* __restrict__ Uv,
                             const T* __restrict__ cwq, const T* __restrict__ cwk, const T* __restrict__ cwv, const T* __restrict__ nq,
                             const T* __restrict__ nk, T* __restrict__ cstate, size_t slot_stride, T* __restrict__ qout,
                             T* __restrict__ kpool, T* __restrict__ vpool) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   // a layer that borrows its keys and values projects and carries q only
   const int Cq = a.H * a.dk, Ck = a.own_kv ? a.G * a.dk : 0, Cv = (a.own_kv && a.own_v) ? a.gv * a.dv : 0, ldst = Cq + Ck + Cv;
   const int HG = a.H + (a.own_kv ? a.G : 0);
@@ -1112,20 +1270,53 @@ __global__ void k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const
     return a.carry ? conv_carry_at(U, ldu, cw, c, n, st + off, ldst, a.taps) : conv_at(U, ldu, cw, c, n, local, st + off, ldst, a.taps);
   };
   float sq = 0.f, sk = 0.f;
-  for (int c = threadIdx.x; c < Cq; c += blockDim.x) {
-    const float v = conv(Uq, Cq, cwq, c, 0);
-    qs[c] = v;
-    sq += v * v;
-  }
-  sq = block_sum(sq, red);
-  if (a.own_kv) {
+  const int page = b.bt[(size_t)slot * b.max_pages + p / PAGE], prow = p % PAGE;
+  T* krow = kpool + ((size_t)page * PAGE + prow) * Ck;
+  T* vrow = vpool + ((size_t)page * PAGE + prow) * Cv;
+  const bool vec = conv_vec_ok<T>(Cq, Ck, Cv, slot_stride, cwq, cwk, cwv, cstate, a.taps);      // a function of the model
+  if (vec) {
+    constexpr int V = Vec16<T>::n;
+    auto all = [&](auto tp) {
+      constexpr int TP = decltype(tp)::value;
+      for (int c = threadIdx.x * V; c < ldst; c += blockDim.x * V) {      // channels of q, then k, then v
+        float v[V];
+        if (c < Cq) {
+          conv_vec<T, TP>(Uq, Cq, cwq, c, n, local, st, ldst, a.carry != 0, v);
+#pragma unroll
+          for (int i = 0; i < V; i++) { qs[c + i] = v[i]; sq += v[i] * v[i]; }
+        } else if (c < Cq + Ck) {
+          conv_vec<T, TP>(Uk, Ck, cwk, c - Cq, n, local, st + Cq, ldst, a.carry != 0, v);
+#pragma unroll
+          for (int i = 0; i < V; i++) { qs[c + i] = v[i]; sk += v[i] * v[i]; }      // (ks follows qs)
+        } else {
+          conv_vec<T, TP>(Uv, Cv, cwv, c - Cq - Ck, n, local, st + Cq + Ck, ldst, a.carry != 0, v);
+          stv(vrow + (c - Cq - Ck), v);
+        }
+      }
+    };
+    switch (a.taps) {
+      case 0: all(std::integral_constant<int, 0>{}); break;
+      case 1: all(std::integral_constant<int, 1>{}); break;
+      case 2: all(std::integral_constant<int, 2>{}); break;
+      case 3: all(std::integral_constant<int, 3>{}); break;
+      default: all(std::integral_constant<int, CONV_MAX_TAPS>{}); break;
+    }
+  } else {
+    for (int c = threadIdx.x; c < Cq; c += blockDim.x) {
+      const float v = conv(Uq, Cq, cwq, c, 0);
+      qs[c] = v;
+      sq += v * v;
+    }
     for (int c = threadIdx.x; c < Ck; c += blockDim.x) {
       const float v = conv(Uk, Ck, cwk, c, Cq);
       ks[c] = v;
       sk += v * v;
     }
-    sk = block_sum(sk, red);
   }
+  if (a.norm == 1) {
+    sq = block_sum(sq, red);
+    if (a.own_kv) sk = block_sum(sk, red);
+  } else __syncthreads();
   for (int i = threadIdx.x; i < a.rot / 2; i += blockDim.x) {
     float sn, cs;
     sincosf((float)p * a.inv_freq[i], &sn, &cs);
@@ -1145,8 +1336,6 @@ __global__ void k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const
   __syncthreads();
   const float rq = a.norm == 1 ? 1.f / sqrtf(sq / (float)Cq + a.eps) : 1.f, rk = (a.norm == 1 && a.own_kv) ? 1.f / sqrtf(sk / (float)Ck + a.eps) : 1.f;
   const float qt = a.qt_every > 0 ? 1.f + a.qt_coef * logf((float)((p + 1) / a.qt_every + 1)) : 1.f;
-  const int page = b.bt[(size_t)slot * b.max_pages + p / PAGE], prow = p % PAGE;
-  T* krow = kpool + ((size_t)page * PAGE + prow) * Ck;
   // element d of head hh (q heads first, then k heads) after the norm
   auto val = [&](int hh, int d) -> float {
     const bool isq = hh < a.H;
@@ -1169,6 +1358,33 @@ __global__ void k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const
       else if (d < a.rot) y = y * cst[d - hr] + val(hh, d - hr) * snt[d - hr];
       put(hh, d, y);
     }
+  } else if (vec && (a.dk & 3) == 0) {      // pairs (2i, 2i+1), two of them a thread
+    const int hr = a.dk / 4;
+    for (int e = threadIdx.x; e < HG * hr; e += blockDim.x) {
+      const int hh = e / hr, d = 4 * (e - hh * hr);
+      const bool isq = hh < a.H;
+      const int c = (isq ? hh : hh - a.H) * a.dk + d;
+      float x[4], w[4];
+      ld4((isq ? qs : ks) + c, x);
+      if (a.norm) {
+        ld4((isq ? nq : nk) + (a.norm == 1 ? c : d), w);
+        const float rr = a.norm == 1 ? (isq ? rq : rk) : hinv[hh];
+#pragma unroll
+        for (int i = 0; i < 4; i++) x[i] = x[i] * rr * w[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i += 2)
+        if (d + i + 1 < a.rot) {
+          const float cs = cst[(d + i) / 2], sn = snt[(d + i) / 2], y0 = x[i] * cs - x[i + 1] * sn, y1 = x[i + 1] * cs + x[i] * sn;
+          x[i] = y0; x[i + 1] = y1;
+        }
+      if (isq) {
+        if (a.qt_every > 0)
+#pragma unroll
+          for (int i = 0; i < 4; i++) x[i] *= qt;
+        st4(qout + (size_t)n * Cq + c, x);
+      } else st4(krow + c, x);
+    }
   } else {
     const int halfk = a.dk / 2;
     // pairs (2i, 2i+1) of every head; odd dk leaves its last dim to the tail loop below
@@ -1185,30 +1401,14 @@ __global__ void k_attn_prep(AttnPrep a, Batch b, const T* __restrict__ Uq, const
     if (a.dk & 1)
       for (int hh = threadIdx.x; hh < HG; hh += blockDim.x) put(hh, a.dk - 1, val(hh, a.dk - 1));
   }
-  if (Cv > 0) {
-    T* vr = vpool + ((size_t)page * PAGE + prow) * Cv;
-    for (int c = threadIdx.x; c < Cv; c += blockDim.x)
-      stf(vr + c, conv(Uv, Cv, cwv, c, Cq + Ck));
-  }
+  if (!vec)
+    for (int c = threadIdx.x; c < Cv; c += blockDim.x) stf(vrow + c, conv(Uv, Cv, cwv, c, Cq + Ck));
 }
 
 // The same for heads that do not rotate and whose norm (if any) is their own: one warp a head of q, k or v walks `tok`
 // consecutive tokens.  A lane owns four adjacent channels (head sizes up to 128, multiples of 4), keeps their weights and the
 // last TAPS - 1 inputs in registers and reads every input row once; the head's sum of squares runs over a lane's four channels
 // in ascending order, then pairwise over the lanes.  Nothing is shared between warps.
-__device__ __forceinline__ void ld4(const float* p, float (&o)[4]) { *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void ld4(const bf16* p, float (&o)[4]) {
-  const uint2 v = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
-  o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-}
-__device__ __forceinline__ void st4(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
-__device__ __forceinline__ void st4(bf16* p, const float (&o)[4]) {
-  uint2 v;
-  *reinterpret_cast<__nv_bfloat162*>(&v.x) = __floats2bfloat162_rn(o[0], o[1]);
-  *reinterpret_cast<__nv_bfloat162*>(&v.y) = __floats2bfloat162_rn(o[2], o[3]);
-  *reinterpret_cast<uint2*>(p) = v;
-}
 constexpr int PREP_MAX_TAPS = 4, PREP_WARPS = 4;
 template <class T, int TAPS>
 __global__ void __launch_bounds__(32 * PREP_WARPS) k_attn_prep_heads(AttnPrep a, Batch b, int tok, const T* __restrict__ Uq, const T* __restrict__ Uk,
@@ -1962,24 +2162,48 @@ struct DeltaPrep {
 };
 // conv + silu on q, k, v; unit-norm q (times dk^-1/2) and k per head; beta = sigmoid(b), decay = exp(-exp(A) softplus(a + dt))
 template <class T>
-__global__ void k_delta_prep(DeltaPrep a, Batch b, const T* __restrict__ Uq, const T* __restrict__ Uk, const T* __restrict__ Uv,
+__global__ void __launch_bounds__(512) k_delta_prep(DeltaPrep a, Batch b, const T* __restrict__ Uq, const T* __restrict__ Uk, const T* __restrict__ Uv,
                              const T* __restrict__ cwq, const T* __restrict__ cwk, const T* __restrict__ cwv, const float* __restrict__ pa,
                              const float* __restrict__ pb, const T* __restrict__ A_log, const T* __restrict__ dt_bias,
                              const T* __restrict__ cstate, size_t slot_stride, float* __restrict__ qn, float* __restrict__ kn,
                              float* __restrict__ vv, float* __restrict__ beta, float* __restrict__ decay) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const int Cq = a.G * a.dk, Cv = a.H * a.dv, ldst = 2 * Cq + Cv;
   float* qs = sm;
   float* ks = sm + Cq;
   const int n = blockIdx.x, slot = b.slot[n];
   const int local = n - b.first[n];
   const T* st = cstate + (size_t)slot * slot_stride;
-  for (int c = threadIdx.x; c < Cq; c += blockDim.x) {
-    qs[c] = silu_f(conv_at(Uq, Cq, cwq, c, n, local, st, ldst, a.taps));
-    ks[c] = silu_f(conv_at(Uk, Cq, cwk, c, n, local, st + Cq, ldst, a.taps));
-  }
-  for (int c = threadIdx.x; c < Cv; c += blockDim.x) {
-    vv[(size_t)n * Cv + c] = silu_f(conv_at(Uv, Cv, cwv, c, n, local, st + 2 * Cq, ldst, a.taps));
+  if (conv_vec_ok<T>(Cq, Cq, Cv, slot_stride, cwq, cwk, cwv, cstate, a.taps)) {      // (a function of the model)
+    constexpr int V = Vec16<T>::n;
+    auto all = [&](auto tp) {
+      constexpr int TP = decltype(tp)::value;
+      for (int c = threadIdx.x * V; c < ldst; c += blockDim.x * V) {      // channels of q, then k (ks follows qs), then v
+        float v[V];
+        const int z = c < Cq ? 0 : c < 2 * Cq ? 1 : 2, cc = c - z * Cq;
+        conv_vec<T, TP>(z == 0 ? Uq : z == 1 ? Uk : Uv, z == 2 ? Cv : Cq, z == 0 ? cwq : z == 1 ? cwk : cwv, cc, n, local, const_cast<T*>(st) + z * Cq, ldst, false, v);
+#pragma unroll
+        for (int i = 0; i < V; i++) v[i] = silu_f(v[i]);
+        float* dst = z == 2 ? vv + (size_t)n * Cv + cc : qs + c;
+#pragma unroll
+        for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      }
+    };
+    switch (a.taps) {
+      case 0: all(std::integral_constant<int, 0>{}); break;
+      case 1: all(std::integral_constant<int, 1>{}); break;
+      case 2: all(std::integral_constant<int, 2>{}); break;
+      case 3: all(std::integral_constant<int, 3>{}); break;
+      default: all(std::integral_constant<int, CONV_MAX_TAPS>{}); break;
+    }
+  } else {
+    for (int c = threadIdx.x; c < Cq; c += blockDim.x) {
+      qs[c] = silu_f(conv_at(Uq, Cq, cwq, c, n, local, st, ldst, a.taps));
+      ks[c] = silu_f(conv_at(Uk, Cq, cwk, c, n, local, st + Cq, ldst, a.taps));
+    }
+    for (int c = threadIdx.x; c < Cv; c += blockDim.x) {
+      vv[(size_t)n * Cv + c] = silu_f(conv_at(Uv, Cv, cwv, c, n, local, st + 2 * Cq, ldst, a.taps));
+    }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
