@@ -101,6 +101,7 @@ _PROTOS = {
     "dn_embed": (_i, [_vp, _vp, _i, _vp, _vp]),
     "dn_layer_forward": (_i, [_vp, _i, _vp, _i, _vp, _vp]),
     "dn_window_forward": (_i, [_vp, C.POINTER(C.c_int32), _i, _vp, _i, _vp, _vp]),
+    "dn_chunk_forward": (_i, [_vp, C.POINTER(C.c_int32), _i, _vp, _i, _vp, _vp]),
     "dn_shard_step": (_i, [_vp, C.POINTER(C.c_int32), _i, _vp, _vp, _i, _i, _vp, _vp, _vp, _i, _vp]),
     "dn_shard_step_hop": (_i, [_vp, C.POINTER(C.c_int32), _i, _vp, _vp, _i, _i, _vp, _vp, _i, _vp, _u32, _vp, _vp, _vp, _u32, _vp]),
     "dn_bind_head_slice": (_i, [_vp, _vp, _i, _i]),

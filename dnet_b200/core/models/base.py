@@ -289,11 +289,12 @@ class BaseRingModel(ABC):
         arr = (C.c_int32 * len(layers))(*layers)
         base = cache.offset
         t0 = 0
-        chunks = _decompose(T, self.max_chunk, self.max_prefill_chunk)
+        big = int(self._lib.dn_model_max_prefill_chunk(self._h))
+        chunks = [min(big, T - i) for i in range(0, T, big)] if big else _decompose(T, self.max_chunk)
         for c in chunks:
             if len(chunks) > 1:
                 cache.seek(base + t0, s)
-            _cabi.check(self._lib.dn_window_forward(self._h, arr, len(layers), x[t0:t0 + c].data_ptr(), c, cache._h, s))
+            _cabi.check(self._lib.dn_chunk_forward(self._h, arr, len(layers), x[t0:t0 + c].data_ptr(), c, cache._h, s))
             t0 += c
         if len(chunks) > 1:
             cache.seek(base, s)

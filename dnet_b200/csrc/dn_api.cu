@@ -6,6 +6,7 @@
 #include "dn_kvquant.cuh"
 #include "dn_megakernel.cuh"
 #include "dn_gemm_tc.cuh"
+#include "dn_rows.cuh"
 #include "dn_attn_tc.cuh"
 #include "dn_attn_q.cuh"
 #include "dn_moe.cuh"
@@ -688,7 +689,7 @@ static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// a prompt chunk's attention over the quantised pages (T >= 16)
+// a prompt chunk's attention over the quantised pages
 template <int BITS>
 static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf16* out, int T, dn_kv* kv, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
@@ -706,7 +707,8 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
 
 // quantised KV: after the (unchanged) append kernels wrote the T new K/V rows as bf16 into the staging pool, quantise
 // them into the packed pool and run the two-pass quantised attention (dn_kvquant.cuh; prompt chunks: dn_attn_q.cuh)
-static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, cudaStream_t s) {
+// (prompt: q and attn_out are the prefill path's)
+static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, bool prompt, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   unsigned char* pool = reinterpret_cast<unsigned char*>(m->kv_pool) + (size_t)li * m->kv_layer_bytes;
   // host mirror: longest context any of the T queries sees (a captured graph is replayed at growing contexts)
@@ -719,7 +721,7 @@ static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_
   } else {
     CK(launch(k_kv_quant_append<4>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
   }
-  if (T >= 16 && g_tc_attn) return c.kv_bits == 8 ? attend_q_tc<8>(m, pool, q, attn_out, T, kv, s) : attend_q_tc<4>(m, pool, q, attn_out, T, kv, s);
+  if (prompt && g_tc_attn) return c.kv_bits == 8 ? attend_q_tc<8>(m, pool, q, attn_out, T, kv, s) : attend_q_tc<4>(m, pool, q, attn_out, T, kv, s);
   static size_t smem_set[2] = {0, 0};
   const int bi = c.kv_bits == 8 ? 1 : 0;
   if (smem > smem_set[bi]) {
@@ -786,7 +788,7 @@ static int layer_forward(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, 
   CK(launch_gemv_T(T, q, q.nrows / 2, s));
   if (evs) CK(cudaEventRecord(evs[1], s));
 
-  if (kvq) { const int rc = kvq_append_and_attend(m, li, m->qbuf, m->attn, T, kv, s); if (rc) return rc; }
+  if (kvq) { const int rc = kvq_append_and_attend(m, li, m->qbuf, m->attn, T, kv, false, s); if (rc) return rc; }
   else CK(launch_attn(m, m->qbuf, pool, kv->block_table, kv->st, T, s));
   if (evs) CK(cudaEventRecord(evs[2], s));
 
@@ -860,6 +862,18 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   return DN_OK;
 }
 
+// the same product(s) for a chunk of at most ROWS_MAX tokens: weights straight from memory
+template <int EPI>
+static cudaError_t rows_product(const TcParams& p, const bf16* x, const bf16* w0, const bf16* w1, const bf16* w2, cudaStream_t s) {
+  RowsParams r;
+  memset(&r, 0, sizeof(r));
+  int blocks = 0;
+  for (int i = 0; i < p.nseg; ++i) { r.seg[i] = p.seg[i]; blocks += (p.seg[i].N + 15) / 16; }
+  r.w[0] = w0; r.w[1] = w1; r.w[2] = w2;
+  r.nseg = p.nseg; r.T = p.T; r.K = p.K; r.x = x; r.resid = p.resid; r.ldr = p.ldr;
+  return p.T <= 8 ? launch(k_rows<EPI, 1>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r) : launch(k_rows<EPI, 2>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r);
+}
+
 static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
   auto it = m->abs2local.find(abs_layer);
   if (it == m->abs2local.end()) return fail(DN_ENOENT, "Layer %d not hosted on this model instance", abs_layer);
@@ -876,8 +890,8 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
 #define EV(i) do { if (ev) CK(cudaEventRecord(ev[i], s)); } while (0)
 
   EV(0);
-  k_rmsnorm_rows<<<T, 256, 0, s>>>(x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps);
-  g_launches++;
+  const bool few = T <= ROWS_MAX;
+  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, few, (const bf16*)x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps));
   TcMaps maps;
   for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = L.tm[i < 3 ? i : 0];
   maps.x = m->tm_xn;
@@ -885,15 +899,13 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   p.seg[0] = TcSeg{qd, qkvd, m->pf_qkv, L.w[DN_W_QB], 0};
   p.seg[1] = TcSeg{kd, qkvd, m->pf_qkv + qd, L.w[DN_W_KB], 0};
   p.seg[2] = TcSeg{kd, qkvd, m->pf_qkv + qd + kd, L.w[DN_W_VB], 0};
-  CK(gemm_tc<EPI_STORE>(maps, p, s));
+  CK(few ? rows_product<EPI_STORE>(p, m->pf_xn, L.w[DN_W_Q], L.w[DN_W_K], L.w[DN_W_V], s) : gemm_tc<EPI_STORE>(maps, p, s));
   const bool kvq = c.kv_bits != 0;
-  k_rope_append<<<dim3(c.n_heads + 2 * c.n_kv_heads, T), 128, 0, s>>>(m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
-                                                                        kvq ? m->kvq_stage_bt : kv->block_table, kv->st, m->inv_freq,
-                                                                        c.n_heads, c.n_kv_heads);
-  g_launches++;
+  CK(launch(k_rope_append, dim3(c.n_heads + 2 * c.n_kv_heads, T), dim3(128), 0, s, few, (const bf16*)m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
+            kvq ? (const int32_t*)m->kvq_stage_bt : (const int32_t*)kv->block_table, (const StepState*)kv->st, (const float*)m->inv_freq, c.n_heads, c.n_kv_heads));
   EV(1);
   if (kvq) {
-    const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, s);
+    const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, true, s);
     if (rc) return rc;
   } else if (g_tc_attn && m->tm_kv_ok) {
     AtParams a;
@@ -915,7 +927,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   EV(2);
   p.K = qd; p.nseg = 1; p.seg[0] = TcSeg{H, H, m->pf_h, nullptr, 0}; p.resid = x; p.ldr = H;
   maps.w[0] = L.tm[3]; maps.x = m->tm_attn;
-  CK(gemm_tc<EPI_RESID>(maps, p, s));
+  CK(few ? rows_product<EPI_RESID>(p, m->pf_attn, L.w[DN_W_O], nullptr, nullptr, s) : gemm_tc<EPI_RESID>(maps, p, s));
   EV(3);
   if (c.n_experts > 0) {
     if (!L.experts_bound) return fail(DN_ENOENT, "MoE layer has no experts bound (dn_bind_layer_experts)");
@@ -923,27 +935,26 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     if (rc == DN_OK) { EV(4); EV(5); }
     return rc;
   }
-  k_rmsnorm_rows<<<T, 256, 0, s>>>(m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps);
-  g_launches++;
+  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, few, (const bf16*)m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   p.K = H; p.seg[0] = TcSeg{c.ffn, c.ffn, m->pf_act, nullptr, 0};
   maps.w[0] = L.tm[4]; maps.w[1] = L.tm[5]; maps.x = m->tm_xn;
-  CK(gemm_tc<EPI_SWIGLU>(maps, p, s));
+  CK(few ? rows_product<EPI_SWIGLU>(p, m->pf_xn, L.w[DN_W_GATE], L.w[DN_W_UP], nullptr, s) : gemm_tc<EPI_SWIGLU>(maps, p, s));
   EV(4);
   p.K = c.ffn; p.seg[0] = TcSeg{H, H, x, nullptr, 0}; p.resid = m->pf_h; p.ldr = H;
   maps.w[0] = L.tm[6]; maps.x = m->tm_act;
-  CK(gemm_tc<EPI_RESID>(maps, p, s));
+  CK(few ? rows_product<EPI_RESID>(p, m->pf_act, L.w[DN_W_DOWN], nullptr, nullptr, s) : gemm_tc<EPI_RESID>(maps, p, s));
   EV(5);
 #undef EV
   CK(cudaGetLastError());
   return DN_OK;
 }
 
-static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv) {
+static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16) {
   if (!m || !x || !kv) return fail(DN_EINVAL, "null argument");
   if (kv->m != m) return fail(DN_EINVAL, "kv belongs to a different model");
-  const bool tc_ok = g_tc_prefill && m->pf_ok && T >= 16 && T <= TPF_MAX;
+  const bool tc_ok = g_tc_prefill && m->pf_ok && T >= tc_from && T <= TPF_MAX;
   if (!tc_ok && (!(T == 1 || T == 2 || T == 4) || T > m->tmax))
-    return fail(DN_EINVAL, "T=%d unsupported (1,2,4 up to %d, or 16..%d on the tensor-core prefill path)", T, m->tmax, TPF_MAX);
+    return fail(DN_EINVAL, "T=%d unsupported (1,2,4 up to %d, or %d..%d on the tensor-core prefill path)", T, m->tmax, tc_from, TPF_MAX);
   if (!g_capturing && kv->host_pos + T > kv->max_tokens)
     return fail(DN_ENOSPC, "KV capacity exceeded: offset %d + %d > %d", kv->host_pos, T, kv->max_tokens);
   if (((uintptr_t)x) & 15) return fail(DN_EINVAL, "activation must be 16-byte aligned");
@@ -1000,6 +1011,19 @@ extern "C" int dn_head_timed(dn_model* m, const void* x, int T, dn_stream s, flo
   CK(cudaEventElapsedTime(ms_out, a, b));
   cudaEventDestroy(a);
   cudaEventDestroy(b);
+  return DN_OK;
+}
+
+// dn_window_forward for a chunk of any size up to dn_model_max_prefill_chunk: 2 .. ROWS_MAX tokens read the weights once, too
+extern "C" int dn_chunk_forward(dn_model* m, const int32_t* abs_layers, int n, void* x_inout, int T, dn_kv* kv, dn_stream s) {
+  int rc = check_fwd(m, x_inout, T, kv, 2);
+  if (rc) return rc;
+  if (n > 0 && !abs_layers) return fail(DN_EINVAL, "null layer list");
+  const bool tc = T > 1 && g_tc_prefill && m->pf_ok;
+  for (int i = 0; i < n; ++i) {
+    rc = tc ? layer_forward_tc(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s) : layer_forward(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s);
+    if (rc) return rc;
+  }
   return DN_OK;
 }
 

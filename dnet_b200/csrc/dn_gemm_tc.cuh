@@ -713,6 +713,8 @@ static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPla
 __global__ void __launch_bounds__(256) k_rmsnorm_rows(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
                                                       int K, float eps) {
   __shared__ float scratch[8];
+  pdl_launch_dependents();
+  pdl_wait();
   const bf16* xr = x + (size_t)blockIdx.x * K;
   bf16* o = out + (size_t)blockIdx.x * K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -747,6 +749,8 @@ __global__ void __launch_bounds__(256) k_rmsnorm_rows(const bf16* __restrict__ x
 __global__ void __launch_bounds__(128) k_rope_append(const bf16* __restrict__ qkv, bf16* __restrict__ q_out, bf16* __restrict__ kv_pool,
                                                      const int32_t* __restrict__ block_table, const StepState* __restrict__ st,
                                                      const float* __restrict__ inv_freq, int n_heads, int n_kv) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.y, slot = blockIdx.x;            // slot: q heads, then k heads, then v heads
   const int pos = st->pos + t;
   const int ld = (n_heads + 2 * n_kv) * HD;

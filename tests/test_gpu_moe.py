@@ -131,3 +131,9 @@ def test_prompt_experts_in_one_grouped_launch(moe, T):
         assert frac < 0.03 and worst <= 2 * 2.0 ** -8, f"T {T}: {frac:.4f} mismatching, worst {worst:.2e}"
     finally:
         rt.unload_model_core()
+
+
+@pytest.mark.parametrize("T", [2, 3, 9, 15])
+def test_experts_of_a_few_tokens_in_one_grouped_launch(moe, T):
+    """the same for chunks of fewer tokens: most experts have no row or one"""
+    test_prompt_experts_in_one_grouped_launch(moe, T)

@@ -50,10 +50,10 @@ def _call(m, kv, x, context):
     return y.float().cpu()
 
 
-def _agree(a, b):
+def _agree(a, b, differing=0.25):
     assert torch.isfinite(a).all()
     assert rel_inf(a, b) <= 3 * 2.0 ** -8, rel_inf(a, b)
-    assert float((a != b).float().mean()) < 0.25
+    assert float((a != b).float().mean()) < differing
 
 
 @pytest.mark.parametrize("group", [1, 2, 4, 5, 7, 8])
@@ -119,3 +119,28 @@ def test_prefill_attention_over_quantised_pages(cuda_lib, bits, group, context, 
         kv.free()
         m.destroy()
     _agree(out[1], out[0])
+
+
+@pytest.mark.parametrize("bits", [0, 8, 4])
+@pytest.mark.parametrize("T", [2, 3, 7, 8, 9, 15, 16, 17])
+@pytest.mark.parametrize("hidden,ffn,kv_heads,group,context", [(256, 512, 1, 2, 0), (768, 27648, 2, 5, 63), (4096, 1280, 2, 4, 700)])
+def test_chunks_of_a_few_tokens(cuda_lib, hidden, ffn, kv_heads, group, context, T, bits):
+    """A chunk of 2 .. 16 tokens in one pass over the weights (k_rows: one or two groups of eight tokens, warps with few columns and with
+    many) against the same tokens one by one (the row kernels) behind the same pages; 17 tokens are the first that the GEMM takes.
+    Over quantised pages a score near a rounding edge flips by 2^-8 of itself, and its weight with it: that moves every result of its
+    token by up to a rounding, half of them over an edge; two or three tokens have no others to average with, so below a half."""
+    x = torch.randn(context + T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    m = _model(kv_heads, group, seed=hidden, hidden=hidden, ffn=ffn, kv_bits=bits)
+    kv = m.make_cache(max_tokens=768)
+    try:
+        one_pass = _call(m, kv, x, context)
+        rows = []
+        for t in range(context, context + T):
+            kv.seek(t)
+            rows.append(m.apply_single_layer(0, x[t:t + 1].clone(), kv))
+        torch.cuda.synchronize()
+        assert cuda_lib.dn_step_error(m._h, 0) == 0
+    finally:
+        kv.free()
+        m.destroy()
+    _agree(one_pass, torch.cat(rows).float().cpu(), 0.5 if bits else 0.25)
