@@ -901,7 +901,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   p.seg[2] = TcSeg{kd, qkvd, m->pf_qkv + qd + kd, L.w[DN_W_VB], 0};
   CK(few ? rows_product<EPI_STORE>(p, m->pf_xn, L.w[DN_W_Q], L.w[DN_W_K], L.w[DN_W_V], s) : gemm_tc<EPI_STORE>(maps, p, s));
   const bool kvq = c.kv_bits != 0;
-  CK(launch(k_rope_append, dim3(c.n_heads + 2 * c.n_kv_heads, T), dim3(128), 0, s, few, (const bf16*)m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
+  CK(launch(k_rope_append, dim3((c.n_heads + 2 * c.n_kv_heads + ROPE_SLOTS - 1) / ROPE_SLOTS, T), dim3(128), 0, s, few, (const bf16*)m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
             kvq ? (const int32_t*)m->kvq_stage_bt : (const int32_t*)kv->block_table, (const StepState*)kv->st, (const float*)m->inv_freq, c.n_heads, c.n_kv_heads));
   EV(1);
   if (kvq) {
