@@ -698,7 +698,7 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
   a.a.n_heads = c.n_heads; a.a.n_kv = c.n_kv_heads; a.a.T = T; a.a.err = m->mk_sync + 2;
   a.pool = pool;
   const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
-  const dim3 grid(c.n_kv_heads, blocks, attn_prefill_split(c.n_kv_heads * blocks, kv->host_pos + T, g_sms));
+  const dim3 grid(c.n_kv_heads, blocks, attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms));
 #define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, a)); break;
   switch (m->G) { PFQ(1) PFQ(2) PFQ(4) PFQ(5) PFQ(7) PFQ(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFQ
@@ -871,7 +871,31 @@ static cudaError_t rows_product(const TcParams& p, const bf16* x, const bf16* w0
   for (int i = 0; i < p.nseg; ++i) { r.seg[i] = p.seg[i]; blocks += (p.seg[i].N + 15) / 16; }
   r.w[0] = w0; r.w[1] = w1; r.w[2] = w2;
   r.nseg = p.nseg; r.T = p.T; r.K = p.K; r.x = x; r.resid = p.resid; r.ldr = p.ldr;
-  return p.T <= 8 ? launch(k_rows<EPI, 1>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r) : launch(k_rows<EPI, 2>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r);
+#define ROWS(NT, U) launch(k_rows<EPI, NT, U>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r)
+  if constexpr (EPI != EPI_SWIGLU)
+    if (rows_mma_deep(blocks, g_sms)) return p.T <= 8 ? ROWS(1, 8) : ROWS(2, 8);
+  return p.T <= 8 ? ROWS(1, 4) : ROWS(2, 4);
+#undef ROWS
+}
+
+// one token's experts: all choices' gate / up products in one launch, all down products in another (a launch a choice, on the row kernels
+// of moe_ffn: 2 x 51 + 2 x 31 us at Mixtral-8x7B sizes, 0.70 and 0.58 of the copy bandwidth; so 70 + 38)
+static int moe_ffn_one(dn_model* m, const LayerW& L, const bf16* h, bf16* out, cudaStream_t s) {
+  const dn_model_cfg& c = m->cfg;
+  const int H = c.hidden, E = c.n_experts, k = c.top_k;
+  CK(launch(k_rmsnorm_rows, dim3(1), dim3(256), 0, s, true, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
+  CK(launch(k_moe_route, dim3(1), dim3(256), 0, s, true, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
+  RowsParams r;
+  memset(&r, 0, sizeof(r));
+  r.nseg = 1; r.T = 1; r.table = (const bf16* const*)L.etable; r.sel = m->moe_psel;
+  r.seg[0] = TcSeg{c.ffn, c.ffn, m->moe_act, nullptr, 0}; r.K = H; r.x = m->pf_xn; r.ldx = 0; r.m0 = 0; r.m1 = E;
+  CK(launch(k_rows<EPI_SWIGLU, 1, 4, true>, dim3(k * ((c.ffn + 15) / 16)), dim3(RM_THREADS), 0, s, true, r));
+  r.seg[0] = TcSeg{H, H, m->moe_out, nullptr, 0}; r.K = c.ffn; r.x = m->moe_act; r.ldx = c.ffn; r.m0 = 2 * E;
+  const int blocks = k * ((H + 15) / 16);
+  if (rows_mma_deep(blocks, g_sms)) CK(launch(k_rows<EPI_STORE, 1, 8, true>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r));
+  else CK(launch(k_rows<EPI_STORE, 1, 4, true>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r));
+  CK(launch(k_moe_join, dim3(1), dim3(256), 0, s, true, (const bf16*)m->moe_out, (const int32_t*)nullptr, (const float*)m->moe_pscore, k, H, h, out));
+  return DN_OK;
 }
 
 static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
@@ -913,7 +937,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.T = T; a.err = err;
     const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
     // (how the keys are shared out only decides the order of the sums; the kernel reads the position from the step state)
-    const int Z = attn_prefill_split(c.n_kv_heads * blocks, kv->host_pos + T, g_sms);
+    const int Z = attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms);
 #define PFT(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_tc<Gv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, m->tm_kv[li], a)); break;
     switch (m->G) { PFT(1) PFT(2) PFT(4) PFT(5) PFT(7) PFT(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT
@@ -931,7 +955,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   EV(3);
   if (c.n_experts > 0) {
     if (!L.experts_bound) return fail(DN_ENOENT, "MoE layer has no experts bound (dn_bind_layer_experts)");
-    const int rc = m->moe_tc_ok && L.emaps_ok ? moe_ffn_tc(m, L, m->pf_h, x, T, s) : moe_ffn(m, L, m->pf_h, x, T, s);
+    const int rc = m->moe_tc_ok && L.emaps_ok ? (T == 1 ? moe_ffn_one(m, L, m->pf_h, x, s) : moe_ffn_tc(m, L, m->pf_h, x, T, s)) : moe_ffn(m, L, m->pf_h, x, T, s);
     if (rc == DN_OK) { EV(4); EV(5); }
     return rc;
   }
@@ -949,6 +973,17 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   return DN_OK;
 }
 
+// The kernels of a chunk.  The prompt kernels take every chunk of two tokens and more, and single tokens of layers with experts or with
+// quantised pages (behind 8,000 8-bit tokens 218 us against 1,650 of the row kernels' attention, a block a head); a single token of a
+// dense layer over bf16 pages is as fast on the row kernels, which form the norm and the rotation in their products' launches
+// (Llama-8B sizes behind 256: 107 us either way).
+static bool use_prompt_kernels(const dn_model* m, int T) {
+  return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.kv_bits != 0 || (m->cfg.n_experts > 0 && m->moe_tc_ok));
+}
+static int one_layer(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
+  return use_prompt_kernels(m, T) ? layer_forward_tc(m, abs_layer, x, T, kv, s, ev) : layer_forward(m, abs_layer, x, T, kv, s, ev);
+}
+
 static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16) {
   if (!m || !x || !kv) return fail(DN_EINVAL, "null argument");
   if (kv->m != m) return fail(DN_EINVAL, "kv belongs to a different model");
@@ -964,8 +999,7 @@ static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16) {
 extern "C" int dn_layer_forward(dn_model* m, int abs_layer, void* x_inout, int T, dn_kv* kv, dn_stream s) {
   int rc = check_fwd(m, x_inout, T, kv);
   if (rc) return rc;
-  if (T >= 16) return layer_forward_tc(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s);
-  return layer_forward(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s);
+  return one_layer(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s);
 }
 
 // Per-kernel device times of one layer (CUDA events between the five launches, on the
@@ -981,8 +1015,7 @@ extern "C" int dn_layer_forward_timed(dn_model* m, int abs_layer, void* x_inout,
   for (int i = 0; i < 6; ++i) CK(cudaEventCreate(&ev[i]));
   const int pdl = g_pdl;
   g_pdl = 0;
-  rc = T >= 16 ? layer_forward_tc(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s, ev)
-               : layer_forward(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s, ev);
+  rc = one_layer(m, abs_layer, (bf16*)x_inout, T, kv, (cudaStream_t)s, ev);
   g_pdl = pdl;
   if (rc == DN_OK) {
     cudaError_t e = cudaStreamSynchronize((cudaStream_t)s);
@@ -1019,9 +1052,8 @@ extern "C" int dn_chunk_forward(dn_model* m, const int32_t* abs_layers, int n, v
   int rc = check_fwd(m, x_inout, T, kv, 2);
   if (rc) return rc;
   if (n > 0 && !abs_layers) return fail(DN_EINVAL, "null layer list");
-  const bool tc = T > 1 && g_tc_prefill && m->pf_ok;
   for (int i = 0; i < n; ++i) {
-    rc = tc ? layer_forward_tc(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s) : layer_forward(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s);
+    rc = one_layer(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s);
     if (rc) return rc;
   }
   return DN_OK;
@@ -1032,8 +1064,7 @@ extern "C" int dn_window_forward(dn_model* m, const int32_t* abs_layers, int n, 
   if (rc) return rc;
   if (n > 0 && !abs_layers) return fail(DN_EINVAL, "null layer list");
   for (int i = 0; i < n; ++i) {
-    rc = T >= 16 ? layer_forward_tc(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s)
-                 : layer_forward(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s);
+    rc = one_layer(m, abs_layers[i], (bf16*)x_inout, T, kv, (cudaStream_t)s);
     if (rc) return rc;
   }
   return DN_OK;

@@ -442,6 +442,8 @@ __global__ void __launch_bounds__(32) k_moe_select(const float* __restrict__ log
 __global__ void __launch_bounds__(256) k_moe_route(const bf16* __restrict__ xn, const bf16* __restrict__ w, int K, int E, int k,
                                                    int32_t* __restrict__ sel, float* __restrict__ score) {
   __shared__ float lg[MOE_MAX_E];
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bf16* x = xn + (size_t)t * K;
   for (int e = warp; e < E; e += 8) {
@@ -457,14 +459,17 @@ __global__ void __launch_bounds__(256) k_moe_route(const bf16* __restrict__ xn, 
   __syncthreads();
   if (threadIdx.x == 0) moe_select(lg, E, k, sel + (size_t)t * k, score + (size_t)t * k);
 }
-// a prompt's tokens: out = T(h + acc), acc = T(acc + T(y_j score_j)) over the token's pairs in selection order (OpDownMoe's rounding)
+// a prompt's tokens: out = T(h + acc), acc = T(acc + T(y_j score_j)) over the token's pairs in selection order (OpDownMoe's rounding);
+// pos: the row of each pair (null: pairs lie in order)
 __global__ void __launch_bounds__(256) k_moe_join(const bf16* __restrict__ y, const int32_t* __restrict__ pos, const float* __restrict__ score,
                                                   int k, int H, const bf16* __restrict__ h, bf16* __restrict__ out) {
   const int t = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   for (int i = threadIdx.x * 8; i < H; i += 256 * 8) {
     float acc[8];
     for (int j = 0; j < k; ++j) {
-      const uint4 v = *reinterpret_cast<const uint4*>(y + (size_t)pos[t * k + j] * H + i);
+      const uint4 v = *reinterpret_cast<const uint4*>(y + (size_t)(pos ? pos[t * k + j] : t * k + j) * H + i);
       const float f[8] = {bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y), bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w)};
       const float sc = score[t * k + j];
 #pragma unroll

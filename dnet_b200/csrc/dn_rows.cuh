@@ -17,26 +17,41 @@ struct RowsParams {
   int nseg, T, K;
   const bf16* x;           // [T][K]
   const bf16* resid; int ldr;
+  // one token's experts (MOE): product i is that of expert sel[i] with the matrices table[m0 + sel], EPI_SWIGLU also table[m1 + sel]; its
+  // result goes to seg[0].Y + i * seg[0].ldy, its row is x + i * ldx
+  const bf16* const* table; const int32_t* sel; int m0, m1, ldx;
 };
 
-template <int EPI, int NT>
-__global__ void __launch_bounds__(RM_THREADS, EPI == EPI_SWIGLU ? 2 : 3) k_rows(const __grid_constant__ RowsParams p) {
+template <int EPI, int NT, int U, bool MOE = false>
+__global__ void __launch_bounds__(RM_THREADS, EPI == EPI_SWIGLU || U == 8 ? 2 : 3) k_rows(const __grid_constant__ RowsParams p) {
   constexpr int TILES = EPI == EPI_SWIGLU ? 2 : 1;
   __shared__ float red[RM_WARPS * TILES * NT * 128];
   pdl_launch_dependents();
   int blk = blockIdx.x, si = 0;
-  if (EPI == EPI_STORE)
+  const bf16* x = p.x;
+  if (MOE) {
+    const int nb = (p.seg[0].N + 15) / 16;
+    si = blk / nb;
+    blk -= si * nb;
+    x += (size_t)si * p.ldx;
+  } else if (EPI == EPI_STORE)
     for (; si + 1 < p.nseg; ++si) {
       const int nb = (p.seg[si].N + 15) / 16;
       if (blk < nb) break;
       blk -= nb;
     }
-  const TcSeg& sg = p.seg[si];
+  const TcSeg& sg = p.seg[MOE ? 0 : si];
   const bf16* w[TILES];
   int r0[TILES];
 #pragma unroll
-  for (int i = 0; i < TILES; ++i) { w[i] = p.w[si + i]; r0[i] = blk * 16; }
-  rows_mma_block<TILES, NT>(w, r0, sg.N, p.x, p.T, p.K, red, [] { pdl_wait(); });
+  for (int i = 0; i < TILES; ++i) { w[i] = MOE ? nullptr : p.w[si + i]; r0[i] = blk * 16; }
+  if (MOE) {      // which matrices is known only behind the wait
+    pdl_wait();
+    const int e = p.sel[si];
+#pragma unroll
+    for (int i = 0; i < TILES; ++i) w[i] = p.table[(i ? p.m1 : p.m0) + e];
+    rows_mma_block<TILES, NT, U>(w, r0, sg.N, x, p.T, p.K, red);
+  } else rows_mma_block<TILES, NT, U>(w, r0, sg.N, x, p.T, p.K, red, [] { pdl_wait(); });
   const int q = threadIdx.x >> 7, at = threadIdx.x & 127, row = at & 15, t = 8 * q + (at >> 4), n = blk * 16 + row;      // neighbouring threads: neighbouring features
   if (q >= NT || t >= p.T || n >= sg.N) return;
   const int slot = row * 8 + (at >> 4);
@@ -49,7 +64,7 @@ __global__ void __launch_bounds__(RM_THREADS, EPI == EPI_SWIGLU ? 2 : 3) k_rows(
     const float sg1 = bf16r(1.0f / (1.0f + expf(-g)));
     y = __fmul_rn(bf16r(__fmul_rn(g, sg1)), u);
   }
-  sg.Y[(size_t)t * sg.ldy + n] = __float2bfloat16_rn(y);
+  sg.Y[(size_t)(MOE ? si : t) * sg.ldy + n] = __float2bfloat16_rn(y);
 }
 
 }  // namespace dn

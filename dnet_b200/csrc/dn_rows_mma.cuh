@@ -21,6 +21,10 @@
 namespace dn {
 
 constexpr int RM_WARPS = 8, RM_THREADS = RM_WARPS * 32;
+// Blocks of one tile: eight blocks of 32 columns in flight a warp and two thread blocks an SM, or four and three.  Two are the faster ones where
+// all thread blocks run at once or in many waves (4,096 x 4,096, 4 tokens: 8.4 us against 8.7; x 14,336: 22.3 / 22.6; 14,336 x 4,096: 20.9 /
+// 22.6), three where only they hold all (6,144 x 4,096: 12.4 / 10.9; 5,120 x 27,648: 58.6 / 46.2).  16 tokens: 4,096 x 14,336 26.6 / 34.9.
+static inline bool rows_mma_deep(int blocks, int sms) { return blocks <= 2 * sms || blocks > 3 * sms; }
 // columns a lane loads at once: 16-byte rows of both operands
 static inline bool rows_mma_ok(int K, const void* X, const void* W, const void* W2) {
   return K % 32 == 0 && ((((uintptr_t)X | (uintptr_t)W | (uintptr_t)(W2 ? W2 : W)) & 15) == 0);
@@ -44,12 +48,11 @@ __device__ __forceinline__ void rm_mma32(float (&d)[4], const uint4& a, const ui
 }
 // One warp's share of TILES tiles of 16 rows for NT groups of 8 tokens.  w: the matrices' rows 0 (row pitch K), r0: a tile's first row,
 // rows: how many the matrix has (rows past it are read again and dropped by the caller); X [N][K]; columns 32 kb0 .. 32 kb1.
-// ready(): called once the first weights are on their way and before the first row is read.  acc: rows g, g + 8 x tokens 2 t, 2 t + 1
+// U: blocks of 32 columns with all their loads in flight.  ready(): called once the first weights are on their way and before the first row is read.  acc: rows g, g + 8 x tokens 2 t, 2 t + 1
 struct RmNow { __device__ __forceinline__ void operator()() const {} };
-template <int TILES, int NT, class Ready>
+template <int TILES, int NT, int U, class Ready>
 __device__ __forceinline__ void rows_mma(const __nv_bfloat16* const (&w)[TILES], const int (&r0)[TILES], int rows, const __nv_bfloat16* X, int N, int K, int kb0,
                                          int kb1, float (&acc)[TILES][NT][4], Ready ready) {
-  constexpr int U = TILES * NT == 1 ? 8 : 4;      // blocks of 32 columns with all their loads in flight
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const __nv_bfloat16 *wa[TILES], *wb[TILES], *x[NT];
   bool live[NT];
@@ -105,12 +108,12 @@ __device__ __forceinline__ void rows_mma(const __nv_bfloat16* const (&w)[TILES],
   if (kb < kb1) go(std::integral_constant<int, 1>{}, kb, false);
 }
 // A block's tiles: every warp its share of the columns, then the sums of the eight.  red: [RM_WARPS][TILES][NT][16 rows][8 tokens] floats
-template <int TILES, int NT = 1, class Ready = RmNow>
+template <int TILES, int NT = 1, int U = 4, class Ready = RmNow>
 __device__ __forceinline__ void rows_mma_block(const __nv_bfloat16* const (&w)[TILES], const int (&r0)[TILES], int rows, const __nv_bfloat16* X, int N, int K,
                                                float* red, Ready ready = Ready()) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = K / 32;
   float acc[TILES][NT][4];
-  rows_mma<TILES, NT>(w, r0, rows, X, N, K, nb * warp / RM_WARPS, nb * (warp + 1) / RM_WARPS, acc, ready);
+  rows_mma<TILES, NT, U>(w, r0, rows, X, N, K, nb * warp / RM_WARPS, nb * (warp + 1) / RM_WARPS, acc, ready);
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int i = 0; i < TILES; ++i)

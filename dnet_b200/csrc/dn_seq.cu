@@ -805,11 +805,12 @@ static cudaError_t linear(dn_seq_model* m, cudaStream_t s, const T* X, const voi
   if constexpr (std::is_same<T, bf16>::value)
     if (N <= 8 && (O >= ROWS_SPLIT || act_two(act)) && dn::rows_mma_ok(K, X, W, act_two(act) ? W2 : nullptr)) {
       const bool own = act == ACT_JOIN || act == ACT_GELU_TAB;      // an epilogue with operands of its own
-#define LM(MODE, EPv) launch(k_linear_mma<MODE, EPv>, dim3((O + (MODE == 1 ? 31 : 15)) / (MODE == 1 ? 32 : 16)), dim3(dn::RM_THREADS), 0, s, (const bf16*)X, (const bf16*)W, \
+#define LM(MODE, U, EPv) launch(k_linear_mma<MODE, U, EPv>, dim3((O + (MODE == 1 ? 31 : 15)) / (MODE == 1 ? 32 : 16)), dim3(dn::RM_THREADS), 0, s, (const bf16*)X, (const bf16*)W, \
                              (const bf16*)W2, Y, out32 ? 1 : 0, N, O, K, act, alim, (const bf16*)bias, epi)
-      if (act_two(act)) return LM(2, false);
-      if (O >= LM_WIDE) return own ? LM(1, true) : LM(1, false);
-      return own ? LM(0, true) : LM(0, false);
+      if (act_two(act)) return LM(2, 4, false);
+      if (O >= LM_WIDE) return own ? LM(1, 4, true) : LM(1, 4, false);
+      if (dn::rows_mma_deep((O + 15) / 16, g_sms)) return own ? LM(0, 8, true) : LM(0, 8, false);
+      return own ? LM(0, 4, true) : LM(0, 4, false);
 #undef LM
     }
   if (N <= 8 && O < ROWS_SPLIT && !act_two(act)) {      // few features: the warps of a block split the reduction
@@ -1317,8 +1318,8 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         if (mma) {
           const int per = rows >= LM_WIDE ? 32 : 16;
           for (int i = 0; i < sg.n; i++) blocks += (sg.O[i] + per - 1) / per;
-          return per == 32 ? launch(k_linear_mma_multi<1>, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W)
-                           : launch(k_linear_mma_multi<0>, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W);
+          auto kern = per == 32 ? k_linear_mma_multi<1, 4> : dn::rows_mma_deep(blocks, g_sms) ? k_linear_mma_multi<0, 8> : k_linear_mma_multi<0, 4>;
+          return launch(kern, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W);
         }
       }
       const bool pair = rows >= ROWS_PAIR;

@@ -1045,7 +1045,7 @@ __global__ void __launch_bounds__(256) k_linear_rows_multi(const T* __restrict__
 // 1: 32 (each token row is read for twice the weights; from LM_WIDE features on, which fill three blocks an SM either way); 2: 16 of two matrices.
 // The order of a feature's sums is the same in all of them.
 constexpr int LM_WIDE = 7104;
-template <int MODE, bool EP>
+template <int MODE, int U, bool EP>
 __device__ __forceinline__ void linear_mma_block(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt, const __nv_bfloat16* __restrict__ W2, void* __restrict__ Y,
                                                  bool out32, int N, int O, int K, int act, int o0, float alim, const __nv_bfloat16* __restrict__ bias,
                                                  const LinEpi<__nv_bfloat16>& ep) {
@@ -1059,7 +1059,7 @@ __device__ __forceinline__ void linear_mma_block(const __nv_bfloat16* __restrict
   int r0[TILES];
 #pragma unroll
   for (int i = 0; i < TILES; i++) { w[i] = MODE == 2 && i == 1 ? W2 : Wt; r0[i] = o0 + (MODE == 1 ? 16 * i : 0); }
-  dn::rows_mma_block<TILES>(w, r0, O, X, N, K, red);
+  dn::rows_mma_block<TILES, 1, U>(w, r0, O, X, N, K, red);
   if (!live) return;
   const float v = dn::rows_mma_sum<TILES>(red, MODE == 1 ? tile : 0, at) + (bias ? ldf(bias + o) : 0.f);
   if (EP) { ea.finish(ep, act, v, n, o, O, Y, out32, alim); return; }
@@ -1067,15 +1067,15 @@ __device__ __forceinline__ void linear_mma_block(const __nv_bfloat16* __restrict
   if (out32) ((float*)Y)[(size_t)n * O + o] = y;
   else stf((__nv_bfloat16*)Y + (size_t)n * O + o, y);
 }
-template <int MODE, bool EP>
-__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 ? 3 : 2) k_linear_mma(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt,
+template <int MODE, int U, bool EP>
+__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 && U == 4 ? 3 : 2) k_linear_mma(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt,
                                                                                 const __nv_bfloat16* __restrict__ W2, void* __restrict__ Y, int out32, int N, int O, int K,
                                                                                 int act, float alim, const __nv_bfloat16* __restrict__ bias,
                                                                                 const __grid_constant__ LinEpi<__nv_bfloat16> ep) {
-  linear_mma_block<MODE, EP>(X, Wt, W2, Y, out32 != 0, N, O, K, act, blockIdx.x * (MODE == 1 ? 32 : 16), alim, bias, ep);
+  linear_mma_block<MODE, U, EP>(X, Wt, W2, Y, out32 != 0, N, O, K, act, blockIdx.x * (MODE == 1 ? 32 : 16), alim, bias, ep);
 }
-template <int MODE>
-__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 ? 3 : 2) k_linear_mma_multi(const __nv_bfloat16* __restrict__ X, LinSegs sg, int N, int K) {
+template <int MODE, int U>
+__global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 && U == 4 ? 3 : 2) k_linear_mma_multi(const __nv_bfloat16* __restrict__ X, LinSegs sg, int N, int K) {
   constexpr int PER = MODE == 1 ? 32 : 16;
   int blk = blockIdx.x, i = 0;
   for (; i < sg.n; i++) {
@@ -1084,7 +1084,7 @@ __global__ void __launch_bounds__(dn::RM_THREADS, MODE == 0 ? 3 : 2) k_linear_mm
     blk -= nb;
   }
   if (i >= sg.n) return;
-  linear_mma_block<MODE, false>(sg.X[i] ? (const __nv_bfloat16*)sg.X[i] : X, (const __nv_bfloat16*)sg.W[i], nullptr, sg.Y[i], sg.out32[i] != 0, N, sg.O[i],
+  linear_mma_block<MODE, U, false>(sg.X[i] ? (const __nv_bfloat16*)sg.X[i] : X, (const __nv_bfloat16*)sg.W[i], nullptr, sg.Y[i], sg.out32[i] != 0, N, sg.O[i],
                                 sg.K[i] > 0 ? sg.K[i] : K, sg.act[i], blk * PER, 0.f, nullptr, LinEpi<__nv_bfloat16>{});
 }
 
