@@ -89,6 +89,7 @@ _PROTOS = {
     "dn_bind_api": (_i, [_vp, _vp, _vp, _vp]),
     "dn_model_max_chunk": (_i, [_vp]),
     "dn_model_max_prefill_chunk": (_i, [_vp]),
+    "dn_model_max_chunk_forward": (_i, [_vp]),
     "dn_kv_create": (_i, [_vp, _i, C.POINTER(_vp)]),
     "dn_kv_free": (_i, [_vp]),
     "dn_kv_reset": (_i, [_vp, _vp]),

@@ -289,7 +289,7 @@ class BaseRingModel(ABC):
         arr = (C.c_int32 * len(layers))(*layers)
         base = cache.offset
         t0 = 0
-        big = int(self._lib.dn_model_max_prefill_chunk(self._h))
+        big = int(self._lib.dn_model_max_chunk_forward(self._h))
         chunks = [min(big, T - i) for i in range(0, T, big)] if big else _decompose(T, self.max_chunk)
         for c in chunks:
             if len(chunks) > 1:

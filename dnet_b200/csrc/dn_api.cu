@@ -116,7 +116,12 @@ struct LayerW {
   bool experts_bound = false;
 };
 
-constexpr int TPF_MAX = 512;   // tokens per tensor-core prefill chunk (weights are streamed once per chunk)
+constexpr int TPF_MAX = 512;   // tokens per chunk of dn_layer_forward and dn_window_forward on the tensor-core path (weights are streamed once per chunk)
+// ... and of dn_chunk_forward.  At 512 tokens a product's tiles fill the 74 CTA pairs badly (gate / up of Llama-8B sizes: 224 tiles, a fourth round
+// for two of them; 105 us against 72 at the measured rate); 2,048 tokens are 896 tiles.  A prompt of
+// 2,048 tokens through two layers and the head: 2,667 us in chunks of 512, 2,033 in one; 777 tokens over 8-bit pages 719 / 644.
+constexpr int CHUNK_MAX = 2048;
+static_assert(CHUNK_MAX >= TPF_MAX && CHUNK_MAX <= (KVQ_STAGE_PAGES - 1) * PAGE, "a chunk's rows lie in the staging pages");
 static int g_tc_prefill = 1;
 static int g_tc_attn = 1;      // prefill attention on tcgen05, else the CUDA-core kernel
 
@@ -160,7 +165,7 @@ struct dn_model {
   // sparse MoE scratch: router logits [E], selected experts [k] + scores [k], running weighted sum [H]
   float* moe_logits = nullptr; int32_t* moe_sel = nullptr; float* moe_score = nullptr; float* moe_y = nullptr;
   const bf16** moe_tables = nullptr;    // [local layers][3][E]
-  // ... of a prompt chunk: P = TPF_MAX top_k pairs; the tokens' rows sorted by expert, the experts' activations and outputs
+  // ... of a prompt chunk: P = CHUNK_MAX top_k pairs; the tokens' rows sorted by expert, the experts' activations and outputs
   bf16 *moe_xg = nullptr, *moe_act = nullptr, *moe_out = nullptr;
   int32_t *moe_psel = nullptr, *moe_plan = nullptr;      // choices [P]; rows of pairs [P], tokens of rows [P], tile table [3][max tiles] + 1
   float* moe_pscore = nullptr;
@@ -179,7 +184,7 @@ struct dn_model {
   std::vector<MkLayer> mk_host;
   MkLayer* mk_dev = nullptr;
   bf16 *xa = nullptr, *xb = nullptr;
-  // tensor-core prefill scratch ([TPF_MAX][...]) and the TMA descriptors of the activation buffers
+  // tensor-core prefill scratch ([CHUNK_MAX][...]) and the TMA descriptors of the activation buffers
   bf16 *pf_xn = nullptr, *pf_qkv = nullptr, *pf_q = nullptr, *pf_attn = nullptr, *pf_h = nullptr, *pf_act = nullptr;
   CUtensorMap tm_xn, tm_attn, tm_act;
   std::vector<CUtensorMap> tm_kv;                // per local layer: KV pool as [pages*2*n_kv*64 rows][128] bf16, box 64 x 64
@@ -437,21 +442,21 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
   CK(util_fill0(m->null_bt, 64));
   {
     const int qkvd = (cfg->n_heads + 2 * cfg->n_kv_heads) * HD;
-    CK(cudaMalloc(&m->pf_xn, (size_t)TPF_MAX * H * 2));
-    CK(cudaMalloc(&m->pf_qkv, (size_t)TPF_MAX * qkvd * 2));
-    CK(cudaMalloc(&m->pf_q, (size_t)TPF_MAX * qd * 2));
-    CK(cudaMalloc(&m->pf_attn, (size_t)TPF_MAX * qd * 2));
-    CK(cudaMalloc(&m->pf_h, (size_t)TPF_MAX * H * 2));
-    CK(cudaMalloc(&m->pf_act, (size_t)TPF_MAX * cfg->ffn * 2));
-    CK(util_fill0(m->pf_xn, (size_t)TPF_MAX * H * 2));
-    CK(util_fill0(m->pf_attn, (size_t)TPF_MAX * qd * 2));
-    CK(util_fill0(m->pf_act, (size_t)TPF_MAX * cfg->ffn * 2));
+    CK(cudaMalloc(&m->pf_xn, (size_t)CHUNK_MAX * H * 2));
+    CK(cudaMalloc(&m->pf_qkv, (size_t)CHUNK_MAX * qkvd * 2));
+    CK(cudaMalloc(&m->pf_q, (size_t)CHUNK_MAX * qd * 2));
+    CK(cudaMalloc(&m->pf_attn, (size_t)CHUNK_MAX * qd * 2));
+    CK(cudaMalloc(&m->pf_h, (size_t)CHUNK_MAX * H * 2));
+    CK(cudaMalloc(&m->pf_act, (size_t)CHUNK_MAX * cfg->ffn * 2));
+    CK(util_fill0(m->pf_xn, (size_t)CHUNK_MAX * H * 2));
+    CK(util_fill0(m->pf_attn, (size_t)CHUNK_MAX * qd * 2));
+    CK(util_fill0(m->pf_act, (size_t)CHUNK_MAX * cfg->ffn * 2));
     m->pf_ok = (H % 128 == 0) && (qd % 128 == 0) && (cfg->ffn % 128 == 0) && ((cfg->n_kv_heads * HD) % 128 == 0) &&
                true;
-    m->pf_ok = m->pf_ok && make_tmap(&m->tm_xn, m->pf_xn, TPF_MAX, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_attn, m->pf_attn, TPF_MAX, qd, TC_XBOX) == DN_OK &&
-               make_tmap(&m->tm_act, m->pf_act, TPF_MAX, cfg->ffn, TC_XBOX) == DN_OK;
+    m->pf_ok = m->pf_ok && make_tmap(&m->tm_xn, m->pf_xn, CHUNK_MAX, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_attn, m->pf_attn, CHUNK_MAX, qd, TC_XBOX) == DN_OK &&
+               make_tmap(&m->tm_act, m->pf_act, CHUNK_MAX, cfg->ffn, TC_XBOX) == DN_OK;
     if (cfg->n_experts > 0 && m->pf_ok) {
-      const int P = TPF_MAX * cfg->top_k, E = cfg->n_experts;
+      const int P = CHUNK_MAX * cfg->top_k, E = cfg->n_experts;
       m->moe_max_tiles = P / 64 + E;
       CK(cudaMalloc(&m->moe_xg, (size_t)P * H * 2));
       CK(cudaMalloc(&m->moe_act, (size_t)P * cfg->ffn * 2));
@@ -487,6 +492,7 @@ extern "C" int dn_model_destroy(dn_model* m) {
 extern "C" int dn_model_max_chunk(dn_model* m) { return m ? m->tmax : 0; }
 // largest chunk for the tensor-core prefill path (0 = unavailable); chunks must be >= 16 tokens
 extern "C" int dn_model_max_prefill_chunk(dn_model* m) { return (m && m->pf_ok && g_tc_prefill) ? TPF_MAX : 0; }
+extern "C" int dn_model_max_chunk_forward(dn_model* m) { return (m && m->pf_ok && g_tc_prefill) ? CHUNK_MAX : 0; }
 
 extern "C" int dn_bind_layer(dn_model* m, int abs_layer, const void* const* dev_ptrs) {
   if (!m || !dev_ptrs) return fail(DN_EINVAL, "null argument");
@@ -819,7 +825,7 @@ static int layer_forward(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, 
 static int head_common(dn_model* m, const void* x, int T, dn_kv* kv, int32_t* token_out, float* logprob_out,
                        float* logits_f32, cudaStream_t s);
 
-// ---- tensor-core prefill path (16 <= T <= TPF_MAX): tcgen05 GEMMs fed by TMA (dn_gemm_tc.cuh)
+// ---- tensor-core prefill path (chunks of up to CHUNK_MAX tokens): tcgen05 GEMMs fed by TMA (dn_gemm_tc.cuh)
 // one launch: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
 static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, cudaStream_t s) {
@@ -838,12 +844,12 @@ static cudaError_t gemm_tc_grouped(const CUtensorMap& x, TcParams& p, int width,
   return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s);
 }
 
-// sparse MoE FFN of a prompt chunk's layer (16 .. TPF_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up
+// sparse MoE FFN of a prompt chunk's layer (2 .. CHUNK_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up
 // products in one grouped launch, all down products in another, join.  Bound by reading the experts' matrices once (Mixtral-8x7B: 2.8 GB,
 // 0.43 ms of copy bandwidth a layer); token by token (moe_ffn) every token reads its own experts': 500 tokens took 86 ms.
 static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, int T, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
-  const int H = c.hidden, E = c.n_experts, k = c.top_k, P = T * k, mt = m->moe_max_tiles, Pmax = TPF_MAX * k;
+  const int H = c.hidden, E = c.n_experts, k = c.top_k, P = T * k, mt = m->moe_max_tiles, Pmax = CHUNK_MAX * k;
   MoePlan pl{m->moe_plan, m->moe_plan + Pmax, m->moe_plan + 2 * Pmax, m->moe_plan + 2 * Pmax + mt, m->moe_plan + 2 * Pmax + 2 * mt, m->moe_plan + 2 * Pmax + 3 * mt};
   const int width = tc_grouped_width((c.ffn + 127) / 128, E, P, g_sms);
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, false, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
@@ -973,23 +979,19 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   return DN_OK;
 }
 
-// The kernels of a chunk.  The prompt kernels take every chunk of two tokens and more, and single tokens of layers with experts or with
-// quantised pages (behind 8,000 8-bit tokens 218 us against 1,650 of the row kernels' attention, a block a head); a single token of a
-// dense layer over bf16 pages is as fast on the row kernels, which form the norm and the rotation in their products' launches
-// (Llama-8B sizes behind 256: 107 us either way).
-static bool use_prompt_kernels(const dn_model* m, int T) {
-  return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.kv_bits != 0 || (m->cfg.n_experts > 0 && m->moe_tc_ok));
-}
+// The kernels of a chunk: the prompt's, single tokens included (Llama-8B sizes behind 256: 99 us against 107 of the row kernels, which form the
+// norm and the rotation in their products' launches; behind 8,000 8-bit tokens 218 against 1,650, Mixtral-8x7B sizes 181 against 236).
+static bool use_prompt_kernels(const dn_model* m, int T) { return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.n_experts == 0 || m->moe_tc_ok); }
 static int one_layer(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
   return use_prompt_kernels(m, T) ? layer_forward_tc(m, abs_layer, x, T, kv, s, ev) : layer_forward(m, abs_layer, x, T, kv, s, ev);
 }
 
-static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16) {
+static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16, int tc_to = TPF_MAX) {
   if (!m || !x || !kv) return fail(DN_EINVAL, "null argument");
   if (kv->m != m) return fail(DN_EINVAL, "kv belongs to a different model");
-  const bool tc_ok = g_tc_prefill && m->pf_ok && T >= tc_from && T <= TPF_MAX;
+  const bool tc_ok = g_tc_prefill && m->pf_ok && T >= tc_from && T <= tc_to;
   if (!tc_ok && (!(T == 1 || T == 2 || T == 4) || T > m->tmax))
-    return fail(DN_EINVAL, "T=%d unsupported (1,2,4 up to %d, or %d..%d on the tensor-core prefill path)", T, m->tmax, tc_from, TPF_MAX);
+    return fail(DN_EINVAL, "T=%d unsupported (1,2,4 up to %d, or %d..%d on the tensor-core prefill path)", T, m->tmax, tc_from, tc_to);
   if (!g_capturing && kv->host_pos + T > kv->max_tokens)
     return fail(DN_ENOSPC, "KV capacity exceeded: offset %d + %d > %d", kv->host_pos, T, kv->max_tokens);
   if (((uintptr_t)x) & 15) return fail(DN_EINVAL, "activation must be 16-byte aligned");
@@ -1047,9 +1049,9 @@ extern "C" int dn_head_timed(dn_model* m, const void* x, int T, dn_stream s, flo
   return DN_OK;
 }
 
-// dn_window_forward for a chunk of any size up to dn_model_max_prefill_chunk: 2 .. ROWS_MAX tokens read the weights once, too
+// dn_window_forward for a chunk of any size up to dn_model_max_chunk_forward: 2 .. ROWS_MAX tokens read the weights once, too
 extern "C" int dn_chunk_forward(dn_model* m, const int32_t* abs_layers, int n, void* x_inout, int T, dn_kv* kv, dn_stream s) {
-  int rc = check_fwd(m, x_inout, T, kv, 2);
+  int rc = check_fwd(m, x_inout, T, kv, 2, CHUNK_MAX);
   if (rc) return rc;
   if (n > 0 && !abs_layers) return fail(DN_EINVAL, "null layer list");
   for (int i = 0; i < n; ++i) {

@@ -126,8 +126,8 @@ __device__ __forceinline__ void kvq_store_row(unsigned char* unit, int tok, int 
 }
 
 // bf16 staging "pool" the unchanged append kernels write into (same page layout as the bf16 pool; logical page p
-// lives in staging page p % KVQ_STAGE_PAGES -- a chunk of <= 512 tokens spans at most 9 logical pages)
-constexpr int KVQ_STAGE_PAGES = 16;
+// lives in staging page p % KVQ_STAGE_PAGES -- a chunk of <= 2,048 tokens spans at most 33 logical pages)
+constexpr int KVQ_STAGE_PAGES = 64;
 __device__ __forceinline__ const bf16* kvq_stage_row(const bf16* stage, int pos, int kv, int kvh, int n_kv) {
   const int sp = (pos / PAGE) % KVQ_STAGE_PAGES;
   return stage + (((size_t)sp * 2 + kv) * n_kv + kvh) * (PAGE * HD) + (size_t)(pos % PAGE) * HD;

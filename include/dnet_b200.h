@@ -137,7 +137,8 @@ int dn_layer_forward(dn_model* m, int abs_layer, void* x_inout, int T, dn_kv* kv
 /* the window loop of FitInMemoryPolicy.process (fit_in_memory.py:78-124) in one call */
 int dn_window_forward(dn_model* m, const int32_t* abs_layers, int n, void* x_inout, int T,
                       dn_kv* kv, dn_stream s);
-/* the same for a chunk of any size, 1 .. dn_model_max_prefill_chunk tokens (where that is 0: the sizes of dn_window_forward) */
+/* the same for a chunk of any size, 1 .. dn_model_max_chunk_forward tokens (where that is 0: the sizes of dn_window_forward) */
+int dn_model_max_chunk_forward(dn_model* m);
 int dn_chunk_forward(dn_model* m, const int32_t* abs_layers, int n, void* x_inout, int T,
                      dn_kv* kv, dn_stream s);
 /* The whole single-token step of this shard -- [embed] + a contiguous run of local layers +

@@ -144,3 +144,25 @@ def test_chunks_of_a_few_tokens(cuda_lib, hidden, ffn, kv_heads, group, context,
         kv.free()
         m.destroy()
     _agree(one_pass, torch.cat(rows).float().cpu(), 0.5 if bits else 0.25)
+
+
+@pytest.mark.parametrize("bits,group,hidden,ffn,T", [(0, 4, 512, 2048, 513), (8, 2, 512, 512, 1029), (0, 5, 768, 1280, 2048), (4, 1, 256, 512, 2050)])
+def test_one_chunk_of_up_to_2048_tokens(cuda_lib, bits, group, hidden, ffn, T):
+    """a prompt in chunks of 2,048 tokens and what is left over (more rows than a launch of 512, staging pages of a whole chunk, two tokens
+    behind the last full one) against the same prompt in chunks of 512"""
+    kv_heads = 2
+    x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    m = _model(kv_heads, group, seed=T, hidden=hidden, ffn=ffn, kv_bits=bits)
+    kv = m.make_cache(max_tokens=2560)
+    try:
+        whole = _call(m, kv, x, 0)
+        parts = []
+        for t in range(0, T, 512):
+            kv.seek(t)
+            parts.append(m.apply_single_layer(0, x[t:t + 512].clone(), kv))
+        torch.cuda.synchronize()
+        assert cuda_lib.dn_step_error(m._h, 0) == 0
+    finally:
+        kv.free()
+        m.destroy()
+    _agree(whole, torch.cat(parts).float().cpu(), 0.5 if bits else 0.25)      # (quantised pages: as above)
