@@ -1480,11 +1480,11 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       // tokens per staged tile: two tiles of `per` floats a token within ~36 KB of shared memory
       const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
       const size_t dsm = (size_t)2 * TB * per * 4;
-#define DR(Rv, Pv) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv>, grid, dim3(32 * Pv), dsm, s, b, lc.heads, lc.kv_heads, lc.dim, lc.vdim, TB, \
+#define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, lc.heads, lc.kv_heads, lc.dim, lc.vdim, TB, \
                          (const float*)m->qn, (const float*)m->kn, (const float*)m->vv, (const float*)m->beta, (const float*)m->decay, st,      \
                          m->delta_stride, m->od))
       PH(DN_SEQ_PH_DELTA_RULE);
-      DR(8, 1); DR(8, 2); DR(8, 4); DR(8, 8); DR(16, 8); DR(16, 16); DR(16, 32); DR(32, 32);
+      DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
 #undef DR
       PH(DN_SEQ_PH_DELTA_OUT);
       CK(launch(k_delta_out<T>, dim3(N, lc.heads), dim3(32), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), lc.heads, lc.vdim,

@@ -2225,40 +2225,92 @@ __global__ void __launch_bounds__(512) k_delta_prep(DeltaPrep a, Batch b, const 
 }
 
 // The recurrence, token by token:  S <- g S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q.
-// Columns of S are independent: a block owns 32 columns of one (entry, head); P adjacent lanes share a column,
-// each holding R consecutive rows (P R >= dk) in registers.  State [slot][head][dk][dv] fp32.
+// Columns of S are independent: a block owns 32 columns of one (entry, head); P adjacent lanes share C columns,
+// each holding R consecutive rows of them (P R >= dk) in registers.  State [slot][head][dk][dv] fp32.
 // The tokens' inputs (k, q, the block's 32 values, decay, beta) come through shared memory in tiles of TB tokens,
 // copied asynchronously one tile ahead, so that the serial chain of a token is registers, shared memory and the
 // lane shuffles only.  k and q lie there as P runs of R values, each run padded by 4 floats: the 16-byte reads of
 // the P lanes of a column then fall into different banks; rows from dk up are zero, so the token loop has no
-// bounds checks.  Sums run in an order fixed by (dk, P): four interleaved partial sums over a thread's rows,
-// then the lanes of a column pairwise -- nothing depends on the tile size or on where a portion was cut.
+// bounds checks.  Sums run in an order fixed by (dk, P): four interleaved partial sums over a thread's rows (two
+// pairs), then the lanes of a column pairwise -- nothing depends on the tile size or on where a portion was cut.
+// Bound by the chain of a token in prompts (a token of one sequence of 32 heads of 128 x 128 takes 309 ns).  With one column a thread (C = 1)
+// the 32 values of k and q that a thread read met 16 rows only; with two they meet 32, two rows an instruction, and the lanes of a column
+// exchange half of their columns in the first step.  Four sequences, 2,048 tokens, the longest 787: C = 1 540 us, 2 373, 4 428 (fewer
+// warps, a longer chain); 4 x 512: 476, 316, 316; one sequence of 2,048: 651, 632, 863.  C = 4 only where registers ask for it (R = 32).
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src));
 }
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
+}
+// two fp32 operations, each rounded as the single one
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{.reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 z, x, y; mov.b64 {%0, %1}, z;}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{.reg .b64 x, y, z, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 w, x, y, z; mov.b64 {%0, %1}, w;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+// The sums over the P lanes of C columns' values, pairwise: while a lane holds more than one column it keeps half of them and gives the other
+// half away; at the end it holds the sum of column lane_col<C>(part).
+template <int C> __device__ __forceinline__ int lane_col(int part) { return C == 4 ? 2 * (part & 1) + ((part >> 1) & 1) : C == 2 ? part & 1 : 0; }
+template <int P, int C>
+__device__ __forceinline__ float sum_lanes(float (&x)[C], int part) {
+  float v;
+  if constexpr (C == 4) {
+    const bool hi = part & 1, hi2 = part & 2;
+    const float a = (hi ? x[2] : x[0]) + __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 1), b = (hi ? x[3] : x[1]) + __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 1);
+    v = (hi2 ? b : a) + __shfl_xor_sync(0xffffffffu, hi2 ? a : b, 2);
+  } else if constexpr (C == 2) v = ((part & 1) ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, (part & 1) ? x[0] : x[1], 1);
+  else v = x[0];
+#pragma unroll
+  for (int d = C; d < P; d <<= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
 
-template <int R, int P>
-__global__ void __launch_bounds__(32 * P) k_delta_rule(Batch b, int H, int G, int dk, int dv, int TB, const float* __restrict__ qn, const float* __restrict__ kn,
+template <int R, int P, int C>
+__global__ void __launch_bounds__(32 * P / C) k_delta_rule(Batch b, int H, int G, int dk, int dv, int TB, const float* __restrict__ qn, const float* __restrict__ kn,
                              const float* __restrict__ vv, const float* __restrict__ beta, const float* __restrict__ decay,
                              float* __restrict__ state, size_t slot_stride, float* __restrict__ o) {
+  static_assert(C <= P && R % 4 == 0, "lanes that share columns");
   extern __shared__ __align__(16) float dsm[];      // 2 x TB x per
   constexpr int KP = P * (R + 4);                   // padded extent of k (and of q)
   constexpr int per = 2 * KP + 36;                      // k q v[32] decay beta, rounded to 16 bytes
   const int e = blockIdx.x / H, h = blockIdx.x % H, g = h / (H / G);
-  const int part = threadIdx.x % P, colb = threadIdx.x / P, col = blockIdx.y * 32 + colb;
+  const int part = threadIdx.x % P, colb = threadIdx.x / P * C, col = blockIdx.y * 32 + colb;
+  const int mine = lane_col<C>(part), own = col + mine;      // the column whose sums this lane ends up with
+  const bool owner = part < C && own < dv;                       // (lanes from C up hold copies)
   const int s0 = b.ent_start[e], s1 = b.ent_start[e + 1];
-  const bool live = col < dv;
   float* Sg = state + (size_t)b.ent_slot[e] * slot_stride + (size_t)h * dk * dv;
   const int r0 = part * R;
-  float S[R];
+  const bool vec = C == 4 && dv % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
+  float2 S[C][R / 2];
 #pragma unroll
-  for (int r = 0; r < R; r++) S[r] = (live && r0 + r < dk) ? Sg[(size_t)(r0 + r) * dv + col] : 0.f;
+  for (int r = 0; r < R; r++) {
+    float x[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) x[c] = 0.f;
+    if (r0 + r < dk) {
+      const float* p = Sg + (size_t)(r0 + r) * dv + col;
+      if (vec) { if (col < dv) { const float4 f = *reinterpret_cast<const float4*>(p); x[0] = f.x; x[C > 1 ? 1 : 0] = f.y; x[C > 2 ? 2 : 0] = f.z; x[C > 3 ? 3 : 0] = f.w; } }
+      else
+#pragma unroll
+        for (int c = 0; c < C; c++) if (col + c < dv) x[c] = p[c];
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++) { if (r & 1) S[c][r / 2].y = x[c]; else S[c][r / 2].x = x[c]; }
+  }
   const int Cq = G * dk, Cv = H * dv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int nwarp = P;
+  constexpr int nwarp = P / C;
   auto stage = [&](int buf, int n0) {
     const int cnt = min(TB, s1 - n0);
     for (int t = warp; t < cnt; t += nwarp) {
@@ -2266,11 +2318,18 @@ __global__ void __launch_bounds__(32 * P) k_delta_rule(Batch b, int H, int G, in
       float* dst = dsm + ((size_t)buf * TB + t) * per;
       const float* kr = kn + (size_t)n * Cq + g * dk;
       const float* qr = qn + (size_t)n * Cq + g * dk;
-      for (int c = lane; c < P * R; c += 32) {
-        const int idx = (c / R) * (R + 4) + (c % R);
-        if (c < dk) { cp_async4(dst + idx, kr + c); cp_async4(dst + KP + idx, qr + c); }
-        else dst[idx] = dst[KP + idx] = 0.f;
-      }
+      if (dk % 4 == 0) {
+        for (int c = 4 * lane; c < P * R; c += 128) {
+          const int idx = (c / R) * (R + 4) + (c % R);
+          if (c < dk) { cp_async16(dst + idx, kr + c); cp_async16(dst + KP + idx, qr + c); }
+          else *reinterpret_cast<float4*>(dst + idx) = *reinterpret_cast<float4*>(dst + KP + idx) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      } else
+        for (int c = lane; c < P * R; c += 32) {
+          const int idx = (c / R) * (R + 4) + (c % R);
+          if (c < dk) { cp_async4(dst + idx, kr + c); cp_async4(dst + KP + idx, qr + c); }
+          else dst[idx] = dst[KP + idx] = 0.f;
+        }
       const int vc = blockIdx.y * 32 + lane;
       if (vc < dv) cp_async4(dst + 2 * KP + lane, vv + (size_t)n * Cv + h * dv + vc);
       else dst[2 * KP + lane] = 0.f;
@@ -2283,7 +2342,9 @@ __global__ void __launch_bounds__(32 * P) k_delta_rule(Batch b, int H, int G, in
   int buf = 0;
   // the read-out of token t is summed over the lanes of its column together with the dot product of token t + 1:
   // two independent shuffle chains in flight instead of one after the other
-  float odp = 0.f;
+  float odp[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) odp[c] = 0.f;
   for (int n0 = s0; n0 < s1; n0 += TB, buf ^= 1) {
     if (n0 + TB < s1) { stage(buf ^ 1, n0 + TB); cp_async_wait<1>(); }
     else cp_async_wait<0>();
@@ -2293,44 +2354,57 @@ __global__ void __launch_bounds__(32 * P) k_delta_rule(Batch b, int H, int G, in
       const float* in = dsm + ((size_t)buf * TB + t) * per;
       const float4* k4 = reinterpret_cast<const float4*>(in + part * (R + 4));
       const float4* q4 = reinterpret_cast<const float4*>(in + KP + part * (R + 4));
-      const float gd = in[2 * KP + 32], bt = in[2 * KP + 33], v = in[2 * KP + colb];
-      float kk[R], qq[R], d4[4] = {0.f, 0.f, 0.f, 0.f};
+      const float gd = in[2 * KP + 32], bt = in[2 * KP + 33], v = in[2 * KP + colb + mine];
+      float2 kk[R / 2], qq[R / 2], d[C][2];
+      const float2 g2 = make_float2(gd, gd), zero = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < R / 4; j++) {
-        const float4 kv = k4[j], qv = q4[j];
-        kk[4 * j] = kv.x; kk[4 * j + 1] = kv.y; kk[4 * j + 2] = kv.z; kk[4 * j + 3] = kv.w;
-        qq[4 * j] = qv.x; qq[4 * j + 1] = qv.y; qq[4 * j + 2] = qv.z; qq[4 * j + 3] = qv.w;
+      for (int i = 0; i < R / 4; i++) {
+        const float4 kv = k4[i], qv = q4[i];
+        kk[2 * i] = make_float2(kv.x, kv.y); kk[2 * i + 1] = make_float2(kv.z, kv.w);
+        qq[2 * i] = make_float2(qv.x, qv.y); qq[2 * i + 1] = make_float2(qv.z, qv.w);
+      }
+      float dot[C];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          S[4 * j + i] *= gd;
-          d4[i] = fmaf(S[4 * j + i], kk[4 * j + i], d4[i]);
+      for (int c = 0; c < C; c++) {
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) {
+          S[c][i] = mul2(S[c][i], g2);
+          d[c][i & 1] = fma2(S[c][i], kk[i], i < 2 ? zero : d[c][i & 1]);
         }
+        dot[c] = (d[c][0].x + d[c][0].y) + (d[c][1].x + d[c][1].y);
       }
-      float dot = (d4[0] + d4[1]) + (d4[2] + d4[3]);
+      const float dsum = sum_lanes<P, C>(dot, part), osum = sum_lanes<P, C>(odp, part);
+      if (owner && n0 + t > s0) o[(size_t)(n0 + t - 1) * Cv + h * dv + own] = osum;
+      const float u = bt * (v - dsum);
 #pragma unroll
-      for (int x = 1; x < P; x <<= 1) {
-        const float a = __shfl_xor_sync(0xffffffffu, dot, x), c = __shfl_xor_sync(0xffffffffu, odp, x);
-        dot += a;
-        odp += c;
-      }
-      if (live && part == 0 && n0 + t > s0) o[(size_t)(n0 + t - 1) * Cv + h * dv + col] = odp;
-      const float u = bt * (v - dot);
-      float o4[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int c = 0; c < C; c++) {
+        const int src = C == 4 ? (c >> 1) | ((c & 1) << 1) : c;      // the lane (of its column group) that holds column c
+        const float uc = C == 1 ? u : __shfl_sync(0xffffffffu, u, (lane & ~(C - 1)) | src);
+        const float2 u2 = make_float2(uc, uc);
 #pragma unroll
-      for (int r = 0; r < R; r++) {
-        S[r] = fmaf(kk[r], u, S[r]);
-        o4[r & 3] = fmaf(S[r], qq[r], o4[r & 3]);
+        for (int i = 0; i < R / 2; i++) {
+          S[c][i] = fma2(kk[i], u2, S[c][i]);
+          d[c][i & 1] = fma2(S[c][i], qq[i], i < 2 ? zero : d[c][i & 1]);
+        }
+        odp[c] = (d[c][0].x + d[c][0].y) + (d[c][1].x + d[c][1].y);
       }
-      odp = (o4[0] + o4[1]) + (o4[2] + o4[3]);
     }
     __syncthreads();      // the tile is read out before the copy after next lands in it
   }
-#pragma unroll
-  for (int x = 1; x < P; x <<= 1) odp += __shfl_xor_sync(0xffffffffu, odp, x);
-  if (live && part == 0 && s1 > s0) o[(size_t)(s1 - 1) * Cv + h * dv + col] = odp;
+  const float osum = sum_lanes<P, C>(odp, part);
+  if (owner && s1 > s0) o[(size_t)(s1 - 1) * Cv + h * dv + own] = osum;
 #pragma unroll
   for (int r = 0; r < R; r++)
-    if (live && r0 + r < dk) Sg[(size_t)(r0 + r) * dv + col] = S[r];
+    if (r0 + r < dk) {
+      float* p = Sg + (size_t)(r0 + r) * dv + col;
+      float x[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) x[c] = (r & 1) ? S[c][r / 2].y : S[c][r / 2].x;
+      if (vec) { if (col < dv) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[C > 1 ? 1 : 0], x[C > 2 ? 2 : 0], x[C > 3 ? 3 : 0]); }
+      else
+#pragma unroll
+        for (int c = 0; c < C; c++) if (col + c < dv) p[c] = x[c];
+    }
 }
 
 // read-out of the recurrence: per head o / rms(o) * w * silu(gate) -> T.  One warp per (token, head).
