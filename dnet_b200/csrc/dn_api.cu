@@ -190,6 +190,7 @@ struct dn_model {
   std::vector<CUtensorMap> tm_kv;                // per local layer: KV pool as [pages*2*n_kv*64 rows][128] bf16, box 64 x 64
   bool tm_kv_ok = false;
   bool pf_ok = false;
+  bool pf_last = false;      // the last chunk ran on the prompt kernels (dn_debug_scratch)
   unsigned long long* mk_dbg = nullptr;
   size_t mk_dbg_words = 0;
   int* mk_bounds = nullptr;      // [4][sms+1] calibrated row partition of the step kernel (null: equal split)
@@ -983,7 +984,8 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
 // norm and the rotation in their products' launches; behind 8,000 8-bit tokens 218 against 1,650, Mixtral-8x7B sizes 181 against 236).
 static bool use_prompt_kernels(const dn_model* m, int T) { return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.n_experts == 0 || m->moe_tc_ok); }
 static int one_layer(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
-  return use_prompt_kernels(m, T) ? layer_forward_tc(m, abs_layer, x, T, kv, s, ev) : layer_forward(m, abs_layer, x, T, kv, s, ev);
+  m->pf_last = use_prompt_kernels(m, T);
+  return m->pf_last ? layer_forward_tc(m, abs_layer, x, T, kv, s, ev) : layer_forward(m, abs_layer, x, T, kv, s, ev);
 }
 
 static int check_fwd(dn_model* m, void* x, int T, dn_kv* kv, int tc_from = 16, int tc_to = TPF_MAX) {
@@ -1375,7 +1377,8 @@ extern "C" int dn_step_error(dn_model* m, dn_stream s) {
 // (which: 0 q after RoPE [tmax][n_heads*128], 1 attention output, 2 h = x + o_proj [tmax][H], 3 SwiGLU output [tmax][ffn])
 extern "C" int dn_debug_scratch(dn_model* m, int which, void* host_out, size_t bytes, dn_stream s) {
   if (!m || !host_out) return fail(DN_EINVAL, "null argument");
-  const bf16* src = which == 0 ? m->qbuf : which == 1 ? m->attn : which == 2 ? m->hbuf : which == 3 ? m->act : nullptr;
+  const bf16* src = which == 0 ? (m->pf_last ? m->pf_q : m->qbuf) : which == 1 ? (m->pf_last ? m->pf_attn : m->attn) : which == 2 ? (m->pf_last ? m->pf_h : m->hbuf)
+                  : which == 3 ? (!m->pf_last ? m->act : m->moe_tc_ok ? m->moe_act : m->pf_act) : nullptr;
   if (!src) return fail(DN_EINVAL, "unknown scratch buffer %d", which);
   CK(cudaMemcpyAsync(host_out, src, bytes, cudaMemcpyDeviceToHost, (cudaStream_t)s));
   CK(cudaStreamSynchronize((cudaStream_t)s));

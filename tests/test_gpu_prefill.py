@@ -166,3 +166,30 @@ def test_one_chunk_of_up_to_2048_tokens(cuda_lib, bits, group, hidden, ffn, T):
         kv.free()
         m.destroy()
     _agree(whole, torch.cat(parts).float().cpu(), 0.5 if bits else 0.25)      # (quantised pages: as above)
+
+
+@pytest.mark.parametrize("T", [1, 4])
+def test_the_scratch_hook_reads_the_last_chunk(cuda_lib, T):
+    """dn_debug_scratch after a chunk, whichever kernels it ran on: the rotated queries, the attention's output, the residual and the
+    SwiGLU output of the chunk itself (a few last roundings of the row kernels')"""
+    import torch as t
+
+    hidden, ffn, heads = 512, 768, 4
+    x = t.randn(70 + T, hidden, generator=t.Generator().manual_seed(T)).to(t.bfloat16).cuda()
+    got = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_prefill", tc)
+            m = _model(2, 2, seed=5, hidden=hidden, ffn=ffn)
+            kv = m.make_cache(max_tokens=128)
+            _call(m, kv, x, 70)
+            for which, n in enumerate((heads * 128, heads * 128, hidden, ffn)):
+                host = t.empty(T, n, dtype=t.bfloat16)
+                assert cuda_lib.dn_debug_scratch(m._h, which, host.data_ptr(), host.numel() * 2, 0) == 0
+                got[tc, which] = host.float()
+            kv.free()
+            m.destroy()
+    finally:
+        cuda_lib.dn_set_option(b"tc_prefill", 1)
+    for which in range(4):
+        assert rel_inf(got[1, which], got[0, which]) <= 4 * 2.0 ** -8, which
