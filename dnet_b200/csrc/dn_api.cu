@@ -43,6 +43,11 @@ static int fail(int code, const char* fmt, ...) {
 
 static std::atomic<long long> g_launches{0};
 static int g_pdl = 0;
+// Launches of a chunk's layer are programmatic whatever the option says (0: never, 1: with the option): a layer is 8 to 10 launches, each of which
+// starts with a wait for the one in front, and the row products ask for their first weights before it.  Three tokens, Llama-8B sizes: 114 us
+// without, 101 with; 45 tokens 165 / 155; one Mixtral-8x7B token 182 / 163; 2,048 tokens of two layers 2,022 / 1,993.  (Prefetching more of the
+// weights into L2 before the wait cost 6 us.)
+constexpr int PDL_CHUNK = 2;
 static int g_l2_prefetch_kb = 64;
 static int g_mk_flags = 0;
 static int g_inflight_hi = 3;   // step kernel: cap while the consumers are starving for weights
@@ -83,7 +88,7 @@ struct dn_graph {
 
 template <typename... KArgs, typename... Args>
 static cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                          bool pdl_ok, Args... args) {
+                          int pdl_ok, Args... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid;
@@ -94,7 +99,7 @@ static cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = (g_pdl && pdl_ok) ? 1 : 0;
+  cfg.numAttrs = pdl_ok == PDL_CHUNK || (g_pdl && pdl_ok) ? 1 : 0;
   if (g_capturing) g_capture_launches++;
   else g_launches++;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
@@ -679,26 +684,28 @@ extern "C" int dn_embed(dn_model* m, const int32_t* ids_dev, int T, void* x_out,
 
 // clusters span the grid's z
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, const Args&... args) {
+static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, int pdl, const Args&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = grid.z;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl == PDL_CHUNK ? 2 : 1;
   if (g_capturing) g_capture_launches++; else g_launches++;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
 // a prompt chunk's attention over the quantised pages
 template <int BITS>
-static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf16* out, int T, dn_kv* kv, cudaStream_t s) {
+static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf16* out, int T, dn_kv* kv, int pdl, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   AqParams a;
   a.a.q = q; a.a.out = out; a.a.block_table = kv->block_table; a.a.st = kv->st;
@@ -706,7 +713,7 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
   a.pool = pool;
   const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
   const dim3 grid(c.n_kv_heads, blocks, attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms));
-#define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, a)); break;
+#define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, pdl, a)); break;
   switch (m->G) { PFQ(1) PFQ(2) PFQ(4) PFQ(5) PFQ(7) PFQ(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFQ
   return DN_OK;
@@ -715,7 +722,7 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
 // quantised KV: after the (unchanged) append kernels wrote the T new K/V rows as bf16 into the staging pool, quantise
 // them into the packed pool and run the two-pass quantised attention (dn_kvquant.cuh; prompt chunks: dn_attn_q.cuh)
 // (prompt: q and attn_out are the prefill path's)
-static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, bool prompt, cudaStream_t s) {
+static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, int pdl, bool prompt, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   unsigned char* pool = reinterpret_cast<unsigned char*>(m->kv_pool) + (size_t)li * m->kv_layer_bytes;
   // host mirror: longest context any of the T queries sees (a captured graph is replayed at growing contexts)
@@ -724,11 +731,11 @@ static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_
   if (smem > 200 * 1024) return fail(DN_EINVAL, "quantised-KV attention outside the step kernel supports contexts up to ~50K tokens (got %d)", kv_len_max);
   const dim3 ga(T, 2 * c.n_kv_heads), gq(c.n_heads, T);
   if (c.kv_bits == 8) {
-    CK(launch(k_kv_quant_append<8>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
+    CK(launch(k_kv_quant_append<8>, ga, dim3(32), 0, s, pdl, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
   } else {
-    CK(launch(k_kv_quant_append<4>, ga, dim3(32), 0, s, false, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
+    CK(launch(k_kv_quant_append<4>, ga, dim3(32), 0, s, pdl, (const bf16*)m->kvq_stage, pool, (const int32_t*)kv->block_table, (const StepState*)kv->st, c.n_kv_heads));
   }
-  if (prompt && g_tc_attn) return c.kv_bits == 8 ? attend_q_tc<8>(m, pool, q, attn_out, T, kv, s) : attend_q_tc<4>(m, pool, q, attn_out, T, kv, s);
+  if (prompt && g_tc_attn) return c.kv_bits == 8 ? attend_q_tc<8>(m, pool, q, attn_out, T, kv, pdl, s) : attend_q_tc<4>(m, pool, q, attn_out, T, kv, pdl, s);
   static size_t smem_set[2] = {0, 0};
   const int bi = c.kv_bits == 8 ? 1 : 0;
   if (smem > smem_set[bi]) {
@@ -795,7 +802,7 @@ static int layer_forward(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, 
   CK(launch_gemv_T(T, q, q.nrows / 2, s));
   if (evs) CK(cudaEventRecord(evs[1], s));
 
-  if (kvq) { const int rc = kvq_append_and_attend(m, li, m->qbuf, m->attn, T, kv, false, s); if (rc) return rc; }
+  if (kvq) { const int rc = kvq_append_and_attend(m, li, m->qbuf, m->attn, T, kv, 0, false, s); if (rc) return rc; }
   else CK(launch_attn(m, m->qbuf, pool, kv->block_table, kv->st, T, s));
   if (evs) CK(cudaEventRecord(evs[2], s));
 
@@ -829,11 +836,11 @@ static int head_common(dn_model* m, const void* x, int T, dn_kv* kv, int32_t* to
 // ---- tensor-core prefill path (chunks of up to CHUNK_MAX tokens): tcgen05 GEMMs fed by TMA (dn_gemm_tc.cuh)
 // one launch: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
-static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, cudaStream_t s) {
+static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, int pdl, cudaStream_t s) {
   int n_tiles = 0;
   for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + tc_tile_rows<EPI>() - 1) / tc_tile_rows<EPI>();
   if (g_capturing) g_capture_launches++; else g_launches++;
-  return tc_launch<EPI, false>(maps, p, tc_plan(n_tiles, p.T, p.K, g_sms), s);
+  return tc_launch<EPI, false>(maps, p, tc_plan(n_tiles, p.T, p.K, g_sms), s, pdl == PDL_CHUNK);
 }
 
 template <int EPI>
@@ -848,13 +855,13 @@ static cudaError_t gemm_tc_grouped(const CUtensorMap& x, TcParams& p, int width,
 // sparse MoE FFN of a prompt chunk's layer (2 .. CHUNK_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up
 // products in one grouped launch, all down products in another, join.  Bound by reading the experts' matrices once (Mixtral-8x7B: 2.8 GB,
 // 0.43 ms of copy bandwidth a layer); token by token (moe_ffn) every token reads its own experts': 500 tokens took 86 ms.
-static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, int T, cudaStream_t s) {
+static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, int T, int pdl, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   const int H = c.hidden, E = c.n_experts, k = c.top_k, P = T * k, mt = m->moe_max_tiles, Pmax = CHUNK_MAX * k;
   MoePlan pl{m->moe_plan, m->moe_plan + Pmax, m->moe_plan + 2 * Pmax, m->moe_plan + 2 * Pmax + mt, m->moe_plan + 2 * Pmax + 2 * mt, m->moe_plan + 2 * Pmax + 3 * mt};
   const int width = tc_grouped_width((c.ffn + 127) / 128, E, P, g_sms);
-  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, false, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
-  CK(launch(k_moe_route, dim3(T), dim3(256), 0, s, false, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
+  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
+  CK(launch(k_moe_route, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
   CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, false, (const int32_t*)m->moe_psel, P, k, E, width, pl, E));
   CK(launch(k_moe_gather<bf16>, dim3(P), dim3(128), 0, s, false, (const bf16*)m->pf_xn, (const int32_t*)pl.row_tok, H, m->moe_xg));
   TcParams p;
@@ -865,20 +872,20 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   CK(gemm_tc_grouped<EPI_SWIGLU>(m->tm_moe_xg, p, width, s));
   p.K = c.ffn; p.seg[0] = TcSeg{H, H, m->moe_out, nullptr, 0}; p.g_mapW = p.g_mapW2 = L.emaps + 2 * E;
   CK(gemm_tc_grouped<EPI_STORE>(m->tm_moe_act, p, width, s));
-  CK(launch(k_moe_join, dim3(T), dim3(256), 0, s, false, (const bf16*)m->moe_out, (const int32_t*)pl.pos, (const float*)m->moe_pscore, k, H, h, out));
+  CK(launch(k_moe_join, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->moe_out, (const int32_t*)pl.pos, (const float*)m->moe_pscore, k, H, h, out));
   return DN_OK;
 }
 
 // the same product(s) for a chunk of at most ROWS_MAX tokens: weights straight from memory
 template <int EPI>
-static cudaError_t rows_product(const TcParams& p, const bf16* x, const bf16* w0, const bf16* w1, const bf16* w2, cudaStream_t s) {
+static cudaError_t rows_product(const TcParams& p, const bf16* x, const bf16* w0, const bf16* w1, const bf16* w2, int pdl, cudaStream_t s) {
   RowsParams r;
   memset(&r, 0, sizeof(r));
   int blocks = 0;
   for (int i = 0; i < p.nseg; ++i) { r.seg[i] = p.seg[i]; blocks += (p.seg[i].N + 15) / 16; }
   r.w[0] = w0; r.w[1] = w1; r.w[2] = w2;
   r.nseg = p.nseg; r.T = p.T; r.K = p.K; r.x = x; r.resid = p.resid; r.ldr = p.ldr;
-#define ROWS(NT, U) launch(k_rows<EPI, NT, U>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r)
+#define ROWS(NT, U) launch(k_rows<EPI, NT, U>, dim3(blocks), dim3(RM_THREADS), 0, s, pdl, r)
   if constexpr (EPI != EPI_SWIGLU)
     if (rows_mma_deep(blocks, g_sms)) return p.T <= 8 ? ROWS(1, 8) : ROWS(2, 8);
   return p.T <= 8 ? ROWS(1, 4) : ROWS(2, 4);
@@ -887,21 +894,21 @@ static cudaError_t rows_product(const TcParams& p, const bf16* x, const bf16* w0
 
 // one token's experts: all choices' gate / up products in one launch, all down products in another (a launch a choice, on the row kernels
 // of moe_ffn: 2 x 51 + 2 x 31 us at Mixtral-8x7B sizes, 0.70 and 0.58 of the copy bandwidth; so 70 + 38)
-static int moe_ffn_one(dn_model* m, const LayerW& L, const bf16* h, bf16* out, cudaStream_t s) {
+static int moe_ffn_one(dn_model* m, const LayerW& L, const bf16* h, bf16* out, int pdl, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   const int H = c.hidden, E = c.n_experts, k = c.top_k;
-  CK(launch(k_rmsnorm_rows, dim3(1), dim3(256), 0, s, true, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
-  CK(launch(k_moe_route, dim3(1), dim3(256), 0, s, true, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
+  CK(launch(k_rmsnorm_rows, dim3(1), dim3(256), 0, s, pdl, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
+  CK(launch(k_moe_route, dim3(1), dim3(256), 0, s, pdl, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
   RowsParams r;
   memset(&r, 0, sizeof(r));
   r.nseg = 1; r.T = 1; r.table = (const bf16* const*)L.etable; r.sel = m->moe_psel;
   r.seg[0] = TcSeg{c.ffn, c.ffn, m->moe_act, nullptr, 0}; r.K = H; r.x = m->pf_xn; r.ldx = 0; r.m0 = 0; r.m1 = E;
-  CK(launch(k_rows<EPI_SWIGLU, 1, 4, true>, dim3(k * ((c.ffn + 15) / 16)), dim3(RM_THREADS), 0, s, true, r));
+  CK(launch(k_rows<EPI_SWIGLU, 1, 4, true>, dim3(k * ((c.ffn + 15) / 16)), dim3(RM_THREADS), 0, s, pdl, r));
   r.seg[0] = TcSeg{H, H, m->moe_out, nullptr, 0}; r.K = c.ffn; r.x = m->moe_act; r.ldx = c.ffn; r.m0 = 2 * E;
   const int blocks = k * ((H + 15) / 16);
-  if (rows_mma_deep(blocks, g_sms)) CK(launch(k_rows<EPI_STORE, 1, 8, true>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r));
-  else CK(launch(k_rows<EPI_STORE, 1, 4, true>, dim3(blocks), dim3(RM_THREADS), 0, s, true, r));
-  CK(launch(k_moe_join, dim3(1), dim3(256), 0, s, true, (const bf16*)m->moe_out, (const int32_t*)nullptr, (const float*)m->moe_pscore, k, H, h, out));
+  if (rows_mma_deep(blocks, g_sms)) CK(launch(k_rows<EPI_STORE, 1, 8, true>, dim3(blocks), dim3(RM_THREADS), 0, s, pdl, r));
+  else CK(launch(k_rows<EPI_STORE, 1, 4, true>, dim3(blocks), dim3(RM_THREADS), 0, s, pdl, r));
+  CK(launch(k_moe_join, dim3(1), dim3(256), 0, s, pdl, (const bf16*)m->moe_out, (const int32_t*)nullptr, (const float*)m->moe_pscore, k, H, h, out));
   return DN_OK;
 }
 
@@ -922,7 +929,8 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
 
   EV(0);
   const bool few = T <= ROWS_MAX;
-  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, few, (const bf16*)x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps));
+  const int pdl = ev ? 0 : PDL_CHUNK;      // (timed one by one: each launch alone)
+  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, (const bf16*)x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps));
   TcMaps maps;
   for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = L.tm[i < 3 ? i : 0];
   maps.x = m->tm_xn;
@@ -930,13 +938,13 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   p.seg[0] = TcSeg{qd, qkvd, m->pf_qkv, L.w[DN_W_QB], 0};
   p.seg[1] = TcSeg{kd, qkvd, m->pf_qkv + qd, L.w[DN_W_KB], 0};
   p.seg[2] = TcSeg{kd, qkvd, m->pf_qkv + qd + kd, L.w[DN_W_VB], 0};
-  CK(few ? rows_product<EPI_STORE>(p, m->pf_xn, L.w[DN_W_Q], L.w[DN_W_K], L.w[DN_W_V], s) : gemm_tc<EPI_STORE>(maps, p, s));
+  CK(few ? rows_product<EPI_STORE>(p, m->pf_xn, L.w[DN_W_Q], L.w[DN_W_K], L.w[DN_W_V], pdl, s) : gemm_tc<EPI_STORE>(maps, p, pdl, s));
   const bool kvq = c.kv_bits != 0;
-  CK(launch(k_rope_append, dim3((c.n_heads + 2 * c.n_kv_heads + ROPE_SLOTS - 1) / ROPE_SLOTS, T), dim3(128), 0, s, few, (const bf16*)m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
+  CK(launch(k_rope_append, dim3((c.n_heads + 2 * c.n_kv_heads + ROPE_SLOTS - 1) / ROPE_SLOTS, T), dim3(128), 0, s, pdl, (const bf16*)m->pf_qkv, m->pf_q, kvq ? m->kvq_stage : pool,
             kvq ? (const int32_t*)m->kvq_stage_bt : (const int32_t*)kv->block_table, (const StepState*)kv->st, (const float*)m->inv_freq, c.n_heads, c.n_kv_heads));
   EV(1);
   if (kvq) {
-    const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, true, s);
+    const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, pdl, true, s);
     if (rc) return rc;
   } else if (g_tc_attn && m->tm_kv_ok) {
     AtParams a;
@@ -945,7 +953,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
     // (how the keys are shared out only decides the order of the sums; the kernel reads the position from the step state)
     const int Z = attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms);
-#define PFT(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_tc<Gv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, m->tm_kv[li], a)); break;
+#define PFT(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_tc<Gv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
     switch (m->G) { PFT(1) PFT(2) PFT(4) PFT(5) PFT(7) PFT(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT
   } else {
@@ -958,22 +966,22 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   EV(2);
   p.K = qd; p.nseg = 1; p.seg[0] = TcSeg{H, H, m->pf_h, nullptr, 0}; p.resid = x; p.ldr = H;
   maps.w[0] = L.tm[3]; maps.x = m->tm_attn;
-  CK(few ? rows_product<EPI_RESID>(p, m->pf_attn, L.w[DN_W_O], nullptr, nullptr, s) : gemm_tc<EPI_RESID>(maps, p, s));
+  CK(few ? rows_product<EPI_RESID>(p, m->pf_attn, L.w[DN_W_O], nullptr, nullptr, pdl, s) : gemm_tc<EPI_RESID>(maps, p, pdl, s));
   EV(3);
   if (c.n_experts > 0) {
     if (!L.experts_bound) return fail(DN_ENOENT, "MoE layer has no experts bound (dn_bind_layer_experts)");
-    const int rc = m->moe_tc_ok && L.emaps_ok ? (T == 1 ? moe_ffn_one(m, L, m->pf_h, x, s) : moe_ffn_tc(m, L, m->pf_h, x, T, s)) : moe_ffn(m, L, m->pf_h, x, T, s);
+    const int rc = m->moe_tc_ok && L.emaps_ok ? (T == 1 ? moe_ffn_one(m, L, m->pf_h, x, pdl, s) : moe_ffn_tc(m, L, m->pf_h, x, T, pdl, s)) : moe_ffn(m, L, m->pf_h, x, T, s);
     if (rc == DN_OK) { EV(4); EV(5); }
     return rc;
   }
-  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, few, (const bf16*)m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
+  CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   p.K = H; p.seg[0] = TcSeg{c.ffn, c.ffn, m->pf_act, nullptr, 0};
   maps.w[0] = L.tm[4]; maps.w[1] = L.tm[5]; maps.x = m->tm_xn;
-  CK(few ? rows_product<EPI_SWIGLU>(p, m->pf_xn, L.w[DN_W_GATE], L.w[DN_W_UP], nullptr, s) : gemm_tc<EPI_SWIGLU>(maps, p, s));
+  CK(few ? rows_product<EPI_SWIGLU>(p, m->pf_xn, L.w[DN_W_GATE], L.w[DN_W_UP], nullptr, pdl, s) : gemm_tc<EPI_SWIGLU>(maps, p, pdl, s));
   EV(4);
   p.K = c.ffn; p.seg[0] = TcSeg{H, H, x, nullptr, 0}; p.resid = m->pf_h; p.ldr = H;
   maps.w[0] = L.tm[6]; maps.x = m->tm_act;
-  CK(few ? rows_product<EPI_RESID>(p, m->pf_act, L.w[DN_W_DOWN], nullptr, nullptr, s) : gemm_tc<EPI_RESID>(maps, p, s));
+  CK(few ? rows_product<EPI_RESID>(p, m->pf_act, L.w[DN_W_DOWN], nullptr, nullptr, pdl, s) : gemm_tc<EPI_RESID>(maps, p, pdl, s));
   EV(5);
 #undef EV
   CK(cudaGetLastError());

@@ -37,6 +37,8 @@ __device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16])
 
 template <int G, int BITS>
 __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParams pq) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int TB = 128 / G;
   const AtParams& p = pq.a;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];

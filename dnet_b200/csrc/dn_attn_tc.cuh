@@ -43,6 +43,8 @@ constexpr float AT_SLACK = 8.f;            // how far (log2) a score may exceed 
 
 template <int G>
 __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_constant__ CUtensorMap mapKV, const AtParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int TB = 128 / G;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);

@@ -251,6 +251,8 @@ template <int EPI, bool GROUPED = false>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant__ TcMaps maps, const __grid_constant__ TcParams p) {
   constexpr bool GLU = epi_two_weights(EPI);
   constexpr int ROWS = tc_tile_rows<EPI>();
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
   float* xch = reinterpret_cast<float*>(smem + TC_RING);
@@ -684,7 +686,7 @@ static inline int tc_grouped_width(int n_tiles, int E, int P, int sms) {
   return best;
 }
 template <int EPI, bool GROUPED>
-static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPlan& pl, cudaStream_t s) {
+static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPlan& pl, cudaStream_t s, bool pdl = false) {
   p.width = pl.width; p.split = pl.split; p.stages = pl.stages;
   for (int i = 0; i < p.nseg; ++i) {
     TcSeg& sg = p.seg[i];
@@ -701,8 +703,11 @@ static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPla
     attr = true;
   }
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   tc_config(&cfg, at, pl.grid, 2 * pl.split, s);
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = pdl ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, k_gemm_tc<EPI, GROUPED>, maps, p);
 }
 

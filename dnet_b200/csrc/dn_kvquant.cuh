@@ -142,6 +142,8 @@ template <int BITS>
 __global__ void __launch_bounds__(32) k_kv_quant_append(const bf16* __restrict__ stage, unsigned char* __restrict__ layer_pool,
                                                         const int32_t* __restrict__ block_table, const StepState* __restrict__ st,
                                                         int n_kv) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x, kv = blockIdx.y / n_kv, kvh = blockIdx.y % n_kv, lane = threadIdx.x;
   const int pos = st->pos + t;
   float w[4], code[4], sc, bi;
