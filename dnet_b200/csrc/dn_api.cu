@@ -285,7 +285,16 @@ static cudaError_t init_kernel_attrs() {
 #define PRS(Gv) PRE((k_shard_step<Gv, MK_ATT_PLAIN>)) PRE((k_shard_step<Gv, MK_ATT_TC>)) PRE((k_shard_step<Gv, MK_ATT_Q8>)) PRE((k_shard_step<Gv, MK_ATT_Q4>))
   PRS(1) PRS(2) PRS(4) PRS(5) PRS(7) PRS(8)
 #undef PRS
+  // (single tokens and small chunks run on these; the GEMMs and attention kernels of larger ones are touched with their limits)
+  PRE(k_rmsnorm_rows) PRE(k_rope_append) PRE(k_kv_quant_append<8>) PRE(k_kv_quant_append<4>) PRE(k_moe_route) PRE(k_moe_join) PRE(k_moe_plan) PRE(k_moe_gather<bf16>)
+#define PRR(E) PRE((k_rows<E, 1, 4>)) PRE((k_rows<E, 1, 8>)) PRE((k_rows<E, 2, 4>)) PRE((k_rows<E, 2, 8>))
+  PRR(EPI_STORE) PRR(EPI_RESID)
+#undef PRR
+  PRE((k_rows<EPI_SWIGLU, 1, 4>)) PRE((k_rows<EPI_SWIGLU, 2, 4>)) PRE((k_rows<EPI_SWIGLU, 1, 4, true>)) PRE((k_rows<EPI_STORE, 1, 4, true>)) PRE((k_rows<EPI_STORE, 1, 8, true>))
 #undef PRE
+#define GEA(E, Gr) if ((e = cudaFuncSetAttribute(k_gemm_tc<E, Gr>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)) != cudaSuccess) return e;
+  GEA(EPI_STORE, false) GEA(EPI_RESID, false) GEA(EPI_SWIGLU, false) GEA(EPI_STORE, true) GEA(EPI_SWIGLU, true)
+#undef GEA
 #define ATA(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
   ATA(1) ATA(2) ATA(4) ATA(5) ATA(7) ATA(8)
 #undef ATA
