@@ -997,8 +997,8 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   return DN_OK;
 }
 
-// The kernels of a chunk: the prompt's, single tokens included (Llama-8B sizes behind 256: 99 us against 107 of the row kernels, which form the
-// norm and the rotation in their products' launches; behind 8,000 8-bit tokens 218 against 1,650, Mixtral-8x7B sizes 181 against 236).
+// The kernels of a chunk: the prompt's, single tokens included (calls timed with their copies: Llama-8B sizes behind 256 130 us against 134 of the row
+// kernels, which form the norm and the rotation in their products' launches, Qwen-32B sizes 218 / 222; behind 8,000 8-bit tokens 218 against 1,650, Mixtral-8x7B sizes 181 against 236).
 static bool use_prompt_kernels(const dn_model* m, int T) { return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.n_experts == 0 || m->moe_tc_ok); }
 static int one_layer(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
   m->pf_last = use_prompt_kernels(m, T);
