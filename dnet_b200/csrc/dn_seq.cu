@@ -1192,9 +1192,11 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
   };
 #define PH(id) CK(mark(m, id, s))
   PH(DN_SEQ_PH_EMBED);
-  CK(launch(W % 4 == 0 ? k_embed<T, 4> : k_embed<T, 1>, dim3(N, (W + (W % 4 == 0 ? 511 : 127)) / (W % 4 == 0 ? 512 : 128)), dim3(128), 0, s, (const T*)m->embed, b, c.embed_scale, W, S1, m->xs, mwp(DN_SQ_EMBED_NORM), mwp(DN_SQ_EMBED_NORM_B),
-            c.embed_norm ? mwp(DN_SQ_EMBED_NORM_ALPHA) : (const T*)nullptr, m->x0, pre ? (T*)nullptr : (T*)m->h,
-            c.bigram_buckets > 0 ? mwp(DN_SQ_BIGRAM) : (const T*)nullptr, c.max_positions > 0 ? mwp(DN_SQ_POS) : (const T*)nullptr));
+  // (a tensor may lie at any address: rows that do not start on four columns are read a number at a time)
+  const T *bigram = c.bigram_buckets > 0 ? mwp(DN_SQ_BIGRAM) : nullptr, *ptab = c.max_positions > 0 ? mwp(DN_SQ_POS) : nullptr;
+  const bool embed4 = W % 4 == 0 && (((uintptr_t)m->embed | (uintptr_t)bigram | (uintptr_t)ptab) & (4 * sizeof(T) - 1)) == 0;
+  CK(launch(embed4 ? k_embed<T, 4> : k_embed<T, 1>, dim3(N, (W + (embed4 ? 511 : 127)) / (embed4 ? 512 : 128)), dim3(128), 0, s, (const T*)m->embed, b, c.embed_scale, W, S1, m->xs,
+            mwp(DN_SQ_EMBED_NORM), mwp(DN_SQ_EMBED_NORM_B), c.embed_norm ? mwp(DN_SQ_EMBED_NORM_ALPHA) : (const T*)nullptr, m->x0, pre ? (T*)nullptr : (T*)m->h, bigram, ptab));
   // the norm before a sublayer and, where the model has them, the sublayer's input convolution with its carried rows
   auto norm_in = [&](SeqLayer& l, const Run& run, int q) -> int {
     auto w = [&](int i) { return (const T*)l.w[i]; };

@@ -180,7 +180,8 @@ struct Batch {
 // embedding -> residual streams
 // nalpha != null: the embedding is dynamic-tanh normed; x0 != null: it is also kept aside (the loop's injection reads it);
 // hout != null: also in the products' number format (models whose sublayers read the residual without a norm)
-// A thread takes four columns (VEC 4: W a multiple of 4) and gridDim.y blocks share a row: every load of a row is in flight at once.
+// A thread takes four columns (VEC 4: W a multiple of 4 and all tables on boundaries of four numbers) and gridDim.y blocks share a row: every
+// load of a row is in flight at once.
 // (One block of 128 threads a row, a number at a time: 21 us for four rows of 4,096 into four streams; now 2.5.)
 template <class T, int VEC>
 __global__ void k_embed(const T* __restrict__ embed, Batch b, float scale, int W, int S1, float* __restrict__ xs, const T* __restrict__ nw,

@@ -1,0 +1,44 @@
+"""-m gpu: layer-list models whose tensors lie at any address.  A checkpoint's tensors may be views into one flat buffer, where a scalar
+in front leaves the next one on an odd element: the kernels then read them a number at a time, with the same results."""
+import pytest
+import torch
+
+from tests import test_gpu_bokenex as bokenex
+from tests import test_gpu_vulanex as vulanex
+
+pytestmark = pytest.mark.gpu
+
+
+def at_an_odd_element(t: torch.Tensor) -> torch.Tensor:
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:] = t.reshape(-1)
+    return flat[1:].view(t.shape)
+
+
+def move(model, names):
+    model.load_weights({k: at_an_odd_element(model._bound[k]) for k in names})
+    torch.cuda.synchronize()      # (the copies ran on torch's stream, the steps run on the engine's)
+
+
+def logits(rig, tokens):
+    """a prompt and a few single tokens behind it"""
+    out = rig.eng.step([("r", tokens[:40], list(range(40)))])
+    for t in tokens[40:]:
+        out = torch.cat([out, rig.eng.step([("r", [t], [0])])])
+    rig.eng.finish("r")
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("family,names", [(bokenex, ["embed"]), (bokenex, ["pos"]), (vulanex, ["embed"]), (vulanex, ["bigram"])])
+def test_embedding_tables(cuda_lib, family, names, dtype):
+    """the token, position and bigram tables: sums of single numbers, so the streams are the same bit for bit; a head that is the embedding
+    table itself goes to another kernel, whose fp32 sums of 48 terms run in another order (48 x 2^-24 of the largest, and as much again)"""
+    tokens = family.toks(44)
+    with family.Rig(family.FULL, dtype) as rig:
+        here = logits(rig, tokens)
+        move(rig.model, names)
+        there = logits(rig, tokens)
+    assert torch.isfinite(there).all()
+    assert float((here - there).abs().max()) <= 2 * 48 * 2.0 ** -24 * float(here.abs().max())
