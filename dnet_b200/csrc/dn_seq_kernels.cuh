@@ -1361,6 +1361,7 @@ __global__ void __launch_bounds__(512) k_attn_prep(AttnPrep a, Batch b, const T*
     }
   } else if (vec && (a.dk & 3) == 0) {      // pairs (2i, 2i+1), two of them a thread
     const int hr = a.dk / 4;
+    const bool nvec = (((uintptr_t)nq | (uintptr_t)nk) & (4 * sizeof(T) - 1)) == 0;      // (norm weights may lie at any address)
     for (int e = threadIdx.x; e < HG * hr; e += blockDim.x) {
       const int hh = e / hr, d = 4 * (e - hh * hr);
       const bool isq = hh < a.H;
@@ -1368,7 +1369,11 @@ __global__ void __launch_bounds__(512) k_attn_prep(AttnPrep a, Batch b, const T*
       float x[4], w[4];
       ld4((isq ? qs : ks) + c, x);
       if (a.norm) {
-        ld4((isq ? nq : nk) + (a.norm == 1 ? c : d), w);
+        const T* wp = (isq ? nq : nk) + (a.norm == 1 ? c : d);
+        if (nvec) ld4(wp, w);
+        else
+#pragma unroll
+          for (int i = 0; i < 4; i++) w[i] = ldf(wp + i);
         const float rr = a.norm == 1 ? (isq ? rq : rk) : hinv[hh];
 #pragma unroll
         for (int i = 0; i < 4; i++) x[i] = x[i] * rr * w[i];

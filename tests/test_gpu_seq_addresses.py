@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from tests import test_gpu_bokenex as bokenex
+from tests import test_gpu_seqmix as moputar
 from tests import test_gpu_vulanex as vulanex
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +43,22 @@ def test_embedding_tables(cuda_lib, family, names, dtype):
         there = logits(rig, tokens)
     assert torch.isfinite(there).all()
     assert float((here - there).abs().max()) <= 2 * 48 * 2.0 ** -24 * float(here.abs().max())
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("family", [moputar, bokenex, vulanex])
+def test_query_and_key_norms(family, dtype):
+    """weights of the q / k norms behind convolutions and rotations (over the whole projection and per head): products of single numbers,
+    the same bit for bit, as the heads' kernels and the blocks' form them"""
+    tokens = family.toks(44)
+    with family.Rig(family.FULL, dtype) as rig:
+        here = logits(rig, tokens)
+        names = [k for k in rig.model._bound if k.endswith((".q.norm", ".k.norm"))]
+        assert names
+        move(rig.model, names)
+        there = logits(rig, tokens)
+    assert torch.isfinite(there).all()
+    if family is moputar:
+        assert torch.equal(here, there)
+    else:      # (the kernel of single heads asks for aligned weights: another one forms the sums of squares in another order)
+        assert family.err(there, here.cpu()) <= family.TOL[dtype]
