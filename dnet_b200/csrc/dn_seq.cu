@@ -1433,8 +1433,9 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       T* pool = (T*)m->kpool[run.kv_index];
       CK(launch(k_latent_prep<T>, dim3(N), dim3(256), 0, s, a, b, (const T*)m->uq, (const T*)m->uk, w(DN_SQ_DKV_NORM), (T*)m->qb, pool));
       // the unrotated query parts into the latent space: qb[n, h, 0:R] = W_uk,h^T q[n, h, 0:dim]
-      // (all strides multiples of 8 numbers: 16-byte operand rows for the MMA form)
-      const bool heads_mma = std::is_same<T, bf16>::value && N >= 16 && dq % 8 == 0 && lc.dim % 8 == 0 && R % 8 == 0 && dr % 8 == 0 && lc.vdim % 8 == 0;
+      // (all strides multiples of 8 numbers and matrices on 16-byte boundaries: 16-byte operand rows for the MMA form)
+      const bool heads_mma = std::is_same<T, bf16>::value && N >= 16 && dq % 8 == 0 && lc.dim % 8 == 0 && R % 8 == 0 && dr % 8 == 0 && lc.vdim % 8 == 0 &&
+                             (((uintptr_t)l.w[DN_SQ_UK] | (uintptr_t)l.w[DN_SQ_UV]) & 15) == 0;
       if (few && (size_t)N * lc.dim * 4 <= 40 * 1024)
         CK(launch(k_absorb_few<T>, dim3((R + 31) / 32, lc.heads), dim3(128), (size_t)(N * lc.dim + 4 * 8 * 32) * 4, s, (const T*)m->uq, w(DN_SQ_UK), (T*)m->qb, N, lc.heads,
                   lc.dim, dq, R, l.Ck));

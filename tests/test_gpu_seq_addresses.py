@@ -1,13 +1,21 @@
 """-m gpu: layer-list models whose tensors lie at any address.  A checkpoint's tensors may be views into one flat buffer, where a scalar
 in front leaves the next one on an odd element: the kernels then read them a number at a time, with the same results."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 from tests import test_gpu_bokenex as bokenex
+from tests import test_gpu_filinex as filinex
+from tests import test_gpu_lutesun as lutesun
 from tests import test_gpu_seqmix as moputar
+from tests import test_gpu_tuguvik as tuguvik
 from tests import test_gpu_vulanex as vulanex
 
 pytestmark = pytest.mark.gpu
+
+# latent attention with head sizes of the tensor-core products between heads and latent space, no routers
+lutesun_dense = SimpleNamespace(**{**vars(lutesun), "FULL": lutesun.config([lutesun.lat(lutesun.DENSE), lutesun.lat(None, heads=2, dim=8, kv_rank=24)])})
 
 
 def at_an_odd_element(t: torch.Tensor) -> torch.Tensor:
@@ -62,3 +70,17 @@ def test_query_and_key_norms(family, dtype):
         assert torch.equal(here, there)
     else:      # (the kernel of single heads asks for aligned weights: another one forms the sums of squares in another order)
         assert family.err(there, here.cpu()) <= family.TOL[dtype]
+
+
+@pytest.mark.parametrize("family,dtype", [(f, "float32") for f in (bokenex, filinex, lutesun, moputar, tuguvik, vulanex)] +
+                         [(f, "bfloat16") for f in (moputar, tuguvik, vulanex)] + [(lutesun_dense, "bfloat16")])
+def test_every_tensor(family, dtype):
+    """all tensors on odd elements against the same ones where they were: no operand may go to TMA or to wide loads, so the products' sums
+    run in another order (the bound of the families' own tests; 16-bit models without routers, whose choices could tip)"""
+    tokens = family.toks(44)
+    with family.Rig(family.FULL, dtype) as rig:
+        here = logits(rig, tokens)
+        move(rig.model, list(rig.model._bound))
+        there = logits(rig, tokens)
+    assert torch.isfinite(there).all()
+    assert family.err(there, here.cpu()) <= family.TOL[dtype]
