@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   tc_fence_before();
   __syncthreads();
+  if (Z > 1) cluster_sync();      // every CTA of the cluster has started: the first walk's end stores into the others' memory
   tc_fence_after();
   const uint32_t tmem = *tmem_slot, tP = tmem + 256, tO = tmem + 320;      // S in two buffers of 128 columns
 
