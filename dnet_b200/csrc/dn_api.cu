@@ -295,8 +295,8 @@ static cudaError_t init_kernel_attrs() {
 #define GEA(E, Gr) if ((e = cudaFuncSetAttribute(k_gemm_tc<E, Gr>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)) != cudaSuccess) return e;
   GEA(EPI_STORE, false) GEA(EPI_RESID, false) GEA(EPI_SWIGLU, false) GEA(EPI_STORE, true) GEA(EPI_SWIGLU, true)
 #undef GEA
-#define ATA(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
-  ATA(1) ATA(2) ATA(4) ATA(5) ATA(7) ATA(8)
+#define ATA(Gv, Pv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv, Pv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
+  ATA(1, 2) ATA(2, 2) ATA(4, 2) ATA(8, 2) ATA(1, 3) ATA(2, 3) ATA(4, 3) ATA(5, 3) ATA(7, 3) ATA(8, 3)
 #undef ATA
 #define ATQ(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess || \
                     (e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess) return e;
@@ -962,8 +962,10 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
     // (how the keys are shared out only decides the order of the sums; the kernel reads the position from the step state)
     const int Z = attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms);
-#define PFT(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_tc<Gv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
-    switch (m->G) { PFT(1) PFT(2) PFT(4) PFT(5) PFT(7) PFT(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
+#define PFT(Gv, Pv) CK(launch_attn_tc(k_attn_prefill_tc<Gv, Pv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
+#define PFT2(Gv) case Gv: if (T < AT_TWO_PARTS_FROM) { PFT(Gv, 3) } else { PFT(Gv, 2) }
+    switch (m->G) { PFT2(1) PFT2(2) PFT2(4) PFT2(8) case 5: PFT(5, 3) case 7: PFT(7, 3) default: return fail(DN_EINVAL, "GQA group unsupported"); }
+#undef PFT2
 #undef PFT
   } else {
     dim3 grid(c.n_kv_heads, (T + 3) / 4);

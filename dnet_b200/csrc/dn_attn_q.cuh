@@ -27,14 +27,6 @@ constexpr int AQT_THREADS = 512, AQT_DQ = 256;
 constexpr int AQT_XCH = (4 * 128 * 2 + 128 * 2 + AT_MAX_Z * 2 * 128) * 4;      // key biases of four tiles, value biases, the ranks' maxima and sums
 constexpr int AQT_SMEM = 5 * AT_TILE + AQT_XCH + 1024 + 256;
 
-__device__ __forceinline__ void tm_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
 template <int G, int BITS>
 __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParams pq) {
   pdl_launch_dependents();
