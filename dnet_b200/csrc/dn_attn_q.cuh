@@ -3,16 +3,20 @@
 //
 // Rows, blocks and the cluster's share of the keys are those of k_attn_prefill_tc (dn_attn_tc.cuh).  The semantics round scores and
 // probabilities to bf16, which an online softmax cannot reproduce: the key tiles are walked twice, first for every row's maximum and
-// sum, then for the probabilities and the output.  Eight warps turn a tile's codes into operands: scale x code has at most 16 mantissa
-// bits, so a pair of bf16 (hi, lo) holds it exactly, and with exact products and fp32 accumulators
-//   s = Q' (hi + lo)^T + bias_0 sum(q'_0) + bias_1 sum(q'_1)      (two groups of 64 dims; the bias terms in fp32 by the row's thread)
-//   o = P (hi + lo) + (sum_j p_j bias_0j, sum_j p_j bias_1j)      (P is bf16 by definition)
-// are the sums that the CUDA-core kernel (k_attn_q) forms, in another order.
+// sum, then for the probabilities and the output.  Rounded numbers land on the other side of an edge by as little as their sums are off, so that
+// the sums are kept as short and as small as the format allows.  With codes less the middle of their range (c' = c - 128 or c - 8, exact in bf16)
+// and b' = bias + middle x scale,
+//   s = scale_0 (Q'_0 c'_0) + scale_1 (Q'_1 c'_1) + b'_0 sum(q'_0) + b'_1 sum(q'_1)      (two groups of 64 dims: an accumulator each, four products
+//       long; scales and biases in fp32 by the row's thread)
+//   o = sum over tiles of P (hi + lo) + (sum_j p_j b'_0j, sum_j p_j b'_1j)      (scale x c' has at most 16 mantissa bits: hi + lo holds it exactly; P is
+//       bf16 by definition; a tile's product and its bias terms join fp32 sums of the row's thread)
+// Eight warps turn a tile's codes into operands.
 //
-// Bound by the tensor cores and the dequantising warps alike: a tile of 128 keys takes 1,024 cycles of products in the first walk and
-// 2,048 in the second, beside 640 and 1,280 cycles of conversion.  A block per (head, token) on the CUDA cores read every key row once
-// per query instead: 777 tokens behind 1,024 of a Llama-3-8B layer took 4.1 ms.
-// Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-7 softmax (a thread a row), warps 8-15 dequantisation.
+// Bound by the softmax warps, a row's thread of which forms every score twice, beside the conversion.  777 tokens behind 1,024 (8 x 4 heads, 8 bits):
+// 247 us; one token behind 8,000 84 us.  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
+// tiles: 240 and 82.  Of the stored results 1.56 % and 2.64 % then were not the nearest to 64 bits; now 0.19 % and 0.17 %; k_attn_q, whose
+// block per (head, token) takes 4.1 ms and 1.4 ms, 0.26 % and 0.66 %.)
+// Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-7 softmax (a thread a row), warps 8-15 conversion.
 #pragma once
 #include "dn_attn_tc.cuh"
 #include "dn_kvquant.cuh"
@@ -24,25 +28,47 @@ struct AqParams {
   const unsigned char* pool;     // this layer's packed pages
 };
 constexpr int AQT_THREADS = 512, AQT_DQ = 256;
-constexpr int AQT_XCH = (4 * 128 * 2 + 128 * 2 + AT_MAX_Z * 2 * 128) * 4;      // key biases of four tiles, value biases, the ranks' maxima and sums
+constexpr int AQT_KB = 4 * 128;      // floats of a key tile: scales of both groups, biases of both groups
+constexpr int AQT_XCH = (4 * AQT_KB + 128 * 2 + AT_MAX_Z * 2 * 128) * 4;      // four key tiles' scales and biases, value biases, the ranks' maxima and sums
 constexpr int AQT_SMEM = 5 * AT_TILE + AQT_XCH + 1024 + 256;
+constexpr int AQT_REGS_MMA = 64, AQT_REGS_SOFTMAX = 224, AQT_REGS_DQ = 112;      // setmaxnreg: of the 128 a thread that 512 threads are launched with
+static_assert(128 * (AQT_REGS_MMA + AQT_REGS_SOFTMAX + 2 * AQT_REGS_DQ) <= AQT_THREADS * 128, "setmaxnreg split exceeds the CTA's launch allocation");
+
+// 16 (8) consecutive 32-bit columns of this warp's TMEM quarter
+__device__ __forceinline__ void tm_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tm_pin16(uint32_t (&r)[16]) {      // no use of r moves above this point
+#pragma unroll
+  for (int i = 0; i < 16; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
+}
+__device__ __forceinline__ void tm_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 
 template <int G, int BITS>
 __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParams pq) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int TB = 128 / G;
+  constexpr float MID = (float)(1 << (BITS - 1));      // what is taken off the codes
   const AtParams& p = pq.a;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  unsigned char *sQ = smem, *sK = smem + AT_TILE, *sV = smem + 3 * AT_TILE;      // K, V: hi tile, lo tile
-  float2* kb = reinterpret_cast<float2*>(smem + 5 * AT_TILE);                    // [4][128]: (bias of group 0, of group 1) of a key row
-  float2* vb = kb + 4 * 128;                                                     // [128]
+  unsigned char *sQ = smem, *sK = smem + AT_TILE, *sV = smem + 3 * AT_TILE;      // K: two tiles in turn; V: hi tile, lo tile
+  float* kb = reinterpret_cast<float*>(smem + 5 * AT_TILE);                      // [4][scale 0, scale 1, bias 0, bias 1][128 keys]
+  float2* vb = reinterpret_cast<float2*>(kb + 4 * AQT_KB);                       // [128]: (bias of group 0, of group 1) of a value row
   float* zx = reinterpret_cast<float*>(vb + 128);                                // [Z][2][128]
   float* zo = reinterpret_cast<float*>(sK);                                      // [Z][128 / Z][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 5 * AT_TILE + AQT_XCH);
-  uint64_t *k_full = bars, *k_empty = bars + 1, *v_full = bars + 2, *v_empty = bars + 3, *s_full = bars + 4, *s_empty = bars + 6, *p_full = bars + 8, *o_full = bars + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 5, *s_full = bars + 6, *s_empty = bars + 8, *p_full = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x, t0 = blockIdx.y * TB, Z = gridDim.z, z = blockIdx.z;
@@ -53,9 +79,8 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   const int j0 = (int)((long long)all * z / Z), n_tiles = (int)((long long)all * (z + 1) / Z) - j0;
 
   if (threadIdx.x == 0) {
-    mbar_init(k_full, AQT_DQ / 32); mbar_init(k_empty, 1); mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
-    mbar_init(p_full, 4); mbar_init(o_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], AQT_DQ / 32); mbar_init(&k_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
+    mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1); mbar_init(p_full, 4);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -79,153 +104,142 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   __syncthreads();
   if (Z > 1) cluster_sync();      // every CTA of the cluster has started: the first walk's end stores into the others' memory
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot, tP = tmem + 256, tO = tmem + 320;      // S in two buffers of 128 columns
+  // S: two halves of a tile in turn, each 64 keys of group 0, then of group 1; P; the tile's product
+  const uint32_t tmem = *tmem_slot, tP = tmem + 256, tO = tmem + 320;
 
-  const uint32_t idesc_s = tc_instr_desc(128, 128), idesc_o = tc_instr_desc(128, 128) | (1u << 16);
-  // ---- S of the it-th tile of both walks
-  auto scores = [&](int it) {
-    mbar_wait(k_full, (uint32_t)it & 1u, p.err);
-    mbar_wait(&s_empty[it & 1], ((uint32_t)(it >> 1) & 1u) ^ 1u, p.err);
-    tc_fence_after();
-#pragma unroll
-    for (int part = 0; part < 2; ++part)
+  if (warp < 4) {
+    // ===================== products =====================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AQT_REGS_MMA));
+    const uint32_t idesc_s = tc_instr_desc(128, 64), idesc_o = tc_instr_desc(128, 128) | (1u << 16);
+    auto scores = [&](int it) {      // of the it-th tile of both walks
+      const int kbuf = it & 1;
+      mbar_wait(&k_full[kbuf], (uint32_t)(it >> 1) & 1u, p.err);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint64_t adesc = tc_smem_desc(sQ + h * 16384), bdesc = tc_smem_desc(sK + part * AT_TILE + h * 16384);
+        mbar_wait(&s_empty[h], ((uint32_t)it & 1u) ^ 1u, p.err);
+        tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < 4; ++k) tc_mma(tmem + (it & 1) * 128, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_s, (part | h | k) ? 1u : 0u);
-      }
-    tc_commit(k_empty);
-    tc_commit(&s_full[it & 1]);
-  };
-  // ---- one tile's codes into operands.  kv 0: keys, 1: values
-  const int dt = (int)threadIdx.x - (AQT_THREADS - AQT_DQ);
-  auto dequant = [&](int j, int kv, unsigned char* dst, float2* bias, uint64_t* empty, uint32_t phase, uint64_t* full) {
-    constexpr int CH = KvQ<BITS>::ROW_BYTES / 16, PER = 128 * CH / AQT_DQ;      // 16-byte chunks of a row, of a thread
-    constexpr int CODES = 128 / BITS;                                           // codes of a chunk: 16 / 32
-    const int key0 = (j0 + j) << 7, pl = 2 * (j0 + j);
-    const int pg0 = p.block_table[pl], pg1 = pl + 1 < pages ? p.block_table[pl + 1] : pg0;
-    uint4 cw[PER];
-    float sc[PER];
-    float2 bv = make_float2(0.f, 0.f);
+        for (int g = 0; g < 2; ++g) {
+          const uint64_t adesc = tc_smem_desc(sQ + g * 16384), bdesc = tc_smem_desc(sK + kbuf * AT_TILE + g * 16384 + h * 8192);
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
-      const unsigned char* unit = kvq_unit<BITS>(pq.pool, row < 64 ? pg0 : pg1, kv, kvh, p.n_kv);
-      const unsigned short* s = reinterpret_cast<const unsigned short*>(unit + KvQ<BITS>::CODES_BYTES);
-      const bool live = key0 + row < kv_max;      // rows that belong to no key: whatever the page holds, it must not enter
-      cw[i] = live ? __ldcg(reinterpret_cast<const uint4*>(unit + (size_t)(row & 63) * KvQ<BITS>::ROW_BYTES) + c) : make_uint4(0u, 0u, 0u, 0u);
-      sc[i] = live ? __uint_as_float((uint32_t)__ldcg(s + (row & 63) * 2 + (c * CODES >= 64 ? 1 : 0)) << 16) : 0.f;
-    }
-    if (dt < 128 && key0 + dt < kv_max) {
-      const unsigned char* unit = kvq_unit<BITS>(pq.pool, dt < 64 ? pg0 : pg1, kv, kvh, p.n_kv);
-      const uint32_t b = __ldcg(reinterpret_cast<const uint32_t*>(unit + KvQ<BITS>::CODES_BYTES + PAGE * 4) + (dt & 63));
-      bv = make_float2(bf_lo(b), bf_hi(b));
-    }
-    mbar_wait(empty, phase, p.err);
-    if (dt < 128) bias[dt] = bv;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
-      const uint32_t u[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
-#pragma unroll
-      for (int o = 0; o < CODES / 8; ++o) {       // eight codes: one 16-byte chunk of each tile
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float a, b;
-          if (BITS == 8) {
-            const uint32_t w = u[(o * 2 + (k >> 1)) & 3] >> (16 * (k & 1));
-            a = (float)(w & 0xffu); b = (float)((w >> 8) & 0xffu);
-          } else {
-            const uint32_t w = u[o & 3] >> (8 * k);
-            a = (float)(w & 0xfu); b = (float)((w >> 4) & 0xfu);
-          }
-          a *= sc[i]; b *= sc[i];
-          hi[k] = pack_bf16x2(a, b);
-          lo[k] = pack_bf16x2(a - __uint_as_float(hi[k] << 16), b - __uint_as_float(hi[k] & 0xffff0000u));
+          for (int k = 0; k < 4; ++k) tc_mma(tmem + h * 128 + g * 64, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_s, k ? 1u : 0u);
         }
-        const uint32_t at = at_swz(row, c * (CODES / 8) + o);
-        *reinterpret_cast<uint4*>(dst + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(dst + AT_TILE + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        if (h == 1) tc_commit(&k_empty[kbuf]);
+        tc_commit(&s_full[h]);
+      }
+    };
+    if (warp == 0 && lane == 0)
+      for (int j = 0; j < n_tiles; ++j) scores(j);
+    __syncwarp();
+    if (Z > 1) cluster_sync();
+    if (warp == 0 && lane == 0) {
+      if (n_tiles > 0) scores(n_tiles);
+      for (int j = 0; j < n_tiles; ++j) {
+        if (j + 1 < n_tiles) scores(n_tiles + j + 1);
+        mbar_wait(v_full, (uint32_t)j & 1u, p.err);
+        mbar_wait(p_full, (uint32_t)j & 1u, p.err);
+        tc_fence_after();
+#pragma unroll
+        for (int part = 1; part >= 0; --part) {      // the small part first: fewer sums are cut at the size of the result
+          const uint64_t vdesc = tc_smem_desc_mn(sV + part * AT_TILE, 16384, 1024);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            tc_mma_ts(tO, tP + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (part == 0 || kk) ? 1u : 0u);
+        }
+        tc_commit(v_empty);
       }
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if (lane == 0) mbar_arrive(full);
-  };
-
-  const int qd = warp & 3, r = qd * 32 + lane;      // softmax: TMEM lane quarter, this thread's row
-  const int rg = r / TB, rt = r % TB;
-  const bool ok = rg < G && rt < nq;
-  const int last = ok ? pos0 + t0 + rt : -1;        // last visible key position
-  const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-  float sq0 = 0.f, sq1 = 0.f, m = -INFINITY, l = 0.f, ob0 = 0.f, ob1 = 0.f;
-  const bool smx = warp >= 4 && warp < 8;
-  if (smx) {
+    if (Z > 1) { cluster_sync(); cluster_sync(); }
+  } else if (warp < 8) {
+    // ===================== softmax, a thread a row =====================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AQT_REGS_SOFTMAX));
+    const int qd = warp & 3, r = qd * 32 + lane;      // TMEM lane quarter, this thread's row
+    const int rg = r / TB, rt = r % TB;
+    const bool ok = rg < G && rt < nq;
+    const int last = ok ? pos0 + t0 + rt : -1;        // last visible key position
+    const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+    float sq0 = 0.f, sq1 = 0.f, m = -INFINITY, l = 0.f, ob0 = 0.f, ob1 = 0.f;
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
       const uint4 v = *reinterpret_cast<const uint4*>(sQ + at_swz(r, c));
       const float f = ((bf_lo(v.x) + bf_hi(v.x)) + (bf_lo(v.y) + bf_hi(v.y))) + ((bf_lo(v.z) + bf_hi(v.z)) + (bf_lo(v.w) + bf_hi(v.w)));
       if (c < 8) sq0 += f; else sq1 += f;
     }
-  }
-  // 32 scores of this row from column c on, rounded to bf16; keys that the row does not see: -inf
-  auto load_scores = [&](int it, int j, int c, float (&s)[32]) {
-    uint32_t v[32];
-    tm_ld32(tmem + (it & 1) * 128 + lane_off + c, v);
-    tm_wait_ld();
-    tm_pin(v);
-    const float4* b4 = reinterpret_cast<const float4*>(kb + (it & 3) * 128 + c);
-    const int key = ((j0 + j) << 7) + c;
+    // Sixteen keys of a half tile at a time: ask for the products of both groups, and, behind tm_wait_ld, the scores rounded to bf16; keys that the
+    // row does not see: -inf.  it, j: the tile, h: its half, c: 0, 16, 32 or 48
+    auto ask = [&](int h, int c, uint32_t (&a)[16], uint32_t (&b)[16]) {
+      tm_ld16(tmem + h * 128 + lane_off + c, a);
+      tm_ld16(tmem + h * 128 + 64 + lane_off + c, b);
+    };
+    auto scores_of = [&](int it, int j, int h, int c, uint32_t (&a)[16], uint32_t (&b)[16], float2 (&s)[8]) {
+      tm_pin16(a);
+      tm_pin16(b);
+      const float4* kf = reinterpret_cast<const float4*>(kb + (it & 3) * AQT_KB + h * 64 + c);
+      const int key = ((j0 + j) << 7) + h * 64 + c;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float4 b = b4[i];
-      s[2 * i] = key + 2 * i <= last ? bf16r(fmaf(b.y, sq1, fmaf(b.x, sq0, __uint_as_float(v[2 * i])))) : -INFINITY;
-      s[2 * i + 1] = key + 2 * i + 1 <= last ? bf16r(fmaf(b.w, sq1, fmaf(b.z, sq0, __uint_as_float(v[2 * i + 1])))) : -INFINITY;
-    }
-  };
-
-  // ===================== first walk: maxima and sums =====================
-  if (warp == 0) {
-    if (lane == 0)
-      for (int j = 0; j < n_tiles; ++j) scores(j);
-  } else if (smx) {
-    for (int j = 0; j < n_tiles; ++j) {
-      // (the key biases were written before the products that these barriers count were issued; their places are used again four tiles later)
-      mbar_wait(&s_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err);
-      __syncwarp();
-      tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < 128; c += 32) {
-        float s[32], mx = m;
-        load_scores(j, j, c, s);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
-        const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
-        float a = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) a += tc_ex2((s[i] - at) * LOG2E);
-        l = fmaf(l, tc_ex2((m - at) * LOG2E), a);
-        m = mx;
+      for (int i = 0; i < 4; ++i) {
+        const float4 s0 = kf[i], s1 = kf[32 + i], b0 = kf[64 + i], b1 = kf[96 + i];
+        auto two = [&](int e, float2 c0, float2 c1, float2 d0, float2 d1) {
+          const float2 x = f2_fma(make_float2(__uint_as_float(a[e]), __uint_as_float(a[e + 1])), c0,
+                                  f2_fma(make_float2(__uint_as_float(b[e]), __uint_as_float(b[e + 1])), c1, f2_fma(d0, f2_of(sq0), f2_mul(d1, f2_of(sq1)))));
+          const uint32_t w = pack_bf16x2(x.x, x.y);
+          s[e / 2] = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+        };
+        two(4 * i, make_float2(s0.x, s0.y), make_float2(s1.x, s1.y), make_float2(b0.x, b0.y), make_float2(b1.x, b1.y));
+        two(4 * i + 2, make_float2(s0.z, s0.w), make_float2(s1.z, s1.w), make_float2(b0.z, b0.w), make_float2(b1.z, b1.w));
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[j & 1]);
+      if (!__all_sync(0xffffffffu, !ok || key + 15 <= last)) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (key + 2 * i > last) s[i].x = -INFINITY;
+          if (key + 2 * i + 1 > last) s[i].y = -INFINITY;
+        }
+      }
+    };
+    // ---- first walk: maxima and sums
+    for (int j = 0; j < n_tiles; ++j) {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        // (the key scales were written before the products that these barriers count were issued; their places are used again four tiles later)
+        mbar_wait(&s_full[h], (uint32_t)j & 1u, p.err);
+        __syncwarp();
+        tc_fence_after();
+        uint32_t a[2][16], b[2][16];
+        ask(h, 0, a[0], b[0]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float2 s[8];
+          tm_wait_ld();
+          if (c < 3) ask(h, 16 * c + 16, a[(c + 1) & 1], b[(c + 1) & 1]);
+          scores_of(j, j, h, 16 * c, a[c & 1], b[c & 1], s);
+          float2 x2 = s[0];
+#pragma unroll
+          for (int i = 1; i < 8; ++i) x2 = make_float2(fmaxf(x2.x, s[i].x), fmaxf(x2.y, s[i].y));
+          const float mx = fmaxf(m, fmaxf(x2.x, x2.y));
+          const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
+          float2 e2 = f2_of(0.f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float2 x = f2_mul(f2_add(s[i], f2_of(-at)), f2_of(LOG2E));
+            e2 = f2_add(e2, make_float2(tc_ex2(x.x), tc_ex2(x.y)));
+          }
+          l = fmaf(l, tc_ex2((m - at) * LOG2E), e2.x + e2.y);
+          m = mx;
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[h]);
+      }
     }
-  } else if (warp >= 8) {
-    for (int j = 0; j < n_tiles; ++j) dequant(j, 0, sK, kb + (j & 3) * 128, k_empty, ((uint32_t)j & 1u) ^ 1u, k_full);
-  }
-  if (Z > 1) {      // the other ranks' keys count too
-    __syncwarp();
-    if (smx)
+    if (Z > 1) {      // the other ranks' keys count too
+      __syncwarp();
       for (int d = 0; d < Z; ++d) {
         dsmem_st(dsmem_addr(zx + z * 256 + r, (uint32_t)d), m);
         dsmem_st(dsmem_addr(zx + z * 256 + 128 + r, (uint32_t)d), l);
       }
-    __syncwarp();
-    cluster_sync();
-    if (smx) {
+      __syncwarp();
+      cluster_sync();
       float M = -INFINITY, L = 0.f;
       for (int d = 0; d < Z; ++d) M = fmaxf(M, zx[d * 256 + r]);
       for (int d = 0; d < Z; ++d) {
@@ -235,111 +249,197 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       m = M;
       l = L;
     }
-  }
-  // ===================== second walk: probabilities and output =====================
-  if (warp == 0) {
-    if (lane == 0) {
-      if (n_tiles > 0) scores(n_tiles);
-      for (int j = 0; j < n_tiles; ++j) {
-        if (j + 1 < n_tiles) scores(n_tiles + j + 1);
-        mbar_wait(v_full, (uint32_t)j & 1u, p.err);
-        mbar_wait(p_full, (uint32_t)j & 1u, p.err);
-        tc_fence_after();
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-          const uint64_t vdesc = tc_smem_desc_mn(sV + part * AT_TILE, 16384, 1024);
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            tc_mma_ts(tO, tP + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (j | part | kk) ? 1u : 0u);
-        }
-        tc_commit(v_empty);
-      }
-      tc_commit(o_full);
-    }
-  } else if (smx) {
+    // ---- second walk: probabilities and output
     const float inv = 1.0f / l;
-    for (int j = 0; j < n_tiles; ++j) {
-      const int it = n_tiles + j;
-      mbar_wait(&s_full[it & 1], (uint32_t)(it >> 1) & 1u, p.err);
-      mbar_wait(v_full, (uint32_t)j & 1u, p.err);             // the value biases are written
-      if (j > 0) mbar_wait(v_empty, (uint32_t)(j - 1) & 1u, p.err);      // the product before has read its probabilities
+    float o[128];
+#pragma unroll
+    for (int i = 0; i < 128; ++i) o[i] = 0.f;
+    auto join = [&](int j) {      // the j-th tile's product joins the row's sums
+      mbar_wait(v_empty, (uint32_t)j & 1u, p.err);
       __syncwarp();
       tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < 128; c += 32) {
-        float s[32];
-        load_scores(it, j, c, s);
-        const float4* b4 = reinterpret_cast<const float4*>(vb + c);
-        uint32_t w[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float a = ok ? tc_ex2((s[2 * i] - m) * LOG2E) * inv : 0.f, d = ok ? tc_ex2((s[2 * i + 1] - m) * LOG2E) * inv : 0.f;
-          w[i] = pack_bf16x2(a, d);
-          const float pa = __uint_as_float(w[i] << 16), pd = __uint_as_float(w[i] & 0xffff0000u);
-          const float4 b = b4[i];
-          ob0 = fmaf(pa, b.x, fmaf(pd, b.z, ob0));
-          ob1 = fmaf(pa, b.y, fmaf(pd, b.w, ob1));
-        }
-        tm_st16(tP + lane_off + c / 2, w);
+      for (int c = 0; c < 4; c += 2) {
+        uint32_t a[32], b[32];
+        tm_ld32(tO + lane_off + c * 32, a);
+        tm_ld32(tO + lane_off + c * 32 + 32, b);
+        tm_wait_ld();
+        tm_pin(a);
+        tm_pin(b);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) { o[c * 32 + i] += __uint_as_float(a[i]); o[c * 32 + 32 + i] += __uint_as_float(b[i]); }
       }
+    };
+    for (int j = 0; j < n_tiles; ++j) {
+      const int it = n_tiles + j;
+      if (j > 0) join(j - 1);      // (it has read its probabilities, too)
+      mbar_wait(v_full, (uint32_t)j & 1u, p.err);             // the value biases are written
+      float2 t0s = f2_of(0.f), t1s = t0s;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        mbar_wait(&s_full[h], (uint32_t)it & 1u, p.err);
+        __syncwarp();
+        tc_fence_after();
+        uint32_t a[2][16], b[2][16];
+        ask(h, 0, a[0], b[0]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float2 s[8];
+          tm_wait_ld();
+          if (c < 3) ask(h, 16 * c + 16, a[(c + 1) & 1], b[(c + 1) & 1]);
+          scores_of(it, j, h, 16 * c, a[c & 1], b[c & 1], s);
+          const float4* b4 = reinterpret_cast<const float4*>(vb + h * 64 + 16 * c);
+          uint32_t w[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float2 x = f2_mul(f2_add(s[i], f2_of(-m)), f2_of(LOG2E)), e = f2_mul(make_float2(tc_ex2(x.x), tc_ex2(x.y)), f2_of(inv));
+            w[i] = ok ? pack_bf16x2(e.x, e.y) : 0u;
+            const float pa = __uint_as_float(w[i] << 16), pd = __uint_as_float(w[i] & 0xffff0000u);
+            const float4 bv = b4[i];
+            t0s = f2_fma(f2_of(pa), make_float2(bv.x, bv.y), t0s);
+            t1s = f2_fma(f2_of(pd), make_float2(bv.z, bv.w), t1s);
+          }
+          tm_st8(tP + lane_off + h * 32 + 8 * c, w);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[h]);
+      }
+      ob0 += t0s.x + t1s.x;
+      ob1 += t0s.y + t1s.y;
       tm_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&s_empty[it & 1]); mbar_arrive(p_full); }
+      if (lane == 0) mbar_arrive(p_full);
     }
-    mbar_wait(o_full, 0u, p.err);
+    if (n_tiles > 0) join(n_tiles - 1);
+#pragma unroll
+    for (int i = 0; i < 128; ++i) o[i] += n_tiles > 0 ? (i < 64 ? ob0 : ob1) : 0.f;
     __syncwarp();
-    tc_fence_after();
-  } else if (warp >= 8) {
-    for (int j = 0; j < n_tiles; ++j) {
-      const int it = n_tiles + j;
-      dequant(j, 0, sK, kb + (it & 3) * 128, k_empty, ((uint32_t)it & 1u) ^ 1u, k_full);
-      dequant(j, 1, sV, vb, v_empty, ((uint32_t)j & 1u) ^ 1u, v_full);
-    }
-  }
-  __syncwarp();
-  if (Z > 1) cluster_sync();      // every rank's products are done: its key buffers may take the other ranks' columns
-  if (smx) {
-    const int per = 128 / Z;      // columns of a rank
-#pragma unroll 1
-    for (int c = 0; c < 128; c += 32) {
-      uint32_t o[32];
-      if (n_tiles > 0) tm_ld32(tO + lane_off + c, o);
-      tm_wait_ld();
-      tm_pin(o);
-      const float ob = c < 64 ? ob0 : ob1;
-      float y[32];
+    if (Z > 1) cluster_sync();      // every rank's products are done: its key buffers may take the other ranks' columns
+    const int per = 128 / Z, lg = 31 - __clz(per);      // columns of a rank: a power of two
+    if (Z > 1) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) y[i] = n_tiles > 0 ? __uint_as_float(o[i]) + ob : 0.f;
-      if (Z > 1) {
+      for (int i = 0; i < 128; ++i) dsmem_st(dsmem_addr(zo + (z * per + (i & (per - 1))) * 128 + r, (uint32_t)(i >> lg)), o[i]);
+      __syncwarp();
+      cluster_sync();
+      if (ok) {
+        bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + z * per;
+        for (int c = 0; c < per; c += 8) {
+          float y[8];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) dsmem_st(dsmem_addr(zo + ((size_t)z * per + (c + i) % per) * 128 + r, (uint32_t)((c + i) / per)), y[i]);
-      } else if (ok) {
-        bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + c;
+          for (int i = 0; i < 8; ++i) y[i] = 0.f;
+          for (int d = 0; d < Z; ++d)
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          *reinterpret_cast<uint4*>(dst + k * 8) = make_uint4(pack_bf16x2(y[8 * k], y[8 * k + 1]), pack_bf16x2(y[8 * k + 2], y[8 * k + 3]),
-                                                             pack_bf16x2(y[8 * k + 4], y[8 * k + 5]), pack_bf16x2(y[8 * k + 6], y[8 * k + 7]));
+            for (int i = 0; i < 8; ++i) y[i] += zo[((size_t)d * per + c + i) * 128 + r];
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]), pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
+        }
       }
+    } else if (ok) {
+      bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD;
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        *reinterpret_cast<uint4*>(dst + k * 8) = make_uint4(pack_bf16x2(o[8 * k], o[8 * k + 1]), pack_bf16x2(o[8 * k + 2], o[8 * k + 3]),
+                                                           pack_bf16x2(o[8 * k + 4], o[8 * k + 5]), pack_bf16x2(o[8 * k + 6], o[8 * k + 7]));
     }
-    tc_fence_before();
-  }
-  if (Z > 1) {
+  } else {
+    // ===================== codes into operands =====================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AQT_REGS_DQ));
+    constexpr int CH = KvQ<BITS>::ROW_BYTES / 16, PER = 128 * CH / AQT_DQ;      // 16-byte chunks of a row, of a thread
+    constexpr int CODES = 128 / BITS;                                           // codes of a chunk: 16 / 32
+    const int dt = (int)threadIdx.x - (AQT_THREADS - AQT_DQ);
+    // the codes, less MID, of eight numbers: o-th of the chunk
+    auto codes8 = [&](const uint4& cw, int o, float (&f)[8]) {
+      const uint32_t u[4] = {cw.x, cw.y, cw.z, cw.w};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t c = BITS == 8 ? (u[(o * 2 + (k >> 2)) & 3] >> (8 * (k & 3))) & 0xffu : (u[o & 3] >> (4 * k)) & 0xfu;
+        f[k] = (float)c - MID;
+      }
+    };
+    auto load = [&](int j, int kv, uint4 (&cw)[PER], uint32_t& sw, uint32_t& bw) {      // sw, bw: scales and biases of row dt (threads 0 .. 127)
+      const int key0 = (j0 + j) << 7, pl = 2 * (j0 + j);
+      const int pg0 = p.block_table[pl], pg1 = pl + 1 < pages ? p.block_table[pl + 1] : pg0;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
+        const unsigned char* unit = kvq_unit<BITS>(pq.pool, row < 64 ? pg0 : pg1, kv, kvh, p.n_kv);
+        cw[i] = key0 + row < kv_max ? __ldcg(reinterpret_cast<const uint4*>(unit + (size_t)(row & 63) * KvQ<BITS>::ROW_BYTES) + c) : make_uint4(0u, 0u, 0u, 0u);
+      }
+      sw = bw = 0u;
+      if (dt < 128 && key0 + dt < kv_max) {      // rows that belong to no key: whatever the page holds, it must not enter
+        const uint32_t* sb = reinterpret_cast<const uint32_t*>(kvq_unit<BITS>(pq.pool, dt < 64 ? pg0 : pg1, kv, kvh, p.n_kv) + KvQ<BITS>::CODES_BYTES);
+        sw = __ldcg(sb + (dt & 63));
+        bw = __ldcg(sb + PAGE + (dt & 63));
+      }
+    };
+    auto keys = [&](int it, int j) {
+      uint4 cw[PER];
+      uint32_t sw, bw;
+      load(j, 0, cw, sw, bw);
+      unsigned char* dst = sK + (it & 1) * AT_TILE;
+      mbar_wait(&k_empty[it & 1], ((uint32_t)(it >> 1) & 1u) ^ 1u, p.err);
+      if (dt < 128) {
+        float* f = kb + (it & 3) * AQT_KB + dt;
+        f[0] = bf_lo(sw); f[128] = bf_hi(sw);
+        f[256] = fmaf(bf_lo(sw), MID, bf_lo(bw)); f[384] = fmaf(bf_hi(sw), MID, bf_hi(bw));
+      }
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
+#pragma unroll
+        for (int o = 0; o < CODES / 8; ++o) {       // eight codes: a 16-byte chunk of the tile
+          float f[8];
+          codes8(cw[i], o, f);
+          *reinterpret_cast<uint4*>(dst + at_swz(row, c * (CODES / 8) + o)) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&k_full[it & 1]);
+    };
+    auto values = [&](int j) {
+      uint4 cw[PER];
+      uint32_t sw, bw;
+      load(j, 1, cw, sw, bw);
+      float sc[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {      // the scale of the chunk's row and group
+        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH, pl = 2 * (j0 + j) + (row >> 6);
+        const unsigned short* su = reinterpret_cast<const unsigned short*>(kvq_unit<BITS>(pq.pool, p.block_table[pl < pages ? pl : pl - 1], 1, kvh, p.n_kv) + KvQ<BITS>::CODES_BYTES);
+        sc[i] = ((j0 + j) << 7) + row < kv_max ? __uint_as_float((uint32_t)__ldcg(su + (row & 63) * 2 + (c * CODES >= 64 ? 1 : 0)) << 16) : 0.f;
+      }
+      mbar_wait(v_empty, ((uint32_t)j & 1u) ^ 1u, p.err);
+      if (dt < 128) vb[dt] = make_float2(fmaf(bf_lo(sw), MID, bf_lo(bw)), fmaf(bf_hi(sw), MID, bf_hi(bw)));
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
+#pragma unroll
+        for (int o = 0; o < CODES / 8; ++o) {       // eight codes: one 16-byte chunk of each tile
+          float f[8];
+          codes8(cw[i], o, f);
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float a = f[2 * k] * sc[i], b = f[2 * k + 1] * sc[i];
+            hi[k] = pack_bf16x2(a, b);
+            lo[k] = pack_bf16x2(a - __uint_as_float(hi[k] << 16), b - __uint_as_float(hi[k] & 0xffff0000u));
+          }
+          const uint32_t at = at_swz(row, c * (CODES / 8) + o);
+          *reinterpret_cast<uint4*>(sV + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(sV + AT_TILE + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(v_full);
+    };
+    for (int j = 0; j < n_tiles; ++j) keys(j, j);
     __syncwarp();
-    cluster_sync();
-    if (smx && ok) {
-      const int per = 128 / Z;
-      bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + z * per;
-      for (int c = 0; c < per; c += 8) {
-        float y[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) y[i] = 0.f;
-        for (int d = 0; d < Z; ++d)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) y[i] += zo[((size_t)d * per + c + i) * 128 + r];
-        *reinterpret_cast<uint4*>(dst + c) = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]), pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
-      }
-    }
+    if (Z > 1) cluster_sync();
+    for (int j = 0; j < n_tiles; ++j) { keys(n_tiles + j, j); values(j); }
+    __syncwarp();
+    if (Z > 1) { cluster_sync(); cluster_sync(); }
   }
   __syncthreads();
   if (warp == 1) {

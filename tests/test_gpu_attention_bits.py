@@ -9,6 +9,8 @@ import math
 import pytest
 import torch
 
+from oracle.llama_oracle import mlx_affine_quantize
+
 pytestmark = pytest.mark.gpu
 
 HD, H, ROLL = 128, 512, 37
@@ -110,3 +112,47 @@ def test_attention_over_16_bit_pages(cuda_lib, group, context, T, eps):
     over = beyond_rounding(got, ref)
     print(f"G {group} context {context} T {T}: beyond rounding / spread {float((over / spread.clamp_min(1e-30)).max()):.2e}, misrounded {float((over > 0).double().mean()):.5f}")
     assert bool((over <= eps * spread + 2.0 ** -22 * total).all())
+
+
+def exact_quantised(q, k, v, context, group, bits):
+    """the quantised semantics in 64 bits: scores and probabilities rounded to bf16"""
+    def deq(x):
+        c, s, b = mlx_affine_quantize(x, bits)
+        g = c.double().view(*x.shape[:-1], 2, 64)
+        return (g * s.double()[..., None] + b.double()[..., None]).view(x.shape)
+
+    def r16(x):      # nearest bf16 of a float64, ties to even
+        m, e = torch.frexp(x)
+        return torch.ldexp(torch.round(torch.ldexp(m, torch.tensor(8))), e - 8)
+
+    kd, vd = deq(k), deq(v)
+    T, heads = q.shape[:2]
+    out = torch.empty(T, heads, HD, dtype=torch.float64)
+    seen = torch.arange(len(k))[None] <= context + torch.arange(T)[:, None]
+    for h in range(heads):
+        qs = (q[:, h].float() * torch.tensor(0.08838834764831845)).to(torch.bfloat16).double()
+        s = r16(qs @ kd[:, h // group].T).masked_fill(~seen, -math.inf)
+        out[:, h] = r16(torch.softmax(s, -1)) @ vd[:, h // group]
+    return out
+
+
+@pytest.mark.parametrize("bits,group,context,T", [(8, 4, 300, 1), (8, 4, 2200, 3), (8, 1, 500, 128), (4, 8, 1500, 16), (8, 5, 2000, 64), (4, 7, 100, 40), (8, 2, 700, 512)])
+def test_attention_over_quantised_pages(cuda_lib, bits, group, context, T):
+    """Scores and probabilities are rounded to bf16, so that a fp32 sum near a rounding edge may land on its other side: how often is what a
+    kernel's precision shows in.  The tensor-core kernel is held to the one of fp32 multiply-adds on the same pages."""
+    x = torch.randn(context + T, H, generator=torch.Generator().manual_seed(context + T)).to(torch.bfloat16).cuda()
+    layer, off = Layer(cuda_lib, 2, group, kv_bits=bits), {}
+    try:
+        k, v = layer.rows(x)
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_attn", tc)
+            q, got = layer.attend(x, context)
+            if tc:
+                ref = exact_quantised(q, k, v, context, group, bits)
+            over = beyond_rounding(got, ref)
+            off[tc] = float((over > 0).double().mean())
+    finally:
+        cuda_lib.dn_set_option(b"tc_attn", 1)
+        layer.close()
+    print(f"bits {bits} G {group} context {context} T {T}: misrounded {off[1]:.5f}, multiply-adds {off[0]:.5f}")
+    assert off[1] <= 2 * off[0] + 1e-3
