@@ -712,6 +712,14 @@ static cudaError_t launch_attn_tc(void (*kern)(KArgs...), dim3 grid, int threads
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// blocks of a prompt chunk's attention, and how many CTAs of a cluster take keys
+static dim3 attn_tc_grid(const dn_model* m, int T, const dn_kv* kv, AtParams& a) {
+  const int tb = 128 / m->G, blocks = (T + tb - 1) / tb, ctas = m->cfg.n_kv_heads * blocks;
+  a.sms = g_sms;
+  a.share = g_capturing ? 0 : attn_prefill_split(ctas, kv->host_pos + T, g_sms);
+  return dim3(m->cfg.n_kv_heads, blocks, g_capturing ? attn_prefill_split_max(ctas, kv->max_tokens, g_sms) : a.share);
+}
+
 // a prompt chunk's attention over the quantised pages
 template <int BITS>
 static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf16* out, int T, dn_kv* kv, int pdl, cudaStream_t s) {
@@ -720,8 +728,7 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
   a.a.q = q; a.a.out = out; a.a.block_table = kv->block_table; a.a.st = kv->st;
   a.a.n_heads = c.n_heads; a.a.n_kv = c.n_kv_heads; a.a.T = T; a.a.err = m->mk_sync + 2;
   a.pool = pool;
-  const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
-  const dim3 grid(c.n_kv_heads, blocks, attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms));
+  const dim3 grid = attn_tc_grid(m, T, kv, a.a);
 #define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, pdl, a)); break;
   switch (m->G) { PFQ(1) PFQ(2) PFQ(4) PFQ(5) PFQ(7) PFQ(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFQ
@@ -959,10 +966,8 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     AtParams a;
     a.q = m->pf_q; a.out = m->pf_attn; a.block_table = kv->block_table; a.st = kv->st;
     a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.T = T; a.err = err;
-    const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
-    // (how the keys are shared out only decides the order of the sums; the kernel reads the position from the step state)
-    const int Z = attn_prefill_split(c.n_kv_heads * blocks, g_capturing ? kv->max_tokens : kv->host_pos + T, g_sms);
-#define PFT(Gv, Pv) CK(launch_attn_tc(k_attn_prefill_tc<Gv, Pv>, dim3(c.n_kv_heads, blocks, Z), AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
+    const dim3 grid = attn_tc_grid(m, T, kv, a);
+#define PFT(Gv, Pv) CK(launch_attn_tc(k_attn_prefill_tc<Gv, Pv>, grid, AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
 #define PFT2(Gv) case Gv: if (T < AT_TWO_PARTS_FROM) { PFT(Gv, 3) } else { PFT(Gv, 2) }
     switch (m->G) { PFT2(1) PFT2(2) PFT2(4) PFT2(8) case 5: PFT(5, 3) case 7: PFT(7, 3) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT2

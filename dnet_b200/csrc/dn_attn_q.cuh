@@ -71,12 +71,13 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, Z = gridDim.z, z = blockIdx.z;
+  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, z = blockIdx.z;
   const int pos0 = p.st->pos;
+  const int Z = p.share > 0 ? p.share : attn_prefill_split((int)(gridDim.x * gridDim.y), pos0 + p.T, p.sms);
   const int nq = min(TB, p.T - t0);
   const int kv_max = pos0 + t0 + nq;
   const int pages = (kv_max + PAGE - 1) / PAGE, all = (kv_max + 127) >> 7;
-  const int j0 = (int)((long long)all * z / Z), n_tiles = (int)((long long)all * (z + 1) / Z) - j0;
+  const int j0 = (int)((long long)all * z / Z), n_tiles = z < Z ? (int)((long long)all * (z + 1) / Z) - j0 : 0;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], AQT_DQ / 32); mbar_init(&k_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     }
     if (Z > 1) {      // the other ranks' keys count too
       __syncwarp();
-      for (int d = 0; d < Z; ++d) {
+      for (int d = 0; d < (z < Z ? Z : 0); ++d) {
         dsmem_st(dsmem_addr(zx + z * 256 + r, (uint32_t)d), m);
         dsmem_st(dsmem_addr(zx + z * 256 + 128 + r, (uint32_t)d), l);
       }
@@ -319,11 +320,12 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     if (Z > 1) cluster_sync();      // every rank's products are done: its key buffers may take the other ranks' columns
     const int per = 128 / Z, lg = 31 - __clz(per);      // columns of a rank: a power of two
     if (Z > 1) {
+      if (z < Z)
 #pragma unroll
-      for (int i = 0; i < 128; ++i) dsmem_st(dsmem_addr(zo + (z * per + (i & (per - 1))) * 128 + r, (uint32_t)(i >> lg)), o[i]);
+        for (int i = 0; i < 128; ++i) dsmem_st(dsmem_addr(zo + (z * per + (i & (per - 1))) * 128 + r, (uint32_t)(i >> lg)), o[i]);
       __syncwarp();
       cluster_sync();
-      if (ok) {
+      if (ok && z < Z) {
         bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + z * per;
         for (int c = 0; c < per; c += 8) {
           float y[8];
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
           *reinterpret_cast<uint4*>(dst + c) = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]), pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
         }
       }
-    } else if (ok) {
+    } else if (ok && z == 0) {
       bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD;
 #pragma unroll
       for (int k = 0; k < 16; ++k)

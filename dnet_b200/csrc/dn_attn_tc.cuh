@@ -34,6 +34,7 @@ struct AtParams {
   const int32_t* block_table;
   const StepState* st;
   int n_heads, n_kv, T;
+  int share, sms;                // CTAs of a cluster that take keys (0: by the position in the step state)
   unsigned int* err;
 };
 
@@ -48,6 +49,33 @@ constexpr int AT_THREADS = 384;
 constexpr int AT_TWO_PARTS_FROM = 16;
 constexpr int AT_REGS_MMA = 56, AT_REGS_SOFTMAX = 224;      // setmaxnreg: of the 168 a thread that 384 threads are launched with
 static_assert(128 * AT_REGS_MMA + 256 * AT_REGS_SOFTMAX <= AT_THREADS * 168, "setmaxnreg split exceeds the CTA's launch allocation");
+
+// CTAs that share a row block's keys: what makes (waves of CTAs) x (key tiles of a CTA + 4 for its start, joining and end) smallest.
+// The grid alone (heads x row blocks) leaves most SMs idle when a chunk is short, and a last wave nearly empty when it is long:
+// 40 heads in groups of 5, 512 tokens give 168 CTAs for 148 SMs.
+// The count takes every SM for usable by every cluster, while 33 clusters of four or 15 of eight run at once: behind 8,192 tokens these 168 row blocks
+// take 234 us with Z = 2 and 269 with the chosen 4 (8 row blocks behind 8,192, one token: 76, 48 and 33 us with 2, 4 and 8).
+__host__ __device__ inline int attn_prefill_split(int ctas, int kv_len, int sms) {
+  const int tiles = (kv_len + 127) / 128;
+  int best = 1, cost = 0;
+  for (int Z = 1; Z <= AT_MAX_Z; Z *= 2) {
+    if (Z > 1 && tiles < 2 * Z) break;
+    const int c = ((ctas * Z + sms - 1) / sms) * ((tiles + Z - 1) / Z + (Z > 1 ? 6 : 4));
+    if (Z == 1 || c < cost) { cost = c; best = Z; }
+  }
+  return best;
+}
+
+// A captured launch is replayed at positions that nobody knows yet: its clusters are as large as the longest share needs, the kernel takes the
+// share of the position it finds (AtParams::share 0), and the CTAs beyond it stay idle -- the sums of a replay are those of an eager launch.
+static inline int attn_prefill_split_max(int ctas, int kv_len, int sms) {
+  int best = 1;
+  for (int n = 128; n < kv_len + 128 && best < AT_MAX_Z; n += 128) {
+    const int z = attn_prefill_split(ctas, n, sms);
+    if (z > best) best = z;
+  }
+  return best;
+}
 
 // two fp32 operations, each rounded as the single one
 __device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
@@ -97,12 +125,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, Z = gridDim.z, z = blockIdx.z;      // the cluster spans the grid's z
+  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, z = blockIdx.z;      // the cluster spans the grid's z
   const int pos0 = p.st->pos;
+  const int Z = p.share > 0 ? p.share : attn_prefill_split((int)(gridDim.x * gridDim.y), pos0 + p.T, p.sms);      // ranks from Z on have no keys and no columns
   const int nq = min(TB, p.T - t0);                         // query tokens of this CTA
   const int kv_max = pos0 + t0 + nq;                        // keys visible to its last query
   const int pages = (kv_max + PAGE - 1) / PAGE, all = (kv_max + 127) >> 7;
-  const int j0 = (int)((long long)all * z / Z), n_tiles = (int)((long long)all * (z + 1) / Z) - j0;      // this CTA's key tiles
+  const int j0 = (int)((long long)all * z / Z), n_tiles = z < Z ? (int)((long long)all * (z + 1) / Z) - j0 : 0;      // this CTA's key tiles
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -344,7 +373,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
       for (int i = 0; i < 32; ++i) y[c * 32 + i] = f0 * __uint_as_float(a[i]) + f1 * __uint_as_float(b[i]);
     }
     if (Z == 1) {
-      if (ok) {
+      if (ok && z == 0) {
         const float inv = 1.0f / L;
         bf16* dst = p.out + ((size_t)(t0 + t) * p.n_heads + kvh * G + g) * HD + sd * 64;
 #pragma unroll
@@ -355,7 +384,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
           *reinterpret_cast<uint4*>(dst + c * 8) = w;
         }
       }
-    } else {
+    } else if (z < Z) {
       const int per = 128 / Z;      // columns of a rank
 #pragma unroll
       for (int i = 0; i < 64; ++i) {
@@ -372,7 +401,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
     if (Z > 1) {
       __syncwarp();
       cluster_sync();
-      if (ok) {
+      if (ok && z < Z) {
         const int per = 128 / Z, half = per / 2;
         float M = -INFINITY, L = 0.f;
         for (int d = 0; d < Z; ++d) M = fmaxf(M, zx[d * 256 + r]);
@@ -404,21 +433,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
-}
-
-// CTAs that share a row block's keys: what makes (waves of CTAs) x (key tiles of a CTA + 4 for its start, joining and end) smallest.
-// The grid alone (heads x row blocks) leaves most SMs idle when a chunk is short, and a last wave nearly empty when it is long:
-// 40 heads in groups of 5, 512 tokens give 168 CTAs for 148 SMs.
-static inline int attn_prefill_split(int ctas, int kv_len, int sms) {
-  const int tiles = (kv_len + 127) / 128;
-  int best = 1;
-  long long cost = 0;
-  for (int Z = 1; Z <= AT_MAX_Z; Z *= 2) {
-    if (Z > 1 && tiles < 2 * Z) break;
-    const long long c = (long long)((ctas * Z + sms - 1) / sms) * ((tiles + Z - 1) / Z + (Z > 1 ? 6 : 4));
-    if (Z == 1 || c < cost) { cost = c; best = Z; }
-  }
-  return best;
 }
 
 }  // namespace dn

@@ -4,6 +4,7 @@ The layer's projections only pick numbers of the normed row (one entry of a powe
 values are the same bits whatever kernel forms the products: the rotated keys of a position are the rotated queries of its group's first
 head, read back with the scratch hook from the token alone at that position, and the values are the same at position 0 (nothing rotates),
 rolled by some dims."""
+import ctypes as C
 import math
 
 import pytest
@@ -156,3 +157,36 @@ def test_attention_over_quantised_pages(cuda_lib, bits, group, context, T):
         layer.close()
     print(f"bits {bits} G {group} context {context} T {T}: misrounded {off[1]:.5f}, multiply-adds {off[0]:.5f}")
     assert off[1] <= 2 * off[0] + 1e-3
+
+
+@pytest.mark.parametrize("bits,group,T", [(0, 4, 1), (0, 5, 1), (0, 4, 3), (0, 7, 15), (0, 4, 16), (0, 5, 200), (8, 4, 1), (4, 1, 2), (8, 5, 64)])
+def test_a_captured_chunk_gives_the_bits_of_an_eager_one(cuda_lib, bits, group, T):
+    """a chunk captured once, for a cache of 4,096 tokens, and replayed at positions whose keys are shared out differently"""
+    n = 2600
+    x = torch.randn(n + T, H, generator=torch.Generator().manual_seed(n + T)).to(torch.bfloat16).cuda()
+    layer, s, graph = Layer(cuda_lib, 2, group, kv_bits=bits, max_tokens=4096), torch.cuda.Stream(), C.c_void_p()
+    try:
+        layer.run(x, 0)      # the cache's rows
+        torch.cuda.synchronize()
+        buf, ids = torch.empty(T, H, dtype=torch.bfloat16, device="cuda"), (C.c_int32 * 1)(0)
+        assert cuda_lib.dn_graph_begin(s.cuda_stream) == 0
+        assert cuda_lib.dn_chunk_forward(layer.m._h, ids, 1, buf.data_ptr(), T, layer.kv._h, s.cuda_stream) == 0
+        assert cuda_lib.dn_graph_end(s.cuda_stream, C.byref(graph)) == 0
+        for at in (0, 300, 1100, n):
+            with torch.cuda.stream(s):
+                out = []
+                for captured in (True, False):
+                    buf.copy_(x[at:at + T])
+                    layer.kv.seek(at, s.cuda_stream)
+                    if captured:
+                        assert cuda_lib.dn_graph_launch(graph, s.cuda_stream) == 0
+                    else:
+                        assert cuda_lib.dn_chunk_forward(layer.m._h, ids, 1, buf.data_ptr(), T, layer.kv._h, s.cuda_stream) == 0
+                    out.append(buf.clone())
+            torch.cuda.synchronize()
+            assert torch.equal(*out), at
+        assert cuda_lib.dn_step_error(layer.m._h, s.cuda_stream) == 0
+    finally:
+        if graph.value:
+            cuda_lib.dn_graph_destroy(graph)
+        layer.close()
