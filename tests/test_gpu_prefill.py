@@ -77,7 +77,7 @@ def test_prefill_attention_groups_and_key_shares(cuda_lib, group, context, T):
     _agree(out[1], out[0])
 
 
-@pytest.mark.parametrize("hidden,ffn,kv_heads,group,T", [(256, 8192, 2, 1, 16), (256, 8192, 2, 1, 45), (768, 1280, 1, 2, 65), (1024, 14336, 2, 4, 129),
+@pytest.mark.parametrize("hidden,ffn,kv_heads,group,T", [(256, 8192, 2, 1, 17), (256, 8192, 2, 1, 45), (768, 1280, 1, 2, 65), (1024, 14336, 2, 4, 129),
                                                          (512, 2048, 2, 2, 300), (768, 27648, 1, 4, 512)])
 def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_heads, group, T):
     """k_gemm_tc (tiles of a CTA pair) against the row kernels: features and tokens that leave part of a tile empty, q, k and v in one launch
@@ -126,24 +126,39 @@ def test_prefill_attention_over_quantised_pages(cuda_lib, bits, group, context, 
 @pytest.mark.parametrize("hidden,ffn,kv_heads,group,context", [(256, 512, 1, 2, 0), (768, 27648, 2, 5, 63), (4096, 1280, 2, 4, 700)])
 def test_chunks_of_a_few_tokens(cuda_lib, hidden, ffn, kv_heads, group, context, T, bits):
     """A chunk of 2 .. 16 tokens in one pass over the weights (k_rows: one or two groups of eight tokens, warps with few columns and with
-    many) against the same tokens one by one (the row kernels) behind the same pages; 17 tokens are the first that the GEMM takes.
-    Over quantised pages a score near a rounding edge flips by 2^-8 of itself, and its weight with it: that moves every result of its
-    token by up to a rounding, half of them over an edge; two or three tokens have no others to average with, so below a half."""
+    many) against the same tokens one by one on the kernels of a model without tensor-core prompts (k_gemv, k_attn or k_attn_q); 17 tokens
+    are the first that the GEMM takes.
+    The row kernels form every product's sums in another order too, so that the flipped roundings start in q, k and v and grow from product
+    to product.  Where every operand of the last one differs in its last place the result is off by 2^-9 / sqrt(3) of its size times sqrt(2),
+    three quarters of a place at the most frequent sizes: about half of the results are stored differently.  Over quantised pages a
+    score near a rounding edge flips by 2^-8 of itself, and its weight with it, which moves every result of its token by up to a rounding,
+    half of them over an edge.  So below a half either way (a wrong weight, row or head changes nearly all, and by more)."""
     x = torch.randn(context + T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
-    m = _model(kv_heads, group, seed=hidden, hidden=hidden, ffn=ffn, kv_bits=bits)
-    kv = m.make_cache(max_tokens=768)
+    out = {}
     try:
-        one_pass = _call(m, kv, x, context)
-        rows = []
-        for t in range(context, context + T):
-            kv.seek(t)
-            rows.append(m.apply_single_layer(0, x[t:t + 1].clone(), kv))
-        torch.cuda.synchronize()
-        assert cuda_lib.dn_step_error(m._h, 0) == 0
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_prefill", tc)
+            m = _model(kv_heads, group, seed=hidden, hidden=hidden, ffn=ffn, kv_bits=bits)
+            kv = m.make_cache(max_tokens=768)
+            if tc:
+                out[tc] = _call(m, kv, x, context)
+            else:
+                assert cuda_lib.dn_model_max_chunk_forward(m._h) == 0      # (the row kernels)
+                rows = []
+                kv.seek(0)
+                if context:
+                    m.apply_single_layer(0, x[:context].clone(), kv)
+                for t in range(context, context + T):
+                    kv.seek(t)
+                    rows.append(m.apply_single_layer(0, x[t:t + 1].clone(), kv))
+                torch.cuda.synchronize()
+                out[tc] = torch.cat(rows).float().cpu()
+            assert cuda_lib.dn_step_error(m._h, 0) == 0
+            kv.free()
+            m.destroy()
     finally:
-        kv.free()
-        m.destroy()
-    _agree(one_pass, torch.cat(rows).float().cpu(), 0.5 if bits else 0.25)
+        cuda_lib.dn_set_option(b"tc_prefill", 1)
+    _agree(out[1], out[0], 0.5)
 
 
 @pytest.mark.parametrize("bits,group,hidden,ffn,T", [(0, 4, 512, 2048, 513), (8, 2, 512, 512, 1029), (0, 5, 768, 1280, 2048), (4, 1, 256, 512, 2050)])
