@@ -5,7 +5,7 @@
   python -m torch.distributed.run --nproc-per-node N ... bench.py --gpus N ...
   python bench.py --impl reference ...                      (CPU port of the reference path, all layers)
 
-Workload (BASELINE.json configs[1] at N shards): Llama-3-8B dims, bf16, random-init weights
+Workload (at N shards): Llama-3-8B dims, bf16, random-init weights
 (synthetic), bs=1 decode after a 128-token synthetic prompt, temperature 0, kv fp16, wire
 dtype bf16, contiguous layer split, k=1, N sequences in flight.  A "step" is one decoded token per
 in-flight sequence.  Weights (15 GB/token) far exceed the 126 MB L2, so no L2 flush is needed
@@ -47,7 +47,7 @@ def layer_bytes(c) -> int:
 
 
 def token_bytes(c) -> int:
-    """SURVEY.md section 8(d): all layers + lm_head + final norm + one embed row."""
+    """all layers + lm_head + final norm + one embed row."""
     H, V = c["hidden_size"], c["vocab_size"]
     return c["num_hidden_layers"] * layer_bytes(c) + 2 * V * H + 2 * H + 2 * H
 
@@ -291,7 +291,7 @@ def run_reference(args, rank: int, world: int) -> None:
         "impl": "reference", "metric": METRIC, "value": tps, "unit": "tok/s", "n_gpus": args.gpus,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": detail["ms_per_token"],
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
-        "config": {"workload": "Llama-3-8B bf16 bs=1 decode (BASELINE configs[1]), reference path = CPU port of "
+        "config": {"workload": "Llama-3-8B bf16 bs=1 decode, reference path = CPU port of "
                                "FitInMemoryPolicy.process + mlx_lm llama block (mlx is not installable here)",
                    "prompt_len": PROMPT_LEN, "mlx_importable": _mlx_probe()},
         "cpu_baseline": {"value": tps, "unit": "tok/s", "cores": cores, "kind": "port", "sample": sample,
@@ -303,7 +303,7 @@ def run_reference(args, rank: int, world: int) -> None:
 
 
 def _mlx_probe() -> dict:
-    """BASELINE.md section 4: if the run box had mlx + mlx_lm, the real reference block could be a third witness."""
+    """if the run box had mlx + mlx_lm, the real reference block could be a third witness."""
     out = {}
     for mod in ("mlx", "mlx.core", "mlx_lm"):
         try:
@@ -489,7 +489,7 @@ def main():
     ap.add_argument("--sched-rounds", type=int, default=8, help="decode rounds per schedule frame (head shard's RingAdapter)")
     ap.add_argument("--sched-depth", type=int, default=4, help="schedule frames in flight")
     ap.add_argument("--config", default="decode", choices=["decode", "swap", "prefill", "moe", "seqmix", "filinex", "lutesun", "vulanex", "bokenex", "tuguvik"],
-                    help="decode: BASELINE configs[1] (the bench contract); swap: configs[3], Llama-3-70B layer swap (bench_swap.py); "
+                    help="decode: Llama-3-8B, bs=1 (the bench contract); swap: Llama-3-70B layer swap (bench_swap.py); "
                          "tuguvik: the Tuguvik family beside Moputar and Lutesun (bench_tuguvik.py; uses --seqmix-sizes / --seqmix-prompt); "
                          "bokenex: the Bokenex family beside Moputar and Lutesun (bench_bokenex.py; uses --seqmix-sizes / --seqmix-prompt); "
                          "vulanex: the Vulanex family beside Moputar (bench_vulanex.py; uses --seqmix-sizes / --seqmix-prompt); lutesun: the Lutesun family beside Filinex (bench_lutesun.py; uses --seqmix-sizes / --seqmix-prompt); filinex: the Filinex family beside Moputar (bench_filinex.py; uses --seqmix-sizes / --seqmix-prompt); seqmix: a layer-list model (Moputar) beside the llama family at equal size (bench_seqmix.py)")

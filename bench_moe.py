@@ -1,4 +1,4 @@
-"""bench_moe.py: Mixtral-8x7B dims (32 layers, 8 experts, top-2), bf16, N shards, several
+"""bench_moe.py -- Mixtral-8x7B dims (32 layers, 8 experts, top-2), bf16, N shards, several
 requests in flight (`bench.py --config moe`, one process per GPU under torchrun).
 
 Every shard is a ShardNode; the model class is ``mixtral`` (dnet_b200/core/models/llama.py MixtralRingModel): attention
@@ -116,7 +116,7 @@ def run_moe(args, rank: int, local_rank: int, world: int) -> None:
         peak, peak_src = B.peaks()
         # steady state bound: with NS >= world requests in flight every shard streams its layers' bytes per token
         bound = 1.0 / (max(len(x) for x in split) * layer_token_bytes / (peak * 1e9))
-        out = {"metric": "decode tok/s Mixtral-8x7B dims bf16, bs=1 per request (BASELINE configs[4])", "value": tps, "unit": "tok/s",
+        out = {"metric": "decode tok/s Mixtral-8x7B dims bf16, bs=1 per request", "value": tps, "unit": "tok/s",
                "n_gpus": world, "steps": K, "warmup": Wm, "ms_per_step": wall / K * 1e3, "higher_is_better": True, "scaling": "weak",
                "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
                "config": {"workload": f"Mixtral-8x7B dims (32 layers, 8 experts top-2), {world} shards x {'/'.join(str(len(x)) for x in split)} "

@@ -1,4 +1,4 @@
-"""bench_prefill.py -- the long-context path (SURVEY.md section 8f N3): a long prompt prefilled through the ring as a
+"""bench_prefill.py -- the long-context path: a long prompt prefilled through the ring as a
 stream of chunks (`bench.py --config prefill`, one process per GPU under torchrun).
 
 The API (`InferenceManager.generate_stream(prefill_chunk=C)`) cuts the prompt into C-token ``tokens`` frames, all but

@@ -329,7 +329,7 @@ def run_ring(args, rank: int, local_rank: int, world: int) -> None:
             "data": "synthetic",
             "config": {"workload": f"Llama-3-8B bf16 bs=1 decode, {world} shard{'s' if world > 1 else ''} x "
                                    f"{'/'.join(str(len(x)) for x in split)} layers ({'1 shard' if world == 1 else args.split + ' contiguous split'}) "
-                                   f"pipelined ring (BASELINE configs[1]), {NS} sequence{'s' if NS > 1 else ''} in flight, each bs=1",
+                                   f"pipelined ring, {NS} sequence{'s' if NS > 1 else ''} in flight, each bs=1",
                        "prompt_len": PROMPT_LEN, "kv": "fp16 paged (64-token pages)", "wire_dtype": "bf16",
                        "l2": "inputs larger than L2 (>=1.7 GB of weights per shard step vs 126 MB L2); no flush",
                        "step_kernel": "k_shard_step via RingAdapter schedule (dn_shard_step_hop: wait + step + hop in one launch)",

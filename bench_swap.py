@@ -1,4 +1,4 @@
-"""bench_swap.py: Llama-3-70B dims on 2 shards x 40 layers with an HBM cap, i.e. the
+"""bench_swap.py -- Llama-3-70B dims on 2 shards x 40 layers with an HBM cap, i.e. the
 layer-swap path end to end (`bench.py --config swap`, one process per GPU under torchrun).
 
 Every shard is a ShardNode (runtime + RingAdapter + gRPC server); the request loads with
@@ -136,7 +136,7 @@ def run_swap(args, rank: int, local_rank: int, world: int) -> None:
     per_rank_gbs = swapped * layer_bytes / (ms_tok / 1e3) / 1e9 if ms_tok else 0.0
     if rank == 0:
         # one sequence: the two shards swap one after the other, so each GPU's copy engine is busy ~1/world of a token
-        out = {"metric": "decode tok/s Llama-3-70B bf16 bs=1, layer swap (BASELINE configs[3])", "value": 1e3 / ms_tok, "unit": "tok/s",
+        out = {"metric": "decode tok/s Llama-3-70B bf16 bs=1, layer swap", "value": 1e3 / ms_tok, "unit": "tok/s",
                "n_gpus": world, "steps": K, "warmup": Wm, "ms_per_step": ms_tok, "higher_is_better": True, "scaling": "weak",
                "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
                "config": {"workload": f"Llama-3-70B dims, {world} shards x {'/'.join(str(len(x)) for x in split)} layers, HBM cap: "

@@ -3,6 +3,6 @@
 Only what the north-star path needs: the C-ABI CUDA library (csrc/, lib/), and the
 host-side mirror of the reference's plug-in seams for that path (ComputePolicy
 registry, BaseRingModel operator API, WeightCache / pools / LayerManager,
-ShardRuntime, ActivationCodec, the ring hop).  See DESIGN.md.
+ShardRuntime, ActivationCodec, the ring hop).
 """
 __version__ = "0.1.0"

@@ -1,6 +1,6 @@
 """The API node's token loop (reference src/dnet/api/inference.py:135-212), on token ids.
 
-Tokenisation, chat templates and the HTTP surface are out of scope (SURVEY.md section 8); what is
+Tokenisation, chat templates and the HTTP surface are out of scope; what is
 rebuilt is the loop that closes the ring: send the prompt, then either
 
 * ``device_loop=False`` -- the reference's loop: await the token, send it back as a one-token

@@ -1,9 +1,9 @@
 """API-side ring adapter: the token loop as the API sees it (reference
 src/dnet/api/strategies/ring.py:101-209; the HALDA solver half of that file is consumed unchanged
-and not rebuilt, SURVEY.md section 8).
+and not rebuilt).
 
 ``send_tokens`` / ``await_token`` / ``resolve_token`` keep the reference's names and meaning.  Two
-additions for the device-closed loop (SURVEY.md section 8f N2): ``lease(nonce, steps)`` lets the ring
+additions for the device-closed loop: ``lease(nonce, steps)`` lets the ring
 decode ``steps`` tokens without the API in the loop -- tokens then arrive unsolicited through
 ``resolve_token`` and queue up per nonce until ``await_token`` takes them in order -- and
 ``end_request`` releases the nonce's lanes on every shard (an ``end_of_request`` frame)."""

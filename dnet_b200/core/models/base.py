@@ -75,8 +75,8 @@ def _stream_ptr(stream) -> int:
 
 
 def _decompose(T: int, tmax: int, big: int = 0) -> List[int]:
-    """Split T into chunk sizes the kernels are instantiated for: chunks of 16..``big`` tokens go
-    to the tensor-core prefill GEMMs, the remainder to the (4, 2, 1)-token GEMV kernels."""
+    """Split T into the chunk sizes of dn_layer_forward and dn_window_forward: 16..``big`` tokens on the tensor-core
+    path (none where ``big`` is 0), the remainder as 4, 2 and 1.  (dn_chunk_forward takes any size.)"""
     out: List[int] = []
     while big >= 16 and T >= 16:
         c = min(T, big)

@@ -73,7 +73,7 @@ class LlamaRingModel(BaseRingModel):
     def lm_project(self, x) -> torch.Tensor:
         """fused final-norm + lm_head on the last position -> (1, 1, V) bf16 logits.
         (The reference projects all T positions and the sampler keeps the last one;
-        last-position-only is result-identical, SURVEY.md Appendix C.)"""
+        last-position-only is result-identical.)"""
         if not isinstance(x, _Normed):
             raise ValueError("lm_project expects the output of normalize()")
         h = x.x.reshape(-1, self.hidden_size)
@@ -126,7 +126,7 @@ class _Normed:
 
 class Qwen2RingModel(LlamaRingModel):
     """qwen2 = llama block + q/k/v bias (mlx_lm.models.qwen2); the reference has no qwen2
-    wrapper, BASELINE config 3 needs one."""
+    wrapper."""
 
     model_type = "qwen2"
 
@@ -134,8 +134,7 @@ class Qwen2RingModel(LlamaRingModel):
 class MixtralRingModel(LlamaRingModel):
     """mixtral = llama attention + a sparse MoE FFN (mlx_lm.models.mixtral: router -> top-k experts -> softmax over
     the selected logits -> SwiGLU experts -> weighted sum).  The reference has no mixtral wrapper; it hosts its MoE
-    families (gpt_oss, deepseek_v2) through this same operator API, and BASELINE.json configs[4] names
-    Mixtral-8x7B.  Expert selection happens on the device, so MoE layers run on the per-op path
+    families (gpt_oss, deepseek_v2) through this same operator API.  Expert selection happens on the device, so MoE layers run on the per-op path
     (dn_window_forward; CUDA-graph capturable), not in the persistent step kernel."""
 
     model_type = "mixtral"

@@ -44,8 +44,8 @@ static int fail(int code, const char* fmt, ...) {
 static std::atomic<long long> g_launches{0};
 static int g_pdl = 0;
 // Launches of a chunk's layer are programmatic whatever the option says (0: never, 1: with the option): a layer is 8 to 10 launches, each of which
-// starts with a wait for the one in front, and the row products ask for their first weights before it.  Three tokens, Llama-8B sizes: 114 us
-// without, 101 with; 45 tokens 165 / 155; one Mixtral-8x7B token 182 / 163; 2,048 tokens of two layers 2,022 / 1,993.  (Prefetching more of the
+// starts with a wait for the one in front, and the row products ask for their first weights before it.  When they became so: three tokens,
+// Llama-8B sizes, 114 us -> 101; 45 tokens 165 -> 155; one Mixtral-8x7B token 182 -> 163; 2,048 tokens of two layers 2,022 -> 1,993.  (Prefetching more of the
 // weights into L2 before the wait cost 6 us.)
 constexpr int PDL_CHUNK = 2;
 static int g_l2_prefetch_kb = 64;
@@ -122,7 +122,7 @@ struct LayerW {
 };
 
 constexpr int TPF_MAX = 512;   // tokens per chunk of dn_layer_forward and dn_window_forward on the tensor-core path (weights are streamed once per chunk)
-// ... and of dn_chunk_forward.  At 512 tokens a product's tiles fill the 74 CTA pairs badly (gate / up of Llama-8B sizes: 224 tiles, a fourth round
+// ... and of dn_chunk_forward (a chunk that does not fit the cache is refused whole).  At 512 tokens a product's tiles fill the 74 CTA pairs badly (gate / up of Llama-8B sizes: 224 tiles, a fourth round
 // for two of them; 105 us against 72 at the measured rate); 2,048 tokens are 896 tiles.  A prompt of
 // 2,048 tokens through two layers and the head: 2,667 us in chunks of 512, 2,033 in one; 777 tokens over 8-bit pages 719 / 644.
 constexpr int CHUNK_MAX = 2048;
@@ -528,7 +528,7 @@ extern "C" int dn_bind_layer(dn_model* m, int abs_layer, const void* const* dev_
     const int rows[7] = {qd, kd, kd, H, c.ffn, c.ffn, H};
     const int cols[7] = {H, H, H, qd, H, H, c.ffn};
     L.tm_ok = m->pf_ok;
-    const int n_tm = m->cfg.n_experts > 0 ? 4 : 7;       // MoE layers: the expert FFN runs token by token, no GEMM descriptors
+    const int n_tm = m->cfg.n_experts > 0 ? 4 : 7;       // MoE layers: the experts' descriptors are made where they are bound
     for (int i = 0; i < n_tm && L.tm_ok; ++i) L.tm_ok = make_tmap(&L.tm[i], L.w[i], rows[i], cols[i], TC_WBOX) == DN_OK;
   }
   MkLayer& ML = m->mk_host[it->second];
@@ -741,7 +741,8 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
 static int kvq_append_and_attend(dn_model* m, int li, const bf16* q, bf16* attn_out, int T, dn_kv* kv, int pdl, bool prompt, cudaStream_t s) {
   const dn_model_cfg& c = m->cfg;
   unsigned char* pool = reinterpret_cast<unsigned char*>(m->kv_pool) + (size_t)li * m->kv_layer_bytes;
-  // host mirror: longest context any of the T queries sees (a captured graph is replayed at growing contexts)
+  // host mirror: longest context any of the T queries sees (a captured graph is replayed at growing contexts).  The bound is that of k_attn_q, whose
+  // scores lie in shared memory; it holds for the prompt kernel, too, so that what a cache may grow to does not hang on an option.
   const int kv_len_max = g_capturing ? kv->max_tokens : kv->host_pos + T;
   const size_t smem = ((size_t)((kv_len_max + 31) / 32 * 32) + AQ_WARPS * 132) * sizeof(float);
   if (smem > 200 * 1024) return fail(DN_EINVAL, "quantised-KV attention outside the step kernel supports contexts up to ~50K tokens (got %d)", kv_len_max);
@@ -1004,8 +1005,9 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   return DN_OK;
 }
 
-// The kernels of a chunk: the prompt's, single tokens included (calls timed with their copies: Llama-8B sizes behind 256 130 us against 134 of the row
-// kernels, which form the norm and the rotation in their products' launches, Qwen-32B sizes 218 / 222; behind 8,000 8-bit tokens 218 against 1,650, Mixtral-8x7B sizes 181 against 236).
+// The kernels of a chunk: the prompt's, single tokens included (calls timed with their copies: Llama-8B sizes behind 256 126 us against 132 of the row
+// kernels, which form the norm and the rotation in their products' launches, behind 8,000 150 / 171 and with 8-bit pages 209 / 1,642; Qwen-32B
+// sizes 198 / 222; Mixtral-8x7B sizes 188 / 247).
 static bool use_prompt_kernels(const dn_model* m, int T) { return m->pf_ok && g_tc_prefill && (T > 1 || m->cfg.n_experts == 0 || m->moe_tc_ok); }
 static int one_layer(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* kv, cudaStream_t s, cudaEvent_t* ev = nullptr) {
   m->pf_last = use_prompt_kernels(m, T);

@@ -633,8 +633,8 @@ static inline int tc_clusters(int S, int sms) {
 // as its bytes from L2, of which all SMs together get 10.8 TB/s (a 256-token tile's MMAs take as long as its bytes); a launch that fills
 // more than half of the SMs with pairs does no better than 120 of them would.  The weights come out of DRAM at 5.6 TB/s at best.  Start and
 // end of a launch cost 6, 10.5 where partial sums meet, and the epilogue of the last tile, which nothing hides, grows with its tokens.
-// Against all widths and splits at 47 shapes (2,048 .. 27,648 features, reductions of 2,048 .. 27,648, 16 .. 2,048 tokens) the plan so
-// chosen was the fastest or within a tenth of it at 45.
+// Against five widths and all splits at 45 shapes (2,048 .. 27,648 features, reductions of 2,048 .. 27,648, 16 .. 2,048 tokens) the plan so
+// chosen is the fastest or within 5 % of it.
 static inline double tc_step(int active, int w) {
   const int bytes = TC_A_BYTES + (w / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
   if (active > 72 && active < 120) active = 120;

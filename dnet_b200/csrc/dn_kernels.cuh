@@ -384,7 +384,7 @@ struct OpGateUp {
 typedef OpOProj OpDown;  // identical dataflow: a=[T][ffn], w=[H][ffn], resid=h, out=x
 
 // ---------------------------------------------------------------------------------
-// Sparse MoE FFN (mixtral; BASELINE configs[4]).  Restated from mlx_lm.models.mixtral.MixtralSparseMoeBlock +
+// Sparse MoE FFN (mixtral).  Restated from mlx_lm.models.mixtral.MixtralSparseMoeBlock +
 // switch_layers.SwitchGLU (oracle/llama_oracle.py moe_block has the rounding points); the reference hosts MoE
 // families through the same operator API (src/dnet/core/models/gpt_oss.py, deepseek_v2.py).  One token at a time
 // (T = 1): the experts a token uses are only known on the device, so the expert ops take a device table of expert
@@ -394,8 +394,9 @@ typedef OpOProj OpDown;  // identical dataflow: a=[T][ffn], w=[H][ffn], resid=h,
 //   OpGateUpMoe   act_j = SwiGLU of expert sel[j]           (j = 0..k-1; same epilogue as the dense OpGateUp)
 //   OpDownMoe     y_j = T(act_j Wd[sel[j]]^T); term_j = T(y_j * score_j); acc = T(acc + term_j) in selection order;
 //                 the last j writes out = T(h + acc)
-// A prompt's tokens (16 and more) take k_moe_route and the grouped GEMM instead: every expert's matrices are read once for all the
-// tokens that chose it (moe_ffn_tc in dn_api.cu), with the same rounding points; k_moe_join adds a token's pairs.
+// Two tokens and more take k_moe_route and the grouped GEMM instead: every expert's matrices are read once for all the tokens that
+// chose it (moe_ffn_tc in dn_api.cu); a single token takes k_moe_route and k_rows over its experts (moe_ffn_one).  The rounding points
+// are the same; k_moe_join adds a token's pairs.
 // ---------------------------------------------------------------------------------
 struct OpRouter {
   static constexpr int ALIGN = 1;

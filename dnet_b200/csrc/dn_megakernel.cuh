@@ -3,7 +3,7 @@
 // Why: ncu on the per-op kernels (profiles/r01_*) shows every weight-streaming kernel moves
 // exactly its algorithmic bytes but is latency bound (59% long-scoreboard stalls, 16 warps/SM)
 // and pays ~10-14 us of launch + prologue + ramp + tail per launch, 160 launches per token.
-// This kernel removes both (DESIGN.md section 3.2 has the measured history):
+// This kernel removes both:
 //   * one CTA per SM (grid = #SMs, cooperative launch), 12 warps = 3 warpgroups.
 //   * warps 8-9 are PRODUCERS: they stream this CTA's share of every weight matrix of every layer
 //     (and the lm_head) through a shared-memory ring with TMA bulk copies (cp.async.bulk + mbarrier
@@ -107,7 +107,7 @@ struct MkParams {
   float* sc_buf;             // [n_heads][sc_stride] bf16-rounded scores of the current layer
   int sc_stride;
   unsigned int* head_tk;     // [n_heads] monotonic arrival counters: the splits of a head exchange (max, sum)
-  // ---- tensor-parallel lm_head over the ring (dn_shard_step_tp; DESIGN.md section 4.2).  Every shard holds
+  // ---- tensor-parallel lm_head over the ring (dn_shard_step_tp).  Every shard holds
   //      vocab/S rows of the lm_head; the last shard broadcasts the final hidden state of a token to all
   //      shards over NVLink, each computes (max, sum-exp, argmax) of its slice and stores that partial into the
   //      head shard's table, which merges them -- so no shard streams the whole 1 GB head.

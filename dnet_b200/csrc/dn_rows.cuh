@@ -1,6 +1,6 @@
 // dn_rows.cuh -- the decoder layer's products for chunks of 1 .. ROWS_MAX tokens: every weight is read once and meets all the tokens on
 // the tensor cores (dn_rows_mma.cuh).  Bound by the weights' bytes.  Three tokens behind 256, Llama-8B sizes: 253 us a layer as chunks of
-// 2 + 1 on the row kernels (two passes), 101 as one; gate and up 37.1 us, 6.3 TB/s.  From 17 tokens on the GEMM takes over (calls timed with
+// 2 + 1 on the row kernels (two passes), 106 as one; gate and up 37.1 us, 6.3 TB/s.  From 17 tokens on the GEMM takes over (calls timed with
 // their copies, before the launches were programmatic: Llama-8B sizes 16 tokens 155 us here, 17 there 179; Qwen-32B sizes 268 / 257).
 // A block takes 16 features (gate / up: the same 16 of both matrices).  The first weights are asked for before the kernel in front has
 // ended (programmatic dependent launch); what that kernel wrote is read after the wait.  Rounding as in the GEMM's epilogues (dn_gemm_tc.cuh).

@@ -25,6 +25,8 @@ constexpr int RM_WARPS = 8, RM_THREADS = RM_WARPS * 32;
 // all thread blocks run at once or in many waves (4,096 x 4,096, 4 tokens: 8.4 us against 8.7; x 14,336: 22.3 / 22.6; 14,336 x 4,096: 20.9 /
 // 22.6), three where only they hold all (6,144 x 4,096: 12.4 / 10.9; 5,120 x 27,648: 58.6 / 46.2).  16 tokens: 4,096 x 14,336 26.6 / 34.9.
 static inline bool rows_mma_deep(int blocks, int sms) { return blocks <= 2 * sms || blocks > 3 * sms; }
+// Features from which a block takes two tiles (each token row is read for twice the weights): tiles of one fill three blocks an SM either way.
+static inline bool rows_mma_wide(int features, int sms) { return features >= 3 * 16 * sms; }
 // columns a lane loads at once: 16-byte rows of both operands
 static inline bool rows_mma_ok(int K, const void* X, const void* W, const void* W2) {
   return K % 32 == 0 && ((((uintptr_t)X | (uintptr_t)W | (uintptr_t)(W2 ? W2 : W)) & 15) == 0);

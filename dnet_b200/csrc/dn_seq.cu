@@ -808,7 +808,7 @@ static cudaError_t linear(dn_seq_model* m, cudaStream_t s, const T* X, const voi
 #define LM(MODE, U, EPv) launch(k_linear_mma<MODE, U, EPv>, dim3((O + (MODE == 1 ? 31 : 15)) / (MODE == 1 ? 32 : 16)), dim3(dn::RM_THREADS), 0, s, (const bf16*)X, (const bf16*)W, \
                              (const bf16*)W2, Y, out32 ? 1 : 0, N, O, K, act, alim, (const bf16*)bias, epi)
       if (act_two(act)) return LM(2, 4, false);
-      if (O >= LM_WIDE) return own ? LM(1, 4, true) : LM(1, 4, false);
+      if (dn::rows_mma_wide(O, g_sms)) return own ? LM(1, 4, true) : LM(1, 4, false);
       if (dn::rows_mma_deep((O + 15) / 16, g_sms)) return own ? LM(0, 8, true) : LM(0, 8, false);
       return own ? LM(0, 4, true) : LM(0, 4, false);
 #undef LM
@@ -1008,7 +1008,7 @@ static cudaError_t mark(dn_seq_model* m, int phase, cudaStream_t s) {
   return cudaEventRecord(ev, s);
 }
 
-// one launch of the tcgen05 GEMM over all experts of a layer (token tiles of MOE_ROWS rows from the plan)
+// one launch of the tcgen05 GEMM over all experts of a layer (token tiles of `width` rows at most, from the plan)
 template <int EPI>
 static cudaError_t gemm_tc_grouped(const CUtensorMap& x, dn::TcParams& p, int width, cudaStream_t s) {
   dn::TcMaps maps;
@@ -1318,7 +1318,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         bool mma = true;
         for (int i = 0; i < sg.n; i++) mma = mma && dn::rows_mma_ok(sg.K[i] > 0 ? sg.K[i] : W, sg.X[i] ? sg.X[i] : m->h, sg.W[i], nullptr);
         if (mma) {
-          const int per = rows >= LM_WIDE ? 32 : 16;
+          const int per = dn::rows_mma_wide(rows, g_sms) ? 32 : 16;
           for (int i = 0; i < sg.n; i++) blocks += (sg.O[i] + per - 1) / per;
           auto kern = per == 32 ? k_linear_mma_multi<1, 4> : dn::rows_mma_deep(blocks, g_sms) ? k_linear_mma_multi<0, 8> : k_linear_mma_multi<0, 4>;
           return launch(kern, dim3(blocks), dim3(dn::RM_THREADS), 0, s, (const bf16*)m->h, sg, N, W);

@@ -1043,9 +1043,8 @@ __global__ void __launch_bounds__(256) k_linear_rows_multi(const T* __restrict__
 }
 
 // The same products on the tensor cores (bf16, K a multiple of 32, 16-byte rows; dn_rows_mma.cuh).  MODE 0: a block takes 16 features;
-// 1: 32 (each token row is read for twice the weights; from LM_WIDE features on, which fill three blocks an SM either way); 2: 16 of two matrices.
+// 1: 32 (each token row is read for twice the weights; rows_mma_wide); 2: 16 of two matrices.
 // The order of a feature's sums is the same in all of them.
-constexpr int LM_WIDE = 7104;
 template <int MODE, int U, bool EP>
 __device__ __forceinline__ void linear_mma_block(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ Wt, const __nv_bfloat16* __restrict__ W2, void* __restrict__ Y,
                                                  bool out32, int N, int O, int K, int act, int o0, float alim, const __nv_bfloat16* __restrict__ bias,

@@ -3,7 +3,7 @@
 Wire format byte-identical to the reference: ``Activation.data`` carries the raw row-major
 element bytes, ``dtype`` names them ("tokens" = int32 ids, "bfloat16"/"float16" tensors).
 The compressed branch (a dtype string containing a pipe character) is dead on the
-reference's live path (SURVEY.md section 2, row 16) and is rejected loudly here.
+reference's live path and is rejected loudly here.
 """
 from __future__ import annotations
 

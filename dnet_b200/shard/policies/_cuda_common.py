@@ -40,7 +40,7 @@ def local_run(rt, current_layer: int) -> List[int]:
 
 
 def more_chunks_follow(msg: ActivationMessage) -> bool:
-    """Chunked prefill (SURVEY.md section 8f N3): a prompt sent as several ``tokens`` frames.  Every frame but
+    """Chunked prefill: a prompt sent as several ``tokens`` frames.  Every frame but
     the last carries ``Activation.batch_size == 0`` (the reference always sends 1 and never reads the field on
     a shard, api/strategies/ring.py:74-140); the flag travels with the activation round the ring
     (build_output copies it), and the finalising shard samples only after the chunk that has it clear."""

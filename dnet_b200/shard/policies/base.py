@@ -56,7 +56,7 @@ class ComputePolicy(ABC):
     @abstractmethod
     def clear(self): ...
 
-    # ---- helpers shared by the fit / offload policies.  Behaviour per SURVEY.md section 8(a) row a5 and the
+    # ---- helpers shared by the fit / offload policies.  Behaviour per the
     #      reference's policy tests (tests/subsystems/test_shard_policy_impl.py:163-257); written against that
     #      behaviour, over this repo's data structures (device-pointer versions, HBM slot recycling).
     @staticmethod

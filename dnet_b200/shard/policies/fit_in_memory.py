@@ -183,7 +183,7 @@ class FitInMemoryPolicy(ComputePolicy):
             ev.record(self.runtime.compute_stream)
 
     def _launch_sched_tp(self, entries, run, arr, first: bool, last: bool) -> None:
-        """Schedule entries with the lm_head tensor-parallel over the ring (DESIGN.md section 4.2).
+        """Schedule entries with the lm_head tensor-parallel over the ring.
 
         Entry i of the ring-wide schedule makes shard r (of S) launch ONE kernel that
           * first serves the head part of the request of entry i - (S - r): by then the last shard has broadcast

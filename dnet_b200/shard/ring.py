@@ -276,7 +276,7 @@ class HeadMesh:
 
 def even_split(num_layers: int, world: int) -> List[List[int]]:
     """contiguous equal splits, k=1 (the manual topology the benchmarks use; HALDA does not
-    balance identical devices, SURVEY.md Appendix B)."""
+    balance identical devices)."""
     base, rem = divmod(num_layers, world)
     out, s = [], 0
     for r in range(world):

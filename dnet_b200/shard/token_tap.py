@@ -1,4 +1,4 @@
-"""TokenTap: how the host *observes* tokens of a device-closed decode loop (SURVEY.md section 8f N2).
+"""TokenTap: how the host *observes* tokens of a device-closed decode loop.
 
 With the token loop closed on the device (the finalising shard's step kernel stores the sampled
 token straight into the head shard's lane slot) no host is on the token's critical path; the API

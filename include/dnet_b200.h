@@ -6,7 +6,7 @@
  * seams are Python plug-in points (ComputePolicy registry, BaseRingModel operator
  * API).  Every entry point below is what a binding for those seams would call; the
  * reference interface each one replaces is cited as file:line relative to
- * /root/reference/.  INTEGRATION.md shows the reference-side ctypes stub.
+ * the reference's tree.
  *
  * Conventions
  *   - plain C: opaque handles, raw device pointers, sizes; no torch / C++ types.
@@ -18,7 +18,7 @@
  *     handles are thread-compatible, not thread-safe.
  *   - activations are row-major [T, hidden] bf16 (the reference's (1,T,H) array with
  *     the unit batch dim dropped); weights are HF/MLX layout [out, in] row-major bf16,
- *     y = x W^T (SURVEY.md Appendix D).
+ *     y = x W^T.
  */
 #ifndef DNET_B200_H
 #define DNET_B200_H
@@ -41,7 +41,7 @@ extern "C" {
 #define DN_DTYPE_BF16 0
 
 /* index of each tensor in the dev_ptrs array handed to dn_bind_layer
- * (SURVEY.md Appendix D; reference utils/model.py:27-43 key regexes) */
+ * (reference utils/model.py:27-43 key regexes) */
 enum {
   DN_W_Q = 0, DN_W_K, DN_W_V, DN_W_O, DN_W_GATE, DN_W_UP, DN_W_DOWN,
   DN_W_LN1, DN_W_LN2,
@@ -67,13 +67,13 @@ typedef struct dn_model_cfg {
   float rms_eps;           /* rms_norm_eps */
   int32_t tie_embeddings;  /* lm_head = embed_tokens (core/models/llama.py:62-66) */
   int32_t dtype;           /* DN_DTYPE_BF16 */
-  int32_t wire_dtype;      /* must equal dtype (mixed wire dtype) */
+  int32_t wire_dtype;      /* must equal dtype (no mixed wire dtype) */
   int32_t kv_page_tokens;  /* 64 */
   int32_t kv_pool_pages;   /* pages in the shard's KV pool (shared by all nonces) */
   int32_t kv_bits;         /* 0: 16-bit KV (mlx_lm KVCache); 4 / 8: affine-quantised KV (QuantizedKVCache,
                               reference utils/model.py:505-554 -- the API's default kv_bits) */
   int32_t kv_group;        /* quantisation group along head_dim: 64 */
-  int32_t n_experts;       /* 0: dense MLP; > 0: sparse MoE FFN (mixtral num_local_experts; BASELINE configs[4]) */
+  int32_t n_experts;       /* 0: dense MLP; > 0: sparse MoE FFN (mixtral num_local_experts) */
   int32_t top_k;           /* experts per token (num_experts_per_tok) */
 } dn_model_cfg;
 
@@ -242,7 +242,7 @@ int dn_hop_send(void* dst_slot, const void* src, size_t bytes, uint32_t* dst_fla
 int dn_hop_wait(const uint32_t* flag, uint32_t seq, uint32_t timeout_ms, uint32_t* err_flag,
                 dn_stream s);
 
-/* measurement hook for the ring-hop latency BASELINE.json's metric names: a (bytes + flag) token makes `iters` trips
+/* measurement hook for the ring-hop latency: a (bytes + flag) token makes `iters` trips
  * around the ring on a lane no request uses, every rank running this on its stream; the origin's *out_ns
  * (device-accessible) receives the elapsed ns of all trips on ITS clock: one hop = out_ns / (iters * ring size). */
 int dn_hop_ring_probe(const void* own_slot, const uint32_t* own_flag, void* next_slot, uint32_t* next_flag,

@@ -6,9 +6,9 @@ product path (dnet_b200/) never does; it fails loudly when the CUDA library is
 missing.
 
 PARITY UNPINNED.  The reference's arithmetic for this path lives in a
-third-party dependency that is absent from /root/reference: ``mlx-lm==0.28.2``
+third-party dependency that the reference's tree does not hold: ``mlx-lm==0.28.2``
 on ``mlx`` (reference pyproject.toml:22,44-46).  The reference's own tests hold
-no golden logits / token ids for any model block (SURVEY.md section 4 and 8c),
+no golden logits / token ids for any model block,
 and mlx cannot be imported here.  This file therefore restates the published
 algorithm of ``mlx_lm.models.llama`` (Attention / MLP / TransformerBlock),
 ``mx.fast.rms_norm``, ``mx.fast.rope`` (non-traditional), ``mx.fast.
@@ -209,7 +209,7 @@ class LlamaOracle:
         # order).  Used only to measure the oracle's own order-sensitivity ("noise floor"):
         # every bf16 rounding point can flip by one ulp when the accumulation order changes,
         # and downstream layers amplify a flip, so two correct implementations of this bf16
-        # pipeline do not agree to 1e-3 end to end (DESIGN.md section "parity").
+        # pipeline do not agree to 1e-3 end to end.
         self.f64_linear = f64_linear
 
     # -- primitives ---------------------------------------------------------
@@ -354,7 +354,7 @@ class LlamaOracle:
 
     def moe_block(self, hn: torch.Tensor, p: str) -> torch.Tensor:
         """Sparse MoE FFN restated from mlx_lm.models.mixtral.MixtralSparseMoeBlock + switch_layers.SwitchGLU
-        (mlx-lm 0.28.2; not in /root/reference -- PARITY UNPINNED like the rest of this file).  The reference hosts
+        (mlx-lm 0.28.2; not in the reference's tree -- PARITY UNPINNED like the rest of this file).  The reference hosts
         MoE families through the same BaseRingModel operator API (core/models/gpt_oss.py, deepseek_v2.py); mixtral is
         BASELINE.json configs[4].
 

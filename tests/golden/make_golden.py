@@ -1,6 +1,6 @@
 """Generate tests/golden/*.npz from the CPU oracle (oracle/llama_oracle.py).
 
-The reference holds no golden vectors for this path (SURVEY.md section 8c: "parity
+The reference holds no golden vectors for this path ("parity
 unpinned"), and mlx cannot be imported here, so the fixtures pin the ORACLE: a later
 change to the oracle or to make_weights() that moves any number fails
 tests/test_oracle.py::test_oracle_matches_golden.  Run from the repo root:

@@ -1,4 +1,4 @@
-"""Chunked prefill, host side (SURVEY.md section 8f N3): the API splits a long prompt into ``tokens`` frames, all but
+"""Chunked prefill, host side: the API splits a long prompt into ``tokens`` frames, all but
 the last flagged ``Activation.batch_size == 0``; the flag survives the proto round trip and the policies' helper reads it."""
 import asyncio
 

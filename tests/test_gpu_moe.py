@@ -1,4 +1,4 @@
-"""-m gpu: sparse MoE FFN layers (mixtral; BASELINE.json configs[4]) through the reference-facing policy / model API
+"""-m gpu: sparse MoE FFN layers (mixtral) through the reference-facing policy / model API
 against the CPU oracle's restatement (oracle/llama_oracle.py moe_block) and the committed fixture
 tests/golden/tiny_mixtral.npz (8 experts, top-2, GQA group 2, 3 layers).  Tolerances as in test_gpu_parity.py:
 per operator on identical inputs the output agrees up to the last bf16 rounding, greedy ids are bit-exact."""
@@ -105,7 +105,7 @@ def test_step_kernel_refuses_moe(moe, cuda_lib):
 
 @pytest.mark.parametrize("T", [16, 63, 65, 200, 512])
 def test_prompt_experts_in_one_grouped_launch(moe, T):
-    """Prompt chunks of 16 tokens and more sort their (token, choice) pairs by expert and run all experts in one grouped launch
+    """Prompt chunks of two tokens and more sort their (token, choice) pairs by expert and run all experts in one grouped launch
     (moe_ffn_tc): experts with no rows, one row, whole tiles and remainders.  Against the oracle's token-by-token loop on the same
     inputs; a result may differ where the last bf16 rounding does (as above)."""
     from oracle.llama_oracle import LlamaOracle, OracleConfig, OracleKV

@@ -383,7 +383,7 @@ def test_error_behaviour_matches_policy_contract(tiny):
 
 
 def test_full_size_llama3_8b_dims_two_layers(cuda_lib):
-    """BASELINE config dims (H=4096, 32/8 heads, FFN 14336, V=128256) on a 2-layer slice:
+    """Llama-3-8B dims (H=4096, 32/8 heads, FFN 14336, V=128256) on a 2-layer slice:
     oracle comparison + the split / graph properties at full width."""
     from dnet_b200.shard.models import ShardLoadModelRequest
     from dnet_b200.shard.runtime import ShardRuntime
@@ -569,8 +569,8 @@ def test_calibrated_partition_does_not_change_results(tiny, cuda_lib):
 
 @pytest.mark.parametrize("plen", [1, 2, 3, 15, 16, 17, 33, 63, 64, 65, 127, 128, 129, 200, 511, 512, 513, 530, 700])
 def test_prompt_length_edges_against_oracle(tiny, cuda_lib, plen):
-    """Ragged prompt lengths around every chunking boundary (GEMV chunks of 1/2/4, tensor-core chunks
-    of 16..512 with 32/64/128-token tiles and out-of-bounds token rows, 64-token KV pages): prefill
+    """Ragged prompt lengths around every boundary of a chunk's kernels (row products up to 16 tokens, the GEMM's
+    token tiles and their out-of-bounds rows, 64-token KV pages): prefill
     logits vs the oracle on the same prompt, then two decode steps that read the KV it wrote."""
     from oracle.llama_oracle import LlamaOracle, OracleConfig, OracleKV
     g, w = tiny
@@ -693,9 +693,9 @@ def test_gpu_error_against_f64_oracle_is_bounded_by_the_fp32_oracles(cuda_lib, n
         asserted         mean_step err(GPU, f64) <= c x mean_step err(fp32, f64),  max_step <= 3 x max_step
     c = 1.5 for the decode path proper (every position through the persistent step kernel): measured 0.95 on
     tiny_llama -- its hidden states are BIT-IDENTICAL to the oracle's for the first five steps (logits differ by
-    1.5e-7, the fp32 rounding of the head) -- and 1.05 on tiny_qwen2_tied (profiles/r02_parity_criterion.txt,
+    1.5e-7, the fp32 rounding of the head) -- and 1.05 on tiny_qwen2_tied (profiles/r02_parity_criterion_first.txt,
     r02_parity_probe.txt).  c = 5 for the paths that run the prompt through the prefill / per-op kernels: measured
-    3.4 on tiny_llama, 1.1 on tiny_qwen2_tied.  tools/perop_bisect.py traced that gap to the per-op attention
+    3.4 on tiny_llama, 1.1 on tiny_qwen2_tied.  That gap comes from the per-op attention
     kernel: on identical q, K, V its fp32 sums differ from the oracle's in the last place, which shows as a
     2-ulp difference in two near-cancelling output elements of layer 1 (everything before is bit-identical) and
     is then amplified by the next RMSNorm + MLP; no rounding point is missing or misplaced."""

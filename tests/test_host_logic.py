@@ -1,5 +1,5 @@
 """GPU-less tests of the host-side mirror.  Each block restates the structural pins the
-reference's own tests hold for this path (SURVEY.md section 8c), mlx-free."""
+reference's own tests hold for this path, mlx-free."""
 import json
 import struct
 import threading

@@ -4,7 +4,7 @@ The first half restates the assertions the reference holds for this layer
 (tests/subsystems/test_ring_adapter.py:43-513, tests/test_stream_manager.py:13-59,
 tests/subsystems/test_shard.py) against the rebuilt classes, mlx-free.  The second half covers
 what the rebuild adds: metadata frames, lane bookkeeping, the head shard's decode schedule, and a
-real two-shard ring over localhost gRPC driven by the API-side adapter (BASELINE config 1)."""
+real two-shard ring over localhost gRPC driven by the API-side adapter."""
 import asyncio
 import queue as pyq
 import types

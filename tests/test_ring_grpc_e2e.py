@@ -1,4 +1,4 @@
-"""BASELINE config 1 end to end through the real transport classes, on CPU: two shards (stub layers)
+"""The pipelined ring end to end through the real transport classes, on CPU: two shards (stub layers)
 and an API node in one process, three localhost gRPC servers, the rebuilt Shard / GrpcServicer /
 RingAdapter / StreamManager on the shards and RingApiAdapter / ShardApiServicer / InferenceManager on
 the API side.  No GPU -> no hop link -> tensor bytes ride the frames (the reference's path); the

@@ -1,4 +1,4 @@
-"""BASELINE config 1 -- two-shard pipelined ring with stub layers, on CPU (no GPU): the wire
+"""Two-shard pipelined ring with stub layers, on CPU (no GPU): the wire
 contract (hand-built protos == reference field numbers), ActivationCodec branches, routing by
 layer_id, the final-token contract, and a world_size-2 gloo run of the same ring.
 

@@ -1,4 +1,4 @@
-"""Layer-swap path (BASELINE config 4 shape): Llama-3-70B dims, one shard holding more layers than
+"""Layer-swap path: Llama-3-70B dims, one shard holding more layers than
 HBM slots; weights live in pinned host memory and are staged per window on the prefetch stream.
 Reports decode tok/s, achieved host->HBM GB/s and the raw pinned cudaMemcpyAsync bandwidth of the box."""
 import ctypes as C, json, os, sys, time

@@ -20,7 +20,6 @@ g = torch.Generator().manual_seed(1234)
 res = {}
 for tc in (1, 0):
     lib.dn_set_option(b"tc_prefill", tc)
-    rt.model.max_prefill_chunk = int(lib.dn_model_max_prefill_chunk(rt.model._h))
     for n in ((128, 2048) if tc else (128,)):
         prompt = torch.randint(0, cfg["vocab_size"], (n,), generator=g).tolist()
         for rep in range(2):

@@ -1,4 +1,4 @@
-"""Measured argument for the wire-dtype restriction (VERDICT r01 item 3, INTEGRATION.md).
+"""Measured argument for the wire-dtype restriction.
 
 The reference's default wire dtype is fp16 (src/dnet/config.py:108-111) and the policy casts the residual
 stream to it after every layer (shard/policies/fit_in_memory.py:105-107).  With bf16 weights MLX promotes
