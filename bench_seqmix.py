@@ -289,7 +289,9 @@ def _run_llama(sz: dict, args, P: int, n_layers: int, flush, dev) -> dict:
     cache.reset()
     x = model.embed(ids)
     t0 = 0
-    for c in _decompose(P, model.max_chunk, model.max_prefill_chunk):
+    big = model.max_prefill_chunk
+    whole, rest = divmod(P, big) if big else (0, P)
+    for c in [big] * whole + ([rest] if big and rest >= 16 else _decompose(rest, model.max_chunk)):
         for li in layers:
             _cabi.check(model._lib.dn_layer_forward_timed(model._h, li, x[t0:t0 + c].data_ptr(), c, cache._h, None, ms5))
             sums = [a + float(b) for a, b in zip(sums, ms5)]

@@ -74,14 +74,9 @@ def _stream_ptr(stream) -> int:
     return int(stream.cuda_stream)
 
 
-def _decompose(T: int, tmax: int, big: int = 0) -> List[int]:
-    """Split T into the chunk sizes of dn_layer_forward and dn_window_forward: 16..``big`` tokens on the tensor-core
-    path (none where ``big`` is 0), the remainder as 4, 2 and 1.  (dn_chunk_forward takes any size.)"""
+def _decompose(T: int, tmax: int) -> List[int]:
+    """Split T into the chunk sizes of the row kernels: 4, 2 and 1, none above ``tmax``."""
     out: List[int] = []
-    while big >= 16 and T >= 16:
-        c = min(T, big)
-        out.append(c)
-        T -= c
     c = 4
     while c > tmax:
         c >>= 1

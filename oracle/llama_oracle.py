@@ -355,8 +355,8 @@ class LlamaOracle:
     def moe_block(self, hn: torch.Tensor, p: str) -> torch.Tensor:
         """Sparse MoE FFN restated from mlx_lm.models.mixtral.MixtralSparseMoeBlock + switch_layers.SwitchGLU
         (mlx-lm 0.28.2; not in the reference's tree -- PARITY UNPINNED like the rest of this file).  The reference hosts
-        MoE families through the same BaseRingModel operator API (core/models/gpt_oss.py, deepseek_v2.py); mixtral is
-        BASELINE.json configs[4].
+        MoE families through the same BaseRingModel operator API (core/models/gpt_oss.py, deepseek_v2.py); mixtral
+        (Mixtral-8x7B) is the one restated here.
 
           gates  = gate(x)                                   Linear, logits rounded to T
           inds   = argpartition(-gates, k-1)[..., :k]        the k largest logits (ties: lowest index first here)

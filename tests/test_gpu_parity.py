@@ -1,7 +1,7 @@
 """-m gpu: the CUDA path (through the reference-facing policy / model API, which calls
 libdnet_b200.so through the C ABI) against the CPU oracle, the committed golden fixtures
 and size-independent properties.  Tolerance for floating point: max|a-b|/max|b| <= 1e-3
-on fp32 logits (north_star); greedy token ids bit-exact."""
+on fp32 logits; greedy token ids bit-exact."""
 import ctypes as C
 import queue
 
@@ -12,7 +12,7 @@ import torch
 from tests.helpers import (load_golden, make_runtime, oracle_weights, rel_inf, ring_generate, token_message)
 
 pytestmark = pytest.mark.gpu
-LOGIT_TOL = 1e-3          # north_star: fp logits within 1e-3 relative -- holds per operator (same inputs)
+LOGIT_TOL = 1e-3          # fp logits within 1e-3 relative -- holds per operator (same inputs)
 
 
 def e2e_tol(g) -> float:
