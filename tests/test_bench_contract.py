@@ -1,4 +1,4 @@
-"""The bench line contract (driver-facing): checked on the committed lines under profiles/, which are
+"""The bench line contract: checked on the committed lines under profiles/, which are
 verbatim stdout of `bench.py` runs on B200 (no GPU needed here)."""
 import json
 from pathlib import Path

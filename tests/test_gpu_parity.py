@@ -261,13 +261,16 @@ def test_offload_and_sliding_fit_match_fit_bit_for_bit(tiny):
             rt.unload_model_core()
 
 
-def test_determinism_graph_vs_eager_and_pdl(tiny, cuda_lib):
+@pytest.mark.parametrize("chunks", [1, 0])
+def test_determinism_graph_vs_eager_and_pdl(tiny, cuda_lib, chunks):
+    """The launches of a chunk's layer are programmatic whatever the option says; those of the row kernels (no tensor-core chunks) are by it."""
     g, w = tiny
     cfgd = g["config"]
     results = []
     for graphs, pdl in ((True, 1), (False, 1), (True, 0), (False, 0), (True, 1)):
-        rt = make_runtime(cfgd, w, range(cfgd["num_hidden_layers"]), cuda_graphs=graphs, megakernel=False)
+        rt = make_runtime(cfgd, w, range(cfgd["num_hidden_layers"]), cuda_graphs=graphs, megakernel=False, max_tokens=2560)
         cuda_lib.dn_set_option(b"pdl", pdl)
+        cuda_lib.dn_set_option(b"tc_prefill", chunks)
         try:
             out = ring_generate([rt], "n0", g["prompt"].tolist(), 10)
             ns = rt._kv_by_nonce["n0"]
@@ -275,6 +278,7 @@ def test_determinism_graph_vs_eager_and_pdl(tiny, cuda_lib):
             torch.cuda.synchronize()
             results.append(([t for t, _, _ in out], [p for _, p, _ in out], f32.cpu()))
         finally:
+            cuda_lib.dn_set_option(b"tc_prefill", 1)
             rt.unload_model_core()
     cuda_lib.dn_set_option(b"pdl", 0)
     for r in results[1:]:
