@@ -154,6 +154,13 @@ static int make_tmap(CUtensorMap* out, const void* base, int rows, int cols, int
   return DN_OK;
 }
 
+// an activation buffer's descriptors, one for each number of rows that a stage may take
+static bool make_xmaps(CUtensorMap (&out)[TC_XMAPS], const void* base, int rows, int cols) {
+  for (int i = 0; i < TC_XMAPS; ++i)
+    if (make_tmap(&out[i], base, rows, cols, TC_XBOX * (i + 1)) != DN_OK) return false;
+  return true;
+}
+
 struct dn_model {
   dn_model_cfg cfg;
   std::vector<int> abs_layers;
@@ -175,7 +182,7 @@ struct dn_model {
   int32_t *moe_psel = nullptr, *moe_plan = nullptr;      // choices [P]; rows of pairs [P], tokens of rows [P], tile table [3][max tiles] + 1
   float* moe_pscore = nullptr;
   CUtensorMap* moe_maps = nullptr;                       // [local layers][3][E]
-  CUtensorMap tm_moe_xg, tm_moe_act;
+  CUtensorMap tm_moe_xg[TC_XMAPS], tm_moe_act[TC_XMAPS];
   int moe_max_tiles = 0;
   bool moe_tc_ok = false;
   StepState* null_state = nullptr;      // zeroed step state + block table for launches without a nonce (head-part only)
@@ -191,7 +198,7 @@ struct dn_model {
   bf16 *xa = nullptr, *xb = nullptr;
   // tensor-core prefill scratch ([CHUNK_MAX][...]) and the TMA descriptors of the activation buffers
   bf16 *pf_xn = nullptr, *pf_qkv = nullptr, *pf_q = nullptr, *pf_attn = nullptr, *pf_h = nullptr, *pf_act = nullptr;
-  CUtensorMap tm_xn, tm_attn, tm_act;
+  CUtensorMap tm_xn[TC_XMAPS], tm_attn[TC_XMAPS], tm_act[TC_XMAPS];
   std::vector<CUtensorMap> tm_kv;                // per local layer: KV pool as [pages*2*n_kv*64 rows][128] bf16, box 64 x 64
   bool tm_kv_ok = false;
   bool pf_ok = false;
@@ -468,8 +475,8 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
     CK(util_fill0(m->pf_act, (size_t)CHUNK_MAX * cfg->ffn * 2));
     m->pf_ok = (H % 128 == 0) && (qd % 128 == 0) && (cfg->ffn % 128 == 0) && ((cfg->n_kv_heads * HD) % 128 == 0) &&
                true;
-    m->pf_ok = m->pf_ok && make_tmap(&m->tm_xn, m->pf_xn, CHUNK_MAX, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_attn, m->pf_attn, CHUNK_MAX, qd, TC_XBOX) == DN_OK &&
-               make_tmap(&m->tm_act, m->pf_act, CHUNK_MAX, cfg->ffn, TC_XBOX) == DN_OK;
+    m->pf_ok = m->pf_ok && make_xmaps(m->tm_xn, m->pf_xn, CHUNK_MAX, H) && make_xmaps(m->tm_attn, m->pf_attn, CHUNK_MAX, qd) &&
+               make_xmaps(m->tm_act, m->pf_act, CHUNK_MAX, cfg->ffn);
     if (cfg->n_experts > 0 && m->pf_ok) {
       const int P = CHUNK_MAX * cfg->top_k, E = cfg->n_experts;
       m->moe_max_tiles = P / 64 + E;
@@ -484,7 +491,7 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
       CK(util_fill0(m->moe_xg, (size_t)P * H * 2));
       CK(util_fill0(m->moe_act, (size_t)P * cfg->ffn * 2));
       for (int i = 0; i < n_layers; ++i) m->layers[i].emaps = m->moe_maps + (size_t)i * 3 * E;
-      m->moe_tc_ok = make_tmap(&m->tm_moe_xg, m->moe_xg, P, H, TC_XBOX) == DN_OK && make_tmap(&m->tm_moe_act, m->moe_act, P, cfg->ffn, TC_XBOX) == DN_OK;
+      m->moe_tc_ok = make_xmaps(m->tm_moe_xg, m->moe_xg, P, H) && make_xmaps(m->tm_moe_act, m->moe_act, P, cfg->ffn);
     }
   }
   *out = m;
@@ -861,10 +868,10 @@ static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, int pdl, cudaStream_
 }
 
 template <int EPI>
-static cudaError_t gemm_tc_grouped(const CUtensorMap& x, TcParams& p, int width, cudaStream_t s) {
+static cudaError_t gemm_tc_grouped(const CUtensorMap (&x)[TC_XMAPS], TcParams& p, int width, cudaStream_t s) {
   TcMaps maps;
-  for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = x;      // (the weights' descriptors lie in global memory)
-  maps.x = x;
+  for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = x[0];      // (the weights' descriptors lie in global memory)
+  memcpy(maps.x, x, sizeof(maps.x));
   if (g_capturing) g_capture_launches++; else g_launches++;
   return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s);
 }
@@ -950,7 +957,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, (const bf16*)x, L.w[DN_W_LN1], m->pf_xn, H, c.rms_eps));
   TcMaps maps;
   for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = L.tm[i < 3 ? i : 0];
-  maps.x = m->tm_xn;
+  memcpy(maps.x, m->tm_xn, sizeof(maps.x));
   p.K = H; p.nseg = 3;      // q, k and v in one launch
   p.seg[0] = TcSeg{qd, qkvd, m->pf_qkv, L.w[DN_W_QB], 0};
   p.seg[1] = TcSeg{kd, qkvd, m->pf_qkv + qd, L.w[DN_W_KB], 0};
@@ -982,7 +989,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   }
   EV(2);
   p.K = qd; p.nseg = 1; p.seg[0] = TcSeg{H, H, m->pf_h, nullptr, 0}; p.resid = x; p.ldr = H;
-  maps.w[0] = L.tm[3]; maps.x = m->tm_attn;
+  maps.w[0] = L.tm[3]; memcpy(maps.x, m->tm_attn, sizeof(maps.x));
   CK(few ? rows_product<EPI_RESID>(p, m->pf_attn, L.w[DN_W_O], nullptr, nullptr, pdl, s) : gemm_tc<EPI_RESID>(maps, p, pdl, s));
   EV(3);
   if (c.n_experts > 0) {
@@ -993,11 +1000,11 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   }
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->pf_h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   p.K = H; p.seg[0] = TcSeg{c.ffn, c.ffn, m->pf_act, nullptr, 0};
-  maps.w[0] = L.tm[4]; maps.w[1] = L.tm[5]; maps.x = m->tm_xn;
+  maps.w[0] = L.tm[4]; maps.w[1] = L.tm[5]; memcpy(maps.x, m->tm_xn, sizeof(maps.x));
   CK(few ? rows_product<EPI_SWIGLU>(p, m->pf_xn, L.w[DN_W_GATE], L.w[DN_W_UP], nullptr, pdl, s) : gemm_tc<EPI_SWIGLU>(maps, p, pdl, s));
   EV(4);
   p.K = c.ffn; p.seg[0] = TcSeg{H, H, x, nullptr, 0}; p.resid = m->pf_h; p.ldr = H;
-  maps.w[0] = L.tm[6]; maps.x = m->tm_act;
+  maps.w[0] = L.tm[6]; memcpy(maps.x, m->tm_act, sizeof(maps.x));
   CK(few ? rows_product<EPI_RESID>(p, m->pf_act, L.w[DN_W_DOWN], nullptr, nullptr, pdl, s) : gemm_tc<EPI_RESID>(maps, p, pdl, s));
   EV(5);
 #undef EV

@@ -7,6 +7,8 @@
 // "swap-AB" orientation: the WEIGHT tile is the MMA's A operand (M = 256 rows per pair of CTAs, 128 each, one TMEM lane a row) and
 // the TOKEN tile is B (up to 256 tokens = TMEM columns, half of them staged by each CTA), because prefill chunks have few tokens
 // and many output features; both operands are K-major in shared memory, exactly what TMA produces from row-major [rows, K] tensors.
+// A stage is three copies of a CTA: 64 + 64 rows of weights, and its half of the tokens in one box.  (With the tokens in boxes of 32 rows the issue of a stage's
+// copies, by one thread, took longer than its MMAs: 18,944 features of 4,096, 2,048 tokens 314 us -> 212; 1,000 tokens 174 -> 120.)
 // An SM takes about 64 bytes a cycle from L2: a 128 x 128 tile of one CTA needs 128 for full tensor rate, 128 x 256 of a pair's
 // half 64.  A tile is therefore as wide in tokens as the chunk allows (TcPlan), and where that leaves too few tiles for the SMs
 // the reduction is split over the S pairs of a cluster, which add their accumulators through distributed shared memory in a fixed
@@ -49,7 +51,8 @@ __host__ __device__ constexpr bool epi_two_weights(int epi) { return epi == EPI_
 
 constexpr int TC_BK = 64;         // k-step: 64 bf16 = 128 bytes = one swizzle span
 constexpr int TC_WBOX = 64;       // rows of a weight descriptor's box
-constexpr int TC_XBOX = 32;       // rows of an activation descriptor's box
+constexpr int TC_XBOX = 32;       // rows of an activation descriptor's box, or twice, three or four times as many (TcMaps::x)
+constexpr int TC_XMAPS = 4;
 constexpr int TC_WMAX = 256;      // tokens of a tile at most
 constexpr int TC_THREADS = 384;
 constexpr int TC_EWARPS = 8;
@@ -69,7 +72,7 @@ struct TcSeg {                    // one product of a launch
 };
 struct TcMaps {
   CUtensorMap w[TC_SEGS];         // two-weight forms: [0] gate, [1] up
-  CUtensorMap x;
+  CUtensorMap x[TC_XMAPS];        // the tokens, in boxes of TC_XBOX (i + 1) rows
 };
 struct TcParams {
   int T, K;                       // tokens, reduction
@@ -328,6 +331,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
         }
         const int r0 = GLU ? tl_.n0 + rank * 64 : tl_.n0 + rank * 128, r1 = GLU ? r0 : r0 + 64;
         const int x0 = tl_.t0 + rank * (tl_.cols / 2), boxes = (tl_.cols / 2 + TC_XBOX - 1) / TC_XBOX;
+        const CUtensorMap* mx = &maps.x[boxes - 1];
         const uint32_t bytes = 2u * (TC_A_BYTES + boxes * (TC_XBOX * TC_BK * 2));
         for (int ks = k0; ks < k1; ++ks) {
           mbar_wait(&empty[stage], phase ^ 1u, p.err);
@@ -336,8 +340,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
           unsigned char* sa = smem + (size_t)stage * stage_bytes;
           tma_load_2d_pair(sa, mw, ks * TC_BK, r0, bar);
           tma_load_2d_pair(sa + TC_A_BYTES / 2, mw2, ks * TC_BK, r1, bar);
-          for (int i = 0; i < boxes; ++i)
-            tma_load_2d_pair(sa + TC_A_BYTES + i * (TC_XBOX * TC_BK * 2), &maps.x, ks * TC_BK, x0 + i * TC_XBOX, bar);
+          tma_load_2d_pair(sa + TC_A_BYTES, mx, ks * TC_BK, x0, bar);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }

@@ -55,7 +55,7 @@ static size_t g_max_smem = 0;
 
 // weight matrices and the activation buffers they multiply get TMA descriptors in bf16 mode
 struct XMaps {
-  CUtensorMap m;
+  CUtensorMap m[dn::TC_XMAPS];       // boxes of dn::TC_XBOX (i + 1) rows
   bool ok = false;
 };
 struct SeqLayer {
@@ -74,8 +74,7 @@ struct SeqLayer {
   const void** etab_d;
   CUtensorMap* emaps_d;              // [3][E] TMA descriptors of the experts' matrices, in device memory (bf16 mode)
   std::vector<char> emap_ok;
-  CUtensorMap x_eact;                // the experts' activations [pairs, ff]
-  bool x_eact_ok;
+  XMaps x_eact;                      // the experts' activations [pairs, ff]
 };
 // One run of a layer.  A layer inside the loop runs loop_times times on the same weights; every run has its own
 // pages, carried inputs and recurrent state.
@@ -93,8 +92,9 @@ struct dn_seq_model {
   std::vector<Run> runs;
   const void *embed = nullptr, *final_norm = nullptr, *head = nullptr;
   const void* mw[16] = {nullptr};     // the other model tensors, by (which - DN_SQ_EMBED)
-  CUtensorMap tm_loop_in, x_xg;       // x_xg: the tokens' rows sorted by expert [pairs, W]
-  bool tm_loop_ok = false, x_xg_ok = false;
+  CUtensorMap tm_loop_in;
+  XMaps x_xg;                         // the tokens' rows sorted by expert [pairs, W]
+  bool tm_loop_ok = false;
   void* xg = nullptr;
   float* attn_part = nullptr;         // partials of split attention rows [AT_SPLIT_ROWS][heads][AT_MAX_SPLITS][2 + vdim padded]
   XMaps x_cat, x_xm[SHIFT_MAX], x_side;
@@ -208,8 +208,10 @@ static bool sig_tc_sizes(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {
   return cfg.dtype == DN_SEQ_BF16 && (c.mixer == DN_MIX_ATTENTION || c.mixer == DN_MIX_PARALLEL) && c.attn_weight == DN_ATTN_SIGMOID && c.softcap <= 0.f && c.pool == 0 && c.keep_first == 0 &&
          (c.dim == 64 || c.dim == 128) && (c.vdim == 64 || c.vdim == 128) && (size_t)c.heads * dist_span(cfg, c) <= DIST_TAB_MAX;
 }
+// an activation buffer's descriptors, one for each number of rows that a stage of the GEMM may take
 static void make_xmaps(XMaps* x, const void* base, int rows, int cols) {
-  x->ok = make_tmap(&x->m, base, rows, cols, dn::TC_XBOX);
+  x->ok = true;
+  for (int i = 0; i < dn::TC_XMAPS; ++i) x->ok = x->ok && make_tmap(&x->m[i], base, rows, cols, dn::TC_XBOX * (i + 1));
 }
 
 static int n_maps(const dn_seq_layer_cfg& c) { return c.maps == 2 ? 2 : 1; }
@@ -325,7 +327,7 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
     l.c = layers[i];
     memset(l.w, 0, sizeof(l.w));
     memset(l.tm_ok, 0, sizeof(l.tm_ok));
-    l.x_eact_ok = false;
+    l.x_eact.ok = false;
     l.Rc = l.Rv = l.Cql = l.Col = 0;
     const dn_seq_layer_cfg& c = l.c;
     if (c.heads <= 0 || c.kv_heads <= 0 || c.heads % c.kv_heads || c.dim <= 0 || c.vdim <= 0) {
@@ -596,10 +598,10 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
       if (fa > 0) make_xmaps(&l.x_act, m->act, m->MB, fa);
     }
     if (m->xg) {
-      m->x_xg_ok = make_tmap(&m->x_xg, m->xg, m->MB * mpairs, cfg->width, dn::TC_XBOX);
+      make_xmaps(&m->x_xg, m->xg, m->MB * mpairs, cfg->width);
       for (auto& l : m->L)
         if (l.c.mlp_kind == DN_MLP_MOE && l.c.ff > 0)
-          l.x_eact_ok = make_tmap(&l.x_eact, m->eact, m->MB * l.c.top, l.c.ff, dn::TC_XBOX);
+          make_xmaps(&l.x_eact, m->eact, m->MB * l.c.top, l.c.ff);
     }
     if (cfg->side_dim > 0) make_xmaps(&m->x_side, m->act, m->MB, cfg->side_dim);
     if (m->cat) make_xmaps(&m->x_cat, m->cat, m->MB, 2 * cfg->width);
@@ -765,7 +767,7 @@ static cudaError_t gemm_tc(const CUtensorMap& w, const CUtensorMap& w2, const XM
   dn::TcMaps maps;
   maps.w[0] = maps.w[2] = maps.w[3] = w;
   maps.w[1] = w2;
-  maps.x = x.m;
+  memcpy(maps.x, x.m, sizeof(maps.x));
   return gemm_tc<EPI>(maps, p, s);
 }
 
@@ -1010,10 +1012,10 @@ static cudaError_t mark(dn_seq_model* m, int phase, cudaStream_t s) {
 
 // one launch of the tcgen05 GEMM over all experts of a layer (token tiles of `width` rows at most, from the plan)
 template <int EPI>
-static cudaError_t gemm_tc_grouped(const CUtensorMap& x, dn::TcParams& p, int width, cudaStream_t s) {
+static cudaError_t gemm_tc_grouped(const XMaps& x, dn::TcParams& p, int width, cudaStream_t s) {
   dn::TcMaps maps;
-  for (int i = 0; i < dn::TC_SEGS; ++i) maps.w[i] = x;      // (the weights' descriptors lie in global memory)
-  maps.x = x;
+  for (int i = 0; i < dn::TC_SEGS; ++i) maps.w[i] = x.m[0];      // (the weights' descriptors lie in global memory)
+  memcpy(maps.x, x.m, sizeof(maps.x));
   g_launches++;
   return dn::tc_launch<EPI, true>(maps, p, dn::TcPlan{width, 1, dn::tc_stages(width), g_sms / 2 * 2}, s);
 }
@@ -1049,7 +1051,7 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
   } else {
     MoePlan pl{m->rpos, m->rtok, m->tiles, m->tiles + m->max_tiles, m->tiles + 2 * m->max_tiles, m->tiles + 3 * m->max_tiles};
     const int mt = std::min(m->max_tiles, P / MOE_ROWS + E + 1);
-    bool tc = std::is_same<T, bf16>::value && m->x_xg_ok && l.x_eact_ok && l.emaps_d && lc.ff >= 32 && W >= 32;
+    bool tc = std::is_same<T, bf16>::value && m->x_xg.ok && l.x_eact.ok && l.emaps_d && lc.ff >= 32 && W >= 32;
     for (size_t i = gated ? 0 : E; i < l.emap_ok.size(); i++) tc = tc && l.emap_ok[i];
     // rows of a token tile: by the plan of the tcgen05 GEMM; the CUDA-core tiles are 64 rows
     const int feat = gated ? 128 : 256, tile_rows = tc ? dn::tc_grouped_width((lc.ff + feat - 1) / feat, E, P, g_sms) : MOE_ROWS;
@@ -1254,7 +1256,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       }
     if (ok && p.nseg > 1) {
       for (int i = p.nseg; i < dn::TC_SEGS; ++i) maps.w[i] = maps.w[0];
-      maps.x = xm.m;
+      memcpy(maps.x, xm.m, sizeof(maps.x));
       p.T = N; p.K = K; p.err = m->tc_err;
       return o32 ? gemm_tc<dn::EPI_STORE_F32>(maps, p, s) : gemm_tc<dn::EPI_STORE>(maps, p, s);
     }
