@@ -883,7 +883,7 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   const dn_model_cfg& c = m->cfg;
   const int H = c.hidden, E = c.n_experts, k = c.top_k, P = T * k, mt = m->moe_max_tiles, Pmax = CHUNK_MAX * k;
   MoePlan pl{m->moe_plan, m->moe_plan + Pmax, m->moe_plan + 2 * Pmax, m->moe_plan + 2 * Pmax + mt, m->moe_plan + 2 * Pmax + 2 * mt, m->moe_plan + 2 * Pmax + 3 * mt};
-  const int width = tc_grouped_width((c.ffn + 127) / 128, E, P, g_sms);
+  const int width = tc_grouped_width(E, P, g_sms);
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   CK(launch(k_moe_route, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
   CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, false, (const int32_t*)m->moe_psel, P, k, E, width, pl, E));

@@ -41,6 +41,7 @@
 // launch).  The number of token tiles is read from device memory, so the host never learns the routing.
 #pragma once
 #include <cuda.h>
+#include <math.h>
 #include <string.h>
 #include "dn_megakernel.cuh"
 
@@ -693,15 +694,22 @@ static inline TcPlan tc_plan(int n_tiles, int T, int K, int sms) {
   best.grid = best.split > 1 ? 2 * best.split * tl.units : 2 * (tl.units < sms / 2 ? tl.units : sms / 2);
   return best;
 }
-// rows of a grouped launch's tiles: P rows over E matrices, taken as equal shares (a tile computes no more rows than it has)
-static inline int tc_grouped_width(int n_tiles, int E, int P, int sms) {
-  const int avg = (P + E - 1) / E, pairs = sms / 2;
+// Rows of a grouped launch's tiles: P rows over E matrices, whose shares are taken to lie within a third of the average.  A matrix with one row more than
+// a tile has takes a second one, which reads its weights again and fills a few columns, so the width keeps a distance from the average; a wider
+// stage leaves fewer of them for the way of 2.5 us that each takes through the ring.  (Mixtral-8x7B, 500 tokens, 125 rows an expert: a layer 813 us with
+// tiles of 128 rows, 709 with 192.)
+static inline int tc_grouped_width(int E, int P, int sms) {
   int best = 64;
-  long long cost = 0;
-  for (int w = 64; w <= TC_WMAX; w *= 2) {
-    const int cols = avg < w ? (avg + 15) & ~15 : w;
-    const long long c = (long long)(n_tiles * E * ((avg + w - 1) / w) + pairs - 1) / pairs * (256 + cols);
-    if (w == 64 || c < cost) { cost = c; best = w; }
+  double cost = 0;
+  for (int w = 64; w <= TC_WMAX; w += 32) {
+    double c = 0;
+    for (int i = -2; i <= 2; ++i) {
+      const int rows = (int)ceil(P * (1.0 + i / 6.0) / E), tiles = (rows + w - 1) / w, cols = rows < w ? (rows + 15) & ~15 : w;
+      const int bytes = TC_A_BYTES + (cols / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
+      const double way = 2.5 / tc_stages(w), copies = sms * (double)bytes / 10.8e6;
+      c += tiles * (way > copies ? way : copies);
+    }
+    if (w == 64 || c < cost * 0.999) { cost = c; best = w; }
   }
   return best;
 }

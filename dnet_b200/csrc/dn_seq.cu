@@ -1054,7 +1054,7 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
     bool tc = std::is_same<T, bf16>::value && m->x_xg.ok && l.x_eact.ok && l.emaps_d && lc.ff >= 32 && W >= 32;
     for (size_t i = gated ? 0 : E; i < l.emap_ok.size(); i++) tc = tc && l.emap_ok[i];
     // rows of a token tile: by the plan of the tcgen05 GEMM; the CUDA-core tiles are 64 rows
-    const int feat = gated ? 128 : 256, tile_rows = tc ? dn::tc_grouped_width((lc.ff + feat - 1) / feat, E, P, g_sms) : MOE_ROWS;
+    const int tile_rows = tc ? dn::tc_grouped_width(E, P, g_sms) : MOE_ROWS;
     CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * Et + 1) * 4, s, (const int32_t*)m->ridx, P, top, Et, tile_rows, pl, E));
     if (tc) {     // bf16 with TMA-able shapes: every expert's tiles in one launch of the tcgen05 GEMM
       CK(launch(k_moe_gather<T>, dim3(P), dim3(128), 0, s, (const T*)m->h, (const int32_t*)m->rtok, W, (T*)m->xg));
