@@ -9,6 +9,7 @@
 #include "dn_rows.cuh"
 #include "dn_attn_tc.cuh"
 #include "dn_attn_q.cuh"
+#include "dn_attn_few.cuh"
 #include "dn_moe.cuh"
 #include "../../include/dnet_b200.h"
 
@@ -202,6 +203,10 @@ struct dn_model {
   std::vector<CUtensorMap> tm_kv;                // per local layer: KV pool as [pages*2*n_kv*64 rows][128] bf16, box 64 x 64
   bool tm_kv_ok = false;
   bool pf_ok = false;
+  // attention of a few tokens: partial outputs of a key head's splits, and how many of them have finished
+  float* few_part = nullptr;
+  unsigned int* few_count = nullptr;
+  int few_splits = 1;
   bool pf_last = false;      // the last chunk ran on the prompt kernels (dn_debug_scratch)
   unsigned long long* mk_dbg = nullptr;
   size_t mk_dbg_words = 0;
@@ -305,6 +310,8 @@ static cudaError_t init_kernel_attrs() {
 #define ATA(Gv, Pv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv, Pv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
   ATA(1, 2) ATA(2, 2) ATA(4, 2) ATA(8, 2) ATA(1, 3) ATA(2, 3) ATA(4, 3) ATA(5, 3) ATA(7, 3) ATA(8, 3)
 #undef ATA
+  if ((e = cudaFuncSetAttribute(k_attn_few<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_attn_few<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess) return e;
 #define ATQ(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess || \
                     (e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess) return e;
   ATQ(1) ATQ(2) ATQ(4) ATQ(5) ATQ(7) ATQ(8)
@@ -470,6 +477,10 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
     CK(cudaMalloc(&m->pf_attn, (size_t)CHUNK_MAX * qd * 2));
     CK(cudaMalloc(&m->pf_h, (size_t)CHUNK_MAX * H * 2));
     CK(cudaMalloc(&m->pf_act, (size_t)CHUNK_MAX * cfg->ffn * 2));
+    m->few_splits = g_sms / cfg->n_kv_heads < 1 ? 1 : g_sms / cfg->n_kv_heads > FEW_SPLITS ? FEW_SPLITS : g_sms / cfg->n_kv_heads;
+    CK(cudaMalloc(&m->few_part, (size_t)cfg->n_kv_heads * m->few_splits * (FEW_ROWS / 16) * FEW_PART * sizeof(float)));
+    CK(cudaMalloc(&m->few_count, (size_t)cfg->n_kv_heads * sizeof(unsigned int)));
+    CK(util_fill0(m->few_count, (size_t)cfg->n_kv_heads * sizeof(unsigned int)));
     CK(util_fill0(m->pf_xn, (size_t)CHUNK_MAX * H * 2));
     CK(util_fill0(m->pf_attn, (size_t)CHUNK_MAX * qd * 2));
     CK(util_fill0(m->pf_act, (size_t)CHUNK_MAX * cfg->ffn * 2));
@@ -502,6 +513,7 @@ extern "C" int dn_model_destroy(dn_model* m) {
   if (!m) return DN_OK;
   cudaFree(m->hbuf); cudaFree(m->qbuf); cudaFree(m->attn); cudaFree(m->act); cudaFree(m->logits_bf16);
   cudaFree(m->part); cudaFree(m->tickets); cudaFree(m->head_part); cudaFree(m->inv_freq); cudaFree(m->kv_pool);
+  cudaFree(m->few_part); cudaFree(m->few_count);
   cudaFree(m->mk_bounds); cudaFree(m->pf_xn); cudaFree(m->pf_qkv); cudaFree(m->pf_q); cudaFree(m->pf_attn); cudaFree(m->pf_h); cudaFree(m->pf_act);
   cudaFree(m->mk_dbg); cudaFree(m->mk_dev); cudaFree(m->xa); cudaFree(m->xb); cudaFree(m->mk_sync);
   cudaFree(m->null_state); cudaFree(m->null_bt);
@@ -970,6 +982,12 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
   if (kvq) {
     const int rc = kvq_append_and_attend(m, li, m->pf_q, m->pf_attn, T, kv, pdl, true, s);
     if (rc) return rc;
+  } else if (g_tc_attn && m->G * T <= FEW_ROWS) {
+    FewParams a;
+    a.q = m->pf_q; a.pool = pool; a.out = m->pf_attn; a.block_table = kv->block_table; a.st = kv->st;
+    a.part = m->few_part; a.count = m->few_count;
+    a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.G = m->G; a.T = T;
+    CK(launch(m->G * T <= 16 ? k_attn_few<1> : k_attn_few<2>, dim3(c.n_kv_heads, m->few_splits), dim3(FEW_THREADS), FEW_SMEM, s, pdl, a));
   } else if (g_tc_attn && m->tm_kv_ok) {
     AtParams a;
     a.q = m->pf_q; a.out = m->pf_attn; a.block_table = kv->block_table; a.st = kv->st;

@@ -77,6 +77,26 @@ def test_prefill_attention_groups_and_key_shares(cuda_lib, group, context, T):
     _agree(out[1], out[0])
 
 
+@pytest.mark.parametrize("group,context,T", [(1, 0, 1), (1, 63, 32), (2, 127, 8), (2, 128, 16), (4, 0, 3), (4, 2552, 8), (4, 500, 4), (5, 1300, 6), (7, 255, 2), (8, 2400, 4)])
+def test_attention_of_a_few_tokens(cuda_lib, group, context, T):
+    """k_attn_few against the CUDA-core kernel: one and two tiles of 16 rows, whole and ragged, one key tile (no partial outputs), page and tile edges
+    inside the new tokens, more key tiles than CTAs of a key head."""
+    m = _model(8 if context > 2500 else 2, group, seed=group)
+    kv = m.make_cache(max_tokens=2560)
+    x = torch.randn(context + T, 512, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    out = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_attn", tc)
+            out[tc] = _call(m, kv, x, context)
+        assert cuda_lib.dn_step_error(m._h, 0) == 0
+    finally:
+        cuda_lib.dn_set_option(b"tc_attn", 1)
+        kv.free()
+        m.destroy()
+    _agree(out[1], out[0])
+
+
 @pytest.mark.parametrize("hidden,ffn,kv_heads,group,T", [(256, 8192, 2, 1, 17), (256, 8192, 2, 1, 45), (768, 1280, 1, 2, 65), (1024, 14336, 2, 4, 129),
                                                          (512, 2048, 2, 2, 300), (768, 27648, 1, 4, 512)])
 def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_heads, group, T):
