@@ -53,14 +53,15 @@ static_assert(128 * AT_REGS_MMA + 256 * AT_REGS_SOFTMAX <= AT_THREADS * 168, "se
 // CTAs that share a row block's keys: what makes (waves of CTAs) x (key tiles of a CTA + 4 for its start, joining and end) smallest.
 // The grid alone (heads x row blocks) leaves most SMs idle when a chunk is short, and a last wave nearly empty when it is long:
 // 40 heads in groups of 5, 512 tokens give 168 CTAs for 148 SMs.
-// The count takes every SM for usable by every cluster, while 33 clusters of four or 15 of eight run at once: behind 8,192 tokens these 168 row blocks
-// take 234 us with Z = 2 and 269 with the chosen 4 (8 row blocks behind 8,192, one token: 76, 48 and 33 us with 2, 4 and 8).
+// Of 148 SMs 74 clusters of two run at once, 33 of four and 15 of eight (asked of the device): behind 8,192 tokens these 168 row blocks take 234 us with
+// Z = 2 and 269 with 4, which a count that takes every SM for usable by every cluster prefers (a layer 798 us so, 770 now).
 __host__ __device__ inline int attn_prefill_split(int ctas, int kv_len, int sms) {
   const int tiles = (kv_len + 127) / 128;
   int best = 1, cost = 0;
   for (int Z = 1; Z <= AT_MAX_Z; Z *= 2) {
     if (Z > 1 && tiles < 2 * Z) break;
-    const int c = ((ctas * Z + sms - 1) / sms) * ((tiles + Z - 1) / Z + (Z > 1 ? 6 : 4));
+    const int at_once = Z == 1 ? sms : Z == 2 ? sms / 2 : Z == 4 ? sms * 33 / 148 : sms * 15 / 148;
+    const int c = ((ctas + at_once - 1) / at_once) * ((tiles + Z - 1) / Z + (Z > 1 ? 6 : 4));
     if (Z == 1 || c < cost) { cost = c; best = Z; }
   }
   return best;
