@@ -12,11 +12,11 @@
 //       bf16 by definition; a tile's product and its bias terms join fp32 sums of the row's thread)
 // Eight warps turn a tile's codes into operands.
 //
-// Bound by the softmax warps, a row's thread of which forms every score twice, beside the conversion.  777 tokens behind 1,024 (8 x 4 heads, 8 bits):
-// 247 us; one token behind 8,000 84 us.  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
+// Bound by the softmax warps, which form every score twice, beside the conversion.  777 tokens behind 1,024 (8 x 4 heads, 8 bits): 237 us with a thread a row,
+// whose one warp a scheduler waits for itself, 198 with two; one token behind 8,000 84 us (a thread a row).  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
 // tiles: 240 and 82.  Of the stored results 1.56 % and 2.64 % then were not the nearest to 64 bits; now 0.19 % and 0.17 %; k_attn_q, whose
 // block per (head, token) takes 4.1 ms and 1.4 ms, 0.26 % and 0.66 %.)
-// Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-7 softmax (a thread a row), warps 8-15 conversion.
+// Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-11 softmax (a thread a row and half of its keys), warps 12-19 conversion.
 #pragma once
 #include "dn_attn_tc.cuh"
 #include "dn_kvquant.cuh"
@@ -27,29 +27,24 @@ struct AqParams {
   AtParams a;
   const unsigned char* pool;     // this layer's packed pages
 };
-constexpr int AQT_THREADS = 512, AQT_DQ = 256;
+constexpr int AQT_THREADS = 640, AQT_DQ = 256;
 constexpr int AQT_KB = 4 * 128;      // floats of a key tile: scales of both groups, biases of both groups
-constexpr int AQT_XCH = (4 * AQT_KB + 128 * 2 + AT_MAX_Z * 2 * 128) * 4;      // four key tiles' scales and biases, value biases, the ranks' maxima and sums
+constexpr int AQT_XCH = (4 * AQT_KB + 128 * 2 + 2 * AT_MAX_Z * 2 * 128 + 2 * 128) * 4;      // four key tiles' scales and biases, value biases, the maxima and sums of
+                                                                                             // both halves of every rank, the halves' bias terms
 constexpr int AQT_SMEM = 5 * AT_TILE + AQT_XCH + 1024 + 256;
-constexpr int AQT_REGS_MMA = 64, AQT_REGS_SOFTMAX = 224, AQT_REGS_DQ = 112;      // setmaxnreg: of the 128 a thread that 512 threads are launched with
-static_assert(128 * (AQT_REGS_MMA + AQT_REGS_SOFTMAX + 2 * AQT_REGS_DQ) <= AQT_THREADS * 128, "setmaxnreg split exceeds the CTA's launch allocation");
+constexpr int AQT_REGS_MMA = 64, AQT_REGS_SOFTMAX = 136, AQT_REGS_DQ = 72;      // setmaxnreg: of the 96 a thread that 640 threads are launched with
+static_assert(128 * (AQT_REGS_MMA + 2 * AQT_REGS_SOFTMAX + 2 * AQT_REGS_DQ) <= AQT_THREADS * 96, "setmaxnreg split exceeds the CTA's launch allocation");
 
-// 16 (8) consecutive 32-bit columns of this warp's TMEM quarter
-__device__ __forceinline__ void tm_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+// 8 (4) consecutive 32-bit columns of this warp's TMEM quarter
+__device__ __forceinline__ void tm_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-__device__ __forceinline__ void tm_pin16(uint32_t (&r)[16]) {      // no use of r moves above this point
-#pragma unroll
-  for (int i = 0; i < 16; i += 8)
-    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
+__device__ __forceinline__ void tm_pin8(uint32_t (&r)[8]) {      // no use of r moves above this point
+  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
 }
-__device__ __forceinline__ void tm_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+__device__ __forceinline__ void tm_st4(uint32_t taddr, const uint32_t (&r)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 
 template <int G, int BITS>
@@ -64,14 +59,15 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   unsigned char *sQ = smem, *sK = smem + AT_TILE, *sV = smem + 3 * AT_TILE;      // K: two tiles in turn; V: hi tile, lo tile
   float* kb = reinterpret_cast<float*>(smem + 5 * AT_TILE);                      // [4][scale 0, scale 1, bias 0, bias 1][128 keys]
   float2* vb = reinterpret_cast<float2*>(kb + 4 * AQT_KB);                       // [128]: (bias of group 0, of group 1) of a value row
-  float* zx = reinterpret_cast<float*>(vb + 128);                                // [Z][2][128]
+  float* zx = reinterpret_cast<float*>(vb + 128);                                // [Z][2 halves][2][128]
+  float* obx = zx + 2 * AT_MAX_Z * 256;                                          // [2][128]
   float* zo = reinterpret_cast<float*>(sK);                                      // [Z][128 / Z][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 5 * AT_TILE + AQT_XCH);
   uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 5, *s_full = bars + 6, *s_empty = bars + 8, *p_full = bars + 10;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, z = blockIdx.z;
+  const int kvh = blockIdx.x, t0 = (int)(gridDim.y - 1 - blockIdx.y) * TB, z = blockIdx.z;      // (the longest row blocks first)
   const int pos0 = p.st->pos;
   const int Z = p.share > 0 ? p.share : attn_prefill_split((int)(gridDim.x * gridDim.y), pos0 + p.T, p.sms);
   const int nq = min(TB, p.T - t0);
@@ -81,7 +77,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], AQT_DQ / 32); mbar_init(&k_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
-    mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1); mbar_init(p_full, 4);
+    mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1); mbar_init(p_full, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -152,10 +148,10 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     }
     __syncwarp();
     if (Z > 1) { cluster_sync(); cluster_sync(); }
-  } else if (warp < 8) {
-    // ===================== softmax, a thread a row =====================
+  } else if (warp < 12) {
+    // ===================== softmax: warps 4-7 take the first half of every tile's keys, warps 8-11 the second, a thread a row =====================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AQT_REGS_SOFTMAX));
-    const int qd = warp & 3, r = qd * 32 + lane;      // TMEM lane quarter, this thread's row
+    const int h = (warp - 4) >> 2, qd = warp & 3, r = qd * 32 + lane;      // half of the keys, and of the output's columns; TMEM lane quarter, this thread's row
     const int rg = r / TB, rt = r % TB;
     const bool ok = rg < G && rt < nq;
     const int last = ok ? pos0 + t0 + rt : -1;        // last visible key position
@@ -167,19 +163,19 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       const float f = ((bf_lo(v.x) + bf_hi(v.x)) + (bf_lo(v.y) + bf_hi(v.y))) + ((bf_lo(v.z) + bf_hi(v.z)) + (bf_lo(v.w) + bf_hi(v.w)));
       if (c < 8) sq0 += f; else sq1 += f;
     }
-    // Sixteen keys of a half tile at a time: ask for the products of both groups, and, behind tm_wait_ld, the scores rounded to bf16; keys that the
-    // row does not see: -inf.  it, j: the tile, h: its half, c: 0, 16, 32 or 48
-    auto ask = [&](int h, int c, uint32_t (&a)[16], uint32_t (&b)[16]) {
-      tm_ld16(tmem + h * 128 + lane_off + c, a);
-      tm_ld16(tmem + h * 128 + 64 + lane_off + c, b);
+    // Eight keys of the half tile at a time: ask for the products of both groups, and, behind tm_wait_ld, the scores rounded to bf16; keys that the
+    // row does not see: -inf.  it, j: the tile, c: 0, 8, .. 56
+    auto ask = [&](int c, uint32_t (&a)[8], uint32_t (&b)[8]) {
+      tm_ld8(tmem + h * 128 + lane_off + c, a);
+      tm_ld8(tmem + h * 128 + 64 + lane_off + c, b);
     };
-    auto scores_of = [&](int it, int j, int h, int c, uint32_t (&a)[16], uint32_t (&b)[16], float2 (&s)[8]) {
-      tm_pin16(a);
-      tm_pin16(b);
+    auto scores_of = [&](int it, int j, int c, uint32_t (&a)[8], uint32_t (&b)[8], float2 (&s)[4]) {
+      tm_pin8(a);
+      tm_pin8(b);
       const float4* kf = reinterpret_cast<const float4*>(kb + (it & 3) * AQT_KB + h * 64 + c);
       const int key = ((j0 + j) << 7) + h * 64 + c;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
         const float4 s0 = kf[i], s1 = kf[32 + i], b0 = kf[64 + i], b1 = kf[96 + i];
         auto two = [&](int e, float2 c0, float2 c1, float2 d0, float2 d1) {
           const float2 x = f2_fma(make_float2(__uint_as_float(a[e]), __uint_as_float(a[e + 1])), c0,
@@ -190,9 +186,9 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
         two(4 * i, make_float2(s0.x, s0.y), make_float2(s1.x, s1.y), make_float2(b0.x, b0.y), make_float2(b1.x, b1.y));
         two(4 * i + 2, make_float2(s0.z, s0.w), make_float2(s1.z, s1.w), make_float2(b0.z, b0.w), make_float2(b1.z, b1.w));
       }
-      if (!__all_sync(0xffffffffu, !ok || key + 15 <= last)) {
+      if (!__all_sync(0xffffffffu, !ok || key + 7 <= last)) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           if (key + 2 * i > last) s[i].x = -INFINITY;
           if (key + 2 * i + 1 > last) s[i].y = -INFINITY;
         }
@@ -200,50 +196,54 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     };
     // ---- first walk: maxima and sums
     for (int j = 0; j < n_tiles; ++j) {
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        // (the key scales were written before the products that these barriers count were issued; their places are used again four tiles later)
-        mbar_wait(&s_full[h], (uint32_t)j & 1u, p.err);
-        __syncwarp();
-        tc_fence_after();
-        uint32_t a[2][16], b[2][16];
-        ask(h, 0, a[0], b[0]);
+      // (the key scales were written before the products that these barriers count were issued; their places are used again four tiles later)
+      mbar_wait(&s_full[h], (uint32_t)j & 1u, p.err);
+      __syncwarp();
+      tc_fence_after();
+      uint32_t a[2][8], b[2][8];
+      ask(0, a[0], b[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float2 s[8];
-          tm_wait_ld();
-          if (c < 3) ask(h, 16 * c + 16, a[(c + 1) & 1], b[(c + 1) & 1]);
-          scores_of(j, j, h, 16 * c, a[c & 1], b[c & 1], s);
-          float2 x2 = s[0];
+      for (int c = 0; c < 8; ++c) {
+        float2 s[4];
+        tm_wait_ld();
+        if (c < 7) ask(8 * c + 8, a[(c + 1) & 1], b[(c + 1) & 1]);
+        scores_of(j, j, 8 * c, a[c & 1], b[c & 1], s);
+        float2 x2 = s[0];
 #pragma unroll
-          for (int i = 1; i < 8; ++i) x2 = make_float2(fmaxf(x2.x, s[i].x), fmaxf(x2.y, s[i].y));
-          const float mx = fmaxf(m, fmaxf(x2.x, x2.y));
-          const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
-          float2 e2 = f2_of(0.f);
+        for (int i = 1; i < 4; ++i) x2 = make_float2(fmaxf(x2.x, s[i].x), fmaxf(x2.y, s[i].y));
+        const float mx = fmaxf(m, fmaxf(x2.x, x2.y));
+        const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
+        float2 e2 = f2_of(0.f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 x = f2_mul(f2_add(s[i], f2_of(-at)), f2_of(LOG2E));
-            e2 = f2_add(e2, make_float2(tc_ex2(x.x), tc_ex2(x.y)));
-          }
-          l = fmaf(l, tc_ex2((m - at) * LOG2E), e2.x + e2.y);
-          m = mx;
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = f2_mul(f2_add(s[i], f2_of(-at)), f2_of(LOG2E));
+          e2 = f2_add(e2, make_float2(tc_ex2(x.x), tc_ex2(x.y)));
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[h]);
+        l = fmaf(l, tc_ex2((m - at) * LOG2E), e2.x + e2.y);
+        m = mx;
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[h]);
     }
-    if (Z > 1) {      // the other ranks' keys count too
+    // the other half's keys count too, and the other ranks'
+    if (Z > 1) {
       __syncwarp();
       for (int d = 0; d < (z < Z ? Z : 0); ++d) {
-        dsmem_st(dsmem_addr(zx + z * 256 + r, (uint32_t)d), m);
-        dsmem_st(dsmem_addr(zx + z * 256 + 128 + r, (uint32_t)d), l);
+        dsmem_st(dsmem_addr(zx + (z * 2 + h) * 256 + r, (uint32_t)d), m);
+        dsmem_st(dsmem_addr(zx + (z * 2 + h) * 256 + 128 + r, (uint32_t)d), l);
       }
       __syncwarp();
       cluster_sync();
+    } else {
+      zx[h * 256 + r] = m;
+      zx[h * 256 + 128 + r] = l;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    {
       float M = -INFINITY, L = 0.f;
-      for (int d = 0; d < Z; ++d) M = fmaxf(M, zx[d * 256 + r]);
-      for (int d = 0; d < Z; ++d) {
+      for (int d = 0; d < 2 * Z; ++d) M = fmaxf(M, zx[d * 256 + r]);
+      for (int d = 0; d < 2 * Z; ++d) {
         const float mm = zx[d * 256 + r];
         if (mm != -INFINITY) L += exp2f((mm - M) * LOG2E) * zx[d * 256 + 128 + r];
       }
@@ -252,23 +252,21 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     }
     // ---- second walk: probabilities and output
     const float inv = 1.0f / l;
-    float o[128];
+    float o[64];      // columns 64 h ..
 #pragma unroll
-    for (int i = 0; i < 128; ++i) o[i] = 0.f;
+    for (int i = 0; i < 64; ++i) o[i] = 0.f;
     auto join = [&](int j) {      // the j-th tile's product joins the row's sums
       mbar_wait(v_empty, (uint32_t)j & 1u, p.err);
       __syncwarp();
       tc_fence_after();
 #pragma unroll
-      for (int c = 0; c < 4; c += 2) {
-        uint32_t a[32], b[32];
-        tm_ld32(tO + lane_off + c * 32, a);
-        tm_ld32(tO + lane_off + c * 32 + 32, b);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t a[32];
+        tm_ld32(tO + lane_off + h * 64 + c * 32, a);
         tm_wait_ld();
         tm_pin(a);
-        tm_pin(b);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) { o[c * 32 + i] += __uint_as_float(a[i]); o[c * 32 + 32 + i] += __uint_as_float(b[i]); }
+        for (int i = 0; i < 32; ++i) o[c * 32 + i] += __uint_as_float(a[i]);
       }
     };
     for (int j = 0; j < n_tiles; ++j) {
@@ -276,36 +274,33 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       if (j > 0) join(j - 1);      // (it has read its probabilities, too)
       mbar_wait(v_full, (uint32_t)j & 1u, p.err);             // the value biases are written
       float2 t0s = f2_of(0.f), t1s = t0s;
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        mbar_wait(&s_full[h], (uint32_t)it & 1u, p.err);
-        __syncwarp();
-        tc_fence_after();
-        uint32_t a[2][16], b[2][16];
-        ask(h, 0, a[0], b[0]);
+      mbar_wait(&s_full[h], (uint32_t)it & 1u, p.err);
+      __syncwarp();
+      tc_fence_after();
+      uint32_t a[2][8], b[2][8];
+      ask(0, a[0], b[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float2 s[8];
-          tm_wait_ld();
-          if (c < 3) ask(h, 16 * c + 16, a[(c + 1) & 1], b[(c + 1) & 1]);
-          scores_of(it, j, h, 16 * c, a[c & 1], b[c & 1], s);
-          const float4* b4 = reinterpret_cast<const float4*>(vb + h * 64 + 16 * c);
-          uint32_t w[8];
+      for (int c = 0; c < 8; ++c) {
+        float2 s[4];
+        tm_wait_ld();
+        if (c < 7) ask(8 * c + 8, a[(c + 1) & 1], b[(c + 1) & 1]);
+        scores_of(it, j, 8 * c, a[c & 1], b[c & 1], s);
+        const float4* b4 = reinterpret_cast<const float4*>(vb + h * 64 + 8 * c);
+        uint32_t w[4];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 x = f2_mul(f2_add(s[i], f2_of(-m)), f2_of(LOG2E)), e = f2_mul(make_float2(tc_ex2(x.x), tc_ex2(x.y)), f2_of(inv));
-            w[i] = ok ? pack_bf16x2(e.x, e.y) : 0u;
-            const float pa = __uint_as_float(w[i] << 16), pd = __uint_as_float(w[i] & 0xffff0000u);
-            const float4 bv = b4[i];
-            t0s = f2_fma(f2_of(pa), make_float2(bv.x, bv.y), t0s);
-            t1s = f2_fma(f2_of(pd), make_float2(bv.z, bv.w), t1s);
-          }
-          tm_st8(tP + lane_off + h * 32 + 8 * c, w);
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = f2_mul(f2_add(s[i], f2_of(-m)), f2_of(LOG2E)), e = f2_mul(make_float2(tc_ex2(x.x), tc_ex2(x.y)), f2_of(inv));
+          w[i] = ok ? pack_bf16x2(e.x, e.y) : 0u;
+          const float pa = __uint_as_float(w[i] << 16), pd = __uint_as_float(w[i] & 0xffff0000u);
+          const float4 bv = b4[i];
+          t0s = f2_fma(f2_of(pa), make_float2(bv.x, bv.y), t0s);
+          t1s = f2_fma(f2_of(pd), make_float2(bv.z, bv.w), t1s);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[h]);
+        tm_st4(tP + lane_off + h * 32 + 4 * c, w);
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[h]);
       ob0 += t0s.x + t1s.x;
       ob1 += t0s.y + t1s.y;
       tm_wait_st();
@@ -314,20 +309,24 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       if (lane == 0) mbar_arrive(p_full);
     }
     if (n_tiles > 0) join(n_tiles - 1);
+    // the bias terms of both halves' keys: this thread's columns are those of group h
+    obx[h * 128 + r] = h ? ob0 : ob1;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const float ob = h ? obx[r] + ob1 : ob0 + obx[128 + r];
 #pragma unroll
-    for (int i = 0; i < 128; ++i) o[i] += n_tiles > 0 ? (i < 64 ? ob0 : ob1) : 0.f;
+    for (int i = 0; i < 64; ++i) o[i] += n_tiles > 0 ? ob : 0.f;
     __syncwarp();
     if (Z > 1) cluster_sync();      // every rank's products are done: its key buffers may take the other ranks' columns
     const int per = 128 / Z, lg = 31 - __clz(per);      // columns of a rank: a power of two
     if (Z > 1) {
       if (z < Z)
 #pragma unroll
-        for (int i = 0; i < 128; ++i) dsmem_st(dsmem_addr(zo + (z * per + (i & (per - 1))) * 128 + r, (uint32_t)(i >> lg)), o[i]);
+        for (int i = 0; i < 64; ++i) dsmem_st(dsmem_addr(zo + (z * per + ((h * 64 + i) & (per - 1))) * 128 + r, (uint32_t)((h * 64 + i) >> lg)), o[i]);
       __syncwarp();
       cluster_sync();
       if (ok && z < Z) {
         bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + z * per;
-        for (int c = 0; c < per; c += 8) {
+        for (int c = h * (per / 2); c < (h + 1) * (per / 2); c += 8) {
           float y[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) y[i] = 0.f;
@@ -338,9 +337,9 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
         }
       }
     } else if (ok && z == 0) {
-      bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD;
+      bf16* dst = p.out + ((size_t)(t0 + rt) * p.n_heads + kvh * G + rg) * HD + h * 64;
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
+      for (int k = 0; k < 8; ++k)
         *reinterpret_cast<uint4*>(dst + k * 8) = make_uint4(pack_bf16x2(o[8 * k], o[8 * k + 1]), pack_bf16x2(o[8 * k + 2], o[8 * k + 3]),
                                                            pack_bf16x2(o[8 * k + 4], o[8 * k + 5]), pack_bf16x2(o[8 * k + 6], o[8 * k + 7]));
     }

@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_attn_prefill_tc(const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x, t0 = blockIdx.y * TB, z = blockIdx.z;      // the cluster spans the grid's z
+  // (the cluster spans the grid's z; the row blocks with the most keys start first, so that the last to run are short)
+  const int kvh = blockIdx.x, t0 = (int)(gridDim.y - 1 - blockIdx.y) * TB, z = blockIdx.z;
   const int pos0 = p.st->pos;
   const int Z = p.share > 0 ? p.share : attn_prefill_split((int)(gridDim.x * gridDim.y), pos0 + p.T, p.sms);      // ranks from Z on have no keys and no columns
   const int nq = min(TB, p.T - t0);                         // query tokens of this CTA
