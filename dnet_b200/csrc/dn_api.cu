@@ -880,12 +880,12 @@ static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, int pdl, cudaStream_
 }
 
 template <int EPI>
-static cudaError_t gemm_tc_grouped(const CUtensorMap (&x)[TC_XMAPS], TcParams& p, int width, cudaStream_t s) {
+static cudaError_t gemm_tc_grouped(const CUtensorMap (&x)[TC_XMAPS], TcParams& p, int width, int pdl, cudaStream_t s) {
   TcMaps maps;
   for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = x[0];      // (the weights' descriptors lie in global memory)
   memcpy(maps.x, x, sizeof(maps.x));
   if (g_capturing) g_capture_launches++; else g_launches++;
-  return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s);
+  return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s, pdl == PDL_CHUNK);
 }
 
 // sparse MoE FFN of a prompt chunk's layer (2 .. CHUNK_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up
@@ -898,16 +898,16 @@ static int moe_ffn_tc(dn_model* m, const LayerW& L, const bf16* h, bf16* out, in
   const int width = tc_grouped_width(E, P, g_sms);
   CK(launch(k_rmsnorm_rows, dim3(T), dim3(256), 0, s, pdl, h, L.w[DN_W_LN2], m->pf_xn, H, c.rms_eps));
   CK(launch(k_moe_route, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->pf_xn, L.router, H, E, k, m->moe_psel, m->moe_pscore));
-  CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, false, (const int32_t*)m->moe_psel, P, k, E, width, pl, E));
-  CK(launch(k_moe_gather<bf16>, dim3(P), dim3(128), 0, s, false, (const bf16*)m->pf_xn, (const int32_t*)pl.row_tok, H, m->moe_xg));
+  CK(launch(k_moe_plan, dim3(1), dim3(1024), (size_t)(2 * E + 1) * 4, s, pdl, (const int32_t*)m->moe_psel, P, k, E, width, pl, E));
+  CK(launch(k_moe_gather<bf16>, dim3(P), dim3(128), 0, s, pdl, (const bf16*)m->pf_xn, (const int32_t*)pl.row_tok, H, m->moe_xg));
   TcParams p;
   memset(&p, 0, sizeof(p));
   p.err = m->mk_sync + 2;
   p.g_tile_e = pl.tile_e; p.g_tile_r0 = pl.tile_r0; p.g_tile_rows = pl.tile_rows; p.g_ntiles = pl.n_tiles;
   p.T = P; p.K = H; p.nseg = 1; p.seg[0] = TcSeg{c.ffn, c.ffn, m->moe_act, nullptr, 0}; p.g_mapW = L.emaps; p.g_mapW2 = L.emaps + E;
-  CK(gemm_tc_grouped<EPI_SWIGLU>(m->tm_moe_xg, p, width, s));
+  CK(gemm_tc_grouped<EPI_SWIGLU>(m->tm_moe_xg, p, width, pdl, s));
   p.K = c.ffn; p.seg[0] = TcSeg{H, H, m->moe_out, nullptr, 0}; p.g_mapW = p.g_mapW2 = L.emaps + 2 * E;
-  CK(gemm_tc_grouped<EPI_STORE>(m->tm_moe_act, p, width, s));
+  CK(gemm_tc_grouped<EPI_STORE>(m->tm_moe_act, p, width, pdl, s));
   CK(launch(k_moe_join, dim3(T), dim3(256), 0, s, pdl, (const bf16*)m->moe_out, (const int32_t*)pl.pos, (const float*)m->moe_pscore, k, H, h, out));
   return DN_OK;
 }

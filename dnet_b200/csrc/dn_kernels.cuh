@@ -19,6 +19,7 @@
 //     and warp 0 runs the fused epilogue (RoPE + paged-KV append, residual add,
 //     SwiGLU, argmax/logsumexp partials).
 #pragma once
+#include "dn_pdl.cuh"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -60,13 +61,6 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-// Programmatic dependent launch: the next kernel's CTAs may start (and prefetch weights,
-// which no kernel ever writes) while this one drains; they block here before touching
-// anything a predecessor produced.  No-ops when launched without the PDL attribute.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

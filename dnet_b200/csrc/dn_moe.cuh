@@ -2,6 +2,7 @@
 // pairs by expert into tiles of rows, and the gather of the tokens' rows in that order.  Both libraries use it.
 #pragma once
 #include <stdint.h>
+#include "dn_pdl.cuh"
 
 namespace dn {
 
@@ -16,6 +17,8 @@ struct MoePlan {
 };
 // E: outputs of the router; experts from Ereal on are identity experts: their pairs get rows but no tiles
 __global__ void __launch_bounds__(1024) k_moe_plan(const int32_t* __restrict__ idx, int P, int top, int E, int rows, MoePlan pl, int Ereal) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ int32_t cnt[];      // [E] counts, [E + 1] offsets
   int32_t* off = cnt + E;
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
@@ -46,6 +49,8 @@ __global__ void __launch_bounds__(1024) k_moe_plan(const int32_t* __restrict__ i
 // the tokens' rows in the order of the plan (the tensor-core tiles read them with one TMA descriptor): xg[row] = h[row_tok[row]]
 template <class T>
 __global__ void k_moe_gather(const T* __restrict__ h, const int32_t* __restrict__ row_tok, int W, T* __restrict__ xg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const T* src = h + (size_t)row_tok[row] * W;
   T* dst = xg + (size_t)row * W;
