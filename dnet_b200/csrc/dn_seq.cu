@@ -3,6 +3,7 @@
 // launch sequence of a layer.  All arithmetic is in dn_seq_kernels.cuh.
 #include "dn_seq_kernels.cuh"
 #include "dn_seq_attn_rows.cuh"
+#include "dn_seq_prep.cuh"
 #include "dn_seq_recur.cuh"
 #include "dn_seq_moe.cuh"
 #include "dn_seq_latent.cuh"
@@ -1349,6 +1350,12 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
           CK(linear<T>(m, s, (const T*)m->h, l.w[DN_SQ_HEAD_GATE], nullptr, m->pa, N, lc.heads, W, true, 0, LinMaps{wm(DN_SQ_HEAD_GATE), nullptr, &m->x_h}));
       }
     }
+    // Channels, convolutions and carried inputs that the kernels of runs take: a function of the model, not of the batch
+    auto run_ok = [&](int vecs) {
+      uintptr_t al = (uintptr_t)cst | (uintptr_t)(m->conv_stride * sizeof(T)) | (uintptr_t)((l.Cq | l.Ck | l.Cv) * sizeof(T));
+      for (int q : {DN_SQ_Q_CONV, DN_SQ_K_CONV, DN_SQ_V_CONV}) al |= (uintptr_t)l.w[q];
+      return std::is_same<T, bf16>::value && lc.conv <= RUN_MAX_TAPS && (al & 15) == 0 && (l.Cq + l.Ck + l.Cv) / 8 <= vecs * (int)prep_threads(l.Cq + l.Ck + l.Cv).x;
+    };
     if (lc.mixer == DN_MIX_ATTENTION || lc.mixer == DN_MIX_PARALLEL) {
       const int maps = n_maps(lc), Hm = lc.heads * maps, Gm = lc.kv_heads * maps;      // heads and key heads, every map counted
       AttnPrep a{Hm, Gm, lc.dim, lc.vdim, lc.conv, lc.rot_dims, l.Ck ? 1 : 0, lc.qk_norm, c.eps, l.inv_freq,
@@ -1381,6 +1388,16 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         const int units = Hm + (l.Ck ? Gm + (lc.v_is_k ? 0 : lc.kv_heads) : 0), per = N > 64 ? 8 : 1;      // (many tokens: eight heads share their cosines and sines)
         CK(launch(k_attn_prep_rot<T>, dim3(N, (units + per * PREP_WARPS - 1) / (per * PREP_WARPS)), dim3(32 * PREP_WARPS), 0, s, a, b, per, (const T*)m->uq, (const T*)m->uk,
                   (const T*)m->uv, w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), (T*)m->qb, (T*)m->kpool[run.kv_index], (T*)m->vpool[run.kv_index]));
+      } else if (run_ok(RUN_VECS) && (lc.qk_norm == DN_QKNORM_WHOLE || lc.qk_norm == 0) && !a.half && lc.dim % 8 == 0 && lc.rot_dims <= RUN_MAX_ROT) {
+        const int tok = N > RUN_FEW ? RUN_TOK : 1;
+        auto go = [&](auto kern) {
+          return launch(kern, dim3((N + tok - 1) / tok), prep_threads(l.Cq + l.Ck + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
+                        (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const bf16*)l.w[DN_SQ_Q_NORM], (const bf16*)l.w[DN_SQ_K_NORM], (bf16*)cst, m->conv_stride, (bf16*)m->qb,
+                        (bf16*)m->kpool[run.kv_index], (bf16*)m->vpool[run.kv_index]);
+        };
+#define PR(TP) (tok == 1 ? go(k_attn_prep_run<TP, 1>) : go(k_attn_prep_run<TP, RUN_TOK>))
+        CK(lc.conv == 0 ? PR(0) : lc.conv == 1 ? PR(1) : lc.conv == 2 ? PR(2) : lc.conv == 3 ? PR(3) : PR(4));
+#undef PR
       } else
         CK(launch(k_attn_prep<T>, dim3(N), prep_threads(l.Cq + l.Ck + l.Cv), sm, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv, w(DN_SQ_Q_CONV),
                   w(DN_SQ_K_CONV), w(DN_SQ_V_CONV), w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), cst, m->conv_stride, (T*)m->qb,
@@ -1476,7 +1493,18 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
     } else if (lc.mixer == DN_MIX_DELTA) {
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
-      CK(launch(k_delta_prep<T>, dim3(N), prep_threads(2 * l.Cq + l.Cv), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
+      if (run_ok(1 << 20) && lc.dim % 8 == 0 && lc.dim <= 256 && (lc.dim & (lc.dim - 1)) == 0) {
+        const int tok = N > RUN_FEW ? RUN_TOK : 1;
+        auto go = [&](auto kern) {
+          return launch(kern, dim3((N + tok - 1) / tok), prep_threads(2 * l.Cq + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
+                        (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const float*)m->pa, (const float*)m->pb, (const bf16*)l.w[DN_SQ_A_LOG],
+                        (const bf16*)l.w[DN_SQ_DT_BIAS], (bf16*)cst, m->conv_stride, m->qn, m->kn, m->vv, m->beta, m->decay);
+        };
+#define PR(TP) (tok == 1 ? go(k_delta_prep_run<TP, 1>) : go(k_delta_prep_run<TP, RUN_TOK>))
+        CK(lc.conv == 0 ? PR(0) : lc.conv == 1 ? PR(1) : lc.conv == 2 ? PR(2) : lc.conv == 3 ? PR(3) : PR(4));
+#undef PR
+      } else
+        CK(launch(k_delta_prep<T>, dim3(N), prep_threads(2 * l.Cq + l.Cv), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
                 w(DN_SQ_Q_CONV), w(DN_SQ_K_CONV), w(DN_SQ_V_CONV), (const float*)m->pa, (const float*)m->pb, w(DN_SQ_A_LOG),
                 w(DN_SQ_DT_BIAS), (const T*)cst, m->conv_stride, m->qn, m->kn, m->vv, m->beta, m->decay));
       int R, P;
@@ -1492,7 +1520,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
 #undef DR
       PH(DN_SEQ_PH_DELTA_OUT);
-      CK(launch(k_delta_out<T>, dim3(N, lc.heads), dim3(32), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), lc.heads, lc.vdim,
+      CK(launch(k_delta_out<T>, dim3((N * lc.heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), N * lc.heads, lc.heads, lc.vdim,
                 c.eps, (T*)m->mo, 0, 0));
     } else {     // DN_MIX_WKV: token-shifted inputs, projections of each, the recurrence read with a bonus
       PH(DN_SEQ_PH_PROJ);
@@ -1522,7 +1550,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       PH(DN_SEQ_PH_RECUR);
       { const int rc = decay_rule(m, b, RECUR_BONUS, lc.heads, lc.dim, lc.vdim, l.w[DN_SQ_BONUS], st, s); if (rc != DN_OK) return rc; }
       PH(DN_SEQ_PH_RECUR_OUT);
-      CK(launch(k_delta_out<T>, dim3(N, lc.heads), dim3(32), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), lc.heads, lc.vdim,
+      CK(launch(k_delta_out<T>, dim3((N * lc.heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), N * lc.heads, lc.heads, lc.vdim,
                 c.eps, (T*)m->mo, lc.vdim, 0));
     }
     if (lc.conv > 1 && !(b.max_len == 1 && (lc.mixer == DN_MIX_ATTENTION || lc.mixer == DN_MIX_PARALLEL))) {      // (those carry in k_attn_prep)
@@ -1614,7 +1642,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
 #undef GD
       }
       PH(DN_SEQ_PH_RECUR_OUT);
-      CK(launch(k_delta_out<T>, dim3(N, lc.r_heads), dim3(32), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_R_NORM), lc.r_heads, lc.r_dim,
+      CK(launch(k_delta_out<T>, dim3((N * lc.r_heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_R_NORM), N * lc.r_heads, lc.r_heads, lc.r_dim,
                 c.eps, (T*)m->mo, lc.r_dim, 1));
       PH(DN_SEQ_PH_OUT_PROJ);
       CK(linear<T>(m, s, (const T*)m->mo, l.w[DN_SQ_R_O], nullptr, m->y2, N, W, l.Rv, true, 0, LinMaps{wm(DN_SQ_R_O), nullptr, &l.x_mo_r}));
@@ -1637,7 +1665,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       PH(DN_SEQ_PH_RECUR);
       { const int rc = decay_rule(m, b, RECUR_AFTER, lc.r_heads, lc.r_dim, lc.r_vdim, nullptr, st, s); if (rc != DN_OK) return rc; }
       PH(DN_SEQ_PH_RECUR_OUT);
-      CK(launch(k_delta_out<T>, dim3(N, lc.r_heads), dim3(32), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_R_NORM), lc.r_heads, lc.r_vdim,
+      CK(launch(k_delta_out<T>, dim3((N * lc.r_heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_R_NORM), N * lc.r_heads, lc.r_heads, lc.r_vdim,
                 c.eps, (T*)m->mo, 0, 0));
       PH(DN_SEQ_PH_OUT_PROJ);
       CK(linear<T>(m, s, (const T*)m->mo, l.w[DN_SQ_R_O], nullptr, m->y2, N, W, l.Rv, true, 0, LinMaps{wm(DN_SQ_R_O), nullptr, &l.x_mo_r}));
