@@ -307,6 +307,9 @@ static cudaError_t init_kernel_attrs() {
 #define GEA(E, Gr) if ((e = cudaFuncSetAttribute(k_gemm_tc<E, Gr>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)) != cudaSuccess) return e;
   GEA(EPI_STORE, false) GEA(EPI_RESID, false) GEA(EPI_SWIGLU, false) GEA(EPI_STORE, true) GEA(EPI_SWIGLU, true)
 #undef GEA
+#define GES(E) if ((e = cudaFuncSetAttribute(k_gemm_tc<E, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM)) != cudaSuccess) return e;
+  GES(EPI_STORE) GES(EPI_RESID) GES(EPI_SWIGLU)
+#undef GES
 #define ATA(Gv, Pv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv, Pv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
   ATA(1, 2) ATA(2, 2) ATA(4, 2) ATA(8, 2) ATA(1, 3) ATA(2, 3) ATA(4, 3) ATA(5, 3) ATA(7, 3) ATA(8, 3)
 #undef ATA
@@ -873,10 +876,9 @@ static int head_common(dn_model* m, const void* x, int T, dn_kv* kv, int32_t* to
 // one launch: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
 static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, int pdl, cudaStream_t s) {
-  int n_tiles = 0;
-  for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + tc_tile_rows<EPI>() - 1) / tc_tile_rows<EPI>();
+  auto tiles = [&](int rows) { int n = 0; for (int i = 0; i < p.nseg; ++i) n += (p.seg[i].N + rows - 1) / rows; return n; };
   if (g_capturing) g_capture_launches++; else g_launches++;
-  return tc_launch<EPI, false>(maps, p, tc_plan(n_tiles, p.T, p.K, g_sms), s, pdl == PDL_CHUNK);
+  return tc_launch<EPI, false>(maps, p, tc_plan(tiles(tc_tile_rows<EPI>(2)), tiles(tc_tile_rows<EPI>(1)), p.T, p.K, g_sms), s, pdl == PDL_CHUNK);
 }
 
 template <int EPI>
@@ -885,7 +887,7 @@ static cudaError_t gemm_tc_grouped(const CUtensorMap (&x)[TC_XMAPS], TcParams& p
   for (int i = 0; i < TC_SEGS; ++i) maps.w[i] = x[0];      // (the weights' descriptors lie in global memory)
   memcpy(maps.x, x, sizeof(maps.x));
   if (g_capturing) g_capture_launches++; else g_launches++;
-  return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2}, s, pdl == PDL_CHUNK);
+  return tc_launch<EPI, true>(maps, p, TcPlan{width, 1, tc_stages(width), g_sms / 2 * 2, 2}, s, pdl == PDL_CHUNK);
 }
 
 // sparse MoE FFN of a prompt chunk's layer (2 .. CHUNK_MAX tokens): route, sort the (token, choice) pairs by expert, all experts' gate / up

@@ -12,7 +12,7 @@
 // An SM takes about 64 bytes a cycle from L2: a 128 x 128 tile of one CTA needs 128 for full tensor rate, 128 x 256 of a pair's
 // half 64.  A tile is therefore as wide in tokens as the chunk allows (TcPlan), and where that leaves too few tiles for the SMs
 // the reduction is split over the S pairs of a cluster, which add their accumulators through distributed shared memory in a fixed
-// order.  Whole rounds of tiles are walked persistently with two accumulator sets in TMEM; the tiles of a last, mostly empty round
+// order.  With few tokens one CTA may take a tile of half as many features (CG = 1, tc_plan).  Whole rounds of tiles are walked persistently with two accumulator sets in TMEM; the tiles of a last, mostly empty round
 // are cut into narrower pieces.
 //
 // Up to TC_SEGS products that read the same X run in one launch (q, k, v): tiles of all of them fill the SMs together.
@@ -248,13 +248,16 @@ __host__ __device__ __forceinline__ TcTiles tc_tiles(int n_tiles, int t_tiles, i
   r.units = r.whole + (total - r.whole) * r.cut;
   return r;
 }
+// bytes of a stage of tiles of w tokens: a CTA's weight rows and its share of the tokens in whole boxes
+__host__ __device__ constexpr int tc_stage_bytes(int w, int cg) { return TC_A_BYTES + (w / cg + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2); }
 template <int EPI>
-__host__ __device__ constexpr int tc_tile_rows() { return epi_two_weights(EPI) ? 128 : 256; }      // output features of a pair's tile
+__host__ __device__ constexpr int tc_tile_rows(int cg = 2) { return (epi_two_weights(EPI) ? 64 : 128) * cg; }      // output features of a tile
 
-template <int EPI, bool GROUPED = false>
+// CG: CTAs that work on one tile (a pair, or one with half of a pair's rows)
+template <int EPI, bool GROUPED = false, int CG = 2>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant__ TcMaps maps, const __grid_constant__ TcParams p) {
   constexpr bool GLU = epi_two_weights(EPI);
-  constexpr int ROWS = tc_tile_rows<EPI>();
+  constexpr int ROWS = tc_tile_rows<EPI>(CG);
   pdl_launch_dependents();
   if (GROUPED) pdl_wait();        // the tiles are a table that the kernel in front has written
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
@@ -267,24 +270,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t crank = cluster_rank(), lead = crank & ~1u;
-  const int rank = (int)(crank & 1u), part = (int)(crank >> 1);      // place in the pair; which share of a split reduction
+  const uint32_t crank = cluster_rank(), lead = crank / CG * CG;
+  const int rank = (int)(crank % CG), part = (int)(crank / CG);      // place in the pair; which share of a split reduction
   const int S = p.split, W = p.width, stages = p.stages;
   int n_tiles = 0;
   for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + ROWS - 1) / ROWS;
-  const int pairs = (int)gridDim.x / (2 * S), pair = (int)blockIdx.x / (2 * S);      // (a cluster counts once)
+  const int pairs = (int)gridDim.x / (CG * S), pair = (int)blockIdx.x / (CG * S);      // (a cluster counts once)
   const TcTiles tl = tc_tiles(n_tiles, GROUPED ? *p.g_ntiles : (p.T + W - 1) / W, W, S, pairs);
   const int k_all = p.K / TC_BK, k0 = (int)((long long)k_all * part / S), k1 = (int)((long long)k_all * (part + 1) / S);
-  const int stage_bytes = TC_A_BYTES + (W / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
+  const int stage_bytes = tc_stage_bytes(W, CG);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < stages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], 2 * TC_EWARPS); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], CG * TC_EWARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {                // TMEM allocation (a warp of each CTA of the pair), address lands in shared memory
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_base_slot)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    if (CG == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_base_slot)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_base_slot)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -335,15 +343,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
           if (GLU) asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(mw2) : "memory");
         }
         const int r0 = GLU ? tl_.n0 + rank * 64 : tl_.n0 + rank * 128, r1 = GLU ? r0 : r0 + 64;
-        const int x0 = tl_.t0 + rank * (tl_.cols / 2), boxes = (tl_.cols / 2 + TC_XBOX - 1) / TC_XBOX;
+        const int x0 = tl_.t0 + rank * (tl_.cols / CG), boxes = (tl_.cols / CG + TC_XBOX - 1) / TC_XBOX;
         const CUtensorMap* mx = &maps.x[boxes - 1];
-        const uint32_t bytes = 2u * (TC_A_BYTES + boxes * (TC_XBOX * TC_BK * 2));
+        const uint32_t bytes = (uint32_t)CG * (TC_A_BYTES + boxes * (TC_XBOX * TC_BK * 2));
         auto weights = [&](int st, int ks) {
           const uint32_t bar = dsmem_addr(&full[st], lead);
           if (rank == 0) mbar_arrive_expect_tx(&full[st], bytes);
           unsigned char* sa = smem + (size_t)st * stage_bytes;
-          tma_load_2d_pair(sa, mw, ks * TC_BK, r0, bar);
-          tma_load_2d_pair(sa + TC_A_BYTES / 2, mw2, ks * TC_BK, r1, bar);
+          if (CG == 2) {
+            tma_load_2d_pair(sa, mw, ks * TC_BK, r0, bar);
+            tma_load_2d_pair(sa + TC_A_BYTES / 2, mw2, ks * TC_BK, r1, bar);
+          } else {
+            tma_load_2d(sa, mw, ks * TC_BK, r0, &full[st]);
+            tma_load_2d(sa + TC_A_BYTES / 2, mw2, ks * TC_BK, r1, &full[st]);
+          }
         };
         if (!GROUPED && u == pair) {
           early = min(stages, k1 - k0);
@@ -356,9 +369,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
             mbar_wait(&empty[stage], phase ^ 1u, p.err);
             weights(stage, ks);
           }
-          const uint32_t bar = dsmem_addr(&full[stage], lead);
-          unsigned char* sa = smem + (size_t)stage * stage_bytes;
-          tma_load_2d_pair(sa + TC_A_BYTES, mx, ks * TC_BK, x0, bar);
+          unsigned char* sx = smem + (size_t)stage * stage_bytes + TC_A_BYTES;
+          if (CG == 2) tma_load_2d_pair(sx, mx, ks * TC_BK, x0, dsmem_addr(&full[stage], lead));
+          else tma_load_2d(sx, mx, ks * TC_BK, x0, &full[stage]);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -370,7 +383,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
       int stage = 0; uint32_t phase = 0;
       uint32_t it = 0;
       for (int u = pair; u < tl.units; u += pairs, ++it) {
-        const uint32_t idesc = tc_instr_desc(256, tile_of(u).cols);
+        const uint32_t idesc = tc_instr_desc(128 * CG, tile_of(u).cols);
         const uint32_t ab = it & 1u, acc_phase = (it >> 1) & 1u, tacc = tmem_base + ab * TC_WMAX;
         mbar_wait_cluster(&tmem_empty[ab], acc_phase ^ 1u, p.err);    // both CTAs' epilogues drained this accumulator set
         tc_fence_after();
@@ -380,12 +393,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
           unsigned char* sa = smem + (size_t)stage * stage_bytes;
           const uint64_t adesc = tc_smem_desc(sa), bdesc = tc_smem_desc(sa + TC_A_BYTES);
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)      // +32 bytes (>>4 = 2) per UMMA_K inside the swizzle span
-            tc_mma_pair(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (ks > k0 || k) ? 1u : 0u);
-          tc_commit_pair(&empty[stage], both);        // both CTAs' stages are reusable once these MMAs retire
+          for (int k = 0; k < TC_BK / 16; ++k) {      // +32 bytes (>>4 = 2) per UMMA_K inside the swizzle span
+            if (CG == 2) tc_mma_pair(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (ks > k0 || k) ? 1u : 0u);
+            else tc_mma(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (ks > k0 || k) ? 1u : 0u);
+          }
+          if (CG == 2) tc_commit_pair(&empty[stage], both);        // both CTAs' stages are reusable once these MMAs retire
+          else tc_commit(&empty[stage]);
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
-        tc_commit_pair(&tmem_full[ab], both);         // accumulator complete -> both epilogues
+        if (CG == 2) tc_commit_pair(&tmem_full[ab], both);         // accumulator complete -> both epilogues
+        else tc_commit(&tmem_full[ab]);
       }
     }
   }
@@ -585,7 +602,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
       const int row = qd * 32 + lane;
       for (int q = 0; q < S; ++q) {
         if (q == part) continue;
-        const uint32_t dst = dsmem_addr(got + (size_t)part * per * 128 + row, (uint32_t)(2 * q + rank));
+        const uint32_t dst = dsmem_addr(got + (size_t)part * per * 128 + row, (uint32_t)(CG * q + rank));
         for (int c = half * (per / 2); c < (half + 1) * (per / 2); c += 8) {
           uint32_t r[8];
           asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -609,16 +626,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
   cluster_sync();                     // nobody leaves while the pair's other CTA may still read its memory or count on its barriers
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
 }
 
 // ---------------------------------------------------------------------------------
 // the plan of a launch (host).  Internal linkage: a process may load both libraries, and the statics of shared inline functions would be one object
 // ---------------------------------------------------------------------------------
-struct TcPlan { int width, split, stages, grid; };
-static inline int tc_stages(int width) {
-  const int s = TC_RING / (TC_A_BYTES + (width / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2));
+struct TcPlan { int width, split, stages, grid, cg; };      // cg: CTAs of a tile
+static inline int tc_stages(int width, int cg = 2) {
+  const int s = TC_RING / tc_stage_bytes(width, cg);
   return s < TC_MAX_STAGES ? s : TC_MAX_STAGES;
 }
 static inline void tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int grid, int cluster, cudaStream_t s) {
@@ -633,22 +651,22 @@ static inline void tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, i
   cfg->attrs = at;
   cfg->numAttrs = 1;
 }
-// clusters of 2 S CTAs that run at once (asked of the device once; the SMs of a processing cluster hold whole ones: 33 of 4, 15 of 8)
-static inline int tc_clusters(int S, int sms) {
-  static int n[5] = {0, 0, 0, 0, 0};
-  if (n[S] == 0) {
+// clusters of n CTAs that run at once (asked of the device once; the SMs of a processing cluster hold whole ones: 33 of 4, 15 of 8)
+static inline int tc_clusters(int n, int sms) {
+  static int at_once[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  if (at_once[n] == 0) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     int c = 0;
-    tc_config(&cfg, at, 2 * S * sms, 2 * S, 0);
+    tc_config(&cfg, at, n * sms, n, 0);
     if (cudaFuncSetAttribute(k_gemm_tc<EPI_STORE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&c, k_gemm_tc<EPI_STORE, false>, &cfg) != cudaSuccess || c < 1) {
       cudaGetLastError();
-      c = sms / (2 * S) * 3 / 4;
+      c = sms / n * 3 / 4;
     }
-    n[S] = c > 0 ? c : 1;
+    at_once[n] = c > 0 ? c : 1;
   }
-  return n[S];
+  return at_once[n];
 }
 // What a plan is expected to take, in microseconds.  A k-step takes at least 0.28 (the way of a stage through the ring) and otherwise as long
 // as its bytes from L2, of which all SMs together get 10.8 TB/s (a 256-token tile's MMAs take as long as its bytes); a launch that fills
@@ -656,42 +674,51 @@ static inline int tc_clusters(int S, int sms) {
 // end of a launch cost 6, 10.5 where partial sums meet, and the epilogue of the last tile, which nothing hides, grows with its tokens.
 // Against five widths and all splits at 45 shapes (2,048 .. 27,648 features, reductions of 2,048 .. 27,648, 16 .. 2,048 tokens) the plan so
 // chosen is the fastest or within 5 % of it.
-static inline double tc_step(int active, int w) {
-  const int bytes = TC_A_BYTES + (w / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
-  if (active > 72 && active < 120) active = 120;
-  const double t = active * (double)bytes / 10.8e6;
+static inline double tc_step(int active, int w, int cg) {
+  if (active > 72 && active < 120 && cg == 2) active = 120;
+  const double t = active * (double)tc_stage_bytes(w, cg) / 10.8e6;
   return t > 0.28 ? t : 0.28;
 }
-static inline double tc_cost(int n_tiles, int T, int K, int w, int S, int sms) {
-  const int pairs = sms / 2, t_tiles = (T + w - 1) / w, ks = K / TC_BK;
-  const double dram = n_tiles * 256.0 * K * 2.0 / 5.6e6 + 7.0;
+static inline double tc_cost(int n_tiles, int T, int K, int w, int S, int cg, int sms) {
+  const int groups = sms / cg, t_tiles = (T + w - 1) / w, ks = K / TC_BK;
+  const double dram = n_tiles * 128.0 * cg * K * 2.0 / 5.6e6 + 7.0;
   double c;
   if (S > 1) {
-    const int at_once = tc_clusters(S, sms), total = n_tiles * t_tiles, rounds = (total + at_once - 1) / at_once;
-    c = rounds * ((ks + S - 1) / S * tc_step((total < at_once ? total : at_once) * 2 * S, w) + 10.5 + 0.035 * w);
+    const int at_once = tc_clusters(cg * S, sms), total = n_tiles * t_tiles, rounds = (total + at_once - 1) / at_once;
+    c = rounds * ((ks + S - 1) / S * tc_step((total < at_once ? total : at_once) * cg * S, w, cg) + 10.5 + 0.035 * w);
   } else {
-    const TcTiles tl = tc_tiles(n_tiles, t_tiles, w, 1, pairs);
-    c = tl.whole / pairs * (ks * tc_step(sms, w)) + 6.0 + 0.024 * w;
-    if (tl.whole % pairs) c += ks * tc_step(2 * (tl.whole % pairs), w);
-    if (tl.cut > 1) c += ks * tc_step(2 * (tl.units - tl.whole), w / tl.cut);
+    const TcTiles tl = tc_tiles(n_tiles, t_tiles, w, 1, groups);
+    c = tl.whole / groups * (ks * tc_step(sms, w, cg)) + 6.0 + 0.024 * w;
+    if (tl.whole % groups) c += ks * tc_step(cg * (tl.whole % groups), w, cg);
+    if (tl.cut > 1) c += ks * tc_step(cg * (tl.units - tl.whole), w / tl.cut, cg);
   }
   return c > dram ? c : dram;
 }
-static inline TcPlan tc_plan(int n_tiles, int T, int K, int sms) {
-  TcPlan best{0, 1, 0, 0};
+// Up to TC_SINGLE_TO tokens one CTA may work on a tile, of half as many features: half as many k-steps of a split reduction fit into the clusters that run at
+// once (4,096 features of 14,336: 16 tiles of pairs meet 15 clusters of eight, so that two pairs share each; 32 tiles of single CTAs meet 33 of four).  45 tokens:
+// 41 us with pairs, 28 so; 4,096 x 4,096 17.1 / 15.2; 5,120 x 27,648 75 / 54; where a split gains nothing both take the same, and from 200 tokens
+// on most shapes want the pairs' halved copies (14,336 x 2 of 4,096, 200 tokens: 58 / 80).
+constexpr int TC_SINGLE_TO = 256;
+// n_pair, n_single: tiles of a pair and of a single CTA along the features
+static inline TcPlan tc_plan(int n_pair, int n_single, int T, int K, int sms) {
+  TcPlan best{0, 1, 0, 0, 2};
   double cost = 0;
   const int ks = K / TC_BK;
-  for (int S = 1; S <= 4; ++S) {
-    if (S > 1 && ks < 8 * S) break;
-    for (int w = 64; w <= TC_WMAX; w += 32) {
-      if (w % (16 * S) || (w > 96 && w >= T + 32)) continue;
-      const double c = tc_cost(n_tiles, T, K, w, S, sms);
-      if (!best.width || c < cost * 0.999) { cost = c; best.width = w; best.split = S; }
+  for (int cg = 2; cg >= 1; --cg) {
+    if (cg == 1 && T > TC_SINGLE_TO) break;
+    for (int S = 1; S <= 4; ++S) {
+      if (S > 1 && ks < 8 * S) break;
+      for (int w = cg == 2 ? 64 : 48; w <= (cg == 2 ? TC_WMAX : 128); w += cg == 2 ? 32 : 16) {
+        if ((S > 1 && w % (16 * S)) || (w > 96 && w >= T + 32)) continue;
+        const double c = tc_cost(cg == 2 ? n_pair : n_single, T, K, w, S, cg, sms);
+        if (!best.width || c < cost * (cg == 1 ? 0.97 : 0.999)) { cost = c; best.width = w; best.split = S; best.cg = cg; }
+      }
     }
   }
-  best.stages = tc_stages(best.width);
-  const TcTiles tl = tc_tiles(n_tiles, (T + best.width - 1) / best.width, best.width, best.split, sms / 2);
-  best.grid = best.split > 1 ? 2 * best.split * tl.units : 2 * (tl.units < sms / 2 ? tl.units : sms / 2);
+  best.stages = tc_stages(best.width, best.cg);
+  const int groups = sms / best.cg;
+  const TcTiles tl = tc_tiles(best.cg == 2 ? n_pair : n_single, (T + best.width - 1) / best.width, best.width, best.split, groups);
+  best.grid = best.split > 1 ? best.cg * best.split * tl.units : best.cg * (tl.units < groups ? tl.units : groups);
   return best;
 }
 // Rows of a grouped launch's tiles: P rows over E matrices, whose shares are taken to lie within a third of the average.  A matrix with one row more than
@@ -705,13 +732,29 @@ static inline int tc_grouped_width(int E, int P, int sms) {
     double c = 0;
     for (int i = -2; i <= 2; ++i) {
       const int rows = (int)ceil(P * (1.0 + i / 6.0) / E), tiles = (rows + w - 1) / w, cols = rows < w ? (rows + 15) & ~15 : w;
-      const int bytes = TC_A_BYTES + (cols / 2 + TC_XBOX - 1) / TC_XBOX * (TC_XBOX * TC_BK * 2);
+      const int bytes = tc_stage_bytes(cols, 2);
       const double way = 2.5 / tc_stages(w), copies = sms * (double)bytes / 10.8e6;
       c += tiles * (way > copies ? way : copies);
     }
     if (w == 64 || c < cost * 0.999) { cost = c; best = w; }
   }
   return best;
+}
+template <int EPI, bool GROUPED, int CG>
+static inline cudaError_t tc_launch_as(const TcMaps& maps, const TcParams& p, const TcPlan& pl, cudaStream_t s, bool pdl) {
+  static bool attr = false;
+  if (!attr) {
+    const cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<EPI, GROUPED, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  tc_config(&cfg, at, pl.grid, CG * pl.split, s);
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k_gemm_tc<EPI, GROUPED, CG>, maps, p);
 }
 template <int EPI, bool GROUPED>
 static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPlan& pl, cudaStream_t s, bool pdl = false) {
@@ -724,19 +767,9 @@ static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPla
     if (EPI == EPI_JOIN) v = v && (((uintptr_t)p.x | (uintptr_t)p.nh) & 15) == 0;
     sg.vec = v;
   }
-  static bool attr = false;
-  if (!attr) {
-    const cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<EPI, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
-  tc_config(&cfg, at, pl.grid, 2 * pl.split, s);
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = pdl ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, k_gemm_tc<EPI, GROUPED>, maps, p);
+  if constexpr (!GROUPED)
+    if (pl.cg == 1) return tc_launch_as<EPI, GROUPED, 1>(maps, p, pl, s, pdl);
+  return tc_launch_as<EPI, GROUPED, 2>(maps, p, pl, s, pdl);
 }
 
 // ---------------------------------------------------------------------------------

@@ -758,10 +758,9 @@ extern "C" int dn_seq_free_slots(dn_seq_model* m) { return m ? (int)m->free_slot
 // one launch of the tcgen05 GEMM: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
 static cudaError_t gemm_tc(const dn::TcMaps& maps, dn::TcParams& p, cudaStream_t s) {
-  int n_tiles = 0;
-  for (int i = 0; i < p.nseg; ++i) n_tiles += (p.seg[i].N + dn::tc_tile_rows<EPI>() - 1) / dn::tc_tile_rows<EPI>();
+  auto tiles = [&](int rows) { int n = 0; for (int i = 0; i < p.nseg; ++i) n += (p.seg[i].N + rows - 1) / rows; return n; };
   g_launches++;
-  return dn::tc_launch<EPI, false>(maps, p, dn::tc_plan(n_tiles, p.T, p.K, g_sms), s);
+  return dn::tc_launch<EPI, false>(maps, p, dn::tc_plan(tiles(dn::tc_tile_rows<EPI>(2)), tiles(dn::tc_tile_rows<EPI>(1)), p.T, p.K, g_sms), s);
 }
 template <int EPI>
 static cudaError_t gemm_tc(const CUtensorMap& w, const CUtensorMap& w2, const XMaps& x, dn::TcParams& p, cudaStream_t s) {
@@ -1018,7 +1017,7 @@ static cudaError_t gemm_tc_grouped(const XMaps& x, dn::TcParams& p, int width, c
   for (int i = 0; i < dn::TC_SEGS; ++i) maps.w[i] = x.m[0];      // (the weights' descriptors lie in global memory)
   memcpy(maps.x, x.m, sizeof(maps.x));
   g_launches++;
-  return dn::tc_launch<EPI, true>(maps, p, dn::TcPlan{width, 1, dn::tc_stages(width), g_sms / 2 * 2}, s);
+  return dn::tc_launch<EPI, true>(maps, p, dn::TcPlan{width, 1, dn::tc_stages(width), g_sms / 2 * 2, 2}, s);
 }
 
 // the expert products of a routed feed-forward: h [N, W] -> m->y [N, W] (routed sum), m->y2 (shared expert, if any);

@@ -479,6 +479,29 @@ def test_command_lines_on_a_checkpoint_folder(tmp_path):
             seq.append(tok)
 
 
+@pytest.mark.parametrize("taps", [0, 1, 2, 3, 4])
+def test_runs_of_tokens_across_entries_and_steps(taps):
+    """The preparations' kernels for runs of tokens (steps of more than 64): entries shorter than a run and than the convolution, runs that span
+    entries, a last run with a remainder, inputs carried from the step before; one vector of channels a thread and two (the wide layer)."""
+    rot = {"base": 500.0, "dims": 16}
+    cfg = config([attn(mixer={"conv": taps, "rot": rot}, mlp=FF), delta(mixer={"dim": 32, "vdim": 24, "conv": taps}),
+                  attn(mixer={"heads": 32, "kv_heads": 16, "dim": 64, "vdim": 64, "conv": taps, "rot": rot})], width=64)
+    if taps == 0:
+        for layer in cfg["layers"]:
+            layer["mixer"].pop("conv")
+    with Rig(cfg, "bfloat16", max_tokens=1024) as r:
+        seqs = [toks(n, seed=i) for i, n in enumerate((4, 3, 73, 68))]
+        first = [1, 2, 3, 66]
+        got = [r.eng.step([(f"s{i}", s[:n], list(range(n))) for i, (s, n) in enumerate(zip(seqs, first))]),
+               r.eng.step([(f"s{i}", s[n:], list(range(len(s) - n))) for i, (s, n) in enumerate(zip(seqs, first))])]
+        r.model.check()
+        at = [0, 0]
+        for i, (s, n) in enumerate(zip(seqs, first)):
+            mine = torch.cat([got[0][at[0]:at[0] + n], got[1][at[1]:at[1] + len(s) - n]])
+            at = [at[0] + n, at[1] + len(s) - n]
+            assert err(mine, r.oracle(s)) < TOL["bfloat16"]
+
+
 def test_decode_graphs_replay_the_same_kernels():
     """decode steps replay a captured graph; the launch-by-launch path gives the same bits, also after a slot and its
     pages went to another request and with a different number of live requests"""
