@@ -119,6 +119,26 @@ def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_h
     _agree(out[1], out[0])
 
 
+@pytest.mark.parametrize("hidden,ffn,T", [(1024, 14336, 17), (2048, 8192, 33), (2048, 8192, 48), (1024, 14336, 64), (768, 8192, 129), (2048, 8192, 250)])
+def test_prefill_products_of_single_ctas(cuda_lib, hidden, ffn, T):
+    """k_gemm_tc with one CTA a tile (few tokens, long reductions) against the row kernels: widths of 48 and 64 tokens and whole rows of a box beside
+    them, reductions shared by two to four CTAs of a cluster, features that leave part of a tile empty, two token tiles."""
+    x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    out = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_prefill", tc)
+            m = _model(2, 2, seed=T, hidden=hidden, ffn=ffn)
+            kv = m.make_cache(max_tokens=576)
+            out[tc] = _call(m, kv, x, 0)
+            assert cuda_lib.dn_step_error(m._h, 0) == 0
+            kv.free()
+            m.destroy()
+    finally:
+        cuda_lib.dn_set_option(b"tc_prefill", 1)
+    _agree(out[1], out[0])
+
+
 @pytest.mark.parametrize("bits", [8, 4])
 @pytest.mark.parametrize("group,context,T", [(4, 0, 16), (1, 0, 130), (2, 100, 29), (5, 129, 64), (7, 1000, 40), (8, 2490, 16), (4, 1500, 512)])
 def test_prefill_attention_over_quantised_pages(cuda_lib, bits, group, context, T):
