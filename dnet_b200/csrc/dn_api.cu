@@ -311,7 +311,7 @@ static cudaError_t init_kernel_attrs() {
   GES(EPI_STORE) GES(EPI_RESID) GES(EPI_SWIGLU)
 #undef GES
 #define ATA(Gv, Pv) if ((e = cudaFuncSetAttribute(k_attn_prefill_tc<Gv, Pv>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM)) != cudaSuccess) return e;
-  ATA(1, 2) ATA(2, 2) ATA(4, 2) ATA(8, 2) ATA(1, 3) ATA(2, 3) ATA(4, 3) ATA(5, 3) ATA(7, 3) ATA(8, 3)
+  ATA(1, 2) ATA(2, 2) ATA(4, 2) ATA(8, 2) ATA(4, 3) ATA(5, 3) ATA(7, 3) ATA(8, 3)
 #undef ATA
   if ((e = cudaFuncSetAttribute(k_attn_few<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_attn_few<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess) return e;
@@ -997,7 +997,7 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     const dim3 grid = attn_tc_grid(m, T, kv, a);
 #define PFT(Gv, Pv) CK(launch_attn_tc(k_attn_prefill_tc<Gv, Pv>, grid, AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
 #define PFT2(Gv) case Gv: if (T < AT_TWO_PARTS_FROM) { PFT(Gv, 3) } else { PFT(Gv, 2) }
-    switch (m->G) { PFT2(1) PFT2(2) PFT2(4) PFT2(8) case 5: PFT(5, 3) case 7: PFT(7, 3) default: return fail(DN_EINVAL, "GQA group unsupported"); }
+    switch (m->G) { case 1: PFT(1, 2) case 2: PFT(2, 2) PFT2(4) PFT2(8) case 5: PFT(5, 3) case 7: PFT(7, 3) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT2
 #undef PFT
   } else {

@@ -45,7 +45,7 @@ constexpr int AT_SMEM = 5 * AT_TILE + AT_XCH + 1024 + 256;
 constexpr int AT_THREADS = 384;
 // A weight is held in two bf16 parts (16 bits of its mantissa; 2^-18 of it at most is lost) or three (all 24).  Three take a third more products.
 // Chunks of fewer tokens than this and groups of 5 and 7 take them: they are as close to 64 bits as fp32 weights on the CUDA cores are (see above;
-// single tokens behind 256 / 8,192: 2.7e-7 / 2.9e-7, k_attn 2.0e-7 / 4.7e-7), for 15.3 us instead of 14.4 with three tokens behind 256.
+// single tokens behind 256 / 8,192: 2.7e-7 / 2.9e-7, k_attn 2.0e-7 / 4.7e-7).  (Chunks whose group has up to FEW_ROWS rows run on k_attn_few.)
 constexpr int AT_TWO_PARTS_FROM = 16;
 constexpr int AT_REGS_MMA = 56, AT_REGS_SOFTMAX = 224;      // setmaxnreg: of the 168 a thread that 384 threads are launched with
 static_assert(128 * AT_REGS_MMA + 256 * AT_REGS_SOFTMAX <= AT_THREADS * 168, "setmaxnreg split exceeds the CTA's launch allocation");
