@@ -50,7 +50,7 @@ __device__ __forceinline__ void conv_run(const bf16* __restrict__ U, int ldu, co
 #pragma unroll
         for (int e = 0; e < 8; e++) x[i][e] += wl[e * TAPS + j] * v[e];
       }
-      if (carry)      // the only token of its entry: its input takes its place among the carried ones
+      if (carry && n0 + i < N)      // the only token of its entry: its input takes its place among the carried ones (places beyond N hold the last token's slot)
 #pragma unroll
         for (int j = 1; j < TAPS; j++) *reinterpret_cast<uint4*>(st[i] + (size_t)(j - 1) * ldst + off + c) = in[j];
     }

@@ -502,6 +502,36 @@ def test_runs_of_tokens_across_entries_and_steps(taps):
             assert err(mine, r.oracle(s)) < TOL["bfloat16"]
 
 
+@pytest.mark.parametrize("n", [65, 66, 67, 68])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_many_one_token_entries_carry_their_inputs(taps, n):
+    """Steps of more than 64 entries of one token each, first tokens among them: the preparations take four tokens a block, of four requests, and
+    carry the convolutions' inputs themselves (narrow and wide layers).  Every request agrees with its oracle at every step, and
+    with itself decoded beside three others, where a block has one token."""
+    rot = {"base": 500.0, "dims": 16}
+    cfg = config([attn(mixer={"conv": taps, "rot": rot}, mlp=FF), delta(mixer={"dim": 32, "vdim": 24, "conv": taps}),
+                  attn(mixer={"heads": 32, "kv_heads": 16, "dim": 64, "vdim": 64, "conv": taps, "rot": rot})], width=64)
+    steps = 6
+    with Rig(cfg, "bfloat16", max_tokens=72 * 64, max_seqs=72) as r:
+        seqs = [toks(steps, seed=i) for i in range(n)]
+        many = torch.stack([r.eng.step([(f"s{i}", [s[t]], [0]) for i, s in enumerate(seqs)]) for t in range(steps)], 1)
+        for i in range(n):
+            r.eng.finish(f"s{i}")
+        few = []
+        for a in range(0, n, 4):
+            part = seqs[a:a + 4]
+            few.append(torch.stack([r.eng.step([(f"f{i}", [s[t]], [0]) for i, s in enumerate(part)]) for t in range(steps)], 1))
+            for i in range(len(part)):
+                r.eng.finish(f"f{i}")
+        r.model.check()
+        few = torch.cat(few)
+        for i, s in enumerate(seqs):
+            ref = r.oracle(s)
+            assert err(many[i], ref) < TOL["bfloat16"], f"request {i} of {n}"
+            assert err(few[i], ref) < TOL["bfloat16"], f"request {i}, four at a time"
+            assert err(many[i], few[i].cpu()) < TOL["bfloat16"], f"request {i} of {n}"
+
+
 def test_decode_graphs_replay_the_same_kernels():
     """decode steps replay a captured graph; the launch-by-launch path gives the same bits, also after a slot and its
     pages went to another request and with a different number of live requests"""
