@@ -521,6 +521,7 @@ extern "C" int dn_model_destroy(dn_model* m) {
   cudaFree(m->mk_dbg); cudaFree(m->mk_dev); cudaFree(m->xa); cudaFree(m->xb); cudaFree(m->mk_sync);
   cudaFree(m->null_state); cudaFree(m->null_bt);
   cudaFree(m->moe_logits); cudaFree(m->moe_sel); cudaFree(m->moe_score); cudaFree(m->moe_y); cudaFree(m->moe_tables);
+  cudaFree(m->moe_xg); cudaFree(m->moe_act); cudaFree(m->moe_out); cudaFree(m->moe_psel); cudaFree(m->moe_pscore); cudaFree(m->moe_plan); cudaFree(m->moe_maps);
   cudaFree(m->kvq_stage); cudaFree(m->kvq_stage_bt); cudaFree(m->kvq_scores); cudaFree(m->kvq_head_tk);
   delete m;
   return DN_OK;

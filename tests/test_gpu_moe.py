@@ -137,3 +137,19 @@ def test_prompt_experts_in_one_grouped_launch(moe, T):
 def test_experts_of_a_few_tokens_in_one_grouped_launch(moe, T):
     """the same for chunks of fewer tokens: most experts have no row or one"""
     test_prompt_experts_in_one_grouped_launch(moe, T)
+
+
+def test_a_destroyed_model_gives_its_device_memory_back(cuda_lib):
+    """a model with experts keeps 2,048 tokens' pairs of rows, activations and outputs (34 MB here): after the first model (the library's own
+    one-time allocations) as much is free behind every further one"""
+    from dnet_b200.core.models.llama import MixtralRingModel
+
+    cfg = dict(hidden_size=1024, num_attention_heads=8, num_key_value_heads=2, head_dim=128, intermediate_size=2048, vocab_size=256, num_hidden_layers=1,
+               rms_norm_eps=1e-5, rope_theta=10000.0, model_type="mixtral", torch_dtype="bfloat16", num_local_experts=4, num_experts_per_tok=2)
+    free = []
+    for _ in range(5):
+        m = MixtralRingModel(cfg, [0], kv_pool_pages=4)
+        m.destroy()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[-1] >= free[0], free
