@@ -1388,7 +1388,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(launch(k_attn_prep_rot<T>, dim3(N, (units + per * PREP_WARPS - 1) / (per * PREP_WARPS)), dim3(32 * PREP_WARPS), 0, s, a, b, per, (const T*)m->uq, (const T*)m->uk,
                   (const T*)m->uv, w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), (T*)m->qb, (T*)m->kpool[run.kv_index], (T*)m->vpool[run.kv_index]));
       } else if (run_ok(RUN_VECS) && (lc.qk_norm == DN_QKNORM_WHOLE || lc.qk_norm == 0) && !a.half && lc.dim % 8 == 0 && lc.rot_dims <= RUN_MAX_ROT) {
-        const int tok = N > RUN_FEW ? RUN_TOK : 1;
+        const int tok = run_tok(N, (int)prep_threads(l.Cq + l.Ck + l.Cv).x, g_sms, RUN_ATTN_FROM);
         auto go = [&](auto kern) {
           return launch(kern, dim3((N + tok - 1) / tok), prep_threads(l.Cq + l.Ck + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
                         (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const bf16*)l.w[DN_SQ_Q_NORM], (const bf16*)l.w[DN_SQ_K_NORM], (bf16*)cst, m->conv_stride, (bf16*)m->qb,
@@ -1493,7 +1493,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
       if (run_ok(1 << 20) && lc.dim % 8 == 0 && lc.dim <= 256 && (lc.dim & (lc.dim - 1)) == 0) {
-        const int tok = N > RUN_FEW ? RUN_TOK : 1;
+        const int tok = 2 * l.Cq + l.Cv > RUN_DELTA_CHANNELS ? run_tok(N, (int)prep_threads(2 * l.Cq + l.Cv).x, g_sms, RUN_DELTA_FROM) : 1;
         auto go = [&](auto kern) {
           return launch(kern, dim3((N + tok - 1) / tok), prep_threads(2 * l.Cq + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
                         (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const float*)m->pa, (const float*)m->pb, (const bf16*)l.w[DN_SQ_A_LOG],

@@ -12,7 +12,15 @@
 namespace dnseq {
 
 constexpr int RUN_VECS = 2, RUN_MAX_TAPS = CONV_MAX_TAPS, RUN_MAX_ROT = 128;      // 16-byte channel groups of a thread; rotated dims of a head
-constexpr int RUN_TOK = 4, RUN_FEW = 64;                                           // tokens of a block in steps of more than RUN_FEW tokens
+constexpr int RUN_TOK = 4;                                                         // tokens of a block where run_tok says so, else one
+// Four tokens a block read less and hold more registers (one block of 512 threads an SM, and spills with four taps), so that a block takes longer: they pay once the
+// blocks of single tokens queue.  us of one / four tokens a block, four taps:
+//   attention, 1,536 channels: 200 tokens 4.7 / 8.4, 600 8.7 / 8.8, 1,000 11.0 / 8.9; 3,072 channels: 200 6.7 / 9.2, 300 9.4 / 9.4, 1,000 19.2 / 13.5;
+//     6,144 channels: 200 10.6 / 14.2, 400 14.7 / 14.4, 2,048 58.8 / 45.3                 -> more than 1,024 threads an SM
+//   delta rule, 1,536 and 3,072 channels (one pass of a block): 2,048 tokens 17.9 / 18.7 and 31.5 / 35.5; 6,144 channels: 600 27.1 / 30.4, 800 34.4 / 32.7,
+//     2,048 83.1 / 67.8                                                                   -> more than 4,096 channels and 2,560 threads an SM
+constexpr int RUN_ATTN_FROM = 1024, RUN_DELTA_FROM = 2560, RUN_DELTA_CHANNELS = 4096;
+inline int run_tok(int tokens, int threads, int sms, int from) { return (long long)tokens * threads > (long long)sms * from ? RUN_TOK : 1; }
 
 // x = the convolution of channels c .. c + 7 (offset `off` among the carried ones) for the block's tokens; U [N][ldu]
 template <int TAPS, int TOK>

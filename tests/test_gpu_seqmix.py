@@ -479,18 +479,25 @@ def test_command_lines_on_a_checkpoint_folder(tmp_path):
             seq.append(tok)
 
 
-@pytest.mark.parametrize("taps", [0, 1, 2, 3, 4])
-def test_runs_of_tokens_across_entries_and_steps(taps):
-    """The preparations' kernels for runs of tokens (steps of more than 64): entries shorter than a run and than the convolution, runs that span
-    entries, a last run with a remainder, inputs carried from the step before; one vector of channels a thread and two (the wide layer)."""
+def runs_config(taps):
+    """layers whose preparations take the kernels of runs: one vector of channels a thread, two (4,096 channels and more: four tokens a block from
+    some 300 tokens on), and a delta rule of 5,632 channels (from some 750 on)"""
     rot = {"base": 500.0, "dims": 16}
-    cfg = config([attn(mixer={"conv": taps, "rot": rot}, mlp=FF), delta(mixer={"dim": 32, "vdim": 24, "conv": taps}),
-                  attn(mixer={"heads": 32, "kv_heads": 16, "dim": 64, "vdim": 64, "conv": taps, "rot": rot})], width=64)
+    cfg = config([attn(mixer={"conv": taps, "rot": rot}, mlp=FF), delta(mixer={"heads": 64, "kv_heads": 64, "dim": 32, "vdim": 24, "conv": taps}),
+                  attn(mixer={"heads": 32, "kv_heads": 16, "dim": 64, "vdim": 64, "conv": taps, "rot": rot}),
+                  attn(mixer={"heads": 32, "kv_heads": 32, "dim": 64, "vdim": 64, "conv": taps, "rot": rot})], width=64)
     if taps == 0:
         for layer in cfg["layers"]:
             layer["mixer"].pop("conv")
-    with Rig(cfg, "bfloat16", max_tokens=1024) as r:
-        seqs = [toks(n, seed=i) for i, n in enumerate((4, 3, 73, 68))]
+    return cfg
+
+
+@pytest.mark.parametrize("taps", [0, 1, 2, 3, 4])
+def test_runs_of_tokens_across_entries_and_steps(taps):
+    """The preparations' kernels for runs of tokens, one token a block in the first step and four in the second: entries shorter than a run and than
+    the convolution, runs that span entries, a last run of three, inputs carried from the step before."""
+    with Rig(runs_config(taps), "bfloat16", max_tokens=1024, max_batch_tokens=768) as r:
+        seqs = [toks(n, seed=i) for i, n in enumerate((4, 3, 73, 735))]
         first = [1, 2, 3, 66]
         got = [r.eng.step([(f"s{i}", s[:n], list(range(n))) for i, (s, n) in enumerate(zip(seqs, first))]),
                r.eng.step([(f"s{i}", s[n:], list(range(len(s) - n))) for i, (s, n) in enumerate(zip(seqs, first))])]
@@ -502,34 +509,29 @@ def test_runs_of_tokens_across_entries_and_steps(taps):
             assert err(mine, r.oracle(s)) < TOL["bfloat16"]
 
 
-@pytest.mark.parametrize("n", [65, 66, 67, 68])
+@pytest.mark.parametrize("n", [65, 297, 298, 299, 300])
 @pytest.mark.parametrize("taps", [2, 3, 4])
 def test_many_one_token_entries_carry_their_inputs(taps, n):
-    """Steps of more than 64 entries of one token each, first tokens among them: the preparations take four tokens a block, of four requests, and
-    carry the convolutions' inputs themselves (narrow and wide layers).  Every request agrees with its oracle at every step, and
-    with itself decoded beside three others, where a block has one token."""
-    rot = {"base": 500.0, "dims": 16}
-    cfg = config([attn(mixer={"conv": taps, "rot": rot}, mlp=FF), delta(mixer={"dim": 32, "vdim": 24, "conv": taps}),
-                  attn(mixer={"heads": 32, "kv_heads": 16, "dim": 64, "vdim": 64, "conv": taps, "rot": rot})], width=64)
+    """Steps of many entries of one token each, first tokens among them: a block of the wide layers takes four tokens, of four requests, and carries
+    the convolutions' inputs itself, in a last block of one to four tokens (65: one token a block).  The requests of the first and of the last blocks and
+    some between agree with their oracle at every step, and with themselves decoded beside three others, where a block has one token."""
     steps = 6
-    with Rig(cfg, "bfloat16", max_tokens=72 * 64, max_seqs=72) as r:
+    with Rig(runs_config(taps), "bfloat16", max_tokens=304 * 64, max_seqs=304) as r:
         seqs = [toks(steps, seed=i) for i in range(n)]
         many = torch.stack([r.eng.step([(f"s{i}", [s[t]], [0]) for i, s in enumerate(seqs)]) for t in range(steps)], 1)
         for i in range(n):
             r.eng.finish(f"s{i}")
-        few = []
-        for a in range(0, n, 4):
-            part = seqs[a:a + 4]
-            few.append(torch.stack([r.eng.step([(f"f{i}", [s[t]], [0]) for i, s in enumerate(part)]) for t in range(steps)], 1))
-            for i in range(len(part)):
+        for a in (*range(0, n - 8, 60), n - 8, n - 4):
+            part = range(a, a + 4)
+            few = torch.stack([r.eng.step([(f"f{i}", [seqs[i][t]], [0]) for i in part]) for t in range(steps)], 1)
+            for i in part:
                 r.eng.finish(f"f{i}")
+            for k, i in enumerate(part):
+                ref = r.oracle(seqs[i])
+                assert err(many[i], ref) < TOL["bfloat16"], f"request {i} of {n}"
+                assert err(few[k], ref) < TOL["bfloat16"], f"request {i}, four at a time"
+                assert err(many[i], few[k].cpu()) < TOL["bfloat16"], f"request {i} of {n}"
         r.model.check()
-        few = torch.cat(few)
-        for i, s in enumerate(seqs):
-            ref = r.oracle(s)
-            assert err(many[i], ref) < TOL["bfloat16"], f"request {i} of {n}"
-            assert err(few[i], ref) < TOL["bfloat16"], f"request {i}, four at a time"
-            assert err(many[i], few[i].cpu()) < TOL["bfloat16"], f"request {i} of {n}"
 
 
 def test_decode_graphs_replay_the_same_kernels():
