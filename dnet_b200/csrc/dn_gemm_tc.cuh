@@ -90,6 +90,7 @@ struct TcParams {
   const CUtensorMap *g_mapW, *g_mapW2;      // [matrices], 64-byte aligned, in global memory
   // the plan (tc_plan)
   int width, split, stages;       // tokens of a tile, pairs that share a tile's reduction, stages of the ring
+  int early;                      // launched programmatically: the first weights are asked for ahead of the tokens
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
@@ -326,7 +327,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
   };
 
   // The producer asks for the weights of a ring's worth of stages before the kernel in front has ended (programmatic dependent launch); what that one
-  // wrote -- tokens, residuals -- is read behind the wait.  45 tokens, Llama-8B sizes, a layer: 157 us without, 148.
+  // wrote -- tokens, residuals -- is read behind the wait.  45 tokens, Llama-8B sizes, a layer: 157 us without, 148.  An ordinary launch has nothing to wait
+  // for, and there the first stage's tokens would come behind the weights of all others.
   if (warp != 0 && !GROUPED) pdl_wait();
   if (warp == 0) {
     // ===================== TMA producer (each CTA its own rows; bytes counted by the leading CTA) =====================
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
           }
         };
         if (!GROUPED && u == pair) {
-          early = min(stages, k1 - k0);
+          if (p.early) early = min(stages, k1 - k0);
           for (int i = 0; i < early; ++i) weights(i, k0 + i);
           pdl_wait();
         }
@@ -758,7 +760,7 @@ static inline cudaError_t tc_launch_as(const TcMaps& maps, const TcParams& p, co
 }
 template <int EPI, bool GROUPED>
 static inline cudaError_t tc_launch(const TcMaps& maps, TcParams& p, const TcPlan& pl, cudaStream_t s, bool pdl = false) {
-  p.width = pl.width; p.split = pl.split; p.stages = pl.stages;
+  p.width = pl.width; p.split = pl.split; p.stages = pl.stages; p.early = pdl;
   for (int i = 0; i < p.nseg; ++i) {
     TcSeg& sg = p.seg[i];
     bool v = sg.ldy % 8 == 0 && ((uintptr_t)sg.Y & 15) == 0;
