@@ -874,12 +874,28 @@ static int head_common(dn_model* m, const void* x, int T, dn_kv* kv, int32_t* to
                        float* logits_f32, cudaStream_t s);
 
 // ---- tensor-core prefill path (chunks of up to CHUNK_MAX tokens): tcgen05 GEMMs fed by TMA (dn_gemm_tc.cuh)
+template <int EPI>
+static TcPlan gemm_plan(const TcParams& p) {
+  auto tiles = [&](int rows) { int n = 0; for (int i = 0; i < p.nseg; ++i) n += (p.seg[i].N + rows - 1) / rows; return n; };
+  return tc_plan(tiles(tc_tile_rows<EPI>(2)), tiles(tc_tile_rows<EPI>(1)), p.T, p.K, g_sms);
+}
 // one launch: the products of p.seg[0 .. nseg) with the weights maps.w (two-weight epilogues: one product, maps.w[0] gate, [1] up)
 template <int EPI>
 static cudaError_t gemm_tc(const TcMaps& maps, TcParams& p, int pdl, cudaStream_t s) {
-  auto tiles = [&](int rows) { int n = 0; for (int i = 0; i < p.nseg; ++i) n += (p.seg[i].N + rows - 1) / rows; return n; };
   if (g_capturing) g_capture_launches++; else g_launches++;
-  return tc_launch<EPI, false>(maps, p, tc_plan(tiles(tc_tile_rows<EPI>(2)), tiles(tc_tile_rows<EPI>(1)), p.T, p.K, g_sms), s, pdl == PDL_CHUNK);
+  return tc_launch<EPI, false>(maps, p, gemm_plan<EPI>(p), s, pdl == PDL_CHUNK);
+}
+extern "C" int dn_debug_gemm_plan(const int32_t* rows, int products, int two_weights, int T, int K, int32_t* out) {
+  if (!rows || !out || products < 1 || products > TC_SEGS || (two_weights && products != 1) || T < 1 || K < TC_BK) return fail(DN_EINVAL, "bad argument");
+  if (g_device < 0) return fail(DN_EINVAL, "dn_init() has not been called");
+  TcParams p;
+  memset(&p, 0, sizeof(p));
+  p.T = T; p.K = K; p.nseg = products;
+  for (int i = 0; i < products; ++i) p.seg[i].N = rows[i];
+  const TcPlan pl = two_weights ? gemm_plan<EPI_SWIGLU>(p) : gemm_plan<EPI_STORE>(p);
+  out[0] = pl.cg; out[1] = pl.width; out[2] = pl.split;
+  out[3] = tc_clusters(4, g_sms); out[4] = tc_clusters(8, g_sms);
+  return DN_OK;
 }
 
 template <int EPI>

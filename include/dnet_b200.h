@@ -196,6 +196,10 @@ int dn_step_error_clear(dn_model* m, dn_stream s);
 /* parity bisection hook: copy a scratch buffer of the per-op path's LAST chunk to the host (0 q after RoPE,
  * 1 attention output, 2 h = x + o_proj, 3 SwiGLU output); synchronises s */
 int dn_debug_scratch(dn_model* m, int which, void* host_out, size_t bytes, dn_stream s);
+/* test hook: the plan of a launch of the prompt GEMM, `products` matrices of rows[i] x K (two_weights: a gate and an up matrix of rows[0]) and T tokens.
+ * out[0] CTAs that work on a tile (1 or 2), out[1] tokens of a tile, out[2] shares of the reduction; out[3], out[4]: clusters of four and of eight CTAs
+ * that the device runs at once, on which the plan rests */
+int dn_debug_gemm_plan(const int32_t* rows, int products, int two_weights, int T, int K, int32_t* out);
 /* per-SM row partition of the step kernel's four weight phases, [4][sms+1] (NULL: equal split); see
  * dnet_b200.shard.calibrate */
 int dn_step_set_bounds(dn_model* m, const int32_t* bounds_host);

@@ -7,6 +7,8 @@ rounding, so results agree to a few last roundings of the largest value.  How ma
 2^-16 of their terms, which flips about p = 1 in 100 of its roundings; a product of such rows is then off by sqrt(p) 2^-9 of its size,
 a tenth of the distance of two roundings, which flips one result in ten, and the feed-forward does the same once more: below a quarter
 (a wrong key, row or head changes all of them)."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -121,8 +123,7 @@ def test_prefill_products_widths_splits_and_segments(cuda_lib, hidden, ffn, kv_h
 
 @pytest.mark.parametrize("hidden,ffn,T", [(1024, 14336, 17), (2048, 8192, 33), (2048, 8192, 48), (1024, 14336, 64), (768, 8192, 129), (2048, 8192, 250)])
 def test_prefill_products_of_single_ctas(cuda_lib, hidden, ffn, T):
-    """k_gemm_tc with one CTA a tile (few tokens, long reductions) against the row kernels: widths of 48 and 64 tokens and whole rows of a box beside
-    them, reductions shared by two to four CTAs of a cluster, features that leave part of a tile empty, two token tiles."""
+    """k_gemm_tc where few tokens meet long reductions, against the row kernels: single CTAs and pairs as the plan takes them, one token tile to six."""
     x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
     out = {}
     try:
@@ -137,6 +138,35 @@ def test_prefill_products_of_single_ctas(cuda_lib, hidden, ffn, T):
     finally:
         cuda_lib.dn_set_option(b"tc_prefill", 1)
     _agree(out[1], out[0])
+
+
+SINGLE = [("gate_up", 512, 2048, 2, 65, (48, 1)), ("o", 4864, 512, 1, 193, (80, 1)), ("down", 4352, 3072, 2, 97, (64, 2)), ("down", 2048, 2048, 2, 65, (48, 3)),
+          ("down", 4096, 4096, 2, 17, (64, 4)), ("down", 4096, 8192, 2, 100, (128, 4))]
+
+
+@pytest.mark.parametrize("product,hidden,ffn,kv_heads,T,plan", SINGLE)
+def test_prefill_products_that_one_cta_a_tile_forms(cuda_lib, product, hidden, ffn, kv_heads, T, plan):
+    """Every width and split that k_gemm_tc takes with one CTA a tile, by the plan that the library reports for the product (with the clusters that the plans
+    rest on; a device that runs another number of them may plan otherwise), against the row kernels."""
+    qd = 2 * kv_heads * 128
+    rows, K = {"o": ([hidden], qd), "gate_up": ([ffn], hidden), "down": ([hidden], ffn)}[product]
+    out = (C.c_int32 * 5)()
+    assert cuda_lib.dn_debug_gemm_plan((C.c_int32 * len(rows))(*rows), len(rows), product == "gate_up", T, K, out) == 0
+    assert list(out)[:3] == [1, *plan] or list(out)[3:] != [33, 15], list(out)
+    x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(T)).to(torch.bfloat16).cuda()
+    got = {}
+    try:
+        for tc in (1, 0):
+            cuda_lib.dn_set_option(b"tc_prefill", tc)
+            m = _model(kv_heads, 2, seed=T, hidden=hidden, ffn=ffn)
+            kv = m.make_cache(max_tokens=576)
+            got[tc] = _call(m, kv, x, 0)
+            assert cuda_lib.dn_step_error(m._h, 0) == 0
+            kv.free()
+            m.destroy()
+    finally:
+        cuda_lib.dn_set_option(b"tc_prefill", 1)
+    _agree(got[1], got[0])
 
 
 @pytest.mark.parametrize("bits", [8, 4])
