@@ -97,8 +97,10 @@ def beyond_rounding(got, ref):
     return ((got.double() - ref).abs() - half).clamp_min(0)
 
 
-# (groups of 5 and 7 and chunks of fewer than 16 tokens hold a weight's 24 bits; the others 16: a weight is off by 2^-18 of itself at most)
+# (groups of 5 and 7, chunks of fewer than 16 tokens and those of up to 32 rows a group, which k_attn_few takes, hold a weight's 24 bits; the others 16: a
+# weight is off by 2^-18 of itself at most)
 @pytest.mark.parametrize("group,context,T,eps", [(4, 300, 1, 2.0 ** -19), (4, 300, 3, 2.0 ** -19), (1, 500, 15, 2.0 ** -19), (5, 640, 8, 2.0 ** -19), (7, 63, 15, 2.0 ** -19), (8, 0, 2, 2.0 ** -19),
+                                                 (8, 2200, 4, 2.0 ** -19), (2, 1100, 16, 2.0 ** -19), (1, 700, 32, 2.0 ** -19), (5, 127, 6, 2.0 ** -19), (7, 1900, 2, 2.0 ** -19),
                                                  (5, 2200, 64, 2.0 ** -18), (7, 300, 40, 2.0 ** -18), (5, 0, 300, 2.0 ** -18),
                                                  (4, 2200, 64, 2.0 ** -16), (8, 1000, 16, 2.0 ** -16), (2, 0, 300, 2.0 ** -16), (1, 129, 130, 2.0 ** -16)])
 def test_attention_over_16_bit_pages(cuda_lib, group, context, T, eps):
