@@ -2,14 +2,15 @@
 // libdnet_b200.so: single tokens outside the step kernel, drafts, the end of a chunked prompt.
 //
 // Bound by latency behind short contexts and by reading the keys and values behind long ones.  A CTA takes one key / value head, all rows of its
-// group (row = token x G + head) and a run of key tiles (128 keys, two pages); the tiles are dealt out over as many CTAs as fill the SMs, whose partial
-// outputs the last one to finish (an atomic count, nobody waits) joins in the order of the keys.  A tile comes by asynchronous copies, the next
+// group (row = token x G + head) and a run of key tiles (128 keys, two pages); the tiles are dealt out over as many CTAs as fill the SMs, FEW_SPLITS a key
+// head at most (one or two key heads leave SMs idle), whose partial outputs the last one to finish (an atomic count, nobody waits) joins in the order of the keys.  A tile comes by asynchronous copies, the next
 // one while it is worked on; each of the eight warps takes 16 of its keys for each 16 rows, on mma.sync:
 //   S = Q K^T   Q stays in registers
 //   P V         a weight goes in three bf16 parts (all 24 bits of its mantissa), the scores' registers being the operand's as they lie
 // Every MMA starts from zero or from the smaller parts, and sums meet in fp32 additions (an accumulator handed on is cut, not rounded, at each step).
 // On the 128-row tiles of k_attn_prefill_tc one CTA a key head walked the tiles: 3 tokens behind 256, eight groups of 4, a layer 105.9 us, 96.0 so; one
-// Mixtral-8x7B token behind 512 169.9 / 154.4.
+// Mixtral-8x7B token behind 512 169.9 / 154.4; one token behind 8,192, eight groups of 4, a layer 133.7 / 106.4.  (One CTA an SM: 255 registers a thread hold the queries,
+// the outputs and a tile's scores.)
 #pragma once
 #include "dn_attn_tc.cuh"
 

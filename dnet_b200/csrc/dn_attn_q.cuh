@@ -13,7 +13,7 @@
 // Eight warps turn a tile's codes into operands.
 //
 // Bound by the softmax warps, which form every score twice, beside the conversion.  777 tokens behind 1,024 (8 x 4 heads, 8 bits): 237 us with a thread a row,
-// whose one warp a scheduler waits for itself, 198 with two; one token behind 8,000 84 us (a thread a row).  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
+// whose one warp a scheduler waits for itself, 198 with two; one token behind 8,000 90 and 86 (traced).  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
 // tiles: 240 and 82.  Of the stored results 1.56 % and 2.64 % then were not the nearest to 64 bits; now 0.19 % and 0.17 %; k_attn_q, whose
 // block per (head, token) takes 4.1 ms and 1.4 ms, 0.26 % and 0.66 %.)
 // Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-11 softmax (a thread a row and half of its keys), warps 12-19 conversion.

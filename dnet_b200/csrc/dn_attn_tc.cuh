@@ -19,7 +19,7 @@
 //
 // Bound by the softmax warps (some six instructions and an exponential a score) beside the products (1,536 cycles a tile with two
 // parts, 2,048 with three).  Measured, 512 tokens behind 8,192: eight groups of 4 heads 109 us with two parts, 148 with three; eight groups of 5
-// 234 with two CTAs a cluster, 269 with the four that attn_prefill_split takes; 2,048 tokens, groups of 4: 90 us.  With one accumulator over all
+// 234 with two CTAs a cluster (what attn_prefill_split takes), 269 with four; 2,048 tokens, groups of 4: 90 us.  With one accumulator over all
 // tiles of a side, and two parts for every group, they were 98, 168, 207 and 80; error against 64 bits before the result is stored, groups of 5
 // behind 8,192 / 300: 5.3e-6 / 2.2e-6 so, 3.0e-7 / 2.6e-7 now, 1.6e-6 / 3.6e-7 on the CUDA cores; groups of 4 behind 8,192 with two parts: 2.6e-6 / 2.1e-6.
 // Roles: warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator, warps 4-7 side 0, warps 8-11 side 1.
@@ -53,7 +53,8 @@ static_assert(128 * AT_REGS_MMA + 256 * AT_REGS_SOFTMAX <= AT_THREADS * 168, "se
 // CTAs that share a row block's keys: what makes (waves of CTAs) x (key tiles of a CTA + 4 for its start, joining and end) smallest.
 // The grid alone (heads x row blocks) leaves most SMs idle when a chunk is short, and a last wave nearly empty when it is long:
 // 40 heads in groups of 5, 512 tokens give 168 CTAs for 148 SMs.
-// Of 148 SMs 74 clusters of two run at once, 33 of four and 15 of eight (asked of the device): behind 8,192 tokens these 168 row blocks take 234 us with
+// Of 148 SMs 74 clusters of two run at once, 33 of four and 15 of eight (what tc_clusters is answered on this board; held here as constants, since the kernel
+// itself counts when it replays a captured chunk: a board whose processing clusters are cut otherwise gets the same results, perhaps later): behind 8,192 tokens these 168 row blocks take 234 us with
 // Z = 2 and 269 with 4, which a count that takes every SM for usable by every cluster prefers (a layer 798 us so, 770 now).
 __host__ __device__ inline int attn_prefill_split(int ctas, int kv_len, int sms) {
   const int tiles = (kv_len + 127) / 128;

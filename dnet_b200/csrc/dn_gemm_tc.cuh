@@ -674,8 +674,9 @@ static inline int tc_clusters(int n, int sms) {
 // as its bytes from L2, of which all SMs together get 10.8 TB/s (a 256-token tile's MMAs take as long as its bytes); a launch that fills
 // more than half of the SMs with pairs does no better than 120 of them would.  The weights come out of DRAM at 5.6 TB/s at best.  Start and
 // end of a launch cost 6, 10.5 where partial sums meet, and the epilogue of the last tile, which nothing hides, grows with its tokens.
-// Against five widths and all splits at 45 shapes (2,048 .. 27,648 features, reductions of 2,048 .. 27,648, 16 .. 2,048 tokens) the plan so
-// chosen is the fastest or within 5 % of it.
+// Against every width and split of pairs and of single CTAs at 304 shapes (512 .. 27,648 features, reductions of 512 .. 27,648, 17 .. 2,048 tokens; launches
+// one behind the other, programmatic or not) the plan so chosen is the fastest or within 5 % of it at nine of ten, within 10 % at 95 of 100, and 19 % off
+// at worst (5,120 features of 27,648, 2,048 tokens, at the power limit; 6,144 of 4,096, 160 tokens 16).
 static inline double tc_step(int active, int w, int cg) {
   if (active > 72 && active < 120 && cg == 2) active = 120;
   const double t = active * (double)tc_stage_bytes(w, cg) / 10.8e6;
@@ -699,7 +700,10 @@ static inline double tc_cost(int n_tiles, int T, int K, int w, int S, int cg, in
 // Up to TC_SINGLE_TO tokens one CTA may work on a tile, of half as many features: half as many k-steps of a split reduction fit into the clusters that run at
 // once (4,096 features of 14,336: 16 tiles of pairs meet 15 clusters of eight, so that two pairs share each; 32 tiles of single CTAs meet 33 of four).  45 tokens:
 // 41 us with pairs, 28 so; 4,096 x 4,096 17.1 / 15.2; 5,120 x 27,648 75 / 54; where a split gains nothing both take the same, and from 200 tokens
-// on most shapes want the pairs' halved copies (14,336 x 2 of 4,096, 200 tokens: 58 / 80).
+// on most shapes want the pairs' halved copies (14,336 x 2 of 4,096, 200 tokens: 58 / 80).  A candidate of single CTAs has to be 3 % cheaper than the best before it,
+// of pairs or of single CTAs, to be taken (asked once, of the best of either, the margin changes two plans of those 304, for 5 % more time).  Of the 67 shapes
+// that single CTAs then take, those with a split reduction gain 12 % on average; those without one (reductions of up to 1,024) lie between 10 % less and
+// 8 % more behind programmatic launches, and are even behind ordinary ones.
 constexpr int TC_SINGLE_TO = 256;
 // n_pair, n_single: tiles of a pair and of a single CTA along the features
 static inline TcPlan tc_plan(int n_pair, int n_single, int T, int K, int sms) {
@@ -725,8 +729,10 @@ static inline TcPlan tc_plan(int n_pair, int n_single, int T, int K, int sms) {
 }
 // Rows of a grouped launch's tiles: P rows over E matrices, whose shares are taken to lie within a third of the average.  A matrix with one row more than
 // a tile has takes a second one, which reads its weights again and fills a few columns, so the width keeps a distance from the average; a wider
-// stage leaves fewer of them for the way of 2.5 us that each takes through the ring.  (Mixtral-8x7B, 500 tokens, 125 rows an expert: a layer 813 us with
-// tiles of 128 rows, 709 with 192.)
+// stage leaves fewer of them for the way of 2.5 us that each takes through the ring.  (Mixtral-8x7B, 500 tokens, 125 rows an expert: a layer 780 to 816 us with
+// tiles of 128 rows, 661 to 676 with 192.  Both products alone, E = 8, 16 and 64, 17 to 2,048 tokens, choices even and uneven up to 1 : E, against tiles
+// of 64, 128 or 256 rows by an average alone: where averages lie just below a tile's rows 2 to 22 % less, where one expert has many times another's share
+// up to 5.6 % more, and the same or within 2 % elsewhere.)
 static inline int tc_grouped_width(int E, int P, int sms) {
   int best = 64;
   double cost = 0;

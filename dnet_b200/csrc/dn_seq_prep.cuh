@@ -1,10 +1,12 @@
 // dn_seq_prep.cuh -- what lies between a mixer's projections and its scores or its recurrence, for runs of tokens (bf16), libdnet_b200_seq.so:
 // short convolution, norm, rotation, cache append (attention); short convolution, SiLU, norm, gates (delta rule).
 //
-// Bound by moving the rows once (2,048 tokens of 4,096 + 2 x 1,024 channels: 25 MB in, 25 out).  A block takes TOK neighbouring tokens and a thread 16 bytes of
+// Bound by latency: 2,048 tokens of 4,096 + 2 x 1,024 channels are 25 MB in and 25 out (50 for the delta rule, whose outputs are fp32) and take 58 and 69 us, 0.9 and
+// 1.1 TB/s, a seventh of the memory's rate.  A thread's loads for four tokens are in flight at once, but with four taps the forms of four tokens hold 128 registers a
+// thread and spill some 100 bytes, so that one block of 512 threads an SM runs at a time (20 % of the warps an SM can hold).  A block takes TOK neighbouring tokens and a thread 16 bytes of
 // adjacent channels of all of them, so that a channel's convolution weights and input rows are read once for TOK tokens, and holds its numbers in
 // registers from the convolution to the store: a thread's channels lie in one head, and so do the pairs that rotate together.  (A block a token, which
-// read four rows and all weights for each and passed its numbers through shared memory: k_attn_prep 87 us, k_delta_prep 96 for these 2,048 tokens; 58 and 69 so.)
+// read four rows and all weights for each and passed its numbers through shared memory: k_attn_prep 87 us, k_delta_prep 96 for these 2,048 tokens.)
 // Every token's numbers are formed in the same order whatever TOK is and whichever tokens come with it.
 #pragma once
 #include "dn_seq_kernels.cuh"
