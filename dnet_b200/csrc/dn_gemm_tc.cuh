@@ -732,7 +732,7 @@ static inline TcPlan tc_plan(int n_pair, int n_single, int T, int K, int sms) {
 // stage leaves fewer of them for the way of 2.5 us that each takes through the ring.  (Mixtral-8x7B, 500 tokens, 125 rows an expert: a layer 780 to 816 us with
 // tiles of 128 rows, 661 to 676 with 192.  Both products alone, E = 8, 16 and 64, 17 to 2,048 tokens, choices even and uneven up to 1 : E, against tiles
 // of 64, 128 or 256 rows by an average alone: where averages lie just below a tile's rows 2 to 22 % less, where one expert has many times another's share
-// up to 5.6 % more, and the same or within 2 % elsewhere.)
+// up to 8 % more, and the same or within 2 % elsewhere.)
 static inline int tc_grouped_width(int E, int P, int sms) {
   int best = 64;
   double cost = 0;
