@@ -8,6 +8,7 @@
 #include "dn_seq_moe.cuh"
 #include "dn_seq_latent.cuh"
 #include "dn_seq_gdelta.cuh"
+#include "dn_seq_delta_chunk.cuh"
 #include "dn_gemm_tc.cuh"      // the tcgen05 / TMA GEMM the llama-family prefill runs on (namespace dn)
 #include "dn_seq_attn_tc.cuh"
 #include "dn_seq_attn_diff.cuh"
@@ -15,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -87,6 +89,7 @@ struct Run {
   size_t canon_off[2];          // ... and of the carried rows of the two sublayers' input convolutions
 };
 
+static bool delta_chunk_sizes(const dn_seq_cfg& c, const dn_seq_layer_cfg& lc);
 struct dn_seq_model {
   dn_seq_cfg cfg;
   std::vector<SeqLayer> L;
@@ -126,6 +129,8 @@ struct dn_seq_model {
   size_t conv_stride = 0;       // elements per slot
   float* delta_state = nullptr;
   size_t delta_stride = 0;
+  bf16* dc_kq = nullptr;                 // what a prompt's delta-rule chunks are made of (k_delta_chunk_prep; null: no layer has its sizes)
+  unsigned char* dc_ta = nullptr;
   std::vector<int> free_pages, free_slots;
   std::vector<std::vector<int>> pages;   // per slot
   std::vector<int> length;               // per slot, -1: closed
@@ -266,7 +271,7 @@ extern "C" int dn_seq_model_destroy(dn_seq_model* m) {
   cudaDeviceSynchronize();
   void* ptrs[] = {m->xs, m->y, m->pa, m->pb, m->qn, m->kn, m->vv, m->od, m->beta, m->decay, m->h, m->uq, m->uk, m->uv, m->qb,
                   m->mo, m->gt, m->act, m->conv_state, m->delta_state, m->stage_d, m->bt_d, m->tc_err, m->y2, m->x0, m->dz, m->rwt,
-                  m->eo, m->cat, m->xm, m->lr, m->eact, m->ridx, m->rpos, m->rtok, m->tiles, m->xg, m->attn_part, m->attn_count, m->dist_tab, m->sgate, m->hn, m->un, m->aun, m->maps32};
+                  m->eo, m->cat, m->xm, m->lr, m->eact, m->ridx, m->rpos, m->rtok, m->tiles, m->xg, m->attn_part, m->attn_count, m->dist_tab, m->sgate, m->hn, m->un, m->aun, m->maps32, m->dc_kq, m->dc_ta};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (auto& g : m->graphs) cudaGraphExecDestroy(g.second.first);
   if (m->lg_buf) cudaFree(m->lg_buf);
@@ -581,6 +586,13 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
   }
   DA(m->h, MB * W * e); DA(m->uq, MB * mq * e); DA(m->uk, MB * mk * e); DA(m->uv, MB * mv * e); DA(m->qb, MB * mq * e);
   DA(m->mo, MB * mo * e); DA(m->gt, MB * mo * e); DA(m->act, MB * mff * e);
+  {
+    size_t kq = 0, ta = 0;
+    for (auto& l : m->L)
+      if (delta_chunk_sizes(*cfg, l.c)) { kq = std::max(kq, (size_t)l.c.kv_heads * 2 * dc_k_bytes(l.c.dim)); ta = std::max(ta, (size_t)l.c.heads * DC_TA_BYTES); }
+    const size_t chunks = MB / DC + MB / DC_FROM;      // (every entry that is cut has DC_FROM tokens or more)
+    if (kq && chunks) { DA(m->dc_kq, chunks * kq); DA(m->dc_ta, chunks * ta); }
+  }
   DA(m->conv_state, (size_t)cfg->max_seqs * coff * e); DA(m->delta_state, (size_t)cfg->max_seqs * doff * 4);
   m->stage_ints = 5 * MB + 3 * (size_t)(cfg->max_seqs + 1) + MB;
   DA(m->stage_d, m->stage_ints * 4); DA(m->bt_d, (size_t)cfg->max_seqs * m->max_pages * 4); DA(m->tc_err, 16);
@@ -1095,6 +1107,29 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
   return DN_OK;
 }
 
+// delta-rule layers whose prompt portions run in chunks of tokens
+static bool delta_chunk_sizes(const dn_seq_cfg& c, const dn_seq_layer_cfg& lc) {
+  return c.dtype == DN_SEQ_BF16 && lc.mixer == DN_MIX_DELTA && (lc.dim == 64 || lc.dim == 128) && lc.vdim % 4 == 0;
+}
+template <int DK>
+static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b, const dn_seq_layer_cfg& lc, int chunks, float* st) {
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(k_delta_chunk_prep<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dc_prep_smem(DK));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_delta_chunk<DK, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dc_smem(DK, 2));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_delta_chunk<DK, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dc_smem(DK, 4));
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  cudaError_t e = launch(k_delta_chunk_prep<DK>, dim3(chunks, lc.kv_heads), dim3(32 * DC_PREP_WARPS), dc_prep_smem(DK), s, b, lc.heads, lc.kv_heads, (const float*)m->qn,
+                         (const float*)m->kn, (const float*)m->beta, (const float*)m->decay, m->dc_kq, m->dc_ta);
+  if (e != cudaSuccess) return e;
+#define DCK(CG) launch(k_delta_chunk<DK, CG>, dim3(b.E * lc.heads, (lc.vdim + 16 * CG - 1) / (16 * CG)), dim3(64 * CG), dc_smem(DK, CG), s, b, lc.heads, lc.kv_heads, lc.vdim, \
+                       (const bf16*)m->dc_kq, (const unsigned char*)m->dc_ta, (const float*)m->vv, st, m->delta_stride, m->od, m->tc_err)
+  return dc_wide(b.E * lc.heads * ((lc.vdim + 63) / 64), g_sms) ? DCK(4) : DCK(2);
+#undef DCK
+}
+
 // rows a lane (R) and lanes a column (P) of the recurrences: the smallest P R >= dk of this table
 static void recur_shape(int dk, int* R, int* P) {
   static const int RP[8][3] = {{8, 8, 1}, {16, 8, 2}, {32, 8, 4}, {64, 8, 8}, {128, 16, 8}, {256, 16, 16}, {512, 16, 32}, {1024, 32, 32}};
@@ -1512,11 +1547,19 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       // tokens per staged tile: two tiles of `per` floats a token within ~36 KB of shared memory
       const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
       const size_t dsm = (size_t)2 * TB * per * 4;
+      PH(DN_SEQ_PH_DELTA_RULE);
+      int chunks = 0, below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
+      if (m->dc_kq && b.max_len >= DC_FROM && delta_chunk_sizes(c, lc)) {
+        below = DC_FROM;
+        for (int n : m->ent_len) chunks += dc_chunks(n);
+        CK(lc.dim == 64 ? delta_chunks<64>(m, s, b, lc, chunks, st) : delta_chunks<128>(m, s, b, lc, chunks, st));
+      }
 #define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, lc.heads, lc.kv_heads, lc.dim, lc.vdim, TB, \
                          (const float*)m->qn, (const float*)m->kn, (const float*)m->vv, (const float*)m->beta, (const float*)m->decay, st,      \
-                         m->delta_stride, m->od))
-      PH(DN_SEQ_PH_DELTA_RULE);
-      DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
+                         m->delta_stride, m->od, below))
+      if (below == INT_MAX || *std::min_element(m->ent_len.begin(), m->ent_len.end()) < below) {
+        DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
+      }
 #undef DR
       PH(DN_SEQ_PH_DELTA_OUT);
       CK(launch(k_delta_out<T>, dim3((N * lc.heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), N * lc.heads, lc.heads, lc.vdim,

@@ -2238,6 +2238,7 @@ __global__ void __launch_bounds__(512) k_delta_prep(DeltaPrep a, Batch b, const 
 // the P lanes of a column then fall into different banks; rows from dk up are zero, so the token loop has no
 // bounds checks.  Sums run in an order fixed by (dk, P): four interleaved partial sums over a thread's rows (two
 // pairs), then the lanes of a column pairwise -- nothing depends on the tile size or on where a portion was cut.
+// Decode steps, short portions, fp32 models and other key sizes than 64 and 128; the prompts of bf16 models run in chunks (dn_seq_delta_chunk.cuh).
 // Bound by the chain of a token in prompts (a token of one sequence of 32 heads of 128 x 128 takes 309 ns).  With one column a thread (C = 1)
 // the 32 values of k and q that a thread read met 16 rows only; with two they meet 32, two rows an instruction, and the lanes of a column
 // exchange half of their columns in the first step.  Four sequences, 2,048 tokens, the longest 787: C = 1 540 us, 2 373, 4 428 (fewer
@@ -2284,7 +2285,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 template <int R, int P, int C>
 __global__ void __launch_bounds__(32 * P / C) k_delta_rule(Batch b, int H, int G, int dk, int dv, int TB, const float* __restrict__ qn, const float* __restrict__ kn,
                              const float* __restrict__ vv, const float* __restrict__ beta, const float* __restrict__ decay,
-                             float* __restrict__ state, size_t slot_stride, float* __restrict__ o) {
+                             float* __restrict__ state, size_t slot_stride, float* __restrict__ o, int below) {
   static_assert(C <= P && R % 4 == 0, "lanes that share columns");
   extern __shared__ __align__(16) float dsm[];      // 2 x TB x per
   constexpr int KP = P * (R + 4);                   // padded extent of k (and of q)
@@ -2294,6 +2295,7 @@ __global__ void __launch_bounds__(32 * P / C) k_delta_rule(Batch b, int H, int G
   const int mine = lane_col<C>(part), own = col + mine;      // the column whose sums this lane ends up with
   const bool owner = part < C && own < dv;                       // (lanes from C up hold copies)
   const int s0 = b.ent_start[e], s1 = b.ent_start[e + 1];
+  if (s1 - s0 >= below) return;      // (k_delta_chunk takes it)
   float* Sg = state + (size_t)b.ent_slot[e] * slot_stride + (size_t)h * dk * dv;
   const int r0 = part * R;
   const bool vec = C == 4 && dv % 4 == 0 && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
