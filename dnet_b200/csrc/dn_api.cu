@@ -10,6 +10,7 @@
 #include "dn_attn_tc.cuh"
 #include "dn_attn_q.cuh"
 #include "dn_attn_few.cuh"
+#include "dn_attn_prompt.cuh"
 #include "dn_moe.cuh"
 #include "../../include/dnet_b200.h"
 
@@ -155,6 +156,19 @@ static int make_tmap(CUtensorMap* out, const void* base, int rows, int cols, int
   return DN_OK;
 }
 
+// [tokens][heads][128], in boxes of 64 dims x `group` heads x `tokens_of_box` tokens
+static int make_tmap_heads(CUtensorMap* out, const void* base, int tokens, int heads, int group, int tokens_of_box) {
+  if (!g_encode) return fail(DN_ECUDA, "cuTensorMapEncodeTiled unavailable");
+  cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)heads, (cuuint64_t)tokens};
+  cuuint64_t strides[2] = {(cuuint64_t)HD * 2, (cuuint64_t)heads * HD * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)group, (cuuint32_t)tokens_of_box};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(DN_ECUDA, "cuTensorMapEncodeTiled failed (%d) tokens=%d heads=%d", (int)r, tokens, heads);
+  return DN_OK;
+}
+
 // an activation buffer's descriptors, one for each number of rows that a stage may take
 static bool make_xmaps(CUtensorMap (&out)[TC_XMAPS], const void* base, int rows, int cols) {
   for (int i = 0; i < TC_XMAPS; ++i)
@@ -205,6 +219,11 @@ struct dn_model {
   bool pf_ok = false;
   // attention of a few tokens (in part's and tickets' memory): partial outputs of a key head's splits, and how many of them have finished
   float* few_part = nullptr;
+  // attention of prompts (there, too): partial outputs of the items that two CTAs or more share, and how many of them have finished
+  float* ap_part = nullptr;
+  unsigned int* ap_count = nullptr;
+  CUtensorMap tm_q;                      // pf_q in boxes of a key head's query heads and as many tokens as 128 rows hold
+  bool tm_q_ok = false;
   unsigned int* few_count = nullptr;
   int few_splits = 1;
   bool pf_last = false;      // the last chunk ran on the prompt kernels (dn_debug_scratch)
@@ -315,6 +334,8 @@ static cudaError_t init_kernel_attrs() {
 #undef ATA
   if ((e = cudaFuncSetAttribute(k_attn_few<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_attn_few<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_attn_prompt<ApPaged, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_attn_prompt<ApPaged, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM)) != cudaSuccess) return e;
 #define ATQ(Gv) if ((e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess || \
                     (e = cudaFuncSetAttribute(k_attn_prefill_q<Gv, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQT_SMEM)) != cudaSuccess) return e;
   ATQ(1) ATQ(2) ATQ(4) ATQ(5) ATQ(7) ATQ(8)
@@ -420,11 +441,15 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
   // (scratch and counters of k_attn_few behind those of k_attn: two allocations less and one clearing less a model, 0.4 ms)
   const size_t part = ((size_t)tmax * cfg->n_heads * ns * PART_STRIDE + 63) / 64 * 64, tickets = (size_t)tmax * cfg->n_kv_heads + 4;
   m->few_splits = g_sms / cfg->n_kv_heads < 1 ? 1 : g_sms / cfg->n_kv_heads > FEW_SPLITS ? FEW_SPLITS : g_sms / cfg->n_kv_heads;
-  CK(cudaMalloc(&m->part, (part + (size_t)cfg->n_kv_heads * m->few_splits * (FEW_ROWS / 16) * FEW_PART) * sizeof(float)));
-  CK(cudaMalloc(&m->tickets, (tickets + cfg->n_kv_heads) * sizeof(unsigned int)));
-  CK(util_fill0(m->tickets, (tickets + cfg->n_kv_heads) * sizeof(unsigned int)));
+  const size_t few = (size_t)cfg->n_kv_heads * m->few_splits * (FEW_ROWS / 16) * FEW_PART, prompt = cfg->kv_bits ? 0 : (size_t)g_sms * 2 * AP_PART;
+  const size_t counts = tickets + cfg->n_kv_heads + (cfg->kv_bits ? 0 : (size_t)cfg->n_kv_heads * AP_MAX_BLOCKS);
+  CK(cudaMalloc(&m->part, (part + few + prompt) * sizeof(float)));
+  CK(cudaMalloc(&m->tickets, counts * sizeof(unsigned int)));
+  CK(util_fill0(m->tickets, counts * sizeof(unsigned int)));
   m->few_part = m->part + part;
   m->few_count = m->tickets + tickets;
+  m->ap_part = m->few_part + few;
+  m->ap_count = m->few_count + cfg->n_kv_heads;
   CK(cudaMalloc(&m->head_part, (size_t)CTAS_PER_SM * g_sms * sizeof(HeadPartial)));
   CK(cudaMalloc(&m->inv_freq, (HD / 2) * sizeof(float)));
   CK(util_h2d(m->inv_freq, inv_freq_host, (HD / 2) * sizeof(float)));
@@ -492,6 +517,7 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
                true;
     m->pf_ok = m->pf_ok && make_xmaps(m->tm_xn, m->pf_xn, CHUNK_MAX, H) && make_xmaps(m->tm_attn, m->pf_attn, CHUNK_MAX, qd) &&
                make_xmaps(m->tm_act, m->pf_act, CHUNK_MAX, cfg->ffn);
+    m->tm_q_ok = m->pf_ok && m->tm_kv_ok && make_tmap_heads(&m->tm_q, m->pf_q, CHUNK_MAX, cfg->n_heads, m->G, 128 / m->G) == DN_OK;
     if (cfg->n_experts > 0 && m->pf_ok) {
       const int P = CHUNK_MAX * cfg->top_k, E = cfg->n_experts;
       m->moe_max_tiles = P / 64 + E;
@@ -1007,13 +1033,22 @@ static int layer_forward_tc(dn_model* m, int abs_layer, bf16* x, int T, dn_kv* k
     a.part = m->few_part; a.count = m->few_count;
     a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.G = m->G; a.T = T;
     CK(launch(m->G * T <= 16 ? k_attn_few<1> : k_attn_few<2>, dim3(c.n_kv_heads, m->few_splits), dim3(FEW_THREADS), FEW_SMEM, s, pdl, a));
+  } else if (g_tc_attn && m->tm_q_ok && attn_prompt_from(m->G, T, c.n_kv_heads)) {
+    ApParams a;
+    a.out = m->pf_attn; a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.G = m->G; a.TB = 128 / m->G; a.scale = 0.08838834764831845f * LOG2E;
+    a.part = m->ap_part; a.count = m->ap_count; a.err = err;
+    ApPaged g;
+    g.block_table = kv->block_table; g.st = kv->st; g.T = T; g.n_kv = c.n_kv_heads; g.pos = 0;
+    const CUtensorMap &q = m->tm_q, &kvm = m->tm_kv[li];
+    if (attn_parts(m->G, T) == 3) CK(launch(k_attn_prompt<ApPaged, 3>, dim3(g_sms), dim3(ApShape<3>::THREADS), AP_SMEM, s, pdl, q, kvm, kvm, a, g));
+    else CK(launch(k_attn_prompt<ApPaged, 2>, dim3(g_sms), dim3(ApShape<2>::THREADS), AP_SMEM, s, pdl, q, kvm, kvm, a, g));
   } else if (g_tc_attn && m->tm_kv_ok) {
     AtParams a;
     a.q = m->pf_q; a.out = m->pf_attn; a.block_table = kv->block_table; a.st = kv->st;
     a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.T = T; a.err = err;
     const dim3 grid = attn_tc_grid(m, T, kv, a);
 #define PFT(Gv, Pv) CK(launch_attn_tc(k_attn_prefill_tc<Gv, Pv>, grid, AT_THREADS, AT_SMEM, s, pdl, m->tm_kv[li], a)); break;
-#define PFT2(Gv) case Gv: if (T < AT_TWO_PARTS_FROM) { PFT(Gv, 3) } else { PFT(Gv, 2) }
+#define PFT2(Gv) case Gv: if (attn_parts(Gv, T) == 3) { PFT(Gv, 3) } else { PFT(Gv, 2) }
     switch (m->G) { case 1: PFT(1, 2) case 2: PFT(2, 2) PFT2(4) PFT2(8) case 5: PFT(5, 3) case 7: PFT(7, 3) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFT2
 #undef PFT

@@ -1,6 +1,8 @@
 // dn_attn_tc.cuh -- causal attention of a prefill chunk over the paged 16-bit KV cache on the 5th-generation tensor cores
 // (tcgen05 + TMEM + TMA), libdnet_b200.so.
 //
+// Chunks of few row blocks, whose keys several CTAs share; those of many run on k_attn_prompt (dn_attn_prompt.cuh, attn_prompt_from).
+//
 // A CTA takes one key / value head, its G query heads and TB = floor(128 / G) consecutive query tokens: the 128 MMA rows are heads
 // x tokens (row = g TB + t), so that a staged key / value tile serves the whole group; with G = 5 or 7 a few rows stay empty.  The
 // key tiles (128 keys, two pages, by TMA through the block table) go in turn to two sides, each with its own running reference,
@@ -47,6 +49,7 @@ constexpr int AT_THREADS = 384;
 // Chunks of fewer tokens than this and groups of 5 and 7 take them: they are as close to 64 bits as fp32 weights on the CUDA cores are (see above;
 // single tokens behind 256 / 8,192: 2.7e-7 / 2.9e-7, k_attn 2.0e-7 / 4.7e-7).  (Chunks whose group has up to FEW_ROWS rows run on k_attn_few.)
 constexpr int AT_TWO_PARTS_FROM = 16;
+static inline int attn_parts(int G, int T) { return G == 5 || G == 7 || (G >= 4 && T < AT_TWO_PARTS_FROM) ? 3 : 2; }
 constexpr int AT_REGS_MMA = 56, AT_REGS_SOFTMAX = 224;      // setmaxnreg: of the 168 a thread that 384 threads are launched with
 static_assert(128 * AT_REGS_MMA + 256 * AT_REGS_SOFTMAX <= AT_THREADS * 168, "setmaxnreg split exceeds the CTA's launch allocation");
 

@@ -12,6 +12,7 @@
 #include "dn_gemm_tc.cuh"      // the tcgen05 / TMA GEMM the llama-family prefill runs on (namespace dn)
 #include "dn_seq_attn_tc.cuh"
 #include "dn_seq_attn_diff.cuh"
+#include "dn_seq_attn_prompt.cuh"
 #include "../../include/dnet_b200_seq.h"
 
 #include <algorithm>
@@ -67,6 +68,8 @@ struct SeqLayer {
   CUtensorMap tm[DN_SQ_COUNT];
   bool tm_ok[DN_SQ_COUNT];
   XMaps x_mo, x_act;            // the mixer's output buffer [MB, Co] and the feed-forward's [MB, ff]
+  CUtensorMap tm_q;             // softmax attention of prompts: the queries in boxes of a key head's query heads and as many tokens as 128 rows hold
+  bool tm_q_ok = false;
   XMaps x_mo_r, x_lr;           // the linear-attention half's [MB, Rv]; the decay projection's inner [MB, rank]
   int Cq, Ck, Cv, Co;           // projection widths: q, k, v and the mixer's output before W_o
   int Rc, Rv;                   // linear-attention half of a parallel mixer: q / k width, v / output width
@@ -110,6 +113,8 @@ struct dn_seq_model {
   float *xs = nullptr, *y = nullptr, *pa = nullptr, *pb = nullptr, *qn = nullptr, *kn = nullptr, *vv = nullptr, *od = nullptr,
         *beta = nullptr, *decay = nullptr, *y2 = nullptr, *x0 = nullptr, *dz = nullptr, *rwt = nullptr, *eo = nullptr, *sgate = nullptr;
   unsigned int* attn_count = nullptr; // blocks of a split row that have finished [AT_SPLIT_ROWS][heads]; zero between launches
+  float* ap_part = nullptr;           // softmax attention of prompts: partial outputs of the items that two CTAs or more share [SMs][2],
+  unsigned int* ap_count = nullptr;   // and how many of them have finished [key heads][blocks]; zero between launches
   int part_dv = 256;            // widest value row (padded to 32) of a split attention row's partials
   void *h = nullptr, *uq = nullptr, *uk = nullptr, *uv = nullptr, *qb = nullptr, *mo = nullptr, *gt = nullptr, *act = nullptr, *cat = nullptr,
        *xm = nullptr, *lr = nullptr, *eact = nullptr;
@@ -120,7 +125,7 @@ struct dn_seq_model {
   std::vector<CUtensorMap> kmap, vmap;   // TMA descriptors of the pools (boxes of one page x 64 columns), where map_ok
   std::vector<char> map_ok;
   float* dist_tab = nullptr;             // [heads][distance]: the tabled bias of the layer whose attention runs (k_dist_table)
-  std::vector<int> ent_len;              // tokens of the current step's entries
+  std::vector<int> ent_len, ent_end;     // tokens of the current step's entries; their sequences' lengths after it
   std::vector<void*> pkpool, pvpool;     // mean-pooled blocks behind a sliding window: [pages][pool_rows][row] (null: the run has none)
   std::vector<int> last_tok;             // per slot: the sequence's last token (-1: none yet), for the bigram row
   void* hn = nullptr;                    // the normed rows before the sublayer's input convolution [MB, W]
@@ -202,6 +207,16 @@ static bool make_tmap(CUtensorMap* out, const void* base, int rows, int cols, in
   return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// [tokens][heads][128], in boxes of 64 dims x `group` heads x as many tokens as 128 rows hold
+static bool make_tmap_heads(CUtensorMap* out, const void* base, int tokens, int heads, int group) {
+  if (!g_encode || !base) return false;
+  cuuint64_t dims[3] = {128, (cuuint64_t)heads, (cuuint64_t)tokens};
+  cuuint64_t strides[2] = {256, (cuuint64_t)heads * 256};
+  cuuint32_t box[3] = {64, (cuuint32_t)group, (cuuint32_t)(128 / group)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 static int dist_span(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {      // distances a visible key can have: 0 .. span - 1
   int span = cfg.pool_pages * PAGE;
   if (cfg.max_positions > 0) span = std::min(span, cfg.max_positions);
@@ -225,6 +240,11 @@ static int n_maps(const dn_seq_layer_cfg& c) { return c.maps == 2 ? 2 : 1; }
 static bool diff_tc_sizes(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {
   return cfg.dtype == DN_SEQ_BF16 && c.mixer == DN_MIX_ATTENTION && n_maps(c) == 2 && c.softcap <= 0.f && c.scale > 0.f && (c.dim == 64 || c.dim == 128) &&
          (c.vdim == 64 || c.vdim == 128);
+}
+// layers whose prompt portions take k_attn_prompt
+static bool soft_tc_sizes(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {
+  return cfg.dtype == DN_SEQ_BF16 && (c.mixer == DN_MIX_ATTENTION || c.mixer == DN_MIX_PARALLEL) && n_maps(c) == 1 && c.attn_weight != DN_ATTN_SIGMOID && c.softcap <= 0.f &&
+         !c.sink && !c.out_gate && !c.dist_bias && c.pool == 0 && c.keep_first == 0 && c.scale > 0.f && c.dim == 128 && c.vdim == 128 && c.heads / c.kv_heads <= 128;
 }
 // rotary frequencies base^(-2j/dims), j = 0 .. dims/2 - 1, optionally scaled.  By a ramp over the pairs (yarn_*): pairs that turn fast
 // within the original context keep theirs, slow ones are divided by the factor, a line between.  By wavelength (band_*): short ones keep
@@ -271,7 +291,7 @@ extern "C" int dn_seq_model_destroy(dn_seq_model* m) {
   cudaDeviceSynchronize();
   void* ptrs[] = {m->xs, m->y, m->pa, m->pb, m->qn, m->kn, m->vv, m->od, m->beta, m->decay, m->h, m->uq, m->uk, m->uv, m->qb,
                   m->mo, m->gt, m->act, m->conv_state, m->delta_state, m->stage_d, m->bt_d, m->tc_err, m->y2, m->x0, m->dz, m->rwt,
-                  m->eo, m->cat, m->xm, m->lr, m->eact, m->ridx, m->rpos, m->rtok, m->tiles, m->xg, m->attn_part, m->attn_count, m->dist_tab, m->sgate, m->hn, m->un, m->aun, m->maps32, m->dc_kq, m->dc_ta};
+                  m->eo, m->cat, m->xm, m->lr, m->eact, m->ridx, m->rpos, m->rtok, m->tiles, m->xg, m->attn_part, m->attn_count, m->dist_tab, m->sgate, m->hn, m->un, m->aun, m->maps32, m->dc_kq, m->dc_ta, m->ap_part, m->ap_count};
   for (void* p : ptrs) if (p) cudaFree(p);
   for (auto& g : m->graphs) cudaGraphExecDestroy(g.second.first);
   if (m->lg_buf) cudaFree(m->lg_buf);
@@ -535,7 +555,7 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
           memset(&vm, 0, sizeof(vm));
           const int prows = cfg->pool_pages * PAGE;
           const void* vp = c.v_is_k ? m->kpool.back() : m->vpool.back();
-          const bool ok = (sig_tc_sizes(*cfg, c) || diff_tc_sizes(*cfg, c)) && make_tmap(&km, m->kpool.back(), prows, l.Ck, PAGE) && make_tmap(&vm, vp, prows, c.v_is_k ? l.Ck : l.Cv, PAGE);
+          const bool ok = (sig_tc_sizes(*cfg, c) || diff_tc_sizes(*cfg, c) || soft_tc_sizes(*cfg, c)) && make_tmap(&km, m->kpool.back(), prows, l.Ck, PAGE) && make_tmap(&vm, vp, prows, c.v_is_k ? l.Ck : l.Cv, PAGE);
           m->kmap.push_back(km);
           m->vmap.push_back(vm);
           m->map_ok.push_back(ok ? 1 : 0);
@@ -566,6 +586,12 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
   DA(m->y2, MB * W * 4); DA(m->dz, MB * mdq * 4); DA(m->lr, MB * mrank * e);
   DA(m->attn_part, (size_t)AT_SPLIT_ROWS * mh * AT_MAX_SPLITS * (2 + m->part_dv) * 4);
   DA(m->attn_count, (size_t)AT_SPLIT_ROWS * mh * 4);
+  {
+    int kv = 0;
+    for (auto& l : m->L) if (soft_tc_sizes(*cfg, l.c)) kv = std::max(kv, l.c.kv_heads);
+    if (kv) { DA(m->ap_part, (size_t)g_sms * 2 * dn::AP_PART * 4); DA(m->ap_count, (size_t)kv * dn::AP_MAX_BLOCKS * 4); }
+    if (kv && rc == DN_OK && cudaMemset(m->ap_count, 0, (size_t)kv * dn::AP_MAX_BLOCKS * 4) != cudaSuccess) rc = fail(DN_ECUDA, "memset failed");
+  }
   if (tab > 0) DA(m->dist_tab, (tab + 32) * 4);      // (rows without a query read up to 32 entries whatever the span)
   DA(m->sgate, MB * 4);
   {
@@ -604,6 +630,7 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
     make_xmaps(&m->x_h, m->h, m->MB, cfg->width);
     for (auto& l : m->L) {
       make_xmaps(&l.x_mo, m->mo, m->MB, l.Co);
+      l.tm_q_ok = soft_tc_sizes(*cfg, l.c) && make_tmap_heads(&l.tm_q, m->qb, m->MB, l.c.heads, l.c.heads / l.c.kv_heads);
       if (l.Rv > 0) make_xmaps(&l.x_mo_r, m->mo, m->MB, l.Rv);
       if (l.c.rank > 0) make_xmaps(&l.x_lr, m->lr, m->MB, l.c.rank);
       if (l.c.mixer == DN_MIX_LATENT && l.c.q_rank > 0) make_xmaps(&l.x_lr, m->lr, m->MB, l.c.q_rank);
@@ -905,6 +932,40 @@ static cudaError_t sig_attn(dn_seq_model* m, cudaStream_t s, const Batch& b, int
   const SigParams p{q, out, m->dist_tab, ex.gate, lc.heads, lc.kv_heads, lc.chunk, ex.window, D, std::min(lc.heads / lc.kv_heads, SG_HEADS), lc.scale, m->tc_err};
   if (lc.dim == 64) return lc.vdim == 64 ? sig_attn_launch<64, 64>(m, s, b, kv, p) : sig_attn_launch<64, 128>(m, s, b, kv, p);
   return lc.vdim == 64 ? sig_attn_launch<128, 64>(m, s, b, kv, p) : sig_attn_launch<128, 128>(m, s, b, kv, p);
+}
+
+// Plain softmax attention, prompt portions: a CTA an SM, from SOFT_FROM keys on that a query of the step sees; below, a row block is a tile or two and k_attn_tiles,
+// whose blocks start and end sooner, is ahead.  Steps of Moputar, two such layers, widths 1,024 / 2,048 / 4,096, k_attn_tiles and k_attn_prompt: a prompt of 64
+// tokens 342, 423, 626 and 351, 432, 636 us; two of 128 together 386, 467, 708 and 389, 474, 713; one of 200 391, 510, 796 and 382, 499, 784; one of 2,048 954, 1,488,
+// 3,366 and 836, 1,310, 3,110.
+constexpr int SOFT_FROM = 160;
+static bool soft_attn_ok(const dn_seq_model* m, const Batch& b, int kv, const SeqLayer& l) {
+  const dn_seq_layer_cfg& lc = l.c;
+  if (!l.tm_q_ok || !m->map_ok[kv] || b.E > AB_MAX_ENTRIES) return false;
+  const int TB = 128 / (lc.heads / lc.kv_heads), ch = lc.chunk;
+  int blocks = 0, seen = 0;
+  for (size_t e = 0; e < m->ent_len.size(); e++) {
+    const int n = m->ent_len[e], end = m->ent_end[e], first = end - n;
+    blocks += (n + TB - 1) / TB;
+    seen = std::max(seen, ch <= 0 ? end : lc.mask_kind == DN_MASK_WINDOW ? std::min(end, ch + n) : first / ch == (end - 1) / ch ? (end - 1) % ch + 1 : ch);
+  }
+  return blocks <= dn::AP_MAX_BLOCKS && seen >= SOFT_FROM;
+}
+static cudaError_t soft_attn(dn_seq_model* m, cudaStream_t s, const Batch& b, int kv, const SeqLayer& l, const bf16* q, bf16* out) {
+  const dn_seq_layer_cfg& lc = l.c;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(dn::k_attn_prompt<ApBatch, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dn::AP_SMEM);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  dn::ApParams p;
+  p.out = (dn::bf16*)out; p.n_heads = lc.heads; p.n_kv = lc.kv_heads; p.G = lc.heads / lc.kv_heads; p.TB = 128 / p.G;
+  p.scale = lc.scale * 1.4426950408889634f;
+  p.part = m->ap_part; p.count = m->ap_count; p.err = m->tc_err;
+  ApBatch g;
+  g.b = b; g.chunk = lc.chunk; g.window = lc.mask_kind == DN_MASK_WINDOW ? 1 : 0;
+  return launch(dn::k_attn_prompt<ApBatch, 2>, dim3(g_sms), dim3(dn::ApShape<2>::THREADS), dn::AP_SMEM, s, l.tm_q, m->kmap[kv], m->vmap[kv], p, g);
 }
 
 // differential attention, prompt portions: a CTA per (block of tokens, key head, up to DA_HEADS of its query heads)
@@ -1444,6 +1505,8 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(diff_attn(m, s, b, run.kv_index, (const bf16*)m->qb, lc, ex, (bf16*)m->mo));
       else if (b.max_len >= 16 && m->map_ok[run.kv_index] && sig_tc_sizes(c, lc))
         CK(sig_attn(m, s, b, run.kv_index, (const bf16*)m->qb, lc, ex, (bf16*)m->mo));
+      else if (b.max_len >= 16 && soft_attn_ok(m, b, run.kv_index, l))
+        CK(soft_attn(m, s, b, run.kv_index, l, (const bf16*)m->qb, (bf16*)m->mo));
       else if (attn_tiles_ok<T>(lc, b))
         CK(attn_tiles(s, b, (const bf16*)m->qb, (const bf16*)m->kpool[run.kv_index], (const bf16*)vpl, lc, ex, (bf16*)m->mo));
       else if (const int st = attn_rows_stages<T>(lc, N))
@@ -1904,6 +1967,8 @@ extern "C" int dn_seq_step(dn_seq_model* m, int E, const int32_t* slots, const i
   CK(cudaEventRecord(m->staged, s));
   int32_t* d = m->stage_d;
   m->ent_len.assign(counts, counts + E);
+  m->ent_end.resize(E);
+  for (int e = 0; e < E; e++) m->ent_end[e] = m->length[slots[e]];
   int max_len = 0, row_tiles = 0;
   for (int e = 0; e < E; e++) { max_len = counts[e] > max_len ? counts[e] : max_len; row_tiles += (counts[e] + AT_ROWS - 1) / AT_ROWS; }
   Batch b{d, d + N, d + 2 * N, d + 3 * N, d + 5 * N, d + 5 * N + E + 1, d + 5 * N + 2 * E + 1, m->bt_d, N, E, m->max_pages, max_len, row_tiles, d + 4 * N};

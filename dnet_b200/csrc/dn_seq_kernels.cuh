@@ -1878,7 +1878,8 @@ __global__ void k_diff_lambda(const T* __restrict__ lq1, const T* __restrict__ l
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The same attention for prompt portions, bf16, on the warp-level tensor-core MMA (m16n8k16, fp32 accumulation).
+// The same attention for prompt portions, bf16, on the warp-level tensor-core MMA (m16n8k16, fp32 accumulation).  Plain softmax attention of head size 128 takes it
+// where few keys are seen (SOFT_FROM); else k_attn_prompt does.
 // A block owns 64 consecutive query rows of one entry and one query head; its four warps take 16 rows each.  Keys
 // and values come page by page (a 64-key tile is exactly one page) through shared memory.  Scores, the running
 // maximum and the running sum are fp32; the weights enter the P V product as a bf16 pair (p = hi + lo, both
