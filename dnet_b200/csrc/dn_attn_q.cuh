@@ -12,8 +12,12 @@
 //       bf16 by definition; a tile's product and its bias terms join fp32 sums of the row's thread)
 // Eight warps turn a tile's codes into operands.
 //
-// Bound by the softmax warps, which form every score twice, beside the conversion.  777 tokens behind 1,024 (8 x 4 heads, 8 bits): 237 us with a thread a row,
-// whose one warp a scheduler waits for itself, 198 with two; one token behind 8,000 90 and 86 (traced).  (With hi + lo keys of scale x code in one accumulator of 16 products, and one output accumulator over all
+// Bound by shared memory: a thread reads sixteen bytes of scales and biases a key in each walk, 262 KB a tile and walk of the 128 bytes a cycle that operands and conversion
+// share, and the softmax warps, which form every score twice.  In the first walk the scores have two places, so that a tile's are formed while the other's are read; in the
+// second the probabilities have two, and a tile's product joins the sums while the next one's probabilities are formed; codes are asked for a unit ahead.  777 tokens
+// behind 1,024 (8 x 4 heads, 8 bits): 237 us with a thread a row, whose one warp a scheduler waits for itself, 190 with two, 161 so; 1,500 behind 3,000 754 and 625; one
+// token behind 8,000 90 and 86 before (traced).  (Code units asked for ahead alone, or the two walks' loops rolled: nothing.  With hi + lo keys of scale x code in one
+// accumulator of 16 products, and one output accumulator over all
 // tiles: 240 and 82.  Of the stored results 1.56 % and 2.64 % then were not the nearest to 64 bits; now 0.19 % and 0.17 %; k_attn_q, whose
 // block per (head, token) takes 4.1 ms and 1.4 ms, 0.26 % and 0.66 %.)
 // Roles: warp 0 MMA issuer, warp 1 TMEM allocator, warps 4-11 softmax (a thread a row and half of its keys), warps 12-19 conversion.
@@ -28,23 +32,28 @@ struct AqParams {
   const unsigned char* pool;     // this layer's packed pages
 };
 constexpr int AQT_THREADS = 640, AQT_DQ = 256;
-constexpr int AQT_KB = 4 * 128;      // floats of a key tile: scales of both groups, biases of both groups
-constexpr int AQT_XCH = (4 * AQT_KB + 128 * 2 + 2 * AT_MAX_Z * 2 * 128 + 2 * 128) * 4;      // four key tiles' scales and biases, value biases, the maxima and sums of
-                                                                                             // both halves of every rank, the halves' bias terms
+constexpr int AQT_KB = 6 * 128;      // floats of a key tile: scales of both groups, biases of both groups, (bias of group 0, of group 1) of each value row
+constexpr int AQT_XCH = (4 * AQT_KB + 2 * AT_MAX_Z * 2 * 128 + 2 * 128) * 4;      // four key tiles' scales and biases, the maxima and sums of both halves of every rank,
+                                                                                 // the halves' bias terms
 constexpr int AQT_SMEM = 5 * AT_TILE + AQT_XCH + 1024 + 256;
-constexpr int AQT_REGS_MMA = 64, AQT_REGS_SOFTMAX = 136, AQT_REGS_DQ = 72;      // setmaxnreg: of the 96 a thread that 640 threads are launched with
+constexpr int AQT_REGS_MMA = 40, AQT_REGS_SOFTMAX = 136, AQT_REGS_DQ = 80;      // setmaxnreg: of the 96 a thread that 640 threads are launched with
 static_assert(128 * (AQT_REGS_MMA + 2 * AQT_REGS_SOFTMAX + 2 * AQT_REGS_DQ) <= AQT_THREADS * 96, "setmaxnreg split exceeds the CTA's launch allocation");
 
-// 8 (4) consecutive 32-bit columns of this warp's TMEM quarter
-__device__ __forceinline__ void tm_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+// 16 (8) consecutive 32-bit columns of this warp's TMEM quarter
+__device__ __forceinline__ void aq_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr));
 }
-__device__ __forceinline__ void tm_pin8(uint32_t (&r)[8]) {      // no use of r moves above this point
-  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
+__device__ __forceinline__ void aq_pin(uint32_t (&r)[16]) {      // no use of r moves above this point
+#pragma unroll
+  for (int i = 0; i < 16; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
 }
-__device__ __forceinline__ void tm_st4(uint32_t taddr, const uint32_t (&r)[4]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+__device__ __forceinline__ void aq_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 
 template <int G, int BITS>
@@ -57,14 +66,14 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char *sQ = smem, *sK = smem + AT_TILE, *sV = smem + 3 * AT_TILE;      // K: two tiles in turn; V: hi tile, lo tile
-  float* kb = reinterpret_cast<float*>(smem + 5 * AT_TILE);                      // [4][scale 0, scale 1, bias 0, bias 1][128 keys]
-  float2* vb = reinterpret_cast<float2*>(kb + 4 * AQT_KB);                       // [128]: (bias of group 0, of group 1) of a value row
-  float* zx = reinterpret_cast<float*>(vb + 128);                                // [Z][2 halves][2][128]
+  float* kb = reinterpret_cast<float*>(smem + 5 * AT_TILE);                      // [4][scale 0, scale 1, bias 0, bias 1, value biases (two)][128 keys]
+  float* zx = kb + 4 * AQT_KB;                                // [Z][2 halves][2][128]
   float* obx = zx + 2 * AT_MAX_Z * 256;                                          // [2][128]
   float* zo = reinterpret_cast<float*>(sK);                                      // [Z][128 / Z][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 5 * AT_TILE + AQT_XCH);
-  uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 5, *s_full = bars + 6, *s_empty = bars + 8, *p_full = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 5, *s_full = bars + 6, *s_empty = bars + 8, *p_full = bars + 10, *o_free = bars + 12,
+           *w_full = bars + 13, *w_empty = bars + 17;      // (w: the first walk's scores, [buffer][half])
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x, t0 = (int)(gridDim.y - 1 - blockIdx.y) * TB, z = blockIdx.z;      // (the longest row blocks first)
@@ -77,7 +86,8 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], AQT_DQ / 32); mbar_init(&k_empty[i], 1); mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); }
-    mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1); mbar_init(p_full, 8);
+    mbar_init(v_full, AQT_DQ / 32); mbar_init(v_empty, 1); mbar_init(&p_full[0], 8); mbar_init(&p_full[1], 8); mbar_init(o_free, 8);
+    for (int i = 0; i < 4; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -101,47 +111,58 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   __syncthreads();
   if (Z > 1) cluster_sync();      // every CTA of the cluster has started: the first walk's end stores into the others' memory
   tc_fence_after();
-  // S: two halves of a tile in turn, each 64 keys of group 0, then of group 1; P; the tile's product
-  const uint32_t tmem = *tmem_slot, tP = tmem + 256, tO = tmem + 320;
+  // S: two halves of a tile, each 64 keys of group 0, then of group 1 (in the first walk two tiles in turn, the second one's in the columns of P and O); P, two in turn;
+  // the tile's product
+  const uint32_t tmem = *tmem_slot, tO = tmem + 256, tP = tmem + 384;
 
   if (warp < 4) {
     // ===================== products =====================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AQT_REGS_MMA));
     const uint32_t idesc_s = tc_instr_desc(128, 64), idesc_o = tc_instr_desc(128, 128) | (1u << 16);
-    auto scores = [&](int it) {      // of the it-th tile of both walks
+    auto scores = [&](int it, uint32_t at, uint64_t* full, uint64_t* empty, uint32_t empty_phase) {      // of the it-th tile of both walks
       const int kbuf = it & 1;
       mbar_wait(&k_full[kbuf], (uint32_t)(it >> 1) & 1u, p.err);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        mbar_wait(&s_empty[h], ((uint32_t)it & 1u) ^ 1u, p.err);
+        mbar_wait(&empty[h], empty_phase, p.err);
         tc_fence_after();
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           const uint64_t adesc = tc_smem_desc(sQ + g * 16384), bdesc = tc_smem_desc(sK + kbuf * AT_TILE + g * 16384 + h * 8192);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) tc_mma(tmem + h * 128 + g * 64, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_s, k ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) tc_mma(at + h * 128 + g * 64, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_s, k ? 1u : 0u);
         }
         if (h == 1) tc_commit(&k_empty[kbuf]);
-        tc_commit(&s_full[h]);
+        tc_commit(&full[h]);
       }
     };
-    if (warp == 0 && lane == 0)
-      for (int j = 0; j < n_tiles; ++j) scores(j);
+    auto scores2 = [&](int j) { scores(n_tiles + j, tmem, s_full, s_empty, ((uint32_t)j & 1u) ^ 1u); };
+    if (warp == 0 && lane == 0) {
+#pragma unroll 1
+      for (int j = 0; j < n_tiles; ++j) scores(j, tmem + (j & 1) * 256, w_full + (j & 1) * 2, w_empty + (j & 1) * 2, ((uint32_t)(j >> 1) & 1u) ^ 1u);
+    }
     __syncwarp();
     if (Z > 1) cluster_sync();
     if (warp == 0 && lane == 0) {
-      if (n_tiles > 0) scores(n_tiles);
+      if (n_tiles > 0) {
+        const uint32_t uses = (uint32_t)(n_tiles + 1) / 2;      // of the first buffer, which has been read
+        mbar_wait(&w_empty[0], (uses - 1) & 1u, p.err);
+        mbar_wait(&w_empty[1], (uses - 1) & 1u, p.err);
+        scores2(0);
+      }
+#pragma unroll 1
       for (int j = 0; j < n_tiles; ++j) {
-        if (j + 1 < n_tiles) scores(n_tiles + j + 1);
+        if (j + 1 < n_tiles) scores2(j + 1);
         mbar_wait(v_full, (uint32_t)j & 1u, p.err);
-        mbar_wait(p_full, (uint32_t)j & 1u, p.err);
+        mbar_wait(&p_full[j & 1], (uint32_t)(j >> 1) & 1u, p.err);
+        mbar_wait(o_free, ((uint32_t)j & 1u) ^ 1u, p.err);
         tc_fence_after();
 #pragma unroll
         for (int part = 1; part >= 0; --part) {      // the small part first: fewer sums are cut at the size of the result
           const uint64_t vdesc = tc_smem_desc_mn(sV + part * AT_TILE, 16384, 1024);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            tc_mma_ts(tO, tP + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (part == 0 || kk) ? 1u : 0u);
+            tc_mma_ts(tO, tP + (j & 1) * 64 + 8 * kk, vdesc + (uint64_t)(kk * (2048 >> 4)), idesc_o, (part == 0 || kk) ? 1u : 0u);
         }
         tc_commit(v_empty);
       }
@@ -163,19 +184,19 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       const float f = ((bf_lo(v.x) + bf_hi(v.x)) + (bf_lo(v.y) + bf_hi(v.y))) + ((bf_lo(v.z) + bf_hi(v.z)) + (bf_lo(v.w) + bf_hi(v.w)));
       if (c < 8) sq0 += f; else sq1 += f;
     }
-    // Eight keys of the half tile at a time: ask for the products of both groups, and, behind tm_wait_ld, the scores rounded to bf16; keys that the
-    // row does not see: -inf.  it, j: the tile, c: 0, 8, .. 56
-    auto ask = [&](int c, uint32_t (&a)[8], uint32_t (&b)[8]) {
-      tm_ld8(tmem + h * 128 + lane_off + c, a);
-      tm_ld8(tmem + h * 128 + 64 + lane_off + c, b);
-    };
-    auto scores_of = [&](int it, int j, int c, uint32_t (&a)[8], uint32_t (&b)[8], float2 (&s)[4]) {
-      tm_pin8(a);
-      tm_pin8(b);
+    // Sixteen keys of the half tile at a time (900 cycles; eight took 530): the products of both groups into the scores
+    // rounded to bf16; keys that the row does not see: -inf.  it, j: the tile, c: 0, 16, 32, 48
+    auto scores_of = [&](uint32_t at, int it, int j, int c, float2 (&s)[8]) {
+      uint32_t a[16], b[16];
+      aq_ld16(at + lane_off + c, a);
+      aq_ld16(at + 64 + lane_off + c, b);
       const float4* kf = reinterpret_cast<const float4*>(kb + (it & 3) * AQT_KB + h * 64 + c);
       const int key = ((j0 + j) << 7) + h * 64 + c;
+      tm_wait_ld();
+      aq_pin(a);
+      aq_pin(b);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < 4; ++i) {
         const float4 s0 = kf[i], s1 = kf[32 + i], b0 = kf[64 + i], b1 = kf[96 + i];
         auto two = [&](int e, float2 c0, float2 c1, float2 d0, float2 d1) {
           const float2 x = f2_fma(make_float2(__uint_as_float(a[e]), __uint_as_float(a[e + 1])), c0,
@@ -186,45 +207,48 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
         two(4 * i, make_float2(s0.x, s0.y), make_float2(s1.x, s1.y), make_float2(b0.x, b0.y), make_float2(b1.x, b1.y));
         two(4 * i + 2, make_float2(s0.z, s0.w), make_float2(s1.z, s1.w), make_float2(b0.z, b0.w), make_float2(b1.z, b1.w));
       }
-      if (!__all_sync(0xffffffffu, !ok || key + 7 <= last)) {
+      if (!__all_sync(0xffffffffu, !ok || key + 15 <= last)) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 8; ++i) {
           if (key + 2 * i > last) s[i].x = -INFINITY;
           if (key + 2 * i + 1 > last) s[i].y = -INFINITY;
         }
       }
     };
     // ---- first walk: maxima and sums
+#pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       // (the key scales were written before the products that these barriers count were issued; their places are used again four tiles later)
-      mbar_wait(&s_full[h], (uint32_t)j & 1u, p.err);
+      const int w = (j & 1) * 2 + h;
+      mbar_wait(&w_full[w], (uint32_t)(j >> 1) & 1u, p.err);
       __syncwarp();
       tc_fence_after();
-      uint32_t a[2][8], b[2][8];
-      ask(0, a[0], b[0]);
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 16) {
+        float2 s[8];
+        scores_of(tmem + (j & 1) * 256 + h * 128, j, j, c, s);
+        float2 x2 = make_float2(fmaxf(s[0].x, s[1].x), fmaxf(s[0].y, s[1].y)), x3 = make_float2(fmaxf(s[2].x, s[3].x), fmaxf(s[2].y, s[3].y));
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float2 s[4];
-        tm_wait_ld();
-        if (c < 7) ask(8 * c + 8, a[(c + 1) & 1], b[(c + 1) & 1]);
-        scores_of(j, j, 8 * c, a[c & 1], b[c & 1], s);
-        float2 x2 = s[0];
-#pragma unroll
-        for (int i = 1; i < 4; ++i) x2 = make_float2(fmaxf(x2.x, s[i].x), fmaxf(x2.y, s[i].y));
-        const float mx = fmaxf(m, fmaxf(x2.x, x2.y));
-        const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
-        float2 e2 = f2_of(0.f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 x = f2_mul(f2_add(s[i], f2_of(-at)), f2_of(LOG2E));
-          e2 = f2_add(e2, make_float2(tc_ex2(x.x), tc_ex2(x.y)));
+        for (int i = 4; i < 8; i += 2) {
+          x2 = make_float2(fmaxf(x2.x, s[i].x), fmaxf(x2.y, s[i].y));
+          x3 = make_float2(fmaxf(x3.x, s[i + 1].x), fmaxf(x3.y, s[i + 1].y));
         }
+        const float mx = fmaxf(m, fmaxf(fmaxf(x2.x, x2.y), fmaxf(x3.x, x3.y)));
+        const float at = mx == -INFINITY ? 0.f : mx;      // (a row that has seen nothing yet adds zeros)
+        float2 e2 = f2_of(0.f), e3 = e2;
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+          const float2 x = f2_mul(f2_add(s[i], f2_of(-at)), f2_of(LOG2E)), y = f2_mul(f2_add(s[i + 1], f2_of(-at)), f2_of(LOG2E));
+          e2 = f2_add(e2, make_float2(tc_ex2(x.x), tc_ex2(x.y)));
+          e3 = f2_add(e3, make_float2(tc_ex2(y.x), tc_ex2(y.y)));
+        }
+        e2 = f2_add(e2, e3);
         l = fmaf(l, tc_ex2((m - at) * LOG2E), e2.x + e2.y);
         m = mx;
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[h]);
+      if (lane == 0) mbar_arrive(&w_empty[w]);
     }
     // the other half's keys count too, and the other ranks'
     if (Z > 1) {
@@ -268,27 +292,25 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[c * 32 + i] += __uint_as_float(a[i]);
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_free);
     };
+#pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int it = n_tiles + j;
-      if (j > 0) join(j - 1);      // (it has read its probabilities, too)
-      mbar_wait(v_full, (uint32_t)j & 1u, p.err);             // the value biases are written
       float2 t0s = f2_of(0.f), t1s = t0s;
-      mbar_wait(&s_full[h], (uint32_t)it & 1u, p.err);
+      mbar_wait(&s_full[h], (uint32_t)j & 1u, p.err);
       __syncwarp();
       tc_fence_after();
-      uint32_t a[2][8], b[2][8];
-      ask(0, a[0], b[0]);
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 16) {
+        float2 s[8];
+        scores_of(tmem + h * 128, it, j, c, s);
+        const float4* b4 = reinterpret_cast<const float4*>(kb + (it & 3) * AQT_KB + 512) + (h * 64 + c) / 2;
+        uint32_t w[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float2 s[4];
-        tm_wait_ld();
-        if (c < 7) ask(8 * c + 8, a[(c + 1) & 1], b[(c + 1) & 1]);
-        scores_of(it, j, 8 * c, a[c & 1], b[c & 1], s);
-        const float4* b4 = reinterpret_cast<const float4*>(vb + h * 64 + 8 * c);
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 8; ++i) {
           const float2 x = f2_mul(f2_add(s[i], f2_of(-m)), f2_of(LOG2E)), e = f2_mul(make_float2(tc_ex2(x.x), tc_ex2(x.y)), f2_of(inv));
           w[i] = ok ? pack_bf16x2(e.x, e.y) : 0u;
           const float pa = __uint_as_float(w[i] << 16), pd = __uint_as_float(w[i] & 0xffff0000u);
@@ -296,7 +318,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
           t0s = f2_fma(f2_of(pa), make_float2(bv.x, bv.y), t0s);
           t1s = f2_fma(f2_of(pd), make_float2(bv.z, bv.w), t1s);
         }
-        tm_st4(tP + lane_off + h * 32 + 4 * c, w);
+        aq_st8(tP + (j & 1) * 64 + lane_off + h * 32 + c / 2, w);      // (the product that read this one's place was joined a tile ago)
       }
       tc_fence_before();
       __syncwarp();
@@ -306,7 +328,8 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       tm_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
+      if (j > 0) join(j - 1);      // (formed while this tile's probabilities were)
     }
     if (n_tiles > 0) join(n_tiles - 1);
     // the bias terms of both halves' keys: this thread's columns are those of group h
@@ -349,82 +372,89 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     constexpr int CH = KvQ<BITS>::ROW_BYTES / 16, PER = 128 * CH / AQT_DQ;      // 16-byte chunks of a row, of a thread
     constexpr int CODES = 128 / BITS;                                           // codes of a chunk: 16 / 32
     const int dt = (int)threadIdx.x - (AQT_THREADS - AQT_DQ);
-    // the codes, less MID, of eight numbers: o-th of the chunk
-    auto codes8 = [&](const uint4& cw, int o, float (&f)[8]) {
+    // The codes, less MID, of eight numbers, the o-th eight of the chunk: a code as the low byte of 2^23 + code, one subtraction for two
+    auto codes8 = [&](const uint4& cw, int o, float2 (&f)[4]) {
       const uint32_t u[4] = {cw.x, cw.y, cw.z, cw.w};
+      const float2 off = f2_of(-(8388608.f + MID));
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t c = BITS == 8 ? (u[(o * 2 + (k >> 2)) & 3] >> (8 * (k & 3))) & 0xffu : (u[o & 3] >> (4 * k)) & 0xfu;
-        f[k] = (float)c - MID;
+      for (int k = 0; k < 4; ++k) {
+        uint32_t a, b;
+        if (BITS == 8) {
+          const uint32_t w = u[(o * 2 + (k >> 1)) & 3];
+          a = __byte_perm(w, 0x4B000000u, 0x7440 + (k & 1) * 2);
+          b = __byte_perm(w, 0x4B000000u, 0x7441 + (k & 1) * 2);
+        } else {
+          a = __byte_perm(u[o & 3] & 0x0f0f0f0fu, 0x4B000000u, 0x7440 + k);
+          b = __byte_perm((u[o & 3] >> 4) & 0x0f0f0f0fu, 0x4B000000u, 0x7440 + k);
+        }
+        f[k] = f2_add(f2_bits(a, b), off);
       }
     };
-    auto load = [&](int j, int kv, uint4 (&cw)[PER], uint32_t& sw, uint32_t& bw) {      // sw, bw: scales and biases of row dt (threads 0 .. 127)
-      const int key0 = (j0 + j) << 7, pl = 2 * (j0 + j);
+    // A unit is a tile's keys or values: those of the first walk, then keys and values of the second in turn.  The next unit's codes are on their way while one is
+    // turned into operands.
+    // codes; keys: scales and biases of row dt (threads 0 .. 127; 128 .. 255: of the second walk's value rows); values: the scale of each chunk's row and group
+    struct Unit { uint4 cw[PER]; uint32_t sw, bw; uint32_t sc[PER]; };
+    const int units = 3 * n_tiles;
+    auto tile_of = [&](int x) { return x < n_tiles ? x : (x - n_tiles) >> 1; };
+    auto load = [&](int x, Unit& U) {
+      const int j = tile_of(x), kv = x >= n_tiles ? (x - n_tiles) & 1 : 0, key0 = (j0 + j) << 7, pl = 2 * (j0 + j);
       const int pg0 = p.block_table[pl], pg1 = pl + 1 < pages ? p.block_table[pl + 1] : pg0;
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
+        const int y = i * AQT_DQ + dt, row = y / CH, c = y % CH;
         const unsigned char* unit = kvq_unit<BITS>(pq.pool, row < 64 ? pg0 : pg1, kv, kvh, p.n_kv);
-        cw[i] = key0 + row < kv_max ? __ldcg(reinterpret_cast<const uint4*>(unit + (size_t)(row & 63) * KvQ<BITS>::ROW_BYTES) + c) : make_uint4(0u, 0u, 0u, 0u);
+        const bool have = key0 + row < kv_max;      // rows that belong to no key: whatever the page holds, it must not enter
+        U.cw[i] = have ? __ldcg(reinterpret_cast<const uint4*>(unit + (size_t)(row & 63) * KvQ<BITS>::ROW_BYTES) + c) : make_uint4(0u, 0u, 0u, 0u);
+        U.sc[i] = kv && have ? (uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(unit + KvQ<BITS>::CODES_BYTES) + (row & 63) * 2 + (c * CODES >= 64 ? 1 : 0)) : 0u;
       }
-      sw = bw = 0u;
-      if (dt < 128 && key0 + dt < kv_max) {      // rows that belong to no key: whatever the page holds, it must not enter
-        const uint32_t* sb = reinterpret_cast<const uint32_t*>(kvq_unit<BITS>(pq.pool, dt < 64 ? pg0 : pg1, kv, kvh, p.n_kv) + KvQ<BITS>::CODES_BYTES);
-        sw = __ldcg(sb + (dt & 63));
-        bw = __ldcg(sb + PAGE + (dt & 63));
+      U.sw = U.bw = 0u;
+      if (!kv && key0 + (dt & 127) < kv_max && (dt < 128 || x >= n_tiles)) {
+        const uint32_t* sb = reinterpret_cast<const uint32_t*>(kvq_unit<BITS>(pq.pool, (dt & 127) < 64 ? pg0 : pg1, dt >> 7, kvh, p.n_kv) + KvQ<BITS>::CODES_BYTES);
+        U.sw = __ldcg(sb + (dt & 63));
+        U.bw = __ldcg(sb + PAGE + (dt & 63));
       }
     };
-    auto keys = [&](int it, int j) {
-      uint4 cw[PER];
-      uint32_t sw, bw;
-      load(j, 0, cw, sw, bw);
+    auto keys = [&](int it, const Unit& U) {
       unsigned char* dst = sK + (it & 1) * AT_TILE;
       mbar_wait(&k_empty[it & 1], ((uint32_t)(it >> 1) & 1u) ^ 1u, p.err);
       if (dt < 128) {
         float* f = kb + (it & 3) * AQT_KB + dt;
-        f[0] = bf_lo(sw); f[128] = bf_hi(sw);
-        f[256] = fmaf(bf_lo(sw), MID, bf_lo(bw)); f[384] = fmaf(bf_hi(sw), MID, bf_hi(bw));
-      }
+        f[0] = bf_lo(U.sw); f[128] = bf_hi(U.sw);
+        f[256] = fmaf(bf_lo(U.sw), MID, bf_lo(U.bw)); f[384] = fmaf(bf_hi(U.sw), MID, bf_hi(U.bw));
+      } else if (it >= n_tiles)
+        *reinterpret_cast<float2*>(kb + (it & 3) * AQT_KB + 512 + 2 * (dt - 128)) = make_float2(fmaf(bf_lo(U.sw), MID, bf_lo(U.bw)), fmaf(bf_hi(U.sw), MID, bf_hi(U.bw)));
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
 #pragma unroll
         for (int o = 0; o < CODES / 8; ++o) {       // eight codes: a 16-byte chunk of the tile
-          float f[8];
-          codes8(cw[i], o, f);
-          *reinterpret_cast<uint4*>(dst + at_swz(row, c * (CODES / 8) + o)) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          float2 f[4];
+          codes8(U.cw[i], o, f);
+          *reinterpret_cast<uint4*>(dst + at_swz(row, c * (CODES / 8) + o)) =
+              make_uint4(upper_halves(f[0].x, f[0].y), upper_halves(f[1].x, f[1].y), upper_halves(f[2].x, f[2].y), upper_halves(f[3].x, f[3].y));      // (exact: eight bits)
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&k_full[it & 1]);
     };
-    auto values = [&](int j) {
-      uint4 cw[PER];
-      uint32_t sw, bw;
-      load(j, 1, cw, sw, bw);
-      float sc[PER];
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {      // the scale of the chunk's row and group
-        const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH, pl = 2 * (j0 + j) + (row >> 6);
-        const unsigned short* su = reinterpret_cast<const unsigned short*>(kvq_unit<BITS>(pq.pool, p.block_table[pl < pages ? pl : pl - 1], 1, kvh, p.n_kv) + KvQ<BITS>::CODES_BYTES);
-        sc[i] = ((j0 + j) << 7) + row < kv_max ? __uint_as_float((uint32_t)__ldcg(su + (row & 63) * 2 + (c * CODES >= 64 ? 1 : 0)) << 16) : 0.f;
-      }
+    auto values = [&](int j, const Unit& U) {
       mbar_wait(v_empty, ((uint32_t)j & 1u) ^ 1u, p.err);
-      if (dt < 128) vb[dt] = make_float2(fmaf(bf_lo(sw), MID, bf_lo(bw)), fmaf(bf_hi(sw), MID, bf_hi(bw)));
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         const int x = i * AQT_DQ + dt, row = x / CH, c = x % CH;
+        const float2 sc = f2_of(__uint_as_float(U.sc[i] << 16));
 #pragma unroll
         for (int o = 0; o < CODES / 8; ++o) {       // eight codes: one 16-byte chunk of each tile
-          float f[8];
-          codes8(cw[i], o, f);
+          float2 f[4];
+          codes8(U.cw[i], o, f);
           uint32_t hi[4], lo[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const float a = f[2 * k] * sc[i], b = f[2 * k + 1] * sc[i];
-            hi[k] = pack_bf16x2(a, b);
-            lo[k] = pack_bf16x2(a - __uint_as_float(hi[k] << 16), b - __uint_as_float(hi[k] & 0xffff0000u));
+            const float2 y = f2_mul(f[k], sc);
+            hi[k] = pack_bf16x2(y.x, y.y);
+            const float2 r = f2_fma(f2_bits(hi[k] << 16, hi[k] & 0xffff0000u), f2_of(-1.f), y);
+            lo[k] = pack_bf16x2(r.x, r.y);
           }
           const uint32_t at = at_swz(row, c * (CODES / 8) + o);
           *reinterpret_cast<uint4*>(sV + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -435,10 +465,18 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
       __syncwarp();
       if (lane == 0) mbar_arrive(v_full);
     };
-    for (int j = 0; j < n_tiles; ++j) keys(j, j);
-    __syncwarp();
-    if (Z > 1) cluster_sync();
-    for (int j = 0; j < n_tiles; ++j) { keys(n_tiles + j, j); values(j); }
+    Unit cur, nxt;
+    if (units > 0) load(0, cur);
+#pragma unroll 1
+    for (int x = 0; x < units; ++x) {
+      if (x + 1 < units) load(x + 1, nxt);
+      if (x < n_tiles) keys(x, cur);
+      else if (((x - n_tiles) & 1) == 0) keys(n_tiles + tile_of(x), cur);
+      else values(tile_of(x), cur);
+      cur = nxt;
+      if (x == n_tiles - 1) { __syncwarp(); if (Z > 1) cluster_sync(); }      // (the end of the first walk)
+    }
+    if (units == 0) { __syncwarp(); if (Z > 1) cluster_sync(); }
     __syncwarp();
     if (Z > 1) { cluster_sync(); cluster_sync(); }
   }
