@@ -1591,7 +1591,7 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
       if (run_ok(1 << 20) && lc.dim % 8 == 0 && lc.dim <= 256 && (lc.dim & (lc.dim - 1)) == 0) {
-        const int tok = 2 * l.Cq + l.Cv > RUN_DELTA_CHANNELS ? run_tok(N, (int)prep_threads(2 * l.Cq + l.Cv).x, g_sms, RUN_DELTA_FROM) : 1;
+        const int tok = run_tok(N, (int)prep_threads(2 * l.Cq + l.Cv).x, g_sms, 2 * l.Cq + l.Cv > RUN_DELTA_CHANNELS ? RUN_DELTA_WIDE_FROM : RUN_DELTA_FROM);
         auto go = [&](auto kern) {
           return launch(kern, dim3((N + tok - 1) / tok), prep_threads(2 * l.Cq + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
                         (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const float*)m->pa, (const float*)m->pb, (const bf16*)l.w[DN_SQ_A_LOG],
