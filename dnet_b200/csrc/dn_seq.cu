@@ -1107,7 +1107,7 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
   auto wm = [&](int i) { return l.tm_ok[i] ? &l.tm[i] : (const CUtensorMap*)nullptr; };
   CK(mark(m, DN_SEQ_PH_ROUTER, s));
   if (scored)
-    CK(launch(k_router_scored<T>, dim3(N), dim3(32 * std::min(32, std::max(4, Et + 1))), (size_t)2 * Et * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_CORR),
+    CK(launch(k_router_scored<T>, dim3(N), dim3(32 * std::min(32, (Et + (lc.shared_gate ? 1 : 0) + ROUTER_ROWS - 1) / ROUTER_ROWS)), (size_t)2 * Et * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_CORR),
               W, Et, top, lc.groups, lc.groups_keep, lc.router_scale, lc.shared_gate ? w(DN_SQ_SH_SG) : (const T*)nullptr, m->ridx, m->rwt, m->rpos, m->sgate, lc.score_kind == DN_SCORE_SIGMOID ? 1 : 0));
   else
     CK(launch(k_router<T>, dim3(N), dim3(32 * std::min(32, std::max(4, E))), (size_t)E * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_B), W, E, top, m->ridx, m->rwt, m->rpos));

@@ -614,17 +614,27 @@ __global__ void k_rms_join(float* __restrict__ x, int W, const float* __restrict
 //   u = y + y2 + sum_j wt[j] (expert output j | the input, for an identity expert) + gate sh        (all but y optional)
 //   x <- x + m u;   h <- RMS norm of x with the next layer's weight (hout null: no norm follows)
 // One block per token, VEC columns a thread; partial sums of squares in the fixed order of k_read_norm.
+constexpr int MOE_JOIN = 16;      // experts of a token at most
 template <class T, int VEC>
 __global__ void k_parallel_join(float* __restrict__ x, int W, float m, const float* __restrict__ y, const float* __restrict__ y2, MoeSrc<T> ms,
                                 const T* __restrict__ nw, int wmode, float eps, T* __restrict__ hout) {
   extern __shared__ __align__(16) float sm[];
   float* v = sm;            // [W]
   float* red = sm + W;      // [33]
+  __shared__ float wts[MOE_JOIN];
+  __shared__ int rows[MOE_JOIN];      // of the chosen experts' outputs; -1: an identity expert
   const size_t n = blockIdx.x, base = n * W;
   auto ld = [](const float* p, float (&o)[VEC]) {
     if (VEC == 4) *reinterpret_cast<float4*>(o) = *reinterpret_cast<const float4*>(p);
     else o[0] = p[0];
   };
+  if (ms.eo) {      // (read once a block, ahead of the rows: weight, place and row one behind the other for each expert took 19 us for 1,000 tokens of 2,048, 4 experts each; 14.7 so)
+    for (int j = threadIdx.x; j < ms.top; j += blockDim.x) {
+      wts[j] = ms.wt[n * ms.top + j];
+      rows[j] = ms.idx[n * ms.top + j] < ms.E ? ms.pos[n * ms.top + j] : -1;
+    }
+    __syncthreads();
+  }
   float ss = 0.f;
   for (int c = threadIdx.x * VEC; c < W; c += blockDim.x * VEC) {
     float u[VEC], t[VEC], xv[VEC];
@@ -636,15 +646,25 @@ __global__ void k_parallel_join(float* __restrict__ x, int W, float m, const flo
       for (int i = 0; i < VEC; i++) u[i] += t[i];
     }
     if (ms.eo) {
-      for (int j = 0; j < ms.top; j++) {
-        const float wj = ms.wt[n * ms.top + j];
-        if (ms.idx[n * ms.top + j] < ms.E) ld(ms.eo + (size_t)ms.pos[n * ms.top + j] * W + c, t);
-        else {
+      for (int j0 = 0; j0 < ms.top; j0 += 4) {
+        float e[4][VEC];
 #pragma unroll
-          for (int i = 0; i < VEC; i++) t[i] = ldf(ms.hid + base + c + i);
+        for (int j = 0; j < 4; j++) {
+          if (j0 + j >= ms.top) continue;
+          const int r = rows[j0 + j];
+          if (r >= 0) ld(ms.eo + (size_t)r * W + c, e[j]);
+          else {
+#pragma unroll
+            for (int i = 0; i < VEC; i++) e[j][i] = ldf(ms.hid + base + c + i);
+          }
         }
 #pragma unroll
-        for (int i = 0; i < VEC; i++) u[i] = fmaf(wj, t[i], u[i]);
+        for (int j = 0; j < 4; j++) {
+          if (j0 + j >= ms.top) continue;
+          const float wj = wts[j0 + j];
+#pragma unroll
+          for (int i = 0; i < VEC; i++) u[i] = fmaf(wj, e[j][i], u[i]);
+        }
       }
     }
     if (ms.sh) {
