@@ -777,7 +777,10 @@ static int attend_q_tc(dn_model* m, const unsigned char* pool, const bf16* q, bf
   a.a.q = q; a.a.out = out; a.a.block_table = kv->block_table; a.a.st = kv->st;
   a.a.n_heads = c.n_heads; a.a.n_kv = c.n_kv_heads; a.a.T = T; a.a.err = m->mk_sync + 2;
   a.pool = pool;
-  const dim3 grid = attn_tc_grid(m, T, kv, a.a);
+  const int tb = 128 / m->G, blocks = (T + tb - 1) / tb;
+  const AqCut cut = attn_q_cut(c.n_kv_heads, blocks, tb, kv->host_pos + T, g_sms);
+  a.a.sms = g_sms; a.a.share = g_capturing ? 0 : cut.Z; a.whole = cut.whole;
+  const dim3 grid(c.n_kv_heads, g_capturing ? blocks : blocks - cut.whole / 2, g_capturing ? attn_q_cut_max(c.n_kv_heads, blocks, tb, kv->max_tokens, g_sms) : cut.Z);
 #define PFQ(Gv) case Gv: CK(launch_attn_tc(k_attn_prefill_q<Gv, BITS>, grid, AQT_THREADS, AQT_SMEM, s, pdl, a)); break;
   switch (m->G) { PFQ(1) PFQ(2) PFQ(4) PFQ(5) PFQ(7) PFQ(8) default: return fail(DN_EINVAL, "GQA group unsupported"); }
 #undef PFQ

@@ -1,7 +1,7 @@
 // dn_attn_q.cuh -- causal attention of a prefill chunk over the 8- / 4-bit quantised KV cache (dn_kvquant.cuh has the format and the
 // semantics) on the 5th-generation tensor cores, libdnet_b200.so.
 //
-// Rows, blocks and the cluster's share of the keys are those of k_attn_prefill_tc (dn_attn_tc.cuh).  The semantics round scores and
+// Rows and row blocks are those of k_attn_prefill_tc (dn_attn_tc.cuh), the cluster's share of the keys is attn_q_cut's.  The semantics round scores and
 // probabilities to bf16, which an online softmax cannot reproduce: the key tiles are walked twice, first for every row's maximum and
 // sum, then for the probabilities and the output.  Rounded numbers land on the other side of an edge by as little as their sums are off, so that
 // the sums are kept as short and as small as the format allows.  With codes less the middle of their range (c' = c - 128 or c - 8, exact in bf16)
@@ -30,7 +30,60 @@ namespace dn {
 struct AqParams {
   AtParams a;
   const unsigned char* pool;     // this layer's packed pages
+  int whole;                     // beside a.share: AqCut::whole
 };
+
+// How a launch's work is cut: Z CTAs share a row block's keys; with `whole`, each of a key head's `whole` longest row blocks (an even number) is one CTA's
+// and only the others are shared.  The CTAs of a launch, longest first, run in rounds of as many as the SMs hold at once; whoever ends first in a round begins first
+// in the next, so that a round's last goes with the next one's first.  Taken is what makes the sum of the rounds smallest, in key tiles (6.9 us each) and 1.5 to 2.5
+// for a CTA's start, exchange and end (weights and the three tiles that halves behind whole blocks are charged: what is taken is then, on average, within 0.1 % of
+// the fastest of all cuts over 380 shapes of 1 to 2,000 tokens behind 0 to 16,000, groups of 1, 4, 5 and 8, and nowhere slower than by the rule of
+// k_attn_prefill_tc, whose tiles take a third as long beside the same start and end: 3.7 % less on average).  8 bits, groups of 4, in us by that rule and so: 8 heads, 777
+// tokens behind 1,024, 200 blocks in rounds of 148 and 52: 159 and 148; one token behind 500 35 and 25; 300 behind 4,000 243 and 212; 160 behind 8,000 234 and
+// 203; 2 heads, 1,500 tokens 90 and 54.
+struct AqCut {
+  int Z, whole;
+};
+__host__ __device__ inline AqCut attn_q_cut(int n_kv, int blocks, int tb, int kv_len, int sms) {
+  const int n = n_kv * blocks, tiles = (kv_len + 127) / 128, keys = tiles * 128;
+  // tenths of a key tile that a CTA of the i-th longest block takes
+  auto weight = [&](int i, int Z) {
+    const int t = (keys - i / n_kv * tb + 127) / 128;
+    return (t + Z - 1) / Z * 10 + (Z == 1 ? 15 : Z == 2 ? 22 : Z == 4 ? 24 : 25);
+  };
+  auto cost = [&](int Z, int whole) {
+    const int at_once = Z == 1 ? sms : Z == 2 ? sms / 2 : Z == 4 ? sms * 33 / 148 : sms * 15 / 148, first = whole * n_kv;
+    const int r1 = (first + sms - 1) / sms, rounds = r1 + (n - first + at_once - 1) / at_once;
+    int sum = 0;
+    for (int r = 0; r < rounds; ++r) {
+      const bool end = !(r & 1) && r + 1 < rounds;      // this round's last counts, else its first
+      if (r < r1) sum += weight(end ? ((r + 1) * sms < first ? (r + 1) * sms : first) - 1 : r * sms, 1);
+      else sum += weight(end ? ((r - r1 + 1) * at_once < n - first ? first + (r - r1 + 1) * at_once : n) - 1 : first + (r - r1) * at_once, Z);
+    }
+    const int longest = weight(0, whole ? 1 : Z);
+    return (sum > longest ? sum : longest) + (whole ? 30 : 0);      // (halves behind whole blocks: their rounds end further apart)
+  };
+  AqCut best{1, 0};
+  int least = cost(1, 0);
+  for (int Z = 2; Z <= AT_MAX_Z && tiles >= 2 * Z; Z *= 2) {
+    const int c = cost(Z, 0);
+    if (c < least) { least = c; best = AqCut{Z, 0}; }
+  }
+  for (int r = 1; r * sms < n && tiles >= 4; ++r) {      // whole rounds of whole blocks, the others in halves
+    const int whole = r * sms / n_kv & ~1, c = whole ? cost(2, whole) : least;
+    if (c < least) { least = c; best = AqCut{2, whole}; }
+  }
+  return best;
+}
+// a captured launch's clusters (as attn_prefill_split_max)
+static inline int attn_q_cut_max(int n_kv, int blocks, int tb, int kv_len, int sms) {
+  int best = 1;
+  for (int n = (blocks - 1) * tb + 1; n < kv_len + 128 && best < AT_MAX_Z; n += 128) {
+    const int z = attn_q_cut(n_kv, blocks, tb, n, sms).Z;
+    if (z > best) best = z;
+  }
+  return best;
+}
 constexpr int AQT_THREADS = 640, AQT_DQ = 256;
 constexpr int AQT_KB = 6 * 128;      // floats of a key tile: scales of both groups, biases of both groups, (bias of group 0, of group 1) of each value row
 constexpr int AQT_XCH = (4 * AQT_KB + 2 * AT_MAX_Z * 2 * 128 + 2 * 128) * 4;      // four key tiles' scales and biases, the maxima and sums of both halves of every rank,
@@ -76,9 +129,13 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x, t0 = (int)(gridDim.y - 1 - blockIdx.y) * TB, z = blockIdx.z;      // (the longest row blocks first)
-  const int pos0 = p.st->pos;
-  const int Z = p.share > 0 ? p.share : attn_prefill_split((int)(gridDim.x * gridDim.y), pos0 + p.T, p.sms);
+  const int pos0 = p.st->pos, blocks = (p.T + TB - 1) / TB;
+  const AqCut cut = p.share > 0 ? AqCut{p.share, pq.whole} : attn_q_cut((int)gridDim.x, blocks, TB, pos0 + p.T, p.sms);
+  // a cluster's block, the longest first: whole ones by twos, one each for the cluster's first two CTAs (the others, as all beyond the share, have nothing to do)
+  const bool alone = 2 * (int)blockIdx.y < cut.whole;
+  const int block = alone ? 2 * (int)blockIdx.y + min((int)blockIdx.z, 1) : (int)blockIdx.y + cut.whole / 2;
+  if (block >= blocks) return;
+  const int kvh = blockIdx.x, t0 = (blocks - 1 - block) * TB, z = alone && blockIdx.z == 1 ? 0 : (int)blockIdx.z, Z = alone ? 1 : cut.Z;
   const int nq = min(TB, p.T - t0);
   const int kv_max = pos0 + t0 + nq;
   const int pages = (kv_max + PAGE - 1) / PAGE, all = (kv_max + 127) >> 7;
