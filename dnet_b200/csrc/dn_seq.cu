@@ -1106,9 +1106,15 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
   auto w = [&](int i) { return (const T*)l.w[i]; };
   auto wm = [&](int i) { return l.tm_ok[i] ? &l.tm[i] : (const CUtensorMap*)nullptr; };
   CK(mark(m, DN_SEQ_PH_ROUTER, s));
-  if (scored)
-    CK(launch(k_router_scored<T>, dim3(N), dim3(32 * std::min(32, (Et + (lc.shared_gate ? 1 : 0) + ROUTER_ROWS - 1) / ROUTER_ROWS)), (size_t)2 * Et * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_CORR),
-              W, Et, top, lc.groups, lc.groups_keep, lc.router_scale, lc.shared_gate ? w(DN_SQ_SH_SG) : (const T*)nullptr, m->ridx, m->rwt, m->rpos, m->sgate, lc.score_kind == DN_SCORE_SIGMOID ? 1 : 0));
+  if (scored) {
+    const int rows = Et + (lc.shared_gate ? 1 : 0);
+    auto go = [&](auto kern, int warps) {
+      return launch(kern, dim3(N), dim3(32 * warps), (size_t)2 * Et * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_CORR), W, Et, top, lc.groups, lc.groups_keep, lc.router_scale,
+                    lc.shared_gate ? w(DN_SQ_SH_SG) : (const T*)nullptr, m->ridx, m->rwt, m->rpos, m->sgate, lc.score_kind == DN_SCORE_SIGMOID ? 1 : 0);
+    };
+    if (router_queues(N, rows, g_sms)) CK(go(k_router_scored<T, ROUTER_ROWS>, std::min(32, (rows + ROUTER_ROWS - 1) / ROUTER_ROWS)));
+    else CK(go(k_router_scored<T, 1>, router_warps_of_rows(rows)));
+  }
   else
     CK(launch(k_router<T>, dim3(N), dim3(32 * std::min(32, std::max(4, E))), (size_t)E * 4, s, (const T*)m->h, w(DN_SQ_ROUTER), w(DN_SQ_ROUTER_B), W, E, top, m->ridx, m->rwt, m->rpos));
   const bool few = N <= 8;
@@ -1484,13 +1490,13 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(launch(k_attn_prep_rot<T>, dim3(N, (units + per * PREP_WARPS - 1) / (per * PREP_WARPS)), dim3(32 * PREP_WARPS), 0, s, a, b, per, (const T*)m->uq, (const T*)m->uk,
                   (const T*)m->uv, w(DN_SQ_Q_NORM), w(DN_SQ_K_NORM), (T*)m->qb, (T*)m->kpool[run.kv_index], (T*)m->vpool[run.kv_index]));
       } else if (run_ok(RUN_VECS) && (lc.qk_norm == DN_QKNORM_WHOLE || lc.qk_norm == 0) && !a.half && lc.dim % 8 == 0 && lc.rot_dims <= RUN_MAX_ROT) {
-        const int tok = run_tok(N, (int)prep_threads(l.Cq + l.Ck + l.Cv).x, g_sms, RUN_ATTN_FROM);
+        const int tok = N <= g_sms ? 1 : run_tok(N, (int)prep_threads(l.Cq + l.Ck + l.Cv).x, g_sms, RUN_ATTN_FROM);
         auto go = [&](auto kern) {
           return launch(kern, dim3((N + tok - 1) / tok), prep_threads(l.Cq + l.Ck + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
                         (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const bf16*)l.w[DN_SQ_Q_NORM], (const bf16*)l.w[DN_SQ_K_NORM], (bf16*)cst, m->conv_stride, (bf16*)m->qb,
                         (bf16*)m->kpool[run.kv_index], (bf16*)m->vpool[run.kv_index]);
         };
-#define PR(TP) (tok == 1 ? go(k_attn_prep_run<TP, 1>) : go(k_attn_prep_run<TP, RUN_TOK>))
+#define PR(TP) (N <= g_sms ? go(k_attn_prep_run<TP, 1, true>) : tok == 1 ? go(k_attn_prep_run<TP, 1>) : go(k_attn_prep_run<TP, RUN_TOK>))
         CK(lc.conv == 0 ? PR(0) : lc.conv == 1 ? PR(1) : lc.conv == 2 ? PR(2) : lc.conv == 3 ? PR(3) : PR(4));
 #undef PR
       } else
@@ -1591,13 +1597,13 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       DeltaPrep a{lc.heads, lc.kv_heads, lc.dim, lc.vdim, lc.conv};
       PH(DN_SEQ_PH_DELTA_PREP);
       if (run_ok(1 << 20) && lc.dim % 8 == 0 && lc.dim <= 256 && (lc.dim & (lc.dim - 1)) == 0) {
-        const int tok = run_tok(N, (int)prep_threads(2 * l.Cq + l.Cv).x, g_sms, 2 * l.Cq + l.Cv > RUN_DELTA_CHANNELS ? RUN_DELTA_WIDE_FROM : RUN_DELTA_FROM);
+        const int tok = N <= g_sms ? 1 : run_tok(N, (int)prep_threads(2 * l.Cq + l.Cv).x, g_sms, 2 * l.Cq + l.Cv > RUN_DELTA_CHANNELS ? RUN_DELTA_WIDE_FROM : RUN_DELTA_FROM);
         auto go = [&](auto kern) {
           return launch(kern, dim3((N + tok - 1) / tok), prep_threads(2 * l.Cq + l.Cv), 0, s, a, b, (const bf16*)m->uq, (const bf16*)m->uk, (const bf16*)m->uv, (const bf16*)l.w[DN_SQ_Q_CONV],
                         (const bf16*)l.w[DN_SQ_K_CONV], (const bf16*)l.w[DN_SQ_V_CONV], (const float*)m->pa, (const float*)m->pb, (const bf16*)l.w[DN_SQ_A_LOG],
                         (const bf16*)l.w[DN_SQ_DT_BIAS], (bf16*)cst, m->conv_stride, m->qn, m->kn, m->vv, m->beta, m->decay);
         };
-#define PR(TP) (tok == 1 ? go(k_delta_prep_run<TP, 1>) : go(k_delta_prep_run<TP, RUN_TOK>))
+#define PR(TP) (N <= g_sms ? go(k_delta_prep_run<TP, 1, true>) : tok == 1 ? go(k_delta_prep_run<TP, 1>) : go(k_delta_prep_run<TP, RUN_TOK>))
         CK(lc.conv == 0 ? PR(0) : lc.conv == 1 ? PR(1) : lc.conv == 2 ? PR(2) : lc.conv == 3 ? PR(3) : PR(4));
 #undef PR
       } else

@@ -95,7 +95,14 @@ __device__ __forceinline__ float warp_dot(const T* __restrict__ x, const T* __re
 // of the `keep` best runs can be chosen (ties: the lower index, for runs and experts alike); the `top` largest c choose;
 // weights = s[chosen] / (their sum + 1e-20) * scale.  sg (optional): one more row, sgate[n] = sigmoid(sg . h).
 constexpr int ROUTER_ROWS = 4;
-template <class T>
+// A block of one token costs the start and end of its warps, where blocks queue, and the way of a warp along its rows, where they do not.  Where not all blocks
+// of a warp a row run at once, a warp therefore takes ROUTER_ROWS rows against one reading of the token and a block has no more warps than that takes; else a
+// warp takes a row.  us of a row / four rows, warm caches: 4,096 columns, 16 experts: 2 tokens 8.4 / 10.6, 444 11.0 / 12.5, 600 16.9 / 12.5; 32 experts: 148 9.8 / 12.5, 300 16.6 / 12.6;
+// 2,048, 16: 444 8.5 / 9.2, 1,000 14.6 / 10.5; 2,048, 8: 1,000 9.4 / 10.4.  In a decode step of two tokens, cold, 4,096 columns: 12.1 / 20.6.
+inline int router_warps_of_rows(int rows) { return rows < 4 ? 4 : rows > 32 ? 32 : rows; }
+inline bool router_queues(int tokens, int rows, int sms) { return (long long)tokens * 32 * router_warps_of_rows(rows) > (long long)sms * 2048; }
+// ROWS: weight rows that a warp takes at a time, 1 or ROUTER_ROWS
+template <class T, int ROWS>
 __global__ void __launch_bounds__(1024) k_router_scored(const T* __restrict__ h, const T* __restrict__ Wr, const T* __restrict__ corr, int W, int Et,
                                                        int top, int groups, int keep, float scale, const T* __restrict__ sg,
                                                        int32_t* __restrict__ idx, float* __restrict__ wt, int32_t* __restrict__ pos,
@@ -105,14 +112,20 @@ __global__ void __launch_bounds__(1024) k_router_scored(const T* __restrict__ h,
   const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const T* x = h + (size_t)n * W;
   const bool vec = W % Vec16<T>::n == 0 && ((((uintptr_t)h | (uintptr_t)Wr | (uintptr_t)(sg ? sg : Wr)) & 15) == 0);
-  // A warp takes ROUTER_ROWS rows at a time against one reading of the token, and a block has no more warps than that takes: starting and ending warps is what a block
-  // of one token costs (1,000 tokens of 2,048 against 16 experts, warm caches: a row a warp, 17 warps, 24.8 us; five warps, one idle, 16.7; four 10.5).
   const int rows = Et + (sg ? 1 : 0);
-  for (int e0 = warp * ROUTER_ROWS; e0 < rows; e0 += nw * ROUTER_ROWS) {
-    float a[ROUTER_ROWS];
-    const T* wr[ROUTER_ROWS];
+  if constexpr (ROWS == 1) {
+    for (int e = warp; e < rows; e += nw) {
+      const float a = warp_dot(x, e < Et ? Wr + (size_t)e * W : sg, W, vec);
+      if (lane == 0) {
+        if (e < Et) zl[e] = a;
+        else sgate[n] = sigmoid_f(a);
+      }
+    }
+  } else for (int e0 = warp * ROWS; e0 < rows; e0 += nw * ROWS) {
+    float a[ROWS];
+    const T* wr[ROWS];
 #pragma unroll
-    for (int k = 0; k < ROUTER_ROWS; k++) {
+    for (int k = 0; k < ROWS; k++) {
       const int e = min(e0 + k, rows - 1);
       wr[k] = e < Et ? Wr + (size_t)e * W : sg;
       a[k] = 0.f;
@@ -122,24 +135,24 @@ __global__ void __launch_bounds__(1024) k_router_scored(const T* __restrict__ h,
 #pragma unroll 2
       for (int c = lane * V; c < W; c += 32 * V) {
         const uint4 xr = *reinterpret_cast<const uint4*>(x + c);
-        uint4 wv[ROUTER_ROWS];
+        uint4 wv[ROWS];
 #pragma unroll
-        for (int k = 0; k < ROUTER_ROWS; k++) wv[k] = *reinterpret_cast<const uint4*>(wr[k] + c);
+        for (int k = 0; k < ROWS; k++) wv[k] = *reinterpret_cast<const uint4*>(wr[k] + c);
         float xv[V];
 #pragma unroll
         for (int j = 0; j < V; j++) xv[j] = ldf(reinterpret_cast<const T*>(&xr) + j);
 #pragma unroll
-        for (int k = 0; k < ROUTER_ROWS; k++)
+        for (int k = 0; k < ROWS; k++)
 #pragma unroll
           for (int j = 0; j < V; j++) a[k] = fmaf(xv[j], ldf(reinterpret_cast<const T*>(&wv[k]) + j), a[k]);
       }
     } else {
       for (int c = lane; c < W; c += 32)
 #pragma unroll
-        for (int k = 0; k < ROUTER_ROWS; k++) a[k] = fmaf(ldf(x + c), ldf(wr[k] + c), a[k]);
+        for (int k = 0; k < ROWS; k++) a[k] = fmaf(ldf(x + c), ldf(wr[k] + c), a[k]);
     }
 #pragma unroll
-    for (int k = 0; k < ROUTER_ROWS; k++) {
+    for (int k = 0; k < ROWS; k++) {
       const float z = warp_sum(a[k]);
       if (lane == 0 && e0 + k < rows) {
         if (e0 + k < Et) zl[e0 + k] = z;

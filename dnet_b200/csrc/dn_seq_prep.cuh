@@ -8,6 +8,8 @@
 // two blocks of 512 threads an SM; four, which read less, hold twice the registers and run alone: 39.5 and 54 us.  (Rows unpacked for every tap and token, the norm's
 // root by every thread, cosines one by one: 72 instructions a channel and 58 and 69 us with four tokens; a block a token that read four rows and all weights for each and passed
 // its numbers through shared memory: 87 and 96.)
+// FEW: steps of no more tokens than SMs, a block of one token an SM: all registers and one path through the convolution, since such a block waits for its code and its loads (single
+// tokens of 3,072 channels, four taps, in a decode step: attention 7.9 us without, 6.6 so; delta rule 7.3 and 6.6).
 // Every token's numbers are formed in the same order whatever TOK is and whichever tokens come with it.
 #pragma once
 #include "dn_seq_kernels.cuh"
@@ -94,8 +96,8 @@ __device__ __forceinline__ void conv_run(const bf16* __restrict__ U, int ldu, co
 }
 
 // k_attn_prep for projections normed as a whole (or not at all) whose pairs (2 i, 2 i + 1) rotate.  Head sizes in whole 16 bytes.
-template <int TAPS, int TOK>
-__global__ void __launch_bounds__(512, 2) k_attn_prep_run(AttnPrep a, Batch b, const bf16* __restrict__ Uq, const bf16* __restrict__ Uk, const bf16* __restrict__ Uv,
+template <int TAPS, int TOK, bool FEW = false>
+__global__ void __launch_bounds__(512, FEW ? 1 : 2) k_attn_prep_run(AttnPrep a, Batch b, const bf16* __restrict__ Uq, const bf16* __restrict__ Uk, const bf16* __restrict__ Uv,
                                                        const bf16* __restrict__ cwq, const bf16* __restrict__ cwk, const bf16* __restrict__ cwv, const bf16* __restrict__ nq,
                                                        const bf16* __restrict__ nk, bf16* __restrict__ cstate, size_t slot_stride, bf16* __restrict__ qout,
                                                        bf16* __restrict__ kpool, bf16* __restrict__ vpool) {
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(512, 2) k_attn_prep_run(AttnPrep a, Batch b, c
     cache[i] = (size_t)b.bt[(size_t)slot * b.max_pages + pos[i] / PAGE] * PAGE + pos[i] % PAGE;
     st[i] = cstate + (size_t)slot * slot_stride;
   }
-  const bool plain = run_plain<TAPS, TOK>(local, n0, b.N, a.carry != 0);
+  const bool plain = !FEW && run_plain<TAPS, TOK>(local, n0, b.N, a.carry != 0);
   float x[RUN_VECS][TOK][8], sq[TOK], sk[TOK];
 #pragma unroll
   for (int i = 0; i < TOK; i++) sq[i] = sk[i] = 0.f;
@@ -206,8 +208,8 @@ __global__ void __launch_bounds__(512, 2) k_attn_prep_run(AttnPrep a, Batch b, c
 }
 
 // k_delta_prep for key sizes of 8, 16, .. 256: a head's sum of squares runs over a thread's eight channels, then pairwise over the head's lanes
-template <int TAPS, int TOK>
-__global__ void __launch_bounds__(512, 2) k_delta_prep_run(DeltaPrep a, Batch b, const bf16* __restrict__ Uq, const bf16* __restrict__ Uk, const bf16* __restrict__ Uv,
+template <int TAPS, int TOK, bool FEW = false>
+__global__ void __launch_bounds__(512, FEW ? 1 : 2) k_delta_prep_run(DeltaPrep a, Batch b, const bf16* __restrict__ Uq, const bf16* __restrict__ Uk, const bf16* __restrict__ Uv,
                                                         const bf16* __restrict__ cwq, const bf16* __restrict__ cwk, const bf16* __restrict__ cwv, const float* __restrict__ pa,
                                                         const float* __restrict__ pb, const bf16* __restrict__ A_log, const bf16* __restrict__ dt_bias,
                                                         bf16* __restrict__ cstate, size_t slot_stride, float* __restrict__ qn, float* __restrict__ kn,
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(512, 2) k_delta_prep_run(DeltaPrep a, Batch b,
     local[i] = n - b.first[n];
     st[i] = cstate + (size_t)b.slot[n] * slot_stride;
   }
-  const bool plain = run_plain<TAPS, TOK>(local, n0, b.N, false);
+  const bool plain = !FEW && run_plain<TAPS, TOK>(local, n0, b.N, false);
   for (int base = 0; base < ldst; base += blockDim.x * 8) {
     const int c = base + threadIdx.x * 8, z = c < Cq ? 0 : c < 2 * Cq ? 1 : 2, off = z * Cq;
     const bool in = c < ldst;
