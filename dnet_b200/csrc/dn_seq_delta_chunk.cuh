@@ -359,6 +359,10 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
       __syncwarp();
       part(sK + ((c + 1) & 1) * KB, c + 1, 0, &k_full[(c + 1) & 1]);
     }
+    // What the halves exchange has one place a warp, and the partner has read the chunk before's: T comes behind t_free, on which every warp arrives after that.
+    // (The wait costs nothing, the copy is under way since the chunk before; a second place would leave room for one block of 32 columns an SM.)
+    dn::mbar_wait(t_full, c & 1, err);
+    __syncwarp();
     // (the sums of the small parts' products join at the end: the fewer additions of full size, the fewer roundings)
     float out[2][4], osm[2][4];      // the outputs of tokens 16 hf ..
     {
@@ -386,8 +390,6 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
 #pragma unroll
         for (int j = 0; j < 4; j++) out[i][j] += other[(16 + 4 * i + j) * 32];
     }
-    dn::mbar_wait(t_full, c & 1, err);
-    __syncwarp();
     // V - G K S0
 #pragma unroll
     for (int i = 0; i < 4; i++) {
