@@ -1178,8 +1178,24 @@ static int moe_ff(dn_seq_model* m, SeqLayer& l, int N, bool fused, NextNorm<T> n
 static bool delta_chunk_sizes(const dn_seq_cfg& c, const dn_seq_layer_cfg& lc) {
   return c.dtype == DN_SEQ_BF16 && lc.mixer == DN_MIX_DELTA && (lc.dim == 64 || lc.dim == 128) && lc.vdim % 4 == 0;
 }
+// how a step's entries go: the chunks of all that are cut, how many are, and whether their blocks take 64 columns or 32.  The others, decoded tokens beside a prompt above
+// all, neither count nor have blocks: blocks that return at once still take their turn on the SMs, so that working ones met on some while others stood idle (one entry of
+// 2,048 tokens beside three of one, 32 heads of 128: 312 us with blocks of 64 columns, 328 with blocks of 32 beside the others' empty ones, 243 so).
+struct DeltaPlan { int chunks, entries, wide; };
+static DeltaPlan delta_plan(const std::vector<int>& counts, int heads, int vdim, int sms) {
+  DeltaPlan p{0, 0, 0};
+  for (int n : counts) { p.chunks += dc_chunks(n); p.entries += dc_chunks(n) > 0; }
+  p.wide = dc_wide(p.entries * heads * ((vdim + 63) / 64), sms);
+  return p;
+}
+extern "C" int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int vdim, int sms, int32_t* out) {
+  if (n_entries < 1 || !counts || heads < 1 || vdim < 1 || sms < 1 || !out) return fail(DN_EINVAL, "bad argument");
+  const DeltaPlan p = delta_plan(std::vector<int>(counts, counts + n_entries), heads, vdim, sms);
+  out[0] = p.chunks; out[1] = p.entries * heads; out[2] = p.wide ? 64 : 32;
+  return DN_OK;
+}
 template <int DK>
-static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b, const dn_seq_layer_cfg& lc, int chunks, float* st) {
+static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b, const dn_seq_layer_cfg& lc, const DeltaPlan& plan, float* st) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_delta_chunk_prep<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dc_prep_smem(DK));
@@ -1188,12 +1204,12 @@ static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b,
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  cudaError_t e = launch(k_delta_chunk_prep<DK>, dim3(chunks, lc.kv_heads), dim3(32 * DC_PREP_WARPS), dc_prep_smem(DK), s, b, lc.heads, lc.kv_heads, (const float*)m->qn,
+  cudaError_t e = launch(k_delta_chunk_prep<DK>, dim3(plan.chunks, lc.kv_heads), dim3(32 * DC_PREP_WARPS), dc_prep_smem(DK), s, b, lc.heads, lc.kv_heads, (const float*)m->qn,
                          (const float*)m->kn, (const float*)m->beta, (const float*)m->decay, m->dc_kq, m->dc_ta);
   if (e != cudaSuccess) return e;
-#define DCK(CG) launch(k_delta_chunk<DK, CG>, dim3(b.E * lc.heads, (lc.vdim + 16 * CG - 1) / (16 * CG)), dim3(64 * CG), dc_smem(DK, CG), s, b, lc.heads, lc.kv_heads, lc.vdim, \
+#define DCK(CG) launch(k_delta_chunk<DK, CG>, dim3(plan.entries * lc.heads, (lc.vdim + 16 * CG - 1) / (16 * CG)), dim3(64 * CG), dc_smem(DK, CG), s, b, lc.heads, lc.kv_heads, lc.vdim, \
                        (const bf16*)m->dc_kq, (const unsigned char*)m->dc_ta, (const float*)m->vv, st, m->delta_stride, m->od, m->tc_err)
-  return dc_wide(b.E * lc.heads * ((lc.vdim + 63) / 64), g_sms) ? DCK(4) : DCK(2);
+  return plan.wide ? DCK(4) : DCK(2);
 #undef DCK
 }
 
@@ -1617,11 +1633,11 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
       const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
       const size_t dsm = (size_t)2 * TB * per * 4;
       PH(DN_SEQ_PH_DELTA_RULE);
-      int chunks = 0, below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
+      int below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
       if (m->dc_kq && b.max_len >= DC_FROM && delta_chunk_sizes(c, lc)) {
         below = DC_FROM;
-        for (int n : m->ent_len) chunks += dc_chunks(n);
-        CK(lc.dim == 64 ? delta_chunks<64>(m, s, b, lc, chunks, st) : delta_chunks<128>(m, s, b, lc, chunks, st));
+        const DeltaPlan plan = delta_plan(m->ent_len, lc.heads, lc.vdim, g_sms);
+        CK(lc.dim == 64 ? delta_chunks<64>(m, s, b, lc, plan, st) : delta_chunks<128>(m, s, b, lc, plan, st));
       }
 #define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, lc.heads, lc.kv_heads, lc.dim, lc.vdim, TB, \
                          (const float*)m->qn, (const float*)m->kn, (const float*)m->vv, (const float*)m->beta, (const float*)m->decay, st,      \

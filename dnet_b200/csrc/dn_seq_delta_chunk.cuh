@@ -43,8 +43,8 @@ __host__ __device__ constexpr size_t dc_smem(int dk, int cg) { return (size_t)3 
 constexpr int DC_PREP_WARPS = 8;
 __host__ __device__ constexpr size_t dc_prep_smem(int dk) { return (size_t)2 * dc_k_bytes(dk) + 2 * DC * (DC + 1) * 8 + DC_PREP_WARPS * 2 * DC * 4; }
 
-// 64 columns a block (of one an SM) where that nearly fills the SMs, else 32 (two an SM): a block of 64 reads K and Q half as often, one of 32 has a
-// warp a scheduler to itself.  Four entries of 32 heads (256 blocks of 64), the longest 788: 173 us with 64, 210 with 32; two of 700 (128): 111, 121; of
+// 64 columns a block (of one an SM) where the blocks of the entries that are cut nearly fill the SMs, else 32 (two an SM): a block of 64 reads K and Q half
+// as often, one of 32 has a warp a scheduler to itself.  Four entries of 32 heads (256 blocks of 64), the longest 788: 173 us with 64, 210 with 32; two of 700 (128): 111, 121; of
 // 16 heads (64): 111, 86; one entry of 2,048, 32 heads: 310, 242.
 __host__ __device__ __forceinline__ bool dc_wide(int blocks, int sms) { return 4 * blocks >= 3 * sms; }
 
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(32 * DC_PREP_WARPS) k_delta_chunk_prep(Batch b
   }
 }
 
-// grid (entries x heads, columns / (16 CG)), 64 CG threads: warp w has the columns of group w % CG and half of their rows (w / CG); the two halves' sums with K
+// grid (entries that are cut x heads, columns / (16 CG)), 64 CG threads: warp w has the columns of group w % CG and half of their rows (w / CG); the two halves' sums with K
 // and Q meet in shared memory, and each finishes half of the tokens' outputs
 template <int DK, int CG>
 __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H, int G, int dv, const bf16* __restrict__ kq, const unsigned char* __restrict__ ta,
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
            *t_free = k_full + 6;      // (free: a warp each has read it out)
   __shared__ int pick;
   const int h = blockIdx.x % H, g = h / (H / G), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cg = warp % CG, hf = warp / CG;
-  // the entry of this place in the order of lengths: the longest start first
+  // the entry of this place in the order of lengths: the longest start first, and those that are not cut come last, behind the grid
   for (int i = threadIdx.x; i < b.E; i += blockDim.x) {
     const int n = b.ent_start[i + 1] - b.ent_start[i];
     int place = 0;
@@ -287,7 +287,6 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
   int base = 0;      // chunks of the entries before this one
   for (int i = 0; i < e; i++) base += dc_chunks(b.ent_start[i + 1] - b.ent_start[i]);
   const int s0 = b.ent_start[e], len = b.ent_start[e + 1] - s0, chunks = dc_chunks(len), Cv = H * dv;
-  if (chunks == 0) return;
   auto part = [&](unsigned char* dst, int c, int z, uint64_t* bar) {      // K (z = 0) or Q of chunk c
     if (lane == 0) {
       dn::mbar_arrive_expect_tx(bar, KB);

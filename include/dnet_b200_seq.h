@@ -271,6 +271,10 @@ int dn_seq_profile_read(dn_seq_model* m, double* ms_out, int reset);
  * results).  The profiler and the layer trace always take the one-by-one path. */
 int dn_seq_set_graphs(dn_seq_model* m, int on);
 
+/* Test hook, on the host alone: how a step whose entries bring counts[e] tokens takes a delta-rule layer on a device of `sms` SMs.
+ * out[0] chunks of the entries that are cut into chunks, out[1] (entry, head) pairs that have blocks, out[2] columns of a head's state that a block takes (32 or 64) */
+int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int vdim, int sms, int32_t* out);
+
 #ifdef __cplusplus
 }
 #endif
