@@ -1194,8 +1194,25 @@ extern "C" int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int
   out[0] = p.chunks; out[1] = p.entries * heads; out[2] = p.wide ? 64 : 32;
   return DN_OK;
 }
+// rows a lane (R) and lanes a column (P) of the recurrences: the smallest P R >= dk of this table
+static void recur_shape(int dk, int* R, int* P) {
+  static const int RP[8][3] = {{8, 8, 1}, {16, 8, 2}, {32, 8, 4}, {64, 8, 8}, {128, 16, 8}, {256, 16, 16}, {512, 16, 32}, {1024, 32, 32}};
+  *R = 32; *P = 32;
+  for (int i = 7; i >= 0; i--) if (dk <= RP[i][0]) { *R = RP[i][1]; *P = RP[i][2]; }
+}
+// the gated delta rule over a step's entries, counts[e] tokens each: inputs, states and what chunks are made of (kq null: all entries token by token)
+struct DeltaIo {
+  int heads, kv_heads, dim, vdim;
+  const float *q, *k, *v, *beta, *decay;
+  float* state;
+  size_t stride;      // of a slot's state
+  float* out;
+  bf16* kq;
+  unsigned char* ta;
+  unsigned int* err;
+};
 template <int DK>
-static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b, const dn_seq_layer_cfg& lc, const DeltaPlan& plan, float* st) {
+static cudaError_t delta_chunks(cudaStream_t s, const Batch& b, const DeltaIo& io, const DeltaPlan& plan) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_delta_chunk_prep<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dc_prep_smem(DK));
@@ -1204,21 +1221,73 @@ static cudaError_t delta_chunks(dn_seq_model* m, cudaStream_t s, const Batch& b,
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  cudaError_t e = launch(k_delta_chunk_prep<DK>, dim3(plan.chunks, lc.kv_heads), dim3(32 * DC_PREP_WARPS), dc_prep_smem(DK), s, b, lc.heads, lc.kv_heads, (const float*)m->qn,
-                         (const float*)m->kn, (const float*)m->beta, (const float*)m->decay, m->dc_kq, m->dc_ta);
+  cudaError_t e = launch(k_delta_chunk_prep<DK>, dim3(plan.chunks, io.kv_heads), dim3(32 * DC_PREP_WARPS), dc_prep_smem(DK), s, b, io.heads, io.kv_heads, io.q, io.k, io.beta, io.decay,
+                         io.kq, io.ta);
   if (e != cudaSuccess) return e;
-#define DCK(CG) launch(k_delta_chunk<DK, CG>, dim3(plan.entries * lc.heads, (lc.vdim + 16 * CG - 1) / (16 * CG)), dim3(64 * CG), dc_smem(DK, CG), s, b, lc.heads, lc.kv_heads, lc.vdim, \
-                       (const bf16*)m->dc_kq, (const unsigned char*)m->dc_ta, (const float*)m->vv, st, m->delta_stride, m->od, m->tc_err)
+#define DCK(CG) launch(k_delta_chunk<DK, CG>, dim3(plan.entries * io.heads, (io.vdim + 16 * CG - 1) / (16 * CG)), dim3(64 * CG), dc_smem(DK, CG), s, b, io.heads, io.kv_heads, io.vdim, \
+                       (const bf16*)io.kq, (const unsigned char*)io.ta, io.v, io.state, io.stride, io.out, io.err)
   return plan.wide ? DCK(4) : DCK(2);
 #undef DCK
 }
-
-// rows a lane (R) and lanes a column (P) of the recurrences: the smallest P R >= dk of this table
-static void recur_shape(int dk, int* R, int* P) {
-  static const int RP[8][3] = {{8, 8, 1}, {16, 8, 2}, {32, 8, 4}, {64, 8, 8}, {128, 16, 8}, {256, 16, 16}, {512, 16, 32}, {1024, 32, 32}};
-  *R = 32; *P = 32;
-  for (int i = 7; i >= 0; i--) if (dk <= RP[i][0]) { *R = RP[i][1]; *P = RP[i][2]; }
+static int delta_rule(cudaStream_t s, const Batch& b, const std::vector<int>& counts, const DeltaIo& io) {
+  int R, P;
+  recur_shape(io.dim, &R, &P);
+  dim3 grid(b.E * io.heads, (io.vdim + 31) / 32);
+  // tokens per staged tile: two tiles of `per` floats a token within ~36 KB of shared memory
+  const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
+  const size_t dsm = (size_t)2 * TB * per * 4;
+  int below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
+  if (io.kq && b.max_len >= DC_FROM) {
+    below = DC_FROM;
+    const DeltaPlan plan = delta_plan(counts, io.heads, io.vdim, g_sms);
+    CK(io.dim == 64 ? delta_chunks<64>(s, b, io, plan) : delta_chunks<128>(s, b, io, plan));
+  }
+#define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, io.heads, io.kv_heads, io.dim, io.vdim, TB, \
+                         io.q, io.k, io.v, io.beta, io.decay, io.state, io.stride, io.out, below))
+  if (below == INT_MAX || *std::min_element(counts.begin(), counts.end()) < below) {
+    DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
+  }
+#undef DR
+  return DN_OK;
 }
+extern "C" int dn_seq_debug_delta(int chunked, int n_entries, const int32_t* counts, int heads, int key_heads, int dim, int vdim, const float* q, const float* k, const float* v,
+                                  const float* beta, const float* decay, float* state, float* out, dn_seq_stream stream) {
+  if (g_sms == 0) return fail(DN_EINVAL, "dn_seq_init() has not been called");
+  if (n_entries < 1 || !counts || heads < 1 || key_heads < 1 || heads % key_heads || dim < 1 || dim > 1024 || vdim < 1 || !q || !k || !v || !beta || !decay || !state || !out)
+    return fail(DN_EINVAL, "bad argument");
+  if (chunked && ((dim != 64 && dim != 128) || vdim % 4)) return fail(DN_EINVAL, "keys of %d, values of %d: no chunks", dim, vdim);
+  const std::vector<int> lens(counts, counts + n_entries);
+  std::vector<int32_t> at(2 * n_entries + 1);
+  int N = 0, longest = 0;
+  for (int e = 0; e < n_entries; e++) {
+    if (lens[e] < 1) return fail(DN_EINVAL, "entry %d brings %d tokens", e, lens[e]);
+    at[e] = N;
+    at[n_entries + 1 + e] = e;
+    N += lens[e];
+    longest = std::max(longest, lens[e]);
+  }
+  at[n_entries] = N;
+  const DeltaPlan plan = delta_plan(lens, heads, vdim, g_sms);
+  cudaStream_t s = (cudaStream_t)stream;
+  int32_t* at_d = nullptr;
+  DeltaIo io{heads, key_heads, dim, vdim, q, k, v, beta, decay, state, (size_t)heads * dim * vdim, out, nullptr, nullptr, nullptr};
+  unsigned int err = 0;
+  int rc = dalloc(&at_d, at.size() * 4);
+  if (rc == DN_OK) rc = dalloc(&io.err, 16);
+  if (rc == DN_OK && chunked) rc = dalloc(&io.kq, (size_t)plan.chunks * key_heads * 2 * dc_k_bytes(dim));
+  if (rc == DN_OK && chunked) rc = dalloc(&io.ta, (size_t)plan.chunks * heads * DC_TA_BYTES);
+  if (rc == DN_OK && (cudaMemcpyAsync(at_d, at.data(), at.size() * 4, cudaMemcpyHostToDevice, s) != cudaSuccess || cudaMemsetAsync(io.err, 0, 16, s) != cudaSuccess)) rc = fail(DN_ECUDA, "copy failed");
+  if (rc == DN_OK) {
+    Batch b{};
+    b.ent_start = at_d; b.ent_slot = at_d + n_entries + 1; b.N = N; b.E = n_entries; b.max_len = longest;
+    rc = delta_rule(s, b, lens, io);
+  }
+  if (rc == DN_OK && (cudaMemcpyAsync(&err, io.err, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)) rc = fail(DN_ECUDA, "the recurrence failed");
+  if (rc == DN_OK && err) rc = fail(DN_ECUDA, "a wait ran out (%u)", err);
+  for (void* p : {(void*)at_d, (void*)io.err, (void*)io.kq, (void*)io.ta}) if (p) cudaFree(p);
+  return rc;
+}
+
 // a decayed outer-product recurrence over the step's entries: inputs m->qn / kn / vv / dz (fp32), output m->od
 static int decay_rule(dn_seq_model* m, const Batch& b, int mode, int H, int dk, int dv, const void* bonus, float* st, cudaStream_t s) {
   int R, P;
@@ -1626,26 +1695,10 @@ static int step_T(dn_seq_model* m, const Batch& b, int n_want, const int32_t* wa
         CK(launch(k_delta_prep<T>, dim3(N), prep_threads(2 * l.Cq + l.Cv), (size_t)2 * l.Cq * 4, s, a, b, (const T*)m->uq, (const T*)m->uk, (const T*)m->uv,
                 w(DN_SQ_Q_CONV), w(DN_SQ_K_CONV), w(DN_SQ_V_CONV), (const float*)m->pa, (const float*)m->pb, w(DN_SQ_A_LOG),
                 w(DN_SQ_DT_BIAS), (const T*)cst, m->conv_stride, m->qn, m->kn, m->vv, m->beta, m->decay));
-      int R, P;
-      recur_shape(lc.dim, &R, &P);
-      dim3 grid(b.E * lc.heads, (lc.vdim + 31) / 32);
-      // tokens per staged tile: two tiles of `per` floats a token within ~36 KB of shared memory
-      const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
-      const size_t dsm = (size_t)2 * TB * per * 4;
       PH(DN_SEQ_PH_DELTA_RULE);
-      int below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
-      if (m->dc_kq && b.max_len >= DC_FROM && delta_chunk_sizes(c, lc)) {
-        below = DC_FROM;
-        const DeltaPlan plan = delta_plan(m->ent_len, lc.heads, lc.vdim, g_sms);
-        CK(lc.dim == 64 ? delta_chunks<64>(m, s, b, lc, plan, st) : delta_chunks<128>(m, s, b, lc, plan, st));
-      }
-#define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, lc.heads, lc.kv_heads, lc.dim, lc.vdim, TB, \
-                         (const float*)m->qn, (const float*)m->kn, (const float*)m->vv, (const float*)m->beta, (const float*)m->decay, st,      \
-                         m->delta_stride, m->od, below))
-      if (below == INT_MAX || *std::min_element(m->ent_len.begin(), m->ent_len.end()) < below) {
-        DR(8, 1, 1); DR(8, 2, 1); DR(8, 4, 1); DR(8, 8, 2); DR(16, 8, 2); DR(16, 16, 2); DR(16, 32, 2); DR(32, 32, 4);
-      }
-#undef DR
+      const DeltaIo io{lc.heads, lc.kv_heads, lc.dim, lc.vdim, m->qn, m->kn, m->vv, m->beta, m->decay, st, m->delta_stride, m->od, delta_chunk_sizes(c, lc) ? m->dc_kq : nullptr, m->dc_ta,
+                       m->tc_err};
+      if (const int rc = delta_rule(s, b, m->ent_len, io)) return rc;
       PH(DN_SEQ_PH_DELTA_OUT);
       CK(launch(k_delta_out<T>, dim3((N * lc.heads + 7) / 8), dim3(256), 0, s, (const float*)m->od, (const T*)m->gt, w(DN_SQ_OUT_NORM), N * lc.heads, lc.heads, lc.vdim,
                 c.eps, (T*)m->mo, 0, 0));

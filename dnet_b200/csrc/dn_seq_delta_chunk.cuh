@@ -12,11 +12,12 @@
 // chunk ahead).
 //
 // fp32 on 16-bit matrix instructions: every operand is three parts of bf16, all 24 bits, and six of the nine products are formed (the others are below
-// 2^-25); the sums of sixteen products of the large parts meet in fp32 additions, the small ones in an accumulator of their own.  T's diagonal, beta, is not
-// part of the product, products of decays are formed in 64 bits and rounded once, and never as quotients: a decay of 0 is as good as any.  Error against
-// 64 bits (2-norm, outputs / states), entries of 1 to 250 tokens of 8 heads of 128 x 128: 7.2e-8 / 3.5e-8, token by token 7.2e-8 / 4.0e-8; decays near 1 and keys that
-// are nearly alike, 1,500 tokens: 2.3e-7 / 2.5e-7, token by token 8.9e-7 / 1.2e-6; decays of about 0.8, 1,500 tokens: 7.3e-8 / 6.8e-8, 6.7e-8 / 6.8e-8.  (Two parts of
-// fp16 and three products are a third faster and three times further off.)
+// 2^-25); the sums of sixteen products of the large parts meet in fp32 additions, the small ones in an accumulator of their own, and the state's products, 32 deep, in one
+// chain, the small ones first: what is added to the state is then rounded once.  T's diagonal, beta, is not part of the product, products of decays are formed in 64 bits and
+// rounded once, A not before it is in parts, and never as quotients: a decay of 0 is as good as any.  Error against 64 bits (2-norm, 1e-8), outputs / states, and token by token:
+//   decays of about 0.8, entries of 81 to 250 tokens, 8 heads of 128 x 128 6.3 / 5.7, 7.1 / 6.3; 64 x 96, 95 and 130 tokens 6.5 / 5.7, 7.3 / 6.0; 1,500 tokens 6.1 / 5.4, 6.7 / 6.8
+//   decays near 1 and keys that are nearly alike, 1,500 tokens 23 / 29, 89 / 122; decays of 0, 1e-20 and 1 5.1 / 4.0, 6.4 / 4.5
+// (Two parts of fp16 and three products are a third faster and three times further off.  tests/test_gpu_delta_chunks.py holds these.)
 //
 // Bound by mma.sync, 348 a chunk and warp at 8.7 cycles each, and the splitting into parts beside them, which one warp a scheduler does not hide.  32 heads of
 // 128 x 128, microseconds, token by token / preparation + chunks: four entries, 2,048 tokens, the longest 788: 450 / 27 + 173; one entry of 2,048: 630 / 27 + 242; one of
@@ -58,6 +59,10 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3], float
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
 }
+// The instruction cuts its sums to fp32 instead of rounding them, so that a product of the large parts is too small by some part of 2^-24 on average: K and Q are made
+// larger by as much as measured best (outputs / states against 64 bits, 1e-8, decays of about 0.8, 1,500 tokens: 0 / 0 6.9 / 6.8, 0.35 / 0.35 6.3 / 5.7, 0.5 / 0.3 6.1 / 5.4,
+// 0.7 / 0.5 8.2 / 5.2; token by token 6.7 / 6.8).
+constexpr float DC_CUT_K = 0.5f / 16777216.f, DC_CUT_Q = 0.3f / 16777216.f;
 __device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -69,13 +74,10 @@ __device__ __forceinline__ void dc_mma0(float (&c)[4], const uint32_t (&a)[4], u
 __device__ __forceinline__ void add_pair(float& x, float& y, float a, float b) {      // two fp32 additions
   asm("{.reg .b64 u, v, w; mov.b64 u, {%0, %1}; mov.b64 v, {%2, %3}; add.rn.f32x2 w, u, v; mov.b64 {%0, %1}, w;}" : "+f"(x), "+f"(y) : "f"(a), "f"(b));
 }
-// sixteen products deep, NT tiles of eight columns: c gets the sums of the large parts' products by fp32 additions, small the other five products that
-// matter (the three left out are below 2^-25 of the result)
+// sixteen products deep, NT tiles of eight columns: small gets the five products of parts that matter beside that of the large ones (the three left out are below 2^-25 of
+// the result)
 template <int NT>
-__device__ __forceinline__ void mma_parts(float (&c)[NT][4], float (&small)[NT][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2 * NT]) {
-  float d[NT][4];
-#pragma unroll
-  for (int n = 0; n < NT; n++) dc_mma0(d[n], a[0], b[0][2 * n], b[0][2 * n + 1]);
+__device__ __forceinline__ void mma_small(float (&small)[NT][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2 * NT]) {
 #pragma unroll
   for (int n = 0; n < NT; n++) dc_mma(small[n], a[2], b[0][2 * n], b[0][2 * n + 1]);
 #pragma unroll
@@ -86,6 +88,14 @@ __device__ __forceinline__ void mma_parts(float (&c)[NT][4], float (&small)[NT][
   for (int n = 0; n < NT; n++) dc_mma(small[n], a[1], b[0][2 * n], b[0][2 * n + 1]);
 #pragma unroll
   for (int n = 0; n < NT; n++) dc_mma(small[n], a[0], b[1][2 * n], b[1][2 * n + 1]);
+}
+// ... and c the sums of the large parts' products by fp32 additions
+template <int NT>
+__device__ __forceinline__ void mma_parts(float (&c)[NT][4], float (&small)[NT][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2 * NT]) {
+  float d[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; n++) dc_mma0(d[n], a[0], b[0][2 * n], b[0][2 * n + 1]);
+  mma_small(small, a, b);
 #pragma unroll
   for (int n = 0; n < NT; n++) {
     add_pair(c[n][0], c[n][1], d[n][0], d[n][1]);
@@ -144,8 +154,9 @@ __global__ void __launch_bounds__(32 * DC_PREP_WARPS) k_delta_chunk_prep(Batch b
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (t < cnt) v = *reinterpret_cast<const float4*>((z ? qn : kn) + ((size_t)(n0 + t) * G + g) * DK + d);
     uint32_t p[3], q[3];
-    split3(v.x, v.y, p);
-    split3(v.z, v.w, q);
+    const float more = z ? DC_CUT_Q : DC_CUT_K;
+    split3(v.x, v.y, p, v.x * more, v.y * more);
+    split3(v.z, v.w, q, v.z * more, v.w * more);
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int at = ((3 * z + j) * DC + t) * HP + d;
@@ -200,10 +211,10 @@ __global__ void __launch_bounds__(32 * DC_PREP_WARPS) k_delta_chunk_prep(Batch b
     __syncwarp();
     unsigned char* base = ta + ((size_t)blockIdx.x * H + h) * DC_TA_BYTES;
     bf16* to = reinterpret_cast<bf16*>(base) + role * 3 * DC * DC_TP;
-    auto store = [&](int t, float x) {      // a number of T or A in its parts
+    auto store = [&](int t, auto x) {      // a number of T (fp32) or A (64 bits) in its parts
 #pragma unroll
       for (int j = 0; j < 3; j++) {
-        const bf16 v = __float2bfloat16_rn(x);
+        const bf16 v = __float2bfloat16_rn((float)x);
         to[(j * DC + t) * DC_TP + lane] = v;
         x -= __bfloat162float(v);
       }
@@ -217,7 +228,7 @@ __global__ void __launch_bounds__(32 * DC_PREP_WARPS) k_delta_chunk_prep(Batch b
         D = lane == t ? 1. : D * gd;
         Gt *= gd;
         if (lane == t) mine = (float)Gt;
-        store(t, lane <= t ? (float)(D * qk[t * (DC + 1) + lane]) : 0.f);
+        store(t, lane <= t ? D * qk[t * (DC + 1) + lane] : 0.);
       }
       float* gm = reinterpret_cast<float*>(base + DC_TA_NUMBERS * 2);
       gm[lane] = mine;
@@ -478,13 +489,12 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
     __syncwarp();
     if (lane == 0) dn::mbar_arrive(t_free);
 #pragma unroll
-    for (int i = 0; i < DK / 64; i++) {      // 32 state rows
-      float d[4][4], small[4][4];
+    for (int i = 0; i < DK / 64; i++) {      // 32 state rows: all products in one chain, the small ones first
+      float d[4][4];
+      uint32_t f[2][3][8];
       zero_tiles(d);
-      zero_tiles(small);
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        uint32_t f[3][8];
 #pragma unroll
         for (int p = 0; p < 3; p++)
 #pragma unroll
@@ -492,14 +502,18 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
             uint32_t w[4];
             ldsm_x4_t(w, Ks + (p * DC + k * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * HP + i * 32 + j * 16 + (lane >> 4) * 8);
 #pragma unroll
-            for (int q = 0; q < 4; q++) f[p][4 * j + q] = w[q];
+            for (int q = 0; q < 4; q++) f[k][p][4 * j + q] = w[q];
           }
-        mma_parts(d, small, a[k], f);
+        mma_small(d, a[k], f[k]);
       }
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+#pragma unroll
+        for (int n = 0; n < 4; n++) dc_mma(d[n], a[k][0], f[k][0][2 * n], f[k][0][2 * n + 1]);
 #pragma unroll
       for (int n = 0; n < 4; n++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) S[4 * i + n][j] = fmaf(S[4 * i + n][j], gl, d[n][j] + small[n][j]);
+        for (int j = 0; j < 4; j++) S[4 * i + n][j] = fmaf(S[4 * i + n][j], gl, d[n][j]);
     }
     __syncwarp();
     if (lane == 0) dn::mbar_arrive(k_free);

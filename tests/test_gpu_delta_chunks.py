@@ -2,9 +2,12 @@
 token-by-token entries in the same step, against the float64 oracle and against the same tokens in portions that all go token by token."""
 from __future__ import annotations
 
+import ctypes as C
+
 import pytest
 import torch
 
+from dnet_b200 import _seqabi
 from tests.test_gpu_seqmix import FF, TOL, Rig, config, delta, err, toks
 
 pytestmark = pytest.mark.gpu
@@ -50,3 +53,70 @@ def test_decays_of_zero_and_repeated_keys():
             got = r.eng.step([("a", tokens, list(range(len(tokens))))])
             assert torch.isfinite(got).all()
             assert err(got, r.oracle(tokens)) < TOL["bfloat16"]
+
+
+# -- the recurrence alone ---------------------------------------------------------------------------------------------
+def recurrence_inputs(kind, lens, heads, groups, dk, dv, seed=0):
+    """fp32 q, k (of unit length), v, beta, decay and one state an entry"""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    nd = lambda *s: torch.randn(*s, generator=g, device="cuda")      # noqa: E731
+    silu, N = torch.nn.functional.silu, sum(lens)
+    unit = lambda x: x / (x.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()      # noqa: E731
+    q, k = unit(silu(nd(N, groups, dk))) * dk ** -0.5, nd(N, groups, dk)
+    beta, decay = torch.sigmoid(nd(N, heads)), torch.exp(-torch.exp(0.5 * nd(N, heads) - 1) * torch.nn.functional.softplus(nd(N, heads)))
+    if kind == "long memory, keys alike":
+        k, beta, decay = nd(1, groups, dk) + 0.1 * k, torch.sigmoid(3 * nd(N, heads) + 3), 1 - 1e-4 * torch.rand(N, heads, generator=g, device="cuda")
+    elif kind == "decays of 0, 1e-20 and 1":
+        u = torch.rand(N, heads, generator=g, device="cuda")
+        decay = torch.where(u < 0.1, 0.0, torch.where(u < 0.55, 1e-20, 1.0))
+    return [x.float().contiguous() for x in (q, unit(silu(k)), silu(nd(N, heads, dv)), beta, decay, 0.3 * nd(len(lens), heads, dk, dv))]
+
+
+def recurrence(chunked, lens, q, k, v, beta, decay, state):
+    state, out = state.clone(), torch.full_like(v, float("nan"))
+    _seqabi.init(0)
+    _seqabi.check(_seqabi.load().dn_seq_debug_delta(chunked, len(lens), (C.c_int32 * len(lens))(*lens), v.shape[1], k.shape[1], k.shape[2], v.shape[2],
+                                                    *(x.data_ptr() for x in (q, k, v, beta, decay, state, out)), torch.cuda.current_stream().cuda_stream))
+    return out, state
+
+
+def recurrence64(lens, q, k, v, beta, decay, state):
+    r = v.shape[1] // k.shape[1]
+    q, k = (x.double().repeat_interleave(r, 1) for x in (q, k))
+    v, beta, decay, state = (x.double() for x in (v, beta, decay, state))
+    out, states, at = torch.empty_like(v), [], 0
+    for n, S in zip(lens, state):
+        for t in range(at, at + n):
+            S = S * decay[t, :, None, None]
+            u = beta[t, :, None] * (v[t] - torch.einsum("hdj,hd->hj", S, k[t]))
+            S = S + k[t, :, :, None] * u[:, None]
+            out[t] = torch.einsum("hdj,hd->hj", S, q[t])
+        states.append(S)
+        at += n
+    return out, torch.stack(states)
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("kind,bound", [("decays of about 0.8", 8e-8), ("long memory, keys alike", 4e-7), ("decays of 0, 1e-20 and 1", 8e-8)])
+@pytest.mark.parametrize("lens,heads,groups,dk,dv", [([100, 83, 96, 81, 250], 8, 2, 128, 128), ([130, 95], 4, 2, 64, 96), ([82, 97], 2, 1, 128, 40), ([1500], 5, 5, 128, 128)])
+def test_recurrence_is_as_close_to_64_bits_as_token_by_token(kind, bound, lens, heads, groups, dk, dv):
+    """Outputs and states in fp32 against float64, 2-norm.  A rounding leaves 2.25e-8 (2^-23 / sqrt(12) over a mantissa of 1.53 rms).  Token by token a number takes two a token,
+    of which a decay of about 0.8 leaves some three tokens' in all: 6e-8 to 7.5e-8, bound 8e-8; with a long memory and keys that are alike errors add up (9e-7 and 1.2e-6 over
+    1,500 tokens).  Chunks are no further off than that, but for a twentieth, the spread of such a norm over inputs, or three roundings, 4e-8, which no order of the sums goes
+    below (u = beta (v - ..), k u): states that a decay of 0 has left with a token or two.  Operands of two parts, 2^-17, are a hundred times off."""
+    x = recurrence_inputs(kind, lens, heads, groups, dk, dv, seed=len(lens) + dk)
+    ref = recurrence64(lens, *x)
+    by_token, chunks = recurrence(0, lens, *x), recurrence(1, lens, *x)
+    for name, a, c, r in zip(("outputs", "states"), by_token, chunks, ref):
+        assert rel(c, r) < min(bound, max(1.05 * rel(a, r), 4e-8)), (name, rel(a, r))
+    assert all(torch.equal(a, b) for a, b in zip(chunks, recurrence(1, lens, *x)))
+
+
+def test_recurrence_hook_refuses_what_has_no_chunks():
+    x = recurrence_inputs("decays of about 0.8", [90], 2, 1, 40, 20)
+    assert all(torch.isfinite(a).all() for a in recurrence(0, [90], *x))
+    with pytest.raises(_seqabi.DnError, match="no chunks"):
+        recurrence(1, [90], *x)
