@@ -20,8 +20,8 @@
 // (Two parts of fp16 and three products are a third faster and three times further off.  tests/test_gpu_delta_chunks.py holds these.)
 //
 // Bound by mma.sync, 348 a chunk and warp at 8.7 cycles each, and the splitting into parts beside them, which one warp a scheduler does not hide.  32 heads of
-// 128 x 128, microseconds, token by token / preparation + chunks: four entries, 2,048 tokens, the longest 788: 450 / 27 + 173; one entry of 2,048: 630 / 27 + 242; one of
-// 100: 36 / 12.6 + 18.7; one of 16: 10.5 / 11 + 8.5.
+// 128 x 128, microseconds, token by token / preparation + chunks: four entries, 2,048 tokens, the longest 788: 450 / 27 + 175; one entry of 2,048: 630 / 27 + 246; one of
+// 100: 36 / 12.6 + 20; one of 16: 10.5 / 11 + 8.5.
 #pragma once
 #include "dn_seq_kernels.cuh"
 #include "dn_megakernel.cuh"
@@ -45,8 +45,8 @@ constexpr int DC_PREP_WARPS = 8;
 __host__ __device__ constexpr size_t dc_prep_smem(int dk) { return (size_t)2 * dc_k_bytes(dk) + 2 * DC * (DC + 1) * 8 + DC_PREP_WARPS * 2 * DC * 4; }
 
 // 64 columns a block (of one an SM) where the blocks of the entries that are cut nearly fill the SMs, else 32 (two an SM): a block of 64 reads K and Q half
-// as often, one of 32 has a warp a scheduler to itself.  Four entries of 32 heads (256 blocks of 64), the longest 788: 173 us with 64, 210 with 32; two of 700 (128): 111, 121; of
-// 16 heads (64): 111, 86; one entry of 2,048, 32 heads: 310, 242.
+// as often, one of 32 has a warp a scheduler to itself.  Four entries of 32 heads (256 blocks of 64), the longest 788: 175 us with 64, 210 with 32; two of 700 (128): 111, 120; of
+// 16 heads (64): 113, 88; one entry of 2,048, 32 heads: 310, 246.
 __host__ __device__ __forceinline__ bool dc_wide(int blocks, int sms) { return 4 * blocks >= 3 * sms; }
 
 // two numbers (x + ex, y + ey, where ex and ey are below the last place) in three parts of bf16: all 24 bits
@@ -115,6 +115,41 @@ __device__ __forceinline__ void a_frag(const float (&x)[4], const float (&y)[4],
     if (i < 2) split3(x[2 * i], x[2 * i + 1], p); else split3(y[2 * i - 4], y[2 * i - 3], p);
     a[0][i] = p[0]; a[1][i] = p[1]; a[2][i] = p[2];
   }
+}
+// Numbers that are not finite.  The zeros above T's and A's diagonals meet the rows of later tokens, and 0 x NaN would carry such a number back to tokens before it: a column's
+// rows from the first one on are taken as zeros, and its outputs from there on and its state become NaN, as token by token they are not finite from there on.  (Above bf16's largest,
+// 3.39e38, is infinite here.)
+constexpr float DC_LARGEST = 0x1.fep127f;
+constexpr int DC_ALL_FINITE = DC | DC << 8;      // the first such token of a thread's two columns, a byte each; 32: none
+// at(i): tokens 8 i + 2 (lane & 3) + {0, 1} of the first column ([0], [1]) and of the second
+template <class At>
+__device__ __forceinline__ int first_not_finite(At at, int lane, int before) {
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) ok = ok && fabsf(at(i)[j]) <= DC_LARGEST;
+  if (__all_sync(0xffffffffu, ok && before == DC_ALL_FINITE)) return before;
+  int a = before & 255, b = before >> 8;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int t = 8 * i + 2 * (lane & 3) + (j & 1);
+      if (fabsf(at(i)[j]) <= DC_LARGEST) continue;
+      if (j < 2) a = min(a, t); else b = min(b, t);
+    }
+#pragma unroll
+  for (int d = 1; d < 4; d <<= 1) {
+    a = min(a, __shfl_xor_sync(0xffffffffu, a, d));
+    b = min(b, __shfl_xor_sync(0xffffffffu, b, d));
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (8 * i + 2 * (lane & 3) + (j & 1) >= (j < 2 ? a : b)) at(i)[j] = 0.f;
+  return a | b << 8;
 }
 // untiled copy into this CTA's shared memory; both addresses on 16 bytes, a multiple of 16 bytes
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -410,6 +445,7 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
         r[i][j] = t < cnt ? fmaf(-((j & 1) ? gt.y : gt.x), r[i][j], Vs[t * VP + col + (j < 2 ? 0 : 8)]) : 0.f;
       }
     }
+    int bad = first_not_finite([&](int i) -> float (&)[4] { return r[i]; }, lane, DC_ALL_FINITE);
     // U = T (..): tokens from 16 on alone see those from 16 on
     auto tile16 = [&](const bf16* m, int j, int k, uint32_t (&f)[3][4]) {      // tokens 16 j .. of T or A, places 16 k ..
 #pragma unroll
@@ -438,6 +474,7 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
           for (int x = 0; x < 4; x++) u[j][i][x] = fmaf((x & 1) ? bt.y : bt.x, r[2 * j + i][x], u[j][i][x] + small[j][i][x]);
         }
     }
+    bad = first_not_finite([&](int i) -> float (&)[4] { return u[i >> 1][i & 1]; }, lane, bad);      // (T's rows, where a key, a decay or beta is the cause)
     if (warp == 1 && c + 1 < chunks) {
       dn::mbar_wait(q_free, c & 1, err);
       __syncwarp();
@@ -466,7 +503,8 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
         for (int j = 0; j < 4; j++) {
           const int t = 16 * hf + 8 * i + 2 * (lane & 3) + (j & 1);
           const float gj = (j & 1) ? gt.y : gt.x;
-          if (t < cnt && (j < 2 ? okA : okB)) od[(size_t)t * Cv + (j < 2 ? 0 : 8)] = fmaf(out[i][j], gj, d[i][j]) + fmaf(osm[i][j], gj, small[i][j]);
+          if (t < cnt && (j < 2 ? okA : okB))
+            od[(size_t)t * Cv + (j < 2 ? 0 : 8)] = t < (j < 2 ? bad & 255 : bad >> 8) ? fmaf(out[i][j], gj, d[i][j]) + fmaf(osm[i][j], gj, small[i][j]) : __int_as_float(0x7fffffff);
         }
       }
     }
@@ -515,6 +553,12 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
 #pragma unroll
         for (int j = 0; j < 4; j++) S[4 * i + n][j] = fmaf(S[4 * i + n][j], gl, d[n][j]);
     }
+    if (bad != DC_ALL_FINITE)
+#pragma unroll
+      for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if ((j < 2 ? bad & 255 : bad >> 8) < DC) S[i][j] = __int_as_float(0x7fffffff);
     __syncwarp();
     if (lane == 0) dn::mbar_arrive(k_free);
     if (warp == 2 && c + 1 < chunks) {

@@ -120,3 +120,24 @@ def test_recurrence_hook_refuses_what_has_no_chunks():
     assert all(torch.isfinite(a).all() for a in recurrence(0, [90], *x))
     with pytest.raises(_seqabi.DnError, match="no chunks"):
         recurrence(1, [90], *x)
+
+
+@pytest.mark.parametrize("where,value", [(w, x) for w in ("q", "k", "v", "beta", "decay", "state") for x in (float("nan"), float("-inf"))] + [("v", 2e38)])
+@pytest.mark.parametrize("token", [37, 64, 95, 120])      # inside, at the edges of and in the last, ragged chunk of an entry
+def test_numbers_that_are_not_finite_touch_what_they_touch_token_by_token(where, value, token):
+    """One such number in an entry's 121 tokens: outputs of earlier tokens, of other columns (values and states), heads and entries are what they are without it, and what is not
+    finite is the same as token by token.  A value of 2e38 is finite and stays so."""
+    lens, at = [90, 121], 90 + token
+    x = recurrence_inputs("decays of about 0.8", lens, 4, 2, 64, 40, seed=3)
+    clean = recurrence(1, lens, *x)
+    tensor = x[["q", "k", "v", "beta", "decay", "state"].index(where)]
+    {"q": lambda: tensor[at, 1, 7:8], "k": lambda: tensor[at, 1, 7:8], "v": lambda: tensor[at, 2, 13:14], "beta": lambda: tensor[at, 2:3], "decay": lambda: tensor[at, 2:3],
+     "state": lambda: tensor[1, 2, 11, 13:14]}[where]().fill_(value)
+    by_token, chunks = recurrence(0, lens, *x), recurrence(1, lens, *x)
+    for name, a, c, w in zip(("outputs", "states"), by_token, chunks, clean):
+        assert torch.equal(torch.isfinite(a), torch.isfinite(c)), name
+        ok = torch.isfinite(a)
+        assert not ok.all() or value == 2e38 or (where, name) == ("q", "states")
+        assert torch.allclose(a[ok], c[ok], rtol=1e-5, atol=1e-6 * (2e38 if value == 2e38 else 1.0)), name
+    if where != "state":
+        assert torch.equal(chunks[0][:at], clean[0][:at])
