@@ -107,3 +107,84 @@ def test_layer_list_attention(heads, kv_heads, mask):
         r.model.check()
         for i, s in enumerate(seqs):
             assert err(torch.cat(got[i]), r.oracle(s)) < TOL["bfloat16"], f"request {i}"
+
+
+# -- items that are cut, several a CTA, and more row blocks than are sorted ---------------------------------------------------------
+def dealt_or_cut(entries, kv_heads, group, first_seen):
+    """how a step's row blocks go over the SMs, from the rule as k_attn_prompt has it: "several" whole items a CTA, "cut" into runs (the most pieces an item comes to), or
+    "unsorted" runs of more row blocks than are sorted"""
+    sms, TB = torch.cuda.get_device_properties(0).multi_processor_count, 128 // group
+    lens = []
+    for pos, n in entries:
+        for i in range(0, n, TB):
+            end = pos + i + min(TB, n - i)
+            lens.append(((end + 63) // 64 - first_seen(pos + i) // 64 + 1) // 2 + 1)
+    items, total = kv_heads * len(lens), kv_heads * sum(lens)
+    per = max(-(-total // sms), 4)
+    if len(lens) > 256:
+        return "unsorted"
+    order = sorted(lens, reverse=True)
+    load = [0] * sms
+    for i in range(items):
+        k, c = divmod(i, sms)
+        load[sms - 1 - c if k & 1 else c] += order[i // kv_heads]
+    return "cut" if max(load) > per + 6 else "several" if items > sms else "whole"
+
+
+def twice(rig, steps):
+    """the same steps two times over, with fresh sequences: the last one's logits"""
+    runs = []
+    for _ in range(2):
+        runs.append([rig.eng.step(s) for s in steps][-1])
+        rig.model.check()
+        for rid in {e[0] for s in steps for e in s}:
+            rig.eng.finish(rid)
+    assert torch.equal(*runs)      # (the counts of finished pieces are zero again, too)
+    return runs[0]
+
+
+@pytest.mark.parametrize("how,heads,kv_heads,mask,first,portions", [
+    ("cut", 4, 1, None, (0, 3, 333), (2000, 1, 40)), ("cut", 4, 1, 1500, (700, 0, 61), (1300, 90, 1)), ("several", 16, 8, None, (0, 100, 0), (1400, 17, 1)),
+    ("unsorted", 16, 1, 700, (0, 0, 65), (2100, 33, 9))])
+def test_layer_list_items_cut_and_joined(how, heads, kv_heads, mask, first, portions):
+    """a long portion beside short ones: their tiles are on the line that runs are cut from, and a run may end in any of them"""
+    mx = {**BASE, "heads": heads, "kv_heads": kv_heads, "conv": 2, "rot": {"base": 500.0, "dims": 32}}
+    if mask:
+        mx["mask"] = {"size": mask}
+    assert dealt_or_cut(list(zip(first, portions)), kv_heads, heads // kv_heads, lambda p: p // mask * mask if mask else 0) == how
+    seqs = [toks(a + n, seed=700 + i) for i, (a, n) in enumerate(zip(first, portions))]
+    with Rig(config([attn(mixer=mx, mlp=FF)], width=64), "bfloat16", max_tokens=6144, max_batch_tokens=2304) as r:
+        steps = [[(f"s{i}", s[:a], []) for i, (s, a) in enumerate(zip(seqs, first)) if a], [(f"s{i}", s[a:], list(range(len(s) - a))) for i, (s, a) in enumerate(zip(seqs, first))]]
+        got, at = twice(r, [s for s in steps if s]), 0
+        for i, (s, a) in enumerate(zip(seqs, first)):
+            assert err(got[at:at + len(s) - a], r.oracle(s)[a:]) < TOL["bfloat16"], f"request {i}"
+            at += len(s) - a
+
+
+def test_layer_list_items_cut_under_a_sliding_window():
+    """a window that starts inside pages: row blocks whose first page is not the sequence's, groups of three (126 of 128 rows), one key head"""
+    from tests.test_gpu_bokenex import Rig as FamilyRig, made_up, random_for, rms1p
+
+    size, heads, W = 1500, 3, 64
+    cls = made_up("TestWindowSoftmax", {"norm": "rms", "qk_norm": False, "mask": "window"})
+    cfg = {"architecture": "TestWindowSoftmax", "vocab": 96, "width": W, "norm": {"eps": 1e-5}, "embedding": {"scale": 1.0},
+           "layers": [{"type": "attention", "mixer": {**BASE, "heads": heads, "kv_heads": 1, "mask": {"size": size}}, "mlp": {"kind": "dense", "ff": 80}}]}
+    w = random_for(cls, cfg, 71)
+    assert dealt_or_cut([(0, 2200), (0, 60)], 1, heads, lambda p: max(0, p - size + 1)) == "cut"
+    t = toks(2200, seed=72)
+    d = {k: v.double() for k, v in w.items()}
+    x = d["embed"][t]
+    h = rms1p(x, d["l0.norm1"], 1e-5)
+    q, k, v = (h @ d[f"l0.mix.{c}"].T for c in "qkv")
+    i = torch.arange(len(t))
+    seen = (i[None] <= i[:, None]) & (i[None] > i[:, None] - size)
+    s = torch.einsum("thd,nd->htn", q.view(-1, heads, 128), k) * BASE["scale"]
+    a = torch.softmax(s.masked_fill(~seen, float("-inf")), -1) @ v
+    x = x + a.transpose(0, 1).reshape(len(t), -1) @ d["l0.mix.o"].T
+    h = rms1p(x, d["l0.norm2"], 1e-5)
+    x = x + (torch.nn.functional.gelu(h @ d["l0.mlp.gate"].T, approximate="tanh") * (h @ d["l0.mlp.up"].T)) @ d["l0.mlp.down"].T
+    ref = rms1p(x, d["final.norm"], 1e-5) @ d["head"].T
+    with FamilyRig(cfg, "bfloat16", weights=w, max_tokens=4096, max_batch_tokens=2304) as r:
+        got = twice(r, [[("a", t, list(range(len(t)))), ("b", t[:60], [59])]])
+    assert err(got[:-1], ref) < TOL["bfloat16"]
+    assert err(got[-1:], ref[59:60]) < TOL["bfloat16"]
