@@ -156,19 +156,6 @@ static int make_tmap(CUtensorMap* out, const void* base, int rows, int cols, int
   return DN_OK;
 }
 
-// [tokens][heads][128], in boxes of 64 dims x `group` heads x `tokens_of_box` tokens
-static int make_tmap_heads(CUtensorMap* out, const void* base, int tokens, int heads, int group, int tokens_of_box) {
-  if (!g_encode) return fail(DN_ECUDA, "cuTensorMapEncodeTiled unavailable");
-  cuuint64_t dims[3] = {(cuuint64_t)HD, (cuuint64_t)heads, (cuuint64_t)tokens};
-  cuuint64_t strides[2] = {(cuuint64_t)HD * 2, (cuuint64_t)heads * HD * 2};
-  cuuint32_t box[3] = {64, (cuuint32_t)group, (cuuint32_t)tokens_of_box};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(DN_ECUDA, "cuTensorMapEncodeTiled failed (%d) tokens=%d heads=%d", (int)r, tokens, heads);
-  return DN_OK;
-}
-
 // an activation buffer's descriptors, one for each number of rows that a stage may take
 static bool make_xmaps(CUtensorMap (&out)[TC_XMAPS], const void* base, int rows, int cols) {
   for (int i = 0; i < TC_XMAPS; ++i)
@@ -517,7 +504,7 @@ extern "C" int dn_model_create(const dn_model_cfg* cfg, const int32_t* abs_layer
                true;
     m->pf_ok = m->pf_ok && make_xmaps(m->tm_xn, m->pf_xn, CHUNK_MAX, H) && make_xmaps(m->tm_attn, m->pf_attn, CHUNK_MAX, qd) &&
                make_xmaps(m->tm_act, m->pf_act, CHUNK_MAX, cfg->ffn);
-    m->tm_q_ok = m->pf_ok && m->tm_kv_ok && make_tmap_heads(&m->tm_q, m->pf_q, CHUNK_MAX, cfg->n_heads, m->G, 128 / m->G) == DN_OK;
+    m->tm_q_ok = m->pf_ok && m->tm_kv_ok && query_map(g_encode, &m->tm_q, m->pf_q, CHUNK_MAX, cfg->n_heads, m->G);
     if (cfg->n_experts > 0 && m->pf_ok) {
       const int P = CHUNK_MAX * cfg->top_k, E = cfg->n_experts;
       m->moe_max_tiles = P / 64 + E;

@@ -89,22 +89,6 @@ __device__ __forceinline__ void mbar_spin(uint64_t* bar, uint32_t parity, unsign
     }
   }
 }
-__device__ __forceinline__ void tm_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-// 16 columns; valid after tm_wait_ld and ap_pin
-__device__ __forceinline__ void tm_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr));
-}
-__device__ __forceinline__ void ap_pin(uint32_t (&r)[16]) {
-#pragma unroll
-  for (int i = 0; i < 16; i += 8)
-    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
-}
 // from FROM registers a thread to TO, by a whole warpgroup (the direction has to be the right one)
 template <int FROM, int TO>
 __device__ __forceinline__ void ap_regs() {
@@ -113,6 +97,18 @@ __device__ __forceinline__ void ap_regs() {
 }
 // 2^(a - b) of whole numbers a <= b (a may be -inf: 0)
 __device__ __forceinline__ float ap_pow(float a, float b) { return a - b < -126.f || a == -INFINITY ? 0.f : __uint_as_float((uint32_t)(127 + (int)(a - b)) << 23); }
+
+// the queries [tokens][heads][128] in boxes of 64 dims x a key head's `group` query heads x as many tokens as 128 rows hold (encode: cuTensorMapEncodeTiled)
+template <class Encode>
+inline bool query_map(Encode encode, CUtensorMap* out, const void* base, int tokens, int heads, int group) {
+  if (!encode || !base) return false;
+  cuuint64_t dims[3] = {128, (cuuint64_t)heads, (cuuint64_t)tokens};
+  cuuint64_t strides[2] = {256, (cuuint64_t)heads * 256};
+  cuuint32_t box[3] = {64, (cuuint32_t)group, (cuuint32_t)(128 / group)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Items from which a launch takes this kernel; fewer stay with k_attn_prefill_tc, whose clusters share a row block's keys.  By the tokens alone, so that a chunk that
 // is captured and replayed at other positions takes the kernel of an eager one.  With eight key heads of groups of 4, 200 tokens (56 items) behind 0 / 1,000 / 3,000 / 8,000:
@@ -394,7 +390,7 @@ __global__ void __launch_bounds__(ApShape<PARTS>::THREADS, 1) k_attn_prompt(cons
           for (int z = 0; z < 2; ++z) {
             uint32_t (&v)[16] = va[z], hi[8], lo[8], x[8];
             tm_wait_ld();
-            ap_pin(v);
+            tm_pin16(v);
             if (z == 0 || c < 96) tm_ld16(tS + c + 16 * z + 16, va[z ^ 1]);      // on its way while this one's weights are formed
 #pragma unroll
             for (int i = 0; i < 8; ++i) {

@@ -92,23 +92,6 @@ constexpr int AQT_SMEM = 5 * AT_TILE + AQT_XCH + 1024 + 256;
 constexpr int AQT_REGS_MMA = 40, AQT_REGS_SOFTMAX = 136, AQT_REGS_DQ = 80;      // setmaxnreg: of the 96 a thread that 640 threads are launched with
 static_assert(128 * (AQT_REGS_MMA + 2 * AQT_REGS_SOFTMAX + 2 * AQT_REGS_DQ) <= AQT_THREADS * 96, "setmaxnreg split exceeds the CTA's launch allocation");
 
-// 16 (8) consecutive 32-bit columns of this warp's TMEM quarter
-__device__ __forceinline__ void aq_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr));
-}
-__device__ __forceinline__ void aq_pin(uint32_t (&r)[16]) {      // no use of r moves above this point
-#pragma unroll
-  for (int i = 0; i < 16; i += 8)
-    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]), "+r"(r[i + 7]));
-}
-__device__ __forceinline__ void aq_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-
 template <int G, int BITS>
 __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParams pq) {
   pdl_launch_dependents();
@@ -245,13 +228,13 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
     // rounded to bf16; keys that the row does not see: -inf.  it, j: the tile, c: 0, 16, 32, 48
     auto scores_of = [&](uint32_t at, int it, int j, int c, float2 (&s)[8]) {
       uint32_t a[16], b[16];
-      aq_ld16(at + lane_off + c, a);
-      aq_ld16(at + 64 + lane_off + c, b);
+      tm_ld16(at + lane_off + c, a);
+      tm_ld16(at + 64 + lane_off + c, b);
       const float4* kf = reinterpret_cast<const float4*>(kb + (it & 3) * AQT_KB + h * 64 + c);
       const int key = ((j0 + j) << 7) + h * 64 + c;
       tm_wait_ld();
-      aq_pin(a);
-      aq_pin(b);
+      tm_pin16(a);
+      tm_pin16(b);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 s0 = kf[i], s1 = kf[32 + i], b0 = kf[64 + i], b1 = kf[96 + i];
@@ -375,7 +358,7 @@ __global__ void __launch_bounds__(AQT_THREADS, 1) k_attn_prefill_q(const AqParam
           t0s = f2_fma(f2_of(pa), make_float2(bv.x, bv.y), t0s);
           t1s = f2_fma(f2_of(pd), make_float2(bv.z, bv.w), t1s);
         }
-        aq_st8(tP + (j & 1) * 64 + lane_off + h * 32 + c / 2, w);      // (the product that read this one's place was joined a tile ago)
+        tm_st8(tP + (j & 1) * 64 + lane_off + h * 32 + c / 2, w);      // (the product that read this one's place was joined a tile ago)
       }
       tc_fence_before();
       __syncwarp();

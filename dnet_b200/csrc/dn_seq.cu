@@ -207,16 +207,6 @@ static bool make_tmap(CUtensorMap* out, const void* base, int rows, int cols, in
   return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// [tokens][heads][128], in boxes of 64 dims x `group` heads x as many tokens as 128 rows hold
-static bool make_tmap_heads(CUtensorMap* out, const void* base, int tokens, int heads, int group) {
-  if (!g_encode || !base) return false;
-  cuuint64_t dims[3] = {128, (cuuint64_t)heads, (cuuint64_t)tokens};
-  cuuint64_t strides[2] = {256, (cuuint64_t)heads * 256};
-  cuuint32_t box[3] = {64, (cuuint32_t)group, (cuuint32_t)(128 / group)};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return g_encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 static int dist_span(const dn_seq_cfg& cfg, const dn_seq_layer_cfg& c) {      // distances a visible key can have: 0 .. span - 1
   int span = cfg.pool_pages * PAGE;
   if (cfg.max_positions > 0) span = std::min(span, cfg.max_positions);
@@ -630,7 +620,7 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
     make_xmaps(&m->x_h, m->h, m->MB, cfg->width);
     for (auto& l : m->L) {
       make_xmaps(&l.x_mo, m->mo, m->MB, l.Co);
-      l.tm_q_ok = soft_tc_sizes(*cfg, l.c) && make_tmap_heads(&l.tm_q, m->qb, m->MB, l.c.heads, l.c.heads / l.c.kv_heads);
+      l.tm_q_ok = soft_tc_sizes(*cfg, l.c) && dn::query_map(g_encode, &l.tm_q, m->qb, m->MB, l.c.heads, l.c.heads / l.c.kv_heads);
       if (l.Rv > 0) make_xmaps(&l.x_mo_r, m->mo, m->MB, l.Rv);
       if (l.c.rank > 0) make_xmaps(&l.x_lr, m->lr, m->MB, l.c.rank);
       if (l.c.mixer == DN_MIX_LATENT && l.c.q_rank > 0) make_xmaps(&l.x_lr, m->lr, m->MB, l.c.q_rank);
