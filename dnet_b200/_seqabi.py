@@ -109,7 +109,7 @@ _PROTOS = {
     "dn_seq_profile": (_i, [_vp, _i]),
     "dn_seq_profile_read": (_i, [_vp, C.POINTER(C.c_double), _i]),
     "dn_seq_set_graphs": (_i, [_vp, _i]),
-    "dn_seq_debug_delta_plan": (_i, [_i, _I32P, _i, _i, _i, _I32P]),
+    "dn_seq_debug_delta_plan": (_i, [_i, _I32P, _i, _i, _i, _i, _I32P]),
     "dn_seq_debug_delta": (_i, [_i, _i, _I32P, _i, _i, _i, _i] + [_vp] * 8),
     "dn_seq_step": (_i, [_vp, _i, _I32P, _I32P, _I32P, _i, _I32P, _vp, _vp, _vp]),
 }

@@ -606,7 +606,7 @@ extern "C" int dn_seq_model_create(const dn_seq_cfg* cfg, const dn_seq_layer_cfg
     size_t kq = 0, ta = 0;
     for (auto& l : m->L)
       if (delta_chunk_sizes(*cfg, l.c)) { kq = std::max(kq, (size_t)l.c.kv_heads * 2 * dc_k_bytes(l.c.dim)); ta = std::max(ta, (size_t)l.c.heads * DC_TA_BYTES); }
-    const size_t chunks = MB / DC + MB / DC_FROM;      // (every entry that is cut has DC_FROM tokens or more)
+    const size_t chunks = MB / DC + MB / DC_FROM;      // (every entry that is cut has DC_FROM tokens or more, the lesser of the two lines)
     if (kq && chunks) { DA(m->dc_kq, chunks * kq); DA(m->dc_ta, chunks * ta); }
   }
   DA(m->conv_state, (size_t)cfg->max_seqs * coff * e); DA(m->delta_state, (size_t)cfg->max_seqs * doff * 4);
@@ -1172,15 +1172,15 @@ static bool delta_chunk_sizes(const dn_seq_cfg& c, const dn_seq_layer_cfg& lc) {
 // all, neither count nor have blocks: blocks that return at once still take their turn on the SMs, so that working ones met on some while others stood idle (one entry of
 // 2,048 tokens beside three of one, 32 heads of 128: 312 us with blocks of 64 columns, 328 with blocks of 32 beside the others' empty ones, 243 so).
 struct DeltaPlan { int chunks, entries, wide; };
-static DeltaPlan delta_plan(const std::vector<int>& counts, int heads, int vdim, int sms) {
+static DeltaPlan delta_plan(const std::vector<int>& counts, int heads, int dim, int vdim, int sms) {
   DeltaPlan p{0, 0, 0};
-  for (int n : counts) { p.chunks += dc_chunks(n); p.entries += dc_chunks(n) > 0; }
+  for (int n : counts) { p.chunks += dc_chunks(n, dim); p.entries += dc_chunks(n, dim) > 0; }
   p.wide = dc_wide(p.entries * heads * ((vdim + 63) / 64), sms);
   return p;
 }
-extern "C" int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int vdim, int sms, int32_t* out) {
-  if (n_entries < 1 || !counts || heads < 1 || vdim < 1 || sms < 1 || !out) return fail(DN_EINVAL, "bad argument");
-  const DeltaPlan p = delta_plan(std::vector<int>(counts, counts + n_entries), heads, vdim, sms);
+extern "C" int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int dim, int vdim, int sms, int32_t* out) {
+  if (n_entries < 1 || !counts || heads < 1 || (dim != 64 && dim != 128) || vdim < 1 || sms < 1 || !out) return fail(DN_EINVAL, "bad argument");
+  const DeltaPlan p = delta_plan(std::vector<int>(counts, counts + n_entries), heads, dim, vdim, sms);
   out[0] = p.chunks; out[1] = p.entries * heads; out[2] = p.wide ? 64 : 32;
   return DN_OK;
 }
@@ -1227,9 +1227,9 @@ static int delta_rule(cudaStream_t s, const Batch& b, const std::vector<int>& co
   const int per = 2 * P * (R + 4) + 36, TB = std::max(1, std::min(16, 4500 / per));
   const size_t dsm = (size_t)2 * TB * per * 4;
   int below = INT_MAX;      // entries of fewer tokens than `below` take k_delta_rule
-  if (io.kq && b.max_len >= DC_FROM) {
-    below = DC_FROM;
-    const DeltaPlan plan = delta_plan(counts, io.heads, io.vdim, g_sms);
+  if (io.kq && b.max_len >= dc_from(io.dim)) {
+    below = dc_from(io.dim);
+    const DeltaPlan plan = delta_plan(counts, io.heads, io.dim, io.vdim, g_sms);
     CK(io.dim == 64 ? delta_chunks<64>(s, b, io, plan) : delta_chunks<128>(s, b, io, plan));
   }
 #define DR(Rv, Pv, Cv_) if (R == Rv && P == Pv) CK(launch(k_delta_rule<Rv, Pv, Cv_>, grid, dim3(32 * Pv / Cv_), dsm, s, b, io.heads, io.kv_heads, io.dim, io.vdim, TB, \
@@ -1257,7 +1257,7 @@ extern "C" int dn_seq_debug_delta(int chunked, int n_entries, const int32_t* cou
     longest = std::max(longest, lens[e]);
   }
   at[n_entries] = N;
-  const DeltaPlan plan = delta_plan(lens, heads, vdim, g_sms);
+  const DeltaPlan plan = delta_plan(lens, heads, dim, vdim, g_sms);
   cudaStream_t s = (cudaStream_t)stream;
   int32_t* at_d = nullptr;
   DeltaIo io{heads, key_heads, dim, vdim, q, k, v, beta, decay, state, (size_t)heads * dim * vdim, out, nullptr, nullptr, nullptr};

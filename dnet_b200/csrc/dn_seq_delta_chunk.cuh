@@ -30,9 +30,13 @@ namespace dnseq {
 
 constexpr int DC = 32;                          // tokens of a chunk
 // Entries from this many tokens on; shorter ones stay with k_delta_rule (a chunk takes as long however few of its tokens there are, and the preparation 11 us).
-// A step of one entry of 64 tokens, width 1,024 / 4,096: 342.8 / 624 us both ways; of 100: 364 / 679, in chunks 360.5 / 676; of 300: 472 / 1,028, 429 / 984.
-constexpr int DC_FROM = 80;
-__host__ __device__ __forceinline__ int dc_chunks(int tokens) { return tokens >= DC_FROM ? (tokens + DC - 1) / DC : 0; }
+// Token by token / preparation + chunks, microseconds, entries x heads of 128 x 128 (64 x 64): one entry of 8 heads, 80 tokens 29 / 29 (25 / 23), 96 35 / 29 (29 / 24), 128 45 / 33
+// (37 / 27); 96 in all, 80 tokens 46 / 50 (29 / 27), 96 54 / 50 (33 / 27), 112 62 / 60; 192, 80 tokens 82 / 68 (33 / 38), 112 111 / 85 (45 / 49), 128 124 / 87 (50 / 50); 512, 80 tokens
+// 168 / 150 (62 / 71), 112 229 / 190 (83 / 91), 128 259 / 191 (94 / 93), 160 319 / 230 (115 / 111).  From these lines on chunks are slower nowhere, but for 5 % with keys of 64
+// and 512 in all whose last chunk is half empty (144 tokens 105 / 109).
+constexpr int DC_FROM = 96, DC_FROM_64 = 128;      // (of keys of 128 and of 64)
+__host__ __device__ __forceinline__ int dc_from(int dk) { return dk == 64 ? DC_FROM_64 : DC_FROM; }
+__host__ __device__ __forceinline__ int dc_chunks(int tokens, int dk) { return tokens >= dc_from(dk) ? (tokens + DC - 1) / DC : 0; }
 constexpr int DC_TP = DC + 8;                   // row pitch of T and A, of K and Q dk + 8: eight rows of 16 bytes fall into different banks
 __host__ __device__ constexpr int dc_k_bytes(int dk) { return 3 * DC * (dk + 8) * 2; }       // [3 parts][32][dk + 8] bf16 of a (chunk, key head): K, then as many of Q
 constexpr int DC_TA_NUMBERS = 6 * DC * DC_TP;                                                // [T, A][3 parts][32][40] bf16 of a (chunk, head),
@@ -158,10 +162,10 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 }
 
 // which entry a chunk belongs to, and which of its chunks it is (false: none)
-__device__ __forceinline__ bool chunk_entry(const Batch& b, int chunk, int& e, int& c) {
+__device__ __forceinline__ bool chunk_entry(const Batch& b, int dk, int chunk, int& e, int& c) {
   c = chunk;
   for (e = 0; e < b.E; e++) {
-    const int nc = dc_chunks(b.ent_start[e + 1] - b.ent_start[e]);
+    const int nc = dc_chunks(b.ent_start[e + 1] - b.ent_start[e], dk);
     if (c < nc) return true;
     c -= nc;
   }
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(32 * DC_PREP_WARPS) k_delta_chunk_prep(Batch b
   float* gb = reinterpret_cast<float*>(qk + DC * (DC + 1));
   static_assert(DC_PREP_WARPS / 2 * DC * LP * 4 <= 2 * dc_k_bytes(DK), "L lies over the parts");
   int e, c;
-  if (!chunk_entry(b, blockIdx.x, e, c)) return;
+  if (!chunk_entry(b, DK, blockIdx.x, e, c)) return;
   const int g = blockIdx.y, n0 = b.ent_start[e] + c * DC, cnt = min(DC, b.ent_start[e + 1] - n0), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bf16* out = kq + ((size_t)blockIdx.x * G + g) * dc_k_bytes(DK);      // (2 x dc_k_bytes bytes)
 #pragma unroll 8
@@ -331,8 +335,8 @@ __global__ void __launch_bounds__(64 * CG, 4 / CG) k_delta_chunk(Batch b, int H,
   __syncthreads();
   const int e = pick;
   int base = 0;      // chunks of the entries before this one
-  for (int i = 0; i < e; i++) base += dc_chunks(b.ent_start[i + 1] - b.ent_start[i]);
-  const int s0 = b.ent_start[e], len = b.ent_start[e + 1] - s0, chunks = dc_chunks(len), Cv = H * dv;
+  for (int i = 0; i < e; i++) base += dc_chunks(b.ent_start[i + 1] - b.ent_start[i], DK);
+  const int s0 = b.ent_start[e], len = b.ent_start[e + 1] - s0, chunks = dc_chunks(len, DK), Cv = H * dv;
   auto part = [&](unsigned char* dst, int c, int z, uint64_t* bar) {      // K (z = 0) or Q of chunk c
     if (lane == 0) {
       dn::mbar_arrive_expect_tx(bar, KB);

@@ -271,9 +271,9 @@ int dn_seq_profile_read(dn_seq_model* m, double* ms_out, int reset);
  * results).  The profiler and the layer trace always take the one-by-one path. */
 int dn_seq_set_graphs(dn_seq_model* m, int on);
 
-/* Test hook, on the host alone: how a step whose entries bring counts[e] tokens takes a delta-rule layer on a device of `sms` SMs.
+/* Test hook, on the host alone: how a step whose entries bring counts[e] tokens takes a delta-rule layer (dim 64 or 128) on a device of `sms` SMs.
  * out[0] chunks of the entries that are cut into chunks, out[1] (entry, head) pairs that have blocks, out[2] columns of a head's state that a block takes (32 or 64) */
-int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int vdim, int sms, int32_t* out);
+int dn_seq_debug_delta_plan(int n_entries, const int32_t* counts, int heads, int dim, int vdim, int sms, int32_t* out);
 /* Test hook: the gated delta rule alone, of entries of counts[e] tokens.  All fp32 on the device: q, k [tokens][key_heads][dim], v, out [tokens][heads][vdim],
  * beta, decay [tokens][heads], state [n_entries][heads][dim][vdim] (updated).  chunked 0: token by token; 1: entries in chunks where a step of a model that has
  * them does so (dim 64 or 128, vdim a multiple of 4).  Synchronises s */

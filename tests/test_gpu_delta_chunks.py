@@ -1,4 +1,4 @@
-"""Prompt portions of the delta rule in chunks of 32 tokens (k_delta_chunk; entries of 80 tokens and more, key sizes 64 and 128) beside
+"""Prompt portions of the delta rule in chunks of 32 tokens (k_delta_chunk; entries of 96 tokens and more with keys of 128, of 128 with keys of 64) beside
 token-by-token entries in the same step, against the float64 oracle and against the same tokens in portions that all go token by token."""
 from __future__ import annotations
 
@@ -22,9 +22,9 @@ def test_chunks_against_the_oracle_and_token_by_token(dk, dv, heads, groups):
     """First portions that end inside, on and behind the edge of a chunk; entries below the line beside them; second portions that start from the first's state."""
     cfg = config([delta(mixer={"heads": heads, "kv_heads": groups, "dim": dk, "vdim": dv, "conv": 3}, mlp=FF),
                   delta(mixer={"heads": heads, "kv_heads": groups, "dim": dk, "vdim": dv, "conv": 0})], width=64)
-    seqs = [toks(n, seed=300 + i) for i, n in enumerate((161, 210, 86, 260))]
-    first = [80, 97, 81, 79]
-    with Rig(cfg, "bfloat16", max_tokens=1024, max_batch_tokens=512) as r:
+    seqs = [toks(n, seed=300 + i) for i, n in enumerate((260, 300, 210, 290))]
+    first = [128, 145, 129, 95]
+    with Rig(cfg, "bfloat16", max_tokens=1536, max_batch_tokens=640) as r:
         parts = [r.eng.step([(f"s{i}", s[a:b], list(range(b - a))) for i, (s, a, b) in enumerate(zip(seqs, lo, hi))])
                  for lo, hi in (([0] * 4, first), (first, [len(s) for s in seqs]))]
         r.model.check()
@@ -101,7 +101,7 @@ def rel(a, b):
 
 
 @pytest.mark.parametrize("kind,bound", [("decays of about 0.8", 8e-8), ("long memory, keys alike", 4e-7), ("decays of 0, 1e-20 and 1", 8e-8)])
-@pytest.mark.parametrize("lens,heads,groups,dk,dv", [([100, 83, 96, 81, 250], 8, 2, 128, 128), ([130, 95], 4, 2, 64, 96), ([82, 97], 2, 1, 128, 40), ([1500], 5, 5, 128, 128)])
+@pytest.mark.parametrize("lens,heads,groups,dk,dv", [([100, 97, 96, 127, 250], 8, 2, 128, 128), ([130, 191], 4, 2, 64, 96), ([98, 113], 2, 1, 128, 40), ([1500], 5, 5, 128, 128)])
 def test_recurrence_is_as_close_to_64_bits_as_token_by_token(kind, bound, lens, heads, groups, dk, dv):
     """Outputs and states in fp32 against float64, 2-norm.  A rounding leaves 2.25e-8 (2^-23 / sqrt(12) over a mantissa of 1.53 rms).  Token by token a number takes two a token,
     of which a decay of about 0.8 leaves some three tokens' in all: 6e-8 to 7.5e-8, bound 8e-8; with a long memory and keys that are alike errors add up (9e-7 and 1.2e-6 over
@@ -123,11 +123,11 @@ def test_recurrence_hook_refuses_what_has_no_chunks():
 
 
 @pytest.mark.parametrize("where,value", [(w, x) for w in ("q", "k", "v", "beta", "decay", "state") for x in (float("nan"), float("-inf"))] + [("v", 2e38)])
-@pytest.mark.parametrize("token", [37, 64, 95, 120])      # inside, at the edges of and in the last, ragged chunk of an entry
+@pytest.mark.parametrize("token", [37, 64, 95, 152])      # inside, at the edges of and in the last, ragged chunk of an entry
 def test_numbers_that_are_not_finite_touch_what_they_touch_token_by_token(where, value, token):
-    """One such number in an entry's 121 tokens: outputs of earlier tokens, of other columns (values and states), heads and entries are what they are without it, and what is not
+    """One such number in an entry's 153 tokens: outputs of earlier tokens, of other columns (values and states), heads and entries are what they are without it, and what is not
     finite is the same as token by token.  A value of 2e38 is finite and stays so."""
-    lens, at = [90, 121], 90 + token
+    lens, at = [90, 153], 90 + token
     x = recurrence_inputs("decays of about 0.8", lens, 4, 2, 64, 40, seed=3)
     clean = recurrence(1, lens, *x)
     tensor = x[["q", "k", "v", "beta", "decay", "state"].index(where)]
