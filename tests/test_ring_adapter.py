@@ -276,6 +276,40 @@ def test_ingress_forwards_frames_for_other_shards(grpc_ok):
     asyncio.run(main())
 
 
+def test_hop_frame_waits_for_the_end_of_the_request_that_had_its_lane(monkeypatch):
+    """the end of a request and the first frame of the next one on its lane come on streams of their own, in any order"""
+    from dnet_b200.shard import ring as link_mod
+
+    ad, rt = make_adapter(assigned_next={1})
+    monkeypatch.setattr(link_mod, "device_view", lambda ptr, shape, dtype: torch.zeros(shape, dtype=dtype))
+    bulk = types.SimpleNamespace(slot=lambda lane: lane, flag=lambda lane: lane, consumed_flag=lambda lane: lane)
+    ad.hop = types.SimpleNamespace(rx_bulk=bulk)
+    ad._streams.configure_lanes(2)
+    ad._teardown_hop = lambda: None
+
+    def frame(nonce):
+        return pb.ActivationRequest(nonce=nonce, activation=pb.Activation(data=fr.pack_hop(fr.HopMeta(lane=0, seq=1, seq0=1)), batch_size=1, shape=[1, 4, 8],
+                                                                          dtype=fr.hop_dtype("bfloat16"), layer_id=0))
+
+    async def main():
+        await ad.start()
+        await ad.ingress_q.put(frame("old"))
+        assert await wait_until(lambda: rt.activation_recv_queue.qsize() == 1)
+        await ad.ingress_q.put(frame("new"))
+        await asyncio.sleep(0.05)
+        assert rt.activation_recv_queue.qsize() == 1 and ad._streams.lane_ctx("new") is None
+        await ad.end_request("old")
+        assert await wait_until(lambda: rt.activation_recv_queue.qsize() == 2)
+        assert [rt.activation_recv_queue.get_nowait().nonce for _ in range(2)] == ["old", "new"]
+        ad.lane_wait_s = 0.01      # an owner that never ends: the frame is refused
+        await ad.ingress_q.put(frame("third"))
+        await asyncio.sleep(0.1)
+        assert rt.activation_recv_queue.empty() and ad._streams.lane_ctx("third") is None
+        await ad.shutdown()
+
+    asyncio.run(main())
+
+
 def test_ingress_deserialize_exception_is_handled(monkeypatch):
     ad, rt = make_adapter(assigned_next={1})
 
